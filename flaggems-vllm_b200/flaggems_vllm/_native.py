@@ -1,4 +1,4 @@
-"""ctypes binding of libdsv4_prologue.so (the C ABI declared in include/dsv4_prologue.h).
+"""ctypes binding of libdsv4_prologue.so (the C ABI declared in include/dsv4_prologue.h) and loader of the native front ends.
 
 There is no fallback: if the library has not been built, or a call is made on a
 machine without a CUDA device, the caller gets an exception, never a silent
@@ -11,6 +11,7 @@ from pathlib import Path
 
 LIB_NAME = "libdsv4_prologue.so"
 LIB_PATH = Path(__file__).resolve().parent / LIB_NAME
+HOST_CALLS_PATH = LIB_PATH.parent / "_host_calls.so"
 
 EXPORTS = (
     "dsv4_qnorm_rope_kv_insert",
@@ -46,6 +47,7 @@ EXPORTS = (
 VARIANT_AUTO, VARIANT_ROWS, VARIANT_BULK = 0, 1, 2
 
 _lib = None
+_host_calls = None
 
 
 class NativeLibraryMissing(RuntimeError):
@@ -133,6 +135,27 @@ def lib() -> ctypes.CDLL:
 def check(code: int) -> None:
     if code != 0:
         raise Dsv4Error(code, lib().dsv4_error_string(code).decode())
+
+
+def host_calls():
+    """The extension module with the native front ends of the operators (csrc/host_calls.cpp), loaded once.  Its functions
+    return None for arguments they do not accept: the Python operator then says which (see `refuse`)."""
+    global _host_calls
+    if _host_calls is None:
+        lib()  # names the missing library; the module is linked against it
+        if not HOST_CALLS_PATH.exists():
+            raise NativeLibraryMissing(f"{HOST_CALLS_PATH} is missing: build it with `python -m flaggems_vllm.build`.")
+        from . import _host_calls as module
+
+        module.bind(check)
+        _host_calls = module
+    return _host_calls
+
+
+def refuse():
+    """Raised by an operator whose native front end refused arguments that its own assertions let pass (a size the
+    library rejects, a tensor without storage)."""
+    raise Dsv4Error(-2, lib().dsv4_error_string(-2).decode())
 
 
 def device_error() -> int:

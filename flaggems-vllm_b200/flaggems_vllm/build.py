@@ -1,6 +1,7 @@
 """Builds the CUDA libraries in place with nvcc for sm_100a: `python -m flaggems_vllm.build`.
 
   libdsv4_prologue.so            the operators (the product)
+  _host_calls.so                 native front ends of the Python operators (CPython extension, plain C++ against torch)
   testing/libdsv4_hbm_probe.so   aids: the bandwidth probe the benchmark compares the kernels with, and the on-device
                                  check of the quantisers' division shortcut that a test runs
 
@@ -13,12 +14,15 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG.parent / "csrc"
 OUT = PKG / "libdsv4_prologue.so"
 PROBE_OUT = PKG / "testing" / "libdsv4_hbm_probe.so"
+HOST_OUT = PKG / "_host_calls.so"
+HOST_SOURCES = ("host_calls.cpp",)
 PROBE_SOURCES = ("hbm_probe.cu", "division_probe.cu")
 SOURCES = ("abi.cu", "prologue_rows.cu", "prologue_bulk.cu", "gather_dequant.cu", "q_kv_rmsnorm.cu", "inv_rope_fp8_quant.cu", "indexer_k_quant.cu",
            "indexer_q_rope_quant.cu", "cp_gather_indexer.cu", "topk_indices.cu", "topk_per_row.cu", "topk_per_row_short.cu", "group_quant_fp8.cu")
@@ -40,6 +44,22 @@ def command(extra_flags=(), out: Path = OUT, sources=SOURCES) -> list[str]:
     ]
 
 
+def host_command(out: Path = HOST_OUT) -> list[str]:
+    """g++ command of the extension module: linked against the operator library beside it (found at load time through
+    $ORIGIN) and against torch's libraries, which the interpreter has loaded by then."""
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc_path()).resolve().parent.parent
+    includes = (root / "include", root / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"])
+    return [
+        shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+        *[f"-I{i}" for i in includes], *[str(CSRC / s) for s in HOST_SOURCES], "-o", str(out),
+        f"-L{OUT.parent}", f"-l:{OUT.name}", f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",
+        "-Wl,-rpath,$ORIGIN",
+    ]
+
+
 def up_to_date(out: Path = OUT, sources=SOURCES) -> bool:
     if not out.exists():
         return False
@@ -48,18 +68,18 @@ def up_to_date(out: Path = OUT, sources=SOURCES) -> bool:
 
 
 def build(force: bool = False, verbose: bool = False, extra_flags=()) -> Path:
-    """Build whichever of the two libraries is older than its sources; returns the operator library's path."""
+    """Build whichever of the libraries is older than its sources; returns the operator library's path."""
     env = dict(os.environ)
     env.pop("CC", None), env.pop("CXX", None)  # let nvcc pick the system host compiler
-    for out, sources in ((OUT, SOURCES), (PROBE_OUT, PROBE_SOURCES)):
+    for out, sources in ((OUT, SOURCES), (HOST_OUT, HOST_SOURCES), (PROBE_OUT, PROBE_SOURCES)):
         if not force and up_to_date(out, sources):
             continue
-        cmd = command(extra_flags, out, sources)
+        cmd = host_command(out) if out == HOST_OUT else command(extra_flags, out, sources)
         res = subprocess.run(cmd, capture_output=True, text=True, env=env)
         if verbose or res.returncode != 0:
             sys.stderr.write(" ".join(cmd) + "\n" + res.stdout + res.stderr)
         if res.returncode != 0:
-            raise RuntimeError(f"nvcc failed building {out.name}")
+            raise RuntimeError(f"{Path(cmd[0]).name} failed building {out.name}")
     return OUT
 
 

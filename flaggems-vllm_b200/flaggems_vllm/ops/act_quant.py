@@ -13,26 +13,24 @@ import torch
 
 from .. import _native
 
+_call = None  # the native front end, looked up once
+
+
+def _bind():
+    global _call
+    _call = _native.host_calls().act_quant
+    return _call
+
 
 def act_quant_triton(x: torch.Tensor, block_size: int = 128, scale_fmt: Optional[str] = None) -> Tuple[torch.Tensor, torch.Tensor]:
+    result = (_call or _bind())(x, block_size, scale_fmt is not None)
+    if result is not None:
+        return result
     assert x.is_contiguous(), "Input tensor must be contiguous"
     assert x.size(-1) % block_size == 0, f"Last dimension size must be divisible by block_size (block_size={block_size})"
     assert x.device.type == "cuda", "this operator has no CPU path"
     assert x.dtype == torch.bfloat16, "bfloat16 only"
-    n = x.size(-1)
-    x_2d = x.view(-1, n)
-    m = x_2d.size(0)
-    y = torch.empty_like(x, dtype=torch.float8_e4m3fn)
-    s = x.new_empty(*x.size()[:-1], n // block_size, dtype=torch.float32)
-    if m == 0 or n == 0:
-        return y, s
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-        _native.check(
-            _native.lib().dsv4_act_quant(x_2d.data_ptr(), x_2d.stride(0), y.data_ptr(), s.data_ptr(), m, n, int(block_size),
-                                         1 if scale_fmt is not None else 0, stream)
-        )
-    return y, s
+    _native.refuse()
 
 
 __all__ = ["act_quant_triton"]

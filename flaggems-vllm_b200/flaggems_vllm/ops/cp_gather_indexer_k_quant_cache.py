@@ -12,13 +12,21 @@ import torch
 
 from .. import _native
 
+_call = None  # the native front end, looked up once
+
+
+def _bind():
+    global _call
+    _call = _native.host_calls().cp_gather_indexer
+    return _call
+
 
 def cp_gather_indexer_k_quant_cache(k_cache: torch.Tensor, k_fp8: torch.Tensor, k_fp8_scale: torch.Tensor,
                                     block_table: torch.Tensor, cu_seqlen: torch.Tensor) -> None:
+    if (_call or _bind())(k_cache, k_fp8, k_fp8_scale, block_table, cu_seqlen) is not None:
+        return
     num_tokens = k_fp8.size(0)
-    block_size = k_cache.size(1)
     head_dim = k_fp8.shape[-1]
-    num_blocks = k_cache.shape[0]
     # the reference takes the scales as uint8 [T, 4*groups]; a float32 [T, groups] tensor is the same bytes
     scale_row_bytes = k_fp8_scale.size(1) * k_fp8_scale.element_size()
     quant_block_size = head_dim * 4 // scale_row_bytes
@@ -38,17 +46,7 @@ def cp_gather_indexer_k_quant_cache(k_cache: torch.Tensor, k_fp8: torch.Tensor, 
     assert cu_seqlen.shape[0] == batch_size + 1
     for t in (k_fp8, k_fp8_scale, block_table, cu_seqlen):
         assert t.device == dev, "all tensors must be on the same device"
-    if num_tokens == 0 or batch_size == 0 or num_blocks == 0:
-        return
-    with torch.cuda.device(dev):
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        _native.check(
-            _native.lib().dsv4_cp_gather_indexer_k_quant_cache(
-                k_cache.data_ptr(), k_cache.stride(0), k_fp8.data_ptr(), k_fp8.stride(0), k_fp8_scale.data_ptr(),
-                k_fp8_scale.stride(0) * k_fp8_scale.element_size(), block_table.data_ptr(), block_table.stride(0),
-                cu_seqlen.data_ptr(), batch_size, num_tokens, block_size, head_dim, num_quant_blocks, stream,
-            )
-        )
+    _native.refuse()
 
 
 __all__ = ["cp_gather_indexer_k_quant_cache"]

@@ -12,6 +12,14 @@ import torch
 
 from .. import _native
 
+_call = None  # the native front end, looked up once
+
+
+def _bind():
+    global _call
+    _call = _native.host_calls().dequantize_and_gather
+    return _call
+
 
 def _default_scale_slots(nope_dim: int) -> int:
     return (nope_dim + 63) // 64 + (1 if nope_dim % 64 == 0 else 0)
@@ -40,6 +48,9 @@ def dequantize_and_gather_k_cache(
     """out[r, offset + i, :nope_dim + rope_dim] = token at position seq_lens[r] - gather_lens[r] + i of
     request r (the whole sequence when gather_lens is None), read from the paged cache through
     block_table[r] and de-quantised: e4m3 * 2^(scale byte - 127) per 64 values -> bf16, RoPE bf16 copied."""
+    call = _call or _bind()
+    if call(out, k_cache, seq_lens, gather_lens, block_table, block_size, offset, rope_dim, nope_dim, scale_slots) is not None:
+        return
     assert out.ndim == 3 and out.dtype == torch.bfloat16
     assert seq_lens.ndim == 1 and block_table.ndim == 2
     assert seq_lens.shape[0] == block_table.shape[0] <= out.shape[0]
@@ -60,19 +71,10 @@ def dequantize_and_gather_k_cache(
         assert gather_lens.dtype == index_dtype and gather_lens.is_contiguous() and gather_lens.shape == seq_lens.shape
     for t in (k_cache_2d, seq_lens, block_table) + ((gather_lens,) if gather_lens is not None else ()):
         assert t.device == out.device, "all tensors must be on the same device"
-    num_reqs = seq_lens.shape[0]
-    if num_reqs == 0 or out.shape[1] == 0:
-        return
-    with torch.cuda.device(out.device):
-        stream = torch.cuda.current_stream(out.device).cuda_stream
-        _native.check(
-            _native.lib().dsv4_dequantize_and_gather_k_cache(
-                out.data_ptr(), out.stride(0), out.stride(1), out.shape[1], k_cache_2d.data_ptr(), seq_lens.data_ptr(),
-                gather_lens.data_ptr() if gather_lens is not None else None, block_table.data_ptr(), num_reqs,
-                block_table.shape[1], int(block_size), k_cache_2d.stride(0), int(offset), int(nope_dim), int(rope_dim),
-                int(scale_slots), 1 if index_dtype == torch.int64 else 0, stream,
-            )
-        )
+    # what is left is a 3-D cache with gaps between its rows, which was copied above
+    if k_cache.ndim == 2 or call(out, k_cache_2d, seq_lens, gather_lens, block_table, block_size, offset, rope_dim, nope_dim,
+                                 scale_slots) is None:
+        _native.refuse()
 
 
 __all__ = ["dequantize_and_gather_k_cache"]

@@ -19,8 +19,7 @@ TOKEN_BYTES = 584  # 448 e4m3 + 64 bf16 + 8 scale bytes per cached token
 
 def _check_arguments(q, kv, k_cache, slot_mapping, position_ids, cos_sin_cache, cache_block_size):
     """The reference's checks (:320-333) in its order and with its exception type, then what the reference leaves
-    to chance and a raw-pointer kernel cannot.  Returns (num_tokens, num_heads, num_tokens_insert, device index).
-    Written for a short call: decode-sized launches run about as long as this function."""
+    to chance and a raw-pointer kernel cannot.  Returns (num_tokens, num_heads, num_tokens_insert)."""
     assert q.is_contiguous() and kv.is_contiguous()
     num_tokens, num_heads, head_dims = q.shape
     assert head_dims == HEAD_DIM
@@ -42,18 +41,16 @@ def _check_arguments(q, kv, k_cache, slot_mapping, position_ids, cos_sin_cache, 
     assert index >= 0 and q.is_cuda, "this operator has no CPU path: tensors must live on a CUDA device"
     assert (kv.get_device() == index and k_cache.get_device() == index and slot_mapping.get_device() == index
             and position_ids.get_device() == index and cos_sin_cache.get_device() == index), "all tensors must be on the same device"
-    return num_tokens, num_heads, num_tokens_insert, index
+    return num_tokens, num_heads, num_tokens_insert
 
 
-# raw handle of the current stream without building a torch.cuda.Stream object
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
-_launch = None  # the bound C entry point, looked up once
+_call = None  # the native front end, looked up once
 
 
 def _bind():
-    global _launch
-    _launch = _native.lib().dsv4_qnorm_rope_kv_insert
-    return _launch
+    global _call
+    _call = _native.host_calls().prologue
+    return _call
 
 
 def fused_deepseek_v4_qnorm_rope_kv_rope_quant_insert(
@@ -84,24 +81,9 @@ def fused_deepseek_v4_qnorm_rope_kv_rope_quant_insert(
         eps: RMSNorm epsilon
         cache_block_size: tokens per cache block
     """
-    num_tokens, num_heads, num_tokens_insert, index = _check_arguments(
-        q, kv, k_cache, slot_mapping, position_ids, cos_sin_cache, cache_block_size)
-    if num_tokens == 0:
-        return
-    launch = _launch or _bind()
-    # the library launches on the current device: switch only when q lives elsewhere (the guard costs
-    # several microseconds, which matters for decode-sized calls outside CUDA graphs)
-    if index == torch.cuda.current_device():
-        code = launch(q.data_ptr(), kv.data_ptr(), k_cache.data_ptr(), slot_mapping.data_ptr(), position_ids.data_ptr(),
-                      cos_sin_cache.data_ptr(), float(eps), num_tokens, num_heads, num_tokens_insert, int(cache_block_size),
-                      k_cache.stride(0), _raw_stream(index))
-    else:
-        with torch.cuda.device(index):
-            code = launch(q.data_ptr(), kv.data_ptr(), k_cache.data_ptr(), slot_mapping.data_ptr(), position_ids.data_ptr(),
-                          cos_sin_cache.data_ptr(), float(eps), num_tokens, num_heads, num_tokens_insert, int(cache_block_size),
-                          k_cache.stride(0), _raw_stream(index))
-    if code != 0:
-        _native.check(code)
+    if (_call or _bind())(q, kv, k_cache, slot_mapping, position_ids, cos_sin_cache, eps, cache_block_size) is None:
+        _check_arguments(q, kv, k_cache, slot_mapping, position_ids, cos_sin_cache, cache_block_size)
+        _native.refuse()
 
 
 def fused_deepseek_v4_qnorm_rope_kv_rope_quant_insert_padded(
@@ -118,7 +100,7 @@ def fused_deepseek_v4_qnorm_rope_kv_rope_quant_insert_padded(
     """The nine-argument, out-of-place form vLLM >= 0.22 uses: q is left untouched and a new tensor
     [num_tokens, padded_heads, 512] is returned whose first num_heads heads hold the normalised, rotated q and
     whose remaining heads are zero; the KV side is the same as in the in-place operator."""
-    num_tokens, num_heads, num_tokens_insert, _ = _check_arguments(
+    num_tokens, num_heads, num_tokens_insert = _check_arguments(
         q, kv, k_cache, slot_mapping, position_ids, cos_sin_cache, cache_block_size)
     dev = q.device
     assert padded_heads >= num_heads
@@ -143,7 +125,7 @@ def fused_deepseek_v4_qnorm_rope_kv_rope_quant_insert_checked(
     """Debug form: same effects, but positions outside the table and slots outside the cache
     are skipped on the device and reported.  Returns a bit mask (bit 0: a bad position, bit 1:
     a bad slot); 0 means every index was in range.  Synchronises to read the mask."""
-    num_tokens, num_heads, num_tokens_insert, _ = _check_arguments(
+    num_tokens, num_heads, num_tokens_insert = _check_arguments(
         q, kv, k_cache, slot_mapping, position_ids, cos_sin_cache, cache_block_size)
     status = torch.zeros(1, dtype=torch.int32, device=q.device)
     if num_tokens == 0:

@@ -10,8 +10,15 @@ import torch
 
 from .. import _native
 
-MXFP4_BLOCK_SIZE = 32
-_WEIGHT_DTYPES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
+_WEIGHT_DTYPES = (torch.bfloat16, torch.float16, torch.float32)
+
+_call = None  # the native front end, looked up once
+
+
+def _bind():
+    global _call
+    _call = _native.host_calls().indexer_q_rope_quant
+    return _call
 
 
 def fused_indexer_q_rope_quant(
@@ -31,6 +38,10 @@ def fused_indexer_q_rope_quant(
     block-scale bytes when D = 128, else uint8 [T, H, D/32] viewed as int32); weights_out = weights *
     softmax_scale * head_scale.
     """
+    result = (_call or _bind())(positions, index_q, index_q_cos_sin_cache, index_weights, index_weights_softmax_scale,
+                                index_weights_head_scale, use_fp4)
+    if result is not None:
+        return result
     assert positions.ndim == 1
     assert index_q.ndim == 3
     assert index_q_cos_sin_cache.ndim == 2
@@ -50,40 +61,7 @@ def fused_indexer_q_rope_quant(
     assert rot_dim % 2 == 0 and rot_dim <= head_dim and (head_dim - rot_dim) % (head_dim // 32) == 0
     for t in (positions, index_q_cos_sin_cache, index_weights):
         assert t.device == index_q.device, "all tensors must be on the same device"
-
-    index_weights_out = torch.empty_like(index_weights, dtype=torch.float32)
-    assert index_weights_out.stride(1) == 1 or num_heads == 1
-    if use_fp4:
-        assert head_dim % MXFP4_BLOCK_SIZE == 0
-        q_out = torch.empty((num_tokens, num_heads, head_dim // 2), dtype=torch.uint8, device=index_q.device)
-        q_scale = torch.empty((num_tokens, num_heads, head_dim // MXFP4_BLOCK_SIZE), dtype=torch.uint8, device=index_q.device)
-        scale_args = (q_scale.data_ptr(), q_scale.stride(0), q_scale.stride(1))
-    else:
-        q_out = torch.empty_like(index_q, dtype=torch.float8_e4m3fn)
-        assert q_out.stride(2) == 1
-        q_scale = None
-        scale_args = (None, 0, 0)
-    if num_tokens > 0:
-        with torch.cuda.device(index_q.device):
-            stream = torch.cuda.current_stream(index_q.device).cuda_stream
-            _native.check(
-                _native.lib().dsv4_fused_indexer_q_rope_quant(
-                    positions.data_ptr(), index_q.data_ptr(), index_q.stride(0), index_q.stride(1),
-                    index_q_cos_sin_cache.data_ptr(), index_q_cos_sin_cache.stride(0),
-                    1 if index_q_cos_sin_cache.dtype == torch.bfloat16 else 0, rot_dim, q_out.data_ptr(), q_out.stride(0),
-                    q_out.stride(1), *scale_args, index_weights.data_ptr(), index_weights.stride(0),
-                    _WEIGHT_DTYPES[index_weights.dtype], index_weights_out.data_ptr(), index_weights_out.stride(0),
-                    float(index_weights_softmax_scale), float(index_weights_head_scale), num_tokens, num_heads, head_dim,
-                    1 if use_fp4 else 0, stream,
-                )
-            )
-    if use_fp4:
-        # four UE8M0 bytes per head (head_dim 128) are handed on as one int32, as the reference does; other
-        # head sizes keep the byte tensor where the reference's int32 view is only defined for multiples of 4
-        if q_scale.shape[-1] % 4 == 0:
-            q_scale = q_scale.view(torch.int32).squeeze(-1)
-        return (q_out, q_scale), index_weights_out
-    return q_out, index_weights_out
+    _native.refuse()
 
 
 __all__ = ["fused_indexer_q_rope_quant"]

@@ -15,9 +15,13 @@ from .. import _native
 
 SUPPORTED_FP8_DTYPE = torch.float8_e4m3fn
 
+_call = None  # the native front end, looked up once
 
-def _get_tma_aligned_size(size: int, align: int) -> int:
-    return ((size + align - 1) // align) * align
+
+def _bind():
+    global _call
+    _call = _native.host_calls().inv_rope_fp8_quant
+    return _call
 
 
 def fused_inv_rope_fp8_quant(
@@ -44,6 +48,11 @@ def fused_inv_rope_fp8_quant(
         o_scale: [num_tokens, n_groups, blocks] float32, or int32 with four UE8M0 bytes per head when
                  tma_aligned_scales; token-major storage padded to a multiple of 4 tokens
     """
+    if dtype is None or dtype == SUPPORTED_FP8_DTYPE:
+        result = (_call or _bind())(o, positions, cos_sin_cache, n_groups, heads_per_group, nope_dim, rope_dim, quant_group_size, eps,
+                                    tma_aligned_scales)
+        if result is not None:
+            return result
     fp8_dtype = SUPPORTED_FP8_DTYPE if dtype is None else dtype
     assert fp8_dtype == torch.float8_e4m3fn, "only torch.float8_e4m3fn is supported"
     assert o.ndim == 3, "`o` must be [num_tokens, num_heads, head_dim]"
@@ -74,30 +83,7 @@ def fused_inv_rope_fp8_quant(
         # with fewer than four the reference's kernel writes one int32 per head into storage sized for one per four
         # groups (:133-143 against :206-217 there): only four groups per head have a defined packed layout
         assert chunks_per_head == 4, "packed UE8M0 scales need four groups per head"
-
-    d = heads_per_group * head_dim
-    num_scale_blocks = d // quant_group_size
-    tma_aligned_t = _get_tma_aligned_size(num_tokens, 4)
-    if tma_aligned_scales:
-        scale_inner, scale_dtype = (num_scale_blocks + 3) // 4, torch.int32
-    else:
-        scale_inner, scale_dtype = num_scale_blocks, torch.float32
-
-    fp8_q = torch.empty((n_groups, num_tokens, d), dtype=fp8_dtype, device=o.device)
-    scale = torch.empty(n_groups * scale_inner * tma_aligned_t, dtype=scale_dtype, device=o.device).as_strided(
-        (n_groups, num_tokens, scale_inner), (scale_inner * tma_aligned_t, 1, tma_aligned_t))
-    if num_tokens > 0:
-        with torch.cuda.device(o.device):
-            stream = torch.cuda.current_stream(o.device).cuda_stream
-            _native.check(
-                _native.lib().dsv4_fused_inv_rope_fp8_quant_geometry(
-                    o.data_ptr(), o.stride(0), o.stride(1), positions.data_ptr(), cos_sin_cache.data_ptr(),
-                    cos_sin_cache.stride(0), fp8_q.data_ptr(), scale.data_ptr(), scale_inner * tma_aligned_t, num_tokens,
-                    tma_aligned_t, n_groups, heads_per_group, int(nope_dim), int(rope_dim), int(quant_group_size), float(eps),
-                    1 if tma_aligned_scales else 0, stream,
-                )
-            )
-    return fp8_q.transpose(0, 1), scale.transpose(0, 1)
+    _native.refuse()
 
 
 __all__ = ["fused_inv_rope_fp8_quant"]

@@ -11,13 +11,21 @@ import torch
 
 from .. import _native
 
+_call = None  # the native front end, looked up once
+
+
+def _bind():
+    global _call
+    _call = _native.host_calls().indexer_k_quant
+    return _call
+
 
 def indexer_k_quant_and_cache(k: torch.Tensor, kv_cache: torch.Tensor, slot_mapping: torch.Tensor, quant_block_size,
                               scale_fmt) -> None:
-    num_blocks = kv_cache.shape[0]
+    if (_call or _bind())(k, kv_cache, slot_mapping, quant_block_size, scale_fmt == "ue8m0") is not None:
+        return
     head_dim = k.shape[-1]
     num_tokens = slot_mapping.shape[0]
-    block_size = kv_cache.shape[1]
     if head_dim % quant_block_size != 0:
         raise ValueError("head_dim must be divisible by quant_block_size")
     assert k.device.type == "cuda", "this operator has no CPU path"
@@ -27,17 +35,7 @@ def indexer_k_quant_and_cache(k: torch.Tensor, kv_cache: torch.Tensor, slot_mapp
     assert kv_cache.dtype == torch.uint8 and kv_cache.dim() == 3 and kv_cache[0].is_contiguous()
     assert kv_cache.shape[2] == head_dim + 4 * (head_dim // quant_block_size), "cache row = values + fp32 scales"
     assert kv_cache.device == k.device and slot_mapping.device == k.device
-    if num_tokens == 0 or num_blocks == 0:
-        return
-    with torch.cuda.device(k.device):
-        stream = torch.cuda.current_stream(k.device).cuda_stream
-        _native.check(
-            _native.lib().dsv4_indexer_k_quant_and_cache(
-                k.data_ptr(), k.stride(0), 1 if k.dtype == torch.float16 else 0, kv_cache.data_ptr(), kv_cache.stride(0),
-                slot_mapping.data_ptr(), num_tokens, block_size, head_dim, int(quant_block_size),
-                1 if scale_fmt == "ue8m0" else 0, stream,
-            )
-        )
+    _native.refuse()
 
 
 __all__ = ["indexer_k_quant_and_cache"]

@@ -15,6 +15,14 @@ from .. import _native
 
 SUPPORTED_FP8_DTYPE = torch.float8_e4m3fn
 
+_call = None  # the native front end, looked up once
+
+
+def _bind():
+    global _call
+    _call = _native.host_calls().group_quant
+    return _call
+
 
 def per_token_group_quant_fp8(
     x: torch.Tensor,
@@ -24,6 +32,10 @@ def per_token_group_quant_fp8(
     column_major_scales: bool = False,
     scale_ue8m0: bool = False,
 ) -> Tuple[torch.Tensor, torch.Tensor]:
+    if dtype is None or dtype == SUPPORTED_FP8_DTYPE:
+        result = (_call or _bind())(x, group_size, eps, column_major_scales, scale_ue8m0)
+        if result is not None:
+            return result
     fp8_dtype = SUPPORTED_FP8_DTYPE if dtype is None else dtype
     assert x.shape[-1] % group_size == 0, (
         f"the last dimension of `x` {x.shape[-1]} must be divisible by `group_size` {group_size}")
@@ -31,27 +43,8 @@ def per_token_group_quant_fp8(
     assert x.device.type == "cuda", "this operator has no CPU path"
     assert x.dtype == torch.bfloat16 and fp8_dtype == torch.float8_e4m3fn, "bfloat16 -> float8_e4m3fn only"
     assert x.dim() >= 2 and (x.dim() == 2 or x.is_contiguous()), "[M, K] with any row stride, or a contiguous tensor of more dimensions"
-    cols = x.shape[-1]
-    x2 = x if x.dim() == 2 else x.view(-1, cols)
-    rows = x2.shape[0]
-    x_q = torch.empty(x.shape, device=x.device, dtype=fp8_dtype)
-    if column_major_scales:
-        shape = (cols // group_size,) + x.shape[:-1]
-        x_s = torch.empty(shape, device=x.device, dtype=torch.float32).permute(-1, -2)
-        assert x.dim() == 2, "column-major scales for [M, K] inputs"
-        stride_row, stride_group = x_s.stride(0), x_s.stride(1)
-    else:
-        x_s = torch.empty(x.shape[:-1] + (cols // group_size,), device=x.device, dtype=torch.float32)
-        stride_row, stride_group = cols // group_size, 1
-    if rows == 0 or cols == 0:
-        return x_q, x_s
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream(x.device).cuda_stream
-        _native.check(
-            _native.lib().dsv4_per_token_group_quant_fp8(x2.data_ptr(), x2.stride(0), x_q.data_ptr(), x_s.data_ptr(), stride_row, stride_group,
-                                                         rows, cols, int(group_size), float(eps), 1 if scale_ue8m0 else 0, stream)
-        )
-    return x_q, x_s
+    assert not column_major_scales or x.dim() == 2, "column-major scales for [M, K] inputs"
+    _native.refuse()
 
 
 __all__ = ["per_token_group_quant_fp8"]

@@ -13,9 +13,20 @@ import torch
 
 from .. import _native
 
+_call = None  # the native front end, looked up once
+
+
+def _bind():
+    global _call
+    _call = _native.host_calls().persistent_topk
+    return _call
+
 
 def persistent_topk(logits: torch.Tensor, lengths: torch.Tensor, output: torch.Tensor, workspace: torch.Tensor, k: int = 512,
                     max_seq_len: int | None = None) -> None:
+    # a row never reaches beyond max_seq_len (the reference sizes its chunks by it)
+    if (_call or _bind())(logits, lengths, output, k, max_seq_len) is not None:
+        return
     assert logits.is_cuda, "persistent_topk: logits must be CUDA tensor"
     assert lengths.is_cuda, "persistent_topk: lengths must be CUDA tensor"
     assert output.is_cuda, "persistent_topk: output must be CUDA tensor"
@@ -33,16 +44,7 @@ def persistent_topk(logits: torch.Tensor, lengths: torch.Tensor, output: torch.T
         f"persistent_topk: output size mismatch: ({output.size(0)}, {output.size(1)}) vs ({num_rows}, {k})")
     assert k in (512, 1024, 2048), f"persistent_topk supports k=512, k=1024, or k=2048, got k={k}"
     assert output.is_contiguous() and logits.device == output.device == lengths.device
-    if num_rows == 0:
-        return
-    # a row never reaches beyond max_seq_len (the reference sizes its chunks by it)
-    width = logits.shape[1] if max_seq_len is None else min(logits.shape[1], int(max_seq_len))
-    with torch.cuda.device(logits.device):
-        stream = torch.cuda.current_stream(logits.device).cuda_stream
-        _native.check(
-            _native.lib().dsv4_top_k_per_row_prefill(logits.data_ptr(), logits.stride(0), logits.stride(1), None, seq_lens.data_ptr(),
-                                                     output.data_ptr(), num_rows, width, int(k), stream)
-        )
+    _native.refuse()
 
 
 __all__ = ["persistent_topk"]

@@ -11,6 +11,14 @@ import torch
 
 from .. import _native
 
+_call = None  # the native front end, looked up once
+
+
+def _bind():
+    global _call
+    _call = _native.host_calls().top_k_decode
+    return _call
+
 
 def _check(logits, indices, num_rows, stride0, stride1, top_k):
     assert num_rows == logits.shape[0]
@@ -22,17 +30,12 @@ def _check(logits, indices, num_rows, stride0, stride1, top_k):
 
 
 def top_k_per_row_decode(logits, next_n, seq_lens, indices, num_rows, stride0, stride1, top_k) -> None:
+    if (_call or _bind())(logits, next_n, seq_lens, indices, num_rows, stride0, stride1, top_k) is not None:
+        return
     _check(logits, indices, num_rows, stride0, stride1, top_k)
     assert seq_lens.dtype == torch.int32 and seq_lens.dim() == 1 and seq_lens.is_contiguous() and seq_lens.device == logits.device
     assert next_n >= 1 and seq_lens.shape[0] * next_n >= num_rows
-    if num_rows == 0 or top_k == 0:
-        return
-    with torch.cuda.device(logits.device):
-        stream = torch.cuda.current_stream(logits.device).cuda_stream
-        _native.check(
-            _native.lib().dsv4_top_k_per_row_decode(logits.data_ptr(), stride0, stride1, int(next_n), seq_lens.data_ptr(),
-                                                    indices.data_ptr(), num_rows, logits.shape[1], int(top_k), stream)
-        )
+    _native.refuse()
 
 
 __all__ = ["top_k_per_row_decode"]

@@ -12,19 +12,22 @@ import torch
 from .. import _native
 from .top_k_per_row_decode import _check
 
+_call = None  # the native front end, looked up once
+
+
+def _bind():
+    global _call
+    _call = _native.host_calls().top_k_prefill
+    return _call
+
 
 def top_k_per_row_prefill(logits, row_starts, row_ends, indices, num_rows, stride0, stride1, top_k) -> None:
+    if (_call or _bind())(logits, row_starts, row_ends, indices, num_rows, stride0, stride1, top_k) is not None:
+        return
     _check(logits, indices, num_rows, stride0, stride1, top_k)
     for t in (row_starts, row_ends):
         assert t.dtype == torch.int32 and t.dim() == 1 and t.is_contiguous() and t.shape[0] >= num_rows and t.device == logits.device
-    if num_rows == 0 or top_k == 0:
-        return
-    with torch.cuda.device(logits.device):
-        stream = torch.cuda.current_stream(logits.device).cuda_stream
-        _native.check(
-            _native.lib().dsv4_top_k_per_row_prefill(logits.data_ptr(), stride0, stride1, row_starts.data_ptr(), row_ends.data_ptr(),
-                                                     indices.data_ptr(), num_rows, logits.shape[1], int(top_k), stream)
-        )
+    _native.refuse()
 
 
 __all__ = ["top_k_per_row_prefill"]
