@@ -8,25 +8,35 @@
 //   decode:  start_i = 0, end_i = seq_lens[i / next_n] - next_n + i % next_n + 1
 //   prefill: start_i = row_starts[i], end_i = row_ends[i]
 //
-// One CTA per row, or a thread-block cluster of 2 / 4 / 8 CTAs for long rows.  Values are ranked by a coarse, monotone 11-bit code (top bits of the fp16 rounding of the value,
-// which spreads real logits over hundreds of bins where the top bits of the fp32 pattern would hit a handful) and,
-// inside a bin, by the order-preserving 32-bit key of their fp32 pattern.
-//   Fast route, ONE read of the row: a sample of the row (128 runs of 32 values) gives a bin b0 above which k values
-//   plus four standard deviations are expected; the row is streamed once and every value in a bin >= b0 is put
-//   into shared memory with its key and position; if at least k and at most kCandidateCap values were collected, a
-//   radix selection in shared memory finishes the job.  In a cluster every CTA streams its share of the row and hands
-//   its candidates to the first CTA through distributed shared memory (two hardware cluster barriers, no spinning).
-//   Histogram route, two reads (the second mostly out of L2), when the sample misjudged the row or k is too large for
-//   the candidate buffer: 1. histogram of the coarse code over the whole row, 2. the bin of the k-th largest value is
-//   located, values in higher bins are emitted, the values of that bin are collected in shared memory, 3. radix
-//   selection among them.
-//   A bin with more values than fit in shared memory (degenerate inputs: thousands of near-equal values) takes three
-//   more histogram reads of the row on the bits of the fp32 key, then one emitting read.
-// The result does not depend on the route; the sample only decides how fast it is reached.
-// HBM traffic on the fast route: the row once (4 bytes per value); top_k * 4 bytes written.
+// Values are ranked by the order-preserving 32-bit key of their fp32 pattern.  ONE read of the row on the normal route:
+//   1. a sample of the row gives a value t that k values plus four standard deviations of that count are expected to
+//      reach (histogram of a coarse, monotone 11-bit code: the top bits of the fp16 rounding of the value, which spreads
+//      real logits over hundreds of bins where the top bits of the fp32 pattern would hit a handful);
+//   2. every value that reaches t goes with its position to a pool in shared memory, where a warp reserves room for all
+//      candidates among 512 values with one atomic; no branches (these kernels are bound by instruction issue and by the
+//      phases between barriers before they are bound by HBM);
+//   3. the candidates (about 1.1 to 3 k of them) are ranked by a histogram of (key - key(t)), whose bins are fine where
+//      the k-th largest is to be expected; the few candidates of its bin are ranked by counting.
+// Three kernels:
+//   topk_short_kernel       one CTA per row, the row in registers; short rows, of which a large part is selected, go without a
+//                           sample: a coarse histogram of all values, then straight to the ranking
+//   topk_registers_kernel   one CTA per row, the row in registers, its sample taken from them
+//   topk_stream_kernel      longer rows: one CTA, or a thread-block cluster of 2 / 4 / 8 CTAs, streams the row past t; the
+//                           first 64 bytes of every thread are on their way while the sample is evaluated.  In a
+//                           cluster every CTA takes the same sample, streams its share and hands its candidates to the
+//                           first CTA through distributed shared memory (two hardware cluster barriers, no spinning).
+// When the sample misjudged the row (fewer than k candidates, or the pool full), or k is too large
+// for the pool, a histogram route reads the row twice more; thousands of near-equal values take a radix selection over the
+// row.  The result does not depend on the route; the sample only decides how fast it is reached.
+// HBM traffic on the normal route: the row once (4 bytes per value); top_k * 4 bytes written.
+// Measured (rows of ragged length, a quarter to the whole of the width; before -> after the pool, the scans by one warp and the
+// choice of CTA sizes): 4096 x 32768, k 2048: 236 -> 123 us; k 512: 192 -> 95 us (3.5 TB/s); 496 x 262144, k 512: 98 -> 74 us;
+// 4096 x 65536, k 1024: 290 -> 150 us (4.5 TB/s); 61 x 16384: 12.8 -> 7.0 us; 1 x 32768: 11.8 -> 7.5 us.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "dsv4_common.cuh"
@@ -36,21 +46,18 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-#ifndef DSV4_TOPK_THREADS
-#define DSV4_TOPK_THREADS 512
-#endif
-constexpr int kTopkThreads = DSV4_TOPK_THREADS;
 constexpr int kBins = 2048;
-constexpr int kCandidateCap = 8192;  // 64 KiB of (key, position) pairs in dynamic shared memory
-constexpr int kSampleChunks = 128;  // x 32 values
 constexpr int kCountingMax = kBins / 2;  // candidates of one bin ranked by counting (they are kept where the histogram was)
+constexpr int kStreamBatch = 4;          // quads (of 4 consecutive values) per thread in flight
+constexpr int kSampleQuads = 1024;       // of the streaming kernel
 
 struct TopkParams {
     const float* logits;
     int64_t stride0, stride1;
     int32_t* indices;  // [num_rows, top_k]
     int32_t num_rows, vocab, top_k;
-    uint32_t pair_capacity;  // (key, position) pairs the dynamic shared memory of this launch holds
+    uint32_t capacity;  // of the candidate pool
+    bool sampled;       // top_k is small enough for it
     // decode
     const int32_t* seq_lens;
     int32_t next_n;
@@ -64,10 +71,27 @@ __device__ __forceinline__ uint32_t order_key(uint32_t bits) { return (bits & 0x
 
 // Coarse monotone code: the top 11 bits of the order key of the value rounded to fp16.
 __device__ __forceinline__ uint32_t coarse_bin(float x) {
-    const uint32_t h = __half_as_ushort(__float2half_rn(x));
-    const uint32_t key = (h & 0x8000u) ? (~h & 0xffffu) : (h | 0x8000u);
-    return key >> 5;
+    const int32_t h = __half_as_short(__float2half_rn(x));  // sign-extended
+    return static_cast<uint32_t>((h ^ ((h >> 15) | 0x8000)) & 0xffff) >> 5;
 }
+
+// A value whose coarse code is `bin`, the lowest one up to the rounding to fp16; -inf for the codes below it.
+__device__ __forceinline__ float value_of_bin(uint32_t bin) {
+    uint32_t key = bin << 5;
+    key = key < 0x0400u ? 0x03ffu : key;  // -inf
+    key = key > 0xfc00u ? 0xfc00u : key;  // +inf
+    const uint32_t h = (key & 0x8000u) ? key & 0x7fffu : ~key & 0xffffu;
+    return __half2float(__ushort_as_half(static_cast<unsigned short>(h)));
+}
+
+// State the threads of a CTA share, apart from the candidates.
+struct Shared {
+    __align__(16) uint32_t hist[kBins];  // later the dense list of the candidates of one bin: kBins / 2 (key, position) pairs
+    uint32_t scratch[32];
+    uint32_t result[4];
+    uint32_t counters[4];  // 0: emitted, 1: collected, 2: ties taken / dense candidates, 3: largest key of the sample
+    uint32_t pooled, below;  // candidates in the pool; those of them below the floor
+};
 
 struct Threshold {
     uint32_t bin;    // the bin holding the k-th largest element
@@ -76,15 +100,18 @@ struct Threshold {
 };
 
 // The bin, counted from the top, in which the running count reaches `want` (1 <= want <= total of hist).
-// All threads call it; hist has kBins entries; `scratch` holds 32 words.  Ends with a barrier.
-__device__ __forceinline__ Threshold find_threshold(const uint32_t* hist, uint32_t want, uint32_t* scratch, uint32_t* result) {
-    constexpr int kPerThread = kBins / kTopkThreads;  // 4 bins per thread, thread 0 owns the highest ones
+// All threads call it; ends with a barrier.
+template <int THREADS>
+__device__ __forceinline__ Threshold find_threshold(Shared& s, uint32_t want) {
+    constexpr int kPerThread = kBins / THREADS;  // thread 0 owns the highest bins
+    constexpr int kWarps = THREADS / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t local[kPerThread], sum = 0;
 #pragma unroll
-    for (int j = 0; j < kPerThread; ++j) {
-        local[j] = hist[kBins - 1 - (tid * kPerThread + j)];
-        sum += local[j];
+    for (int j = 0; j < kPerThread; j += 4) {
+        const uint4 v = *reinterpret_cast<const uint4*>(&s.hist[kBins - 4 - (tid * kPerThread + j)]);
+        local[j] = v.w, local[j + 1] = v.z, local[j + 2] = v.y, local[j + 3] = v.x;
+        sum += v.x + v.y + v.z + v.w;
     }
     uint32_t incl = sum;
 #pragma unroll
@@ -92,35 +119,98 @@ __device__ __forceinline__ Threshold find_threshold(const uint32_t* hist, uint32
         const uint32_t up = __shfl_up_sync(0xffffffffu, incl, m);
         if (lane >= m) incl += up;
     }
-    if (lane == 31) scratch[warp] = incl;
+    if (lane == 31) s.scratch[warp] = incl;
     __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < kTopkThreads / 32 ? scratch[lane] : 0u, wi = w;
-#pragma unroll
-        for (int m = 1; m < 32; m <<= 1) {
-            const uint32_t up = __shfl_up_sync(0xffffffffu, wi, m);
-            if (lane >= m) wi += up;
-        }
-        scratch[lane] = wi - w;  // exclusive prefix of the warp totals
-    }
-    __syncthreads();
-    uint32_t above = scratch[warp] + incl - sum;  // elements in bins higher than this thread's
+    // every warp adds up the totals of the warps in front of it
+    uint32_t before = lane < warp && lane < kWarps ? s.scratch[lane] : 0u;
+    before = __reduce_add_sync(0xffffffffu, before);
+    uint32_t above = before + incl - sum;  // elements in bins higher than this thread's
     if (above < want && want <= above + sum) {
 #pragma unroll
         for (int j = 0; j < kPerThread; ++j) {
             if (above < want && want <= above + local[j]) {
-                result[0] = kBins - 1 - (tid * kPerThread + j);
-                result[1] = want - above;
-                result[2] = local[j];
+                s.result[0] = kBins - 1 - (tid * kPerThread + j);
+                s.result[1] = want - above;
+                s.result[2] = local[j];
             }
             above += local[j];
         }
     }
     __syncthreads();
     Threshold t;
-    t.bin = result[0], t.need = result[1], t.count = result[2];
-    __syncthreads();
+    t.bin = s.result[0], t.need = s.result[1], t.count = s.result[2];
     return t;
+}
+
+// The same by one warp (all its lanes call it), 32 bins at a time: from bin `start` down until the running count reaches
+// `want` >= 1.  One warp's work instead of the CTA's, and short where the bin lies near the start.
+__device__ __forceinline__ Threshold scan_down(const uint32_t* hist, int start, uint32_t want) {
+    const int lane = threadIdx.x & 31;
+    Threshold t{0u, 1u, 1u};
+    uint32_t above = 0u;
+    for (int top = start; top >= 0; top -= 32) {
+        const uint32_t mine = top - lane >= 0 ? hist[top - lane] : 0u;
+        const uint32_t total = __reduce_add_sync(0xffffffffu, mine);
+        if (above + total < want) {
+            above += total;
+            continue;
+        }
+        uint32_t incl = mine;
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, incl, m);
+            if (lane >= m) incl += up;
+        }
+        const int at = __ffs(__ballot_sync(0xffffffffu, above + incl >= want)) - 1;
+        t.bin = static_cast<uint32_t>(top - at);
+        t.count = __shfl_sync(0xffffffffu, mine, at);
+        t.need = want - (above + __shfl_sync(0xffffffffu, incl - mine, at));
+        break;
+    }
+    return t;
+}
+
+// The same from bin 0 up: `skip` elements are left out, the next one is the smallest of those selected.
+__device__ __forceinline__ Threshold scan_up(const uint32_t* hist, uint32_t skip) {
+    const int lane = threadIdx.x & 31;
+    Threshold t{kBins - 1u, 1u, 1u};
+    uint32_t below = 0u;
+    for (int b = 0; b < kBins; b += 32) {
+        const uint32_t mine = hist[b + lane];
+        const uint32_t total = __reduce_add_sync(0xffffffffu, mine);
+        if (below + total <= skip) {
+            below += total;
+            continue;
+        }
+        uint32_t incl = mine;
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, incl, m);
+            if (lane >= m) incl += up;
+        }
+        const int at = __ffs(__ballot_sync(0xffffffffu, below + incl > skip)) - 1;
+        t.bin = static_cast<uint32_t>(b + at);
+        t.count = __shfl_sync(0xffffffffu, mine, at);
+        t.need = t.count - (skip - (below + __shfl_sync(0xffffffffu, incl - mine, at)));
+        break;
+    }
+    return t;
+}
+
+template <int THREADS>
+__device__ __forceinline__ void clear_histogram(Shared& s) {
+    for (int i = threadIdx.x; i < kBins / 4; i += THREADS) reinterpret_cast<uint4*>(s.hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Appends `value` of the lanes whose `take` is set to list[], one atomic per warp.  Whole warps call it.
+__device__ __forceinline__ void append(int32_t* list, uint32_t* counter, bool take, int32_t value) {
+    const uint32_t mask = __ballot_sync(0xffffffffu, take);
+    if (mask == 0u) return;
+    const int lane = threadIdx.x & 31;
+    uint32_t base = 0u;
+    if (lane == 0) base = atomicAdd(counter, __popc(mask));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (take) list[base + __popc(mask & ((1u << lane) - 1u))] = value;
 }
 
 // Histogram increment shared by the lanes of a warp that hit the same bin (degenerate inputs put a whole warp
@@ -133,43 +223,44 @@ __device__ __forceinline__ void add_aggregated(uint32_t* hist, uint32_t bin, boo
 }
 
 // The `want` largest of the n candidates (key, position) in shared memory; their positions are appended to out
-// through counters[0], ties at the smallest selected key through counters[2].  Radix selection in digits of up to
-// 11 bits on key - min(key), starting at the highest bit in which the candidates differ at all (they share sign,
+// through counters[0], ties at the smallest selected key through counters[2] (zero on entry).  Radix selection in digits of
+// up to 11 bits on key - min(key), starting at the highest bit in which the candidates differ at all (they share sign,
 // exponent and leading mantissa bits, which a selection on fixed bit positions would waste passes and atomic
 // conflicts on).
-__device__ __forceinline__ void select_in_shared(const uint2* cand, uint32_t n, uint32_t want, uint32_t* hist, uint32_t* scratch,
-                                                 uint32_t* result, uint32_t* counters, int32_t* out) {
+template <int THREADS>
+__device__ __noinline__ void select_radix(Shared& s, const uint2* cand, uint32_t n, uint32_t want, int32_t* out) {
     const int tid = threadIdx.x;
+    __syncthreads();
     if (want >= n) {
-        for (uint32_t i = tid; i < n; i += kTopkThreads) out[atomicAdd(&counters[0], 1u)] = static_cast<int32_t>(cand[i].y);
+        for (uint32_t i = tid; i < n; i += THREADS) out[atomicAdd(&s.counters[0], 1u)] = static_cast<int32_t>(cand[i].y);
         return;
     }
     // range of the keys
-    if (tid == 0) result[0] = 0xffffffffu, result[1] = 0u;
+    if (tid == 0) s.result[0] = 0xffffffffu, s.result[1] = 0u;
     __syncthreads();
     uint32_t lo = 0xffffffffu, hi = 0u;
-    for (uint32_t i = tid; i < n; i += kTopkThreads) {
+    for (uint32_t i = tid; i < n; i += THREADS) {
         const uint32_t key = cand[i].x;
         lo = key < lo ? key : lo, hi = key > hi ? key : hi;
     }
     lo = __reduce_min_sync(0xffffffffu, lo), hi = __reduce_max_sync(0xffffffffu, hi);
-    if ((tid & 31) == 0) atomicMin(&result[0], lo), atomicMax(&result[1], hi);
+    if ((tid & 31) == 0) atomicMin(&s.result[0], lo), atomicMax(&s.result[1], hi);
     __syncthreads();
-    const uint32_t base = result[0], range = result[1] - result[0];
+    const uint32_t base = s.result[0], range = s.result[1] - s.result[0];
     __syncthreads();
     uint32_t need = want, prefix = 0u, prefix_mask = 0u;
     int top = 32 - __clz(range | 1u);  // bits of (key - base) that can be set
     while (top > 0) {
         const int shift = top > 11 ? top - 11 : 0;
         const uint32_t digit_mask = (1u << (top - shift)) - 1u;
-        for (int i = tid; i < kBins; i += kTopkThreads) hist[i] = 0u;
+        clear_histogram<THREADS>(s);
         __syncthreads();
-        for (uint32_t i = tid; i < n; i += kTopkThreads) {
+        for (uint32_t i = tid; i < n; i += THREADS) {
             const uint32_t rel = cand[i].x - base;
-            if ((rel & prefix_mask) == prefix) atomicAdd(&hist[(rel >> shift) & digit_mask], 1u);
+            if ((rel & prefix_mask) == prefix) atomicAdd(&s.hist[(rel >> shift) & digit_mask], 1u);
         }
         __syncthreads();
-        const Threshold t = find_threshold(hist, need, scratch, result);
+        const Threshold t = find_threshold<THREADS>(s, need);
         prefix |= t.bin << shift;
         prefix_mask |= digit_mask << shift;
         need = t.need;
@@ -177,265 +268,672 @@ __device__ __forceinline__ void select_in_shared(const uint2* cand, uint32_t n, 
         if (t.need == t.count) break;  // every candidate with this prefix is taken: the lower bits do not matter
     }
     // keys above the prefix (on the bits examined) are in; `need` of those equal to it are in
-    for (uint32_t i = tid; i < n; i += kTopkThreads) {
+    for (uint32_t i = tid; i < n; i += THREADS) {
         const uint2 e = cand[i];
         const uint32_t rel_hi = (e.x - base) & prefix_mask;
-        if (rel_hi > prefix || (rel_hi == prefix && atomicAdd(&counters[2], 1u) < need)) out[atomicAdd(&counters[0], 1u)] = static_cast<int32_t>(e.y);
+        if (rel_hi > prefix || (rel_hi == prefix && atomicAdd(&s.counters[2], 1u) < need)) out[atomicAdd(&s.counters[0], 1u)] = static_cast<int32_t>(e.y);
     }
-}
-
-__device__ __forceinline__ uint32_t coarse_bin_of_key(uint32_t key) {  // key -> value -> bin
-    return coarse_bin(__uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key));
 }
 
 // The `want` largest of n candidates by counting: a candidate's rank is the number of candidates ahead of it in the
 // total order (key descending, position ascending); one pass, no histogram.
-__device__ __forceinline__ void rank_by_counting(const uint2* dense, uint32_t n, uint32_t want, uint32_t* counters, int32_t* out) {
-    for (uint32_t a = threadIdx.x; a < n; a += kTopkThreads) {
+template <int THREADS>
+__device__ __forceinline__ void rank_by_counting(Shared& s, const uint2* dense, uint32_t n, uint32_t want, int32_t* out) {
+    for (uint32_t a = threadIdx.x; a < n; a += THREADS) {
         const uint2 e = dense[a];
         uint32_t ahead = 0u;
-#pragma unroll 8
+#pragma unroll 4
         for (uint32_t b = 0; b < n; ++b) {
             const uint2 o = dense[b];  // the same address for all lanes: a broadcast
             ahead += (o.x > e.x || (o.x == e.x && o.y < e.y)) ? 1u : 0u;
         }
-        if (ahead < want) out[atomicAdd(&counters[0], 1u)] = static_cast<int32_t>(e.y);
+        if (ahead < want) out[atomicAdd(&s.counters[0], 1u)] = static_cast<int32_t>(e.y);
     }
 }
 
-// The `want` largest of the n <= kCandidateCap candidates in `cand`, in two levels: a histogram of their coarse codes
-// finds the bin of the want-th largest; candidates above it are emitted; those inside it are copied to where the
-// histogram was and ranked by counting: a candidate's rank is the number of them ahead of it in the total order (key
-// descending, position ascending).  A crowded bin goes to the radix selection instead.
-// counters[1] must be zero on entry; `hist_ready` says that hist already holds the histogram.
-__device__ __forceinline__ void select_two_level(const uint2* cand, uint32_t n, uint32_t want, uint32_t* hist, uint32_t* scratch,
-                                                 uint32_t* result, uint32_t* counters, int32_t* out, bool hist_ready) {
-    const int tid = threadIdx.x;
-    if (!hist_ready) {
-        for (int i = tid; i < kBins; i += kTopkThreads) hist[i] = 0u;
-        __syncthreads();
-        for (uint32_t i = tid; i < n; i += kTopkThreads) atomicAdd(&hist[coarse_bin_of_key(cand[i].x)], 1u);
-        __syncthreads();
+__device__ __forceinline__ float4 load_quad(const float* p) {
+    const uint4 q = ld_stream16(p);
+    return make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w));
+}
+
+// The valid range of a row, seen as 16-byte quads of 4 consecutive values counted from the 16-byte boundary at or below its
+// first value (`lead` = values between the two).  Rows whose values are not adjacent have lead 0 and are loaded value by value.
+struct Row {
+    const float* x;
+    int64_t stride;
+    int32_t len, lead, quads;
+
+    __device__ __forceinline__ Row(const float* first, int64_t stride1, int32_t length) : x(first), stride(stride1), len(length), lead(0) {
+        if (stride1 == 1) lead = static_cast<int32_t>((reinterpret_cast<uintptr_t>(first) & 15u) >> 2);
+        quads = (len + lead + 3) >> 2;
     }
-    const Threshold coarse = find_threshold(hist, want, scratch, result);
-    const bool take_all = coarse.need == coarse.count;
-    if (!take_all && coarse.count > kCountingMax) {
-        select_in_shared(cand, n, want, hist, scratch, result, counters, out);
-        return;
+    // Quads [first_whole(), end_whole()) lie inside the row and are one 16-byte load each.
+    __device__ __forceinline__ int32_t first_whole() const { return stride != 1 ? quads : lead > 0 ? 1 : 0; }
+    __device__ __forceinline__ int32_t end_whole() const { return stride != 1 ? quads : (len + lead) >> 2; }
+    __device__ __forceinline__ float value(int32_t i) const { return __uint_as_float(ld_stream4(x + static_cast<int64_t>(i) * stride)); }
+    __device__ __forceinline__ int32_t position(int32_t quad) const { return 4 * quad - lead; }  // of the quad's first value
+    // Values outside the row are -inf (their positions tell them from values that are).
+    __device__ __forceinline__ float4 load(int32_t quad) const {
+        const int32_t p = position(quad);
+        if (stride == 1 && p >= 0 && p + 4 <= len) return load_quad(x + p);
+        return make_float4(edge(p), edge(p + 1), edge(p + 2), edge(p + 3));
     }
-    uint2* dense = reinterpret_cast<uint2*>(hist);  // the histogram is no longer needed: kBins / 2 entries
-    for (uint32_t i = tid; i < n; i += kTopkThreads) {
-        const uint2 e = cand[i];
-        const uint32_t c = coarse_bin_of_key(e.x);
-        if (c > coarse.bin || (take_all && c == coarse.bin)) out[atomicAdd(&counters[0], 1u)] = static_cast<int32_t>(e.y);
-        else if (c == coarse.bin) dense[atomicAdd(&counters[1], 1u)] = e;
+    __device__ __forceinline__ bool inside(int32_t i) const { return static_cast<uint32_t>(i) < static_cast<uint32_t>(len); }
+    __device__ __forceinline__ float edge(int32_t i) const { return inside(i) ? value(i) : -INFINITY; }
+};
+
+// The candidates a CTA has found: (bits of the value, position) pairs in shared memory.  `size` counts past `capacity` when
+// it does not hold all of them.
+struct Pool {
+    uint2* entries;
+    uint32_t* size;
+    uint32_t capacity;
+
+    // Takes the values of N quads per lane that reach `floor` (> -inf); quad u holds the positions from p + u * step on, and what
+    // is no part of the row is -inf.  NaNs of either sign pass the comparison, as the largest values should.  Whole warps call
+    // it: a lane counts, the warp adds up and reserves room with one atomic, the lane writes; three instructions per value,
+    // the writes predicated, no branches.
+    template <int N>
+    __device__ __forceinline__ void take(const float4 (&v)[N], int32_t p, int32_t step, float floor) const {
+        const int lane = threadIdx.x & 31;
+        uint32_t mine = 0u;
+#pragma unroll
+        for (int u = 0; u < N; ++u) count(mine, v[u].x, floor), count(mine, v[u].y, floor), count(mine, v[u].z, floor), count(mine, v[u].w, floor);
+        uint32_t upto = mine;
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1)
+            asm volatile(
+                "{.reg .u32 r;\n"
+                ".reg .pred t;\n"
+                "shfl.sync.up.b32 r|t, %0, %1, 0, 0xffffffff;\n"
+                "@t add.u32 %0, %0, r;}"
+                : "+r"(upto)
+                : "r"(m));
+        uint32_t at = 0u;
+        if (lane == 31 && upto > 0u) at = atomicAdd(size, upto);
+        at += upto;  // lane 31: the end of the warp's part
+        const uint32_t end = __shfl_sync(0xffffffffu, at, 31), total = __shfl_sync(0xffffffffu, upto, 31);
+        if (total == 0u || end > capacity) return;
+        uint32_t address = static_cast<uint32_t>(__cvta_generic_to_shared(entries + (end - total + upto - mine)));
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const int32_t q = p + u * step;
+            put(address, v[u].x, q, floor), put(address, v[u].y, q + 1, floor), put(address, v[u].z, q + 2, floor), put(address, v[u].w, q + 3, floor);
+        }
+    }
+
+private:
+    static __device__ __forceinline__ void count(uint32_t& n, float v, float floor) {
+        asm("{.reg .pred t;\n"
+            "setp.geu.f32 t, %1, %2;\n"
+            "@t add.u32 %0, %0, 1;}"
+            : "+r"(n)
+            : "f"(v), "f"(floor));
+    }
+    static __device__ __forceinline__ void put(uint32_t& address, float v, int32_t p, float floor) {
+        asm volatile(
+            "{.reg .pred t;\n"
+            "setp.geu.f32 t, %1, %2;\n"
+            "@t st.shared.f32 [%0], %1;\n"
+            "@t st.shared.u32 [%0+4], %3;\n"
+            "@t add.u32 %0, %0, 8;}"
+            : "+r"(address)
+            : "f"(v), "f"(floor), "r"(p)
+            : "memory");
+    }
+};
+
+// Bin of a candidate in the histogram that ranks them: linear in the key from `anchor` on, the first and the last bin open.
+__device__ __forceinline__ uint32_t fine_bin(uint32_t key, uint32_t anchor, int shift) {
+    const uint32_t bin = key > anchor ? (key - anchor) >> shift : 0u;
+    return bin < kBins - 1u ? bin : kBins - 1u;
+}
+// 2048 bins between the key candidates start at and one near the top of the row (the largest of the sample) leave a handful
+// of candidates in the bin of the k-th largest.
+__device__ __forceinline__ int fine_shift(uint32_t floor_key, uint32_t top_key) {
+    const int bits = 32 - __clz(top_key > floor_key ? top_key - floor_key : 1u);
+    return bits > 11 ? bits - 11 : 0;
+}
+
+// What the sample says: the value to collect from, its key, and the anchor and shift of fine_bin().  The sample is in hist and its largest
+// key in counters[3], a barrier ago; `size` values of it stand for `len` values of the row.  Clears hist; the caller's next
+// barrier completes that.
+struct Floor {
+    float value;
+    uint32_t key, anchor;
+    int shift;
+};
+template <int THREADS>
+__device__ __forceinline__ Floor floor_from_sample(Shared& s, int32_t k, int32_t size, int32_t len) {
+    if (threadIdx.x < 32) {
+        // rank inside the sample that stands for k values of the row, plus four standard deviations of that count
+        const float mean = static_cast<float>(k) * static_cast<float>(size) / static_cast<float>(len);
+        const uint32_t rank = static_cast<uint32_t>(mean + 4.0f * sqrtf(mean)) + 3u;
+        const uint32_t limit = static_cast<uint32_t>(size);
+        const uint32_t top_key = s.counters[3];
+        const uint32_t bin = scan_down(s.hist, coarse_bin(__uint_as_float((top_key & 0x80000000u) ? top_key & 0x7fffffffu : ~top_key)), rank < limit ? rank : limit).bin;
+        if (threadIdx.x == 0) {
+            const uint32_t bits = __float_as_uint(value_of_bin(bin));
+            // a row hardly longer than k: all finite values are candidates (no more of them than expected)
+            s.result[0] = rank < limit ? bits : 0xff7fffffu;
+            s.result[1] = order_key(bits), s.result[2] = fine_shift(order_key(bits), top_key);
+        }
     }
     __syncthreads();
-    if (take_all) return;
-    rank_by_counting(dense, coarse.count, coarse.need, counters, out);
+    Floor f;
+    f.value = __uint_as_float(s.result[0]), f.key = order_key(s.result[0]), f.anchor = s.result[1], f.shift = static_cast<int>(s.result[2]);
+    clear_histogram<THREADS>(s);
+    return f;
 }
 
-template <bool DECODE>
-__global__ void __launch_bounds__(kTopkThreads) topk_per_row_kernel(const TopkParams p) {
-    __shared__ __align__(8) uint32_t hist[kBins];
-    extern __shared__ uint2 cand[];  // kCandidateCap entries: (order key, position)
-    __shared__ uint32_t scratch[32];
-    __shared__ uint32_t result[4];
-    __shared__ uint32_t counters[4];  // 0: emitted, 1: candidates collected, 2: ties taken
-    cg::cluster_group cluster = cg::this_cluster();
-    const uint32_t ctas = cluster.num_blocks(), rank = cluster.block_rank();  // the CTAs of a cluster share one row
+// Histogram route: two reads of the row by one CTA, any k, any distribution.  `cand` holds `capacity` pairs.
+template <int THREADS>
+__device__ __noinline__ void select_from_histogram(Shared& s, uint2* cand, uint32_t capacity, const Row row, int32_t k, int32_t* out) {
     const int tid = threadIdx.x;
-    const int row = blockIdx.x / ctas;
-    int64_t start, end;
-    if (DECODE) {
-        start = 0;
-        end = static_cast<int64_t>(p.seq_lens[row / p.next_n]) - p.next_n + row % p.next_n + 1;
-    } else {
-        start = p.row_starts ? p.row_starts[row] : 0;
-        end = p.row_ends[row];
-    }
-    start = start < 0 ? 0 : start;
-    end = end > p.vocab ? p.vocab : end;
-    const int32_t len = end > start ? static_cast<int32_t>(end - start) : 0;
-    const int32_t k = len < p.top_k ? len : p.top_k;
-    int32_t* out = p.indices + static_cast<int64_t>(row) * p.top_k;
-    // Everything up to the first cluster barrier depends on the row only, so the CTAs of a cluster leave together.
-    if (rank == 0)
-        for (int i = k + tid; i < p.top_k; i += kTopkThreads) out[i] = -1;
-    if (len <= p.top_k) {  // everything is selected
-        if (rank == 0)
-            for (int i = tid; i < len; i += kTopkThreads) out[i] = i;
-        return;
-    }
-    const float* x = p.logits + static_cast<int64_t>(row) * p.stride0 + start * p.stride1;
-    const auto load = [&](int32_t i) { return __uint_as_float(ld_stream4(x + static_cast<int64_t>(i) * p.stride1)); };
-    // Calls visit(position, value) for the elements [from, to) of the row; 16-byte loads where the layout allows.
-    const auto for_each = [&](int32_t from, int32_t to, auto&& visit) {
-        if (p.stride1 == 1) {
-            int32_t head = from + static_cast<int32_t>(((16u - (reinterpret_cast<uintptr_t>(x + from) & 15u)) & 15u) >> 2);  // first 16-byte boundary
-            head = head < to ? head : to;
-            const int32_t vecs = (to - head) >> 2;
-            const float* body = x + head;
-            int32_t v = tid;
-            for (; v + 3 * kTopkThreads < vecs; v += 4 * kTopkThreads) {  // four 16-byte loads per thread in flight
-                uint4 q[4];
+    __syncthreads();
+    clear_histogram<THREADS>(s);
+    if (tid < 4) s.counters[tid] = 0u;
+    __syncthreads();
+    // four quads per thread in flight; whole warps stay together for append()
+    const auto for_each_quad = [&](auto&& visit) {
+        for (int32_t q = tid; q - (tid & 31) < row.quads; q += kStreamBatch * THREADS) {
+            float4 v[kStreamBatch];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) q[u] = ld_stream16(body + 4 * (v + u * kTopkThreads));
+            for (int u = 0; u < kStreamBatch; ++u)
+                if (q + u * THREADS < row.quads) v[u] = row.load(q + u * THREADS);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int32_t i = head + 4 * (v + u * kTopkThreads);
-                    visit(i, __uint_as_float(q[u].x)), visit(i + 1, __uint_as_float(q[u].y)), visit(i + 2, __uint_as_float(q[u].z)), visit(i + 3, __uint_as_float(q[u].w));
-                }
+            for (int u = 0; u < kStreamBatch; ++u) {
+                const int32_t p = q + u * THREADS < row.quads ? row.position(q + u * THREADS) : -8;
+                visit(v[u].x, p), visit(v[u].y, p + 1), visit(v[u].z, p + 2), visit(v[u].w, p + 3);
             }
-            for (; v < vecs; v += kTopkThreads) {
-                const uint4 a = ld_stream16(body + 4 * v);
-                const int32_t ia = head + 4 * v;
-                visit(ia, __uint_as_float(a.x)), visit(ia + 1, __uint_as_float(a.y)), visit(ia + 2, __uint_as_float(a.z)), visit(ia + 3, __uint_as_float(a.w));
-            }
-            for (int32_t i = from + tid; i < head; i += kTopkThreads) visit(i, load(i));
-            for (int32_t i = head + 4 * vecs + tid; i < to; i += kTopkThreads) visit(i, load(i));
-        } else {
-            for (int32_t i = from + tid; i < to; i += kTopkThreads) visit(i, load(i));
         }
     };
-
-    const bool fast = 2 * k + 512 <= kCandidateCap;
-    if (rank != 0 && (!fast || len <= kCandidateCap)) return;  // these rows are handled by the first CTA alone
-    for (int i = tid; i < kBins; i += kTopkThreads) hist[i] = 0u;
-    if (tid < 4) counters[tid] = 0u;
-    __syncthreads();
-
-    // ---- fast route -------------------------------------------------------------------------------------------
-    if (fast && len <= kCandidateCap) {
-        // The whole row fits into shared memory (keys only: a value's position is its place in the buffer): one read
-        // fills it and the coarse histogram; values above the bin of the k-th largest are emitted, the few inside it
-        // are copied to where the histogram was and ranked by counting.
-        uint32_t* keys = reinterpret_cast<uint32_t*>(cand);
-        for_each(0, len, [&](int32_t i, float v) {
-            keys[i] = order_key(__float_as_uint(v));
-            atomicAdd(&hist[coarse_bin(v)], 1u);
-        });
-        __syncthreads();
-        const Threshold coarse = find_threshold(hist, static_cast<uint32_t>(k), scratch, result);
-        const bool take_all = coarse.need == coarse.count;
-        if (take_all || coarse.count <= kCountingMax) {
-            uint2* dense = reinterpret_cast<uint2*>(hist);
-            for (int32_t i = tid; i < len; i += kTopkThreads) {
-                const uint32_t key = keys[i];
-                const uint32_t c = coarse_bin_of_key(key);
-                if (c > coarse.bin || (take_all && c == coarse.bin)) out[atomicAdd(&counters[0], 1u)] = i;
-                else if (c == coarse.bin) dense[atomicAdd(&counters[1], 1u)] = make_uint2(key, static_cast<uint32_t>(i));
-            }
-            __syncthreads();
-            if (!take_all) rank_by_counting(dense, coarse.count, coarse.need, counters, out);
-            return;
-        }
-        // a crowded bin: over to the histogram route, which has the histogram it needs already
-    } else if (fast) {
-        // every CTA of the cluster takes the same sample, hence the same b0: candidates are the values in bins >= b0
-        // the sample: kSampleChunks runs of 32 consecutive values (one 128-byte line each) spread evenly over the row
-        const int32_t stride = (len / kSampleChunks) & ~31;  // len > kCandidateCap, so the runs do not overlap
-        for (int32_t j = tid; j < kSampleChunks * 32; j += kTopkThreads) atomicAdd(&hist[coarse_bin(load((j >> 5) * stride + (j & 31)))], 1u);
-        __syncthreads();
-        // rank inside the sample that stands for k values of the row, plus four standard deviations of that count
-        const float mean = static_cast<float>(k) * (kSampleChunks * 32) / static_cast<float>(len);
-        const uint32_t sample_rank = static_cast<uint32_t>(mean + 4.0f * sqrtf(mean)) + 3u;
-        const uint32_t b0 = find_threshold(hist, sample_rank < kSampleChunks * 32u ? sample_rank : kSampleChunks * 32u, scratch, result).bin;
-        cluster.sync();  // the first CTA's counters are zero before anybody reserves space in its buffer
-        // this CTA's share of the row, a multiple of 4 elements so that the 16-byte loads stay aligned
-        const int32_t share = (((len + static_cast<int32_t>(ctas) - 1) / static_cast<int32_t>(ctas)) + 3) & ~3;
-        const int32_t from = static_cast<int32_t>(rank) * share < len ? static_cast<int32_t>(rank) * share : len;
-        const int32_t to = from + share < len ? from + share : len;
-        for_each(from, to, [&](int32_t i, float v) {
-            if (coarse_bin(v) >= b0) {
-                const uint32_t at = atomicAdd(&counters[1], 1u);
-                if (at < kCandidateCap) cand[at] = make_uint2(order_key(__float_as_uint(v)), static_cast<uint32_t>(i));
-            }
-        });
-        __syncthreads();
-        if (rank != 0) {
-            // hand the candidates over to the first CTA through distributed shared memory
-            const uint32_t mine = counters[1];
-            if (tid == 0) result[3] = atomicAdd(cluster.map_shared_rank(&counters[1], 0), mine);
-            __syncthreads();
-            const uint32_t at = result[3];
-            if (mine <= kCandidateCap && at + mine <= kCandidateCap) {
-                uint2* remote = cluster.map_shared_rank(cand, 0);
-                for (uint32_t j = tid; j < mine; j += kTopkThreads) remote[at + j] = cand[j];
-            }
-        }
-        cluster.sync();  // all candidates have arrived
-        if (rank != 0) return;
-        const uint32_t collected = counters[1];
-        if (collected >= static_cast<uint32_t>(k) && collected <= kCandidateCap) {
-            __syncthreads();
-            if (tid == 0) counters[1] = 0u;
-            select_two_level(cand, collected, static_cast<uint32_t>(k), hist, scratch, result, counters, out, false);
-            return;
-        }
-        // the sample misjudged the row: the first CTA starts over on the histogram route
-        __syncthreads();
-        for (int i = tid; i < kBins; i += kTopkThreads) hist[i] = 0u;
-        if (tid < 4) counters[tid] = 0u;
-        __syncthreads();
-    }
-
-    // ---- histogram route --------------------------------------------------------------------------------------
-    if (!(fast && len <= kCandidateCap)) {  // (a short row arrives with its histogram)
-        for_each(0, len, [&](int32_t, float v) { atomicAdd(&hist[coarse_bin(v)], 1u); });
-        __syncthreads();
-    }
-    const Threshold coarse = find_threshold(hist, static_cast<uint32_t>(k), scratch, result);
-    const bool collect = coarse.count <= p.pair_capacity && coarse.need < coarse.count;
-    const bool take_all = coarse.need == coarse.count;  // the whole bin belongs to the top k
-    // emit everything above the bin (and the bin itself if it is taken whole); collect the bin's candidates
-    for_each(0, len, [&](int32_t i, float v) {
-        const uint32_t c = coarse_bin(v);
-        if (c > coarse.bin || (take_all && c == coarse.bin)) {
-            out[atomicAdd(&counters[0], 1u)] = i;
-        } else if (collect && c == coarse.bin) {
-            cand[atomicAdd(&counters[1], 1u)] = make_uint2(order_key(__float_as_uint(v)), static_cast<uint32_t>(i));
-        }
+    for_each_quad([&](float v, int32_t i) {
+        if (row.inside(i)) atomicAdd(&s.hist[coarse_bin(v)], 1u);
     });
     __syncthreads();
+    const Threshold coarse = find_threshold<THREADS>(s, static_cast<uint32_t>(k));
+    const bool collect_bin = coarse.count <= capacity && coarse.need < coarse.count;
+    const bool take_all = coarse.need == coarse.count;  // the whole bin belongs to the top k
+    // emit everything above the bin (and the bin itself if it is taken whole); collect the bin's candidates
+    for_each_quad([&](float v, int32_t i) {
+        const uint32_t c = coarse_bin(v);
+        append(out, &s.counters[0], row.inside(i) && (c > coarse.bin || (take_all && c == coarse.bin)), i);
+        if (row.inside(i) && collect_bin && c == coarse.bin) cand[atomicAdd(&s.counters[1], 1u)] = make_uint2(order_key(__float_as_uint(v)), static_cast<uint32_t>(i));
+    });
     if (take_all) return;
-    if (collect) {
-        select_in_shared(cand, coarse.count, coarse.need, hist, scratch, result, counters, out);
+    if (collect_bin) {
+        select_radix<THREADS>(s, cand, coarse.count, coarse.need, out);
         return;
     }
-
-    // Slow route: the bin is too crowded for shared memory.  Radix selection on the fp32 key over the row itself,
-    // restricted to the elements of the bin: bits 31-21, 20-10, 9-0.
+    // The bin is too crowded for shared memory.  Radix selection on the fp32 key over the row itself, restricted to the
+    // elements of the bin: bits 31-21, 20-10, 9-0.
     uint32_t need = coarse.need, prefix = 0u, prefix_mask = 0u;
     const int shifts[3] = {21, 10, 0};
     const uint32_t widths[3] = {11, 11, 10};
     for (int pass = 0; pass < 3; ++pass) {
-        for (int i = tid; i < kBins; i += kTopkThreads) hist[i] = 0u;
         __syncthreads();
-        const int32_t padded = (len + 31) & ~31;  // whole warps stay together for the aggregated increment
-        for (int32_t i = tid; i < padded; i += kTopkThreads) {
+        clear_histogram<THREADS>(s);
+        __syncthreads();
+        for (int32_t i = tid; i - (tid & 31) < row.len; i += THREADS) {  // whole warps stay together for the aggregated increment
             bool active = false;
             uint32_t bin = 0u;
-            if (i < len) {
-                const float v = load(i);
+            if (i < row.len) {
+                const float v = row.value(i);
                 const uint32_t key = order_key(__float_as_uint(v));
                 active = coarse_bin(v) == coarse.bin && (key & prefix_mask) == prefix;
                 bin = (key >> shifts[pass]) & ((1u << widths[pass]) - 1u);
             }
-            add_aggregated(hist, bin, active);
+            add_aggregated(s.hist, bin, active);
         }
         __syncthreads();
-        const Threshold t = find_threshold(hist, need, scratch, result);
+        const Threshold t = find_threshold<THREADS>(s, need);
         prefix |= t.bin << shifts[pass];
         prefix_mask |= ((1u << widths[pass]) - 1u) << shifts[pass];
         need = t.need;
     }
-    for (int32_t i = tid; i < len; i += kTopkThreads) {
-        const float v = load(i);
+    for (int32_t i = tid; i < row.len; i += THREADS) {
+        const float v = row.value(i);
         if (coarse_bin(v) != coarse.bin) continue;
         const uint32_t key = order_key(__float_as_uint(v));
-        if (key > prefix || (key == prefix && atomicAdd(&counters[2], 1u) < need)) out[atomicAdd(&counters[0], 1u)] = i;
+        if (key > prefix || (key == prefix && atomicAdd(&s.counters[2], 1u) < need)) out[atomicAdd(&s.counters[0], 1u)] = i;
     }
+}
+
+// Ranks the `size` candidates and emits the k largest; false (in every thread) when the pool does not hold them.  hist and the
+// counters are zero on entry, a barrier ago or more.  A negative NaN, the smallest key, may be among the candidates: keys
+// below the floor do not count.
+template <int THREADS>
+__device__ __forceinline__ bool select(Shared& s, const uint2* pool, uint32_t size, uint32_t capacity, uint32_t k, const Floor& f, int32_t* out) {
+    const int tid = threadIdx.x;
+    const uint32_t floor_key = f.key;
+    if (size < k || size > capacity) return false;
+    for (uint32_t i = tid; i < size; i += THREADS) {
+        const uint32_t key = order_key(pool[i].x);
+        if (key >= floor_key) atomicAdd(&s.hist[fine_bin(key, f.anchor, f.shift)], 1u);
+        else atomicAdd(&s.below, 1u);
+    }
+    __syncthreads();
+    if (size - s.below < k) return false;
+    Threshold t;
+    if (f.shift > 16) {  // the bins cover many octaves: the candidates reach down to values near zero
+        t = find_threshold<THREADS>(s, k);
+    } else {
+        if (tid < 32) {
+            t = scan_up(s.hist, size - s.below - k);
+            if (tid == 0) s.result[0] = t.bin, s.result[1] = t.need, s.result[2] = t.count;
+        }
+        __syncthreads();
+        t.bin = s.result[0], t.need = s.result[1], t.count = s.result[2];
+    }
+    const bool take_all = t.need == t.count;
+    if (!take_all && t.count > kCountingMax) return false;
+    const uint32_t lowest = take_all ? t.bin : t.bin + 1u;  // of the bins taken whole
+    uint2* dense = reinterpret_cast<uint2*>(s.hist);  // the histogram is no longer needed
+    for (uint32_t i = tid; i - (tid & 31) < size; i += THREADS) {  // whole warps stay together for append()
+        const uint2 e = i < size ? pool[i] : make_uint2(0u, 0u);
+        const uint32_t key = order_key(e.x), bin = fine_bin(key, f.anchor, f.shift);
+        const bool in = i < size && key >= floor_key;
+        append(out, &s.counters[0], in && bin >= lowest, static_cast<int32_t>(e.y));
+        if (in && !take_all && bin == t.bin) dense[atomicAdd(&s.counters[2], 1u)] = make_uint2(key, e.y);
+    }
+    if (take_all) return true;
+    __syncthreads();
+    rank_by_counting<THREADS>(s, dense, t.count, t.need, out);
+    return true;
+}
+
+// The valid range of row `r`: its first value's index and its length.
+template <bool DECODE>
+__device__ __forceinline__ int32_t row_range(const TopkParams& p, int r, int64_t* first) {
+    int64_t start, end;
+    if (DECODE) {
+        start = 0;
+        const int request = p.next_n == 1 ? r : r / p.next_n;
+        end = static_cast<int64_t>(p.seq_lens[request]) - p.next_n + (r - request * p.next_n) + 1;
+    } else {
+        start = p.row_starts ? p.row_starts[r] : 0;
+        end = p.row_ends[r];
+    }
+    start = start < 0 ? 0 : start;
+    end = end > p.vocab ? p.vocab : end;
+    *first = start;
+    return end > start ? static_cast<int32_t>(end - start) : 0;
+}
+
+// One CTA per row, the row in registers, no sample: the coarse histogram of all values gives the bin of the k-th largest,
+// what lies above it is emitted from the registers, and the values of the bin are ranked by counting.  For short rows, of which
+// a large part is selected: fewer phases, and about 25 instructions per value.
+template <bool DECODE, int THREADS, int QUADS>
+__global__ void __launch_bounds__(THREADS) topk_short_kernel(const TopkParams p) {
+    __shared__ Shared s;
+    extern __shared__ uint2 dynamic[];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int r = blockIdx.x;
+    int64_t first;
+    const int32_t len = row_range<DECODE>(p, r, &first);
+    const int32_t k = len < p.top_k ? len : p.top_k;
+    int32_t* out = p.indices + static_cast<int64_t>(r) * p.top_k;
+    for (int i = k + tid; i < p.top_k; i += THREADS) out[i] = -1;
+    if (len <= p.top_k) {  // everything is selected
+        for (int i = tid; i < len; i += THREADS) out[i] = i;
+        return;
+    }
+    const Row row(p.logits + static_cast<int64_t>(r) * p.stride0 + first * p.stride1, p.stride1, len);
+    float4 v[QUADS];
+#pragma unroll
+    for (int u = 0; u < QUADS; ++u)
+        if (tid + u * THREADS < row.quads) v[u] = row.load(tid + u * THREADS);
+    clear_histogram<THREADS>(s);
+    if (tid < 4) s.counters[tid] = 0u;
+    __syncthreads();
+    uint32_t largest = 0u;
+    const auto for_each = [&](auto&& visit) {  // visit(number of the value in the thread, value, position)
+#pragma unroll
+        for (int u = 0; u < QUADS; ++u) {
+            if ((tid & ~31) + u * THREADS >= row.quads) break;  // nothing left for the warp
+            const int32_t i = tid + u * THREADS < row.quads ? row.position(tid + u * THREADS) : -8;
+            visit(4 * u, v[u].x, i), visit(4 * u + 1, v[u].y, i + 1), visit(4 * u + 2, v[u].z, i + 2), visit(4 * u + 3, v[u].w, i + 3);
+        }
+    };
+    for_each([&](int, float x, int32_t i) {
+        if (!row.inside(i)) return;
+        const uint32_t bin = coarse_bin(x);
+        atomicAdd(&s.hist[bin], 1u);
+        largest = bin > largest ? bin : largest;
+    });
+    largest = __reduce_max_sync(0xffffffffu, largest);
+    if (lane == 0) atomicMax(&s.counters[3], largest);
+    __syncthreads();
+    Threshold t;
+    if (4 * k > len) {  // far from the top, perhaps behind the many bins of values near zero
+        t = find_threshold<THREADS>(s, static_cast<uint32_t>(k));
+    } else {
+        if (tid < 32) {
+            t = scan_down(s.hist, static_cast<int>(s.counters[3]), static_cast<uint32_t>(k));
+            if (tid == 0) s.result[0] = t.bin, s.result[1] = t.need, s.result[2] = t.count;
+        }
+        __syncthreads();
+        t.bin = s.result[0], t.need = s.result[1], t.count = s.result[2];
+    }
+    const bool take_all = t.need == t.count;
+    if (!take_all && t.count > kCountingMax) {
+        select_from_histogram<THREADS>(s, dynamic, p.capacity, row, k, out);
+        return;
+    }
+    const uint32_t lowest = take_all ? t.bin : t.bin + 1u;  // of the bins taken whole
+    uint2* dense = reinterpret_cast<uint2*>(s.hist);  // the histogram is no longer needed
+    uint32_t mask = 0u;
+    for_each([&](int n, float x, int32_t i) {
+        const uint32_t bin = row.inside(i) ? coarse_bin(x) : 0u;
+        if (row.inside(i) && bin >= lowest) mask |= 1u << n;
+        else if (row.inside(i) && bin == t.bin) dense[atomicAdd(&s.counters[2], 1u)] = make_uint2(order_key(__float_as_uint(x)), static_cast<uint32_t>(i));
+    });
+    uint32_t at = __popc(mask);
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, at, m);
+        if (lane >= m) at += up;
+    }
+    uint32_t base = 0u;
+    if (lane == 31 && at > 0u) base = atomicAdd(&s.counters[0], at);
+    at += __shfl_sync(0xffffffffu, base, 31) - __popc(mask);
+    for_each([&](int n, float, int32_t i) {
+        if (mask & (1u << n)) out[at++] = i;
+    });
+    if (take_all) return;
+    __syncthreads();
+    rank_by_counting<THREADS>(s, dense, t.count, t.need, out);
+}
+
+// One CTA per row, the row in registers: QUADS x 4 values per thread.  The sample is the first value of every quad.
+template <bool DECODE, int THREADS, int QUADS>
+__global__ void __launch_bounds__(THREADS) topk_registers_kernel(const TopkParams p) {
+    __shared__ Shared s;
+    extern __shared__ uint2 dynamic[];
+    const int tid = threadIdx.x;
+    const int r = blockIdx.x;
+    int64_t first;
+    const int32_t len = row_range<DECODE>(p, r, &first);
+    const int32_t k = len < p.top_k ? len : p.top_k;
+    int32_t* out = p.indices + static_cast<int64_t>(r) * p.top_k;
+    for (int i = k + tid; i < p.top_k; i += THREADS) out[i] = -1;
+    if (len <= p.top_k) {  // everything is selected
+        for (int i = tid; i < len; i += THREADS) out[i] = i;
+        return;
+    }
+    const Row row(p.logits + static_cast<int64_t>(r) * p.stride0 + first * p.stride1, p.stride1, len);
+    float4 v[QUADS];
+#pragma unroll
+    for (int u = 0; u < QUADS; ++u) {
+        const int32_t quad = tid + u * THREADS;
+        v[u] = quad < row.quads ? row.load(quad) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    }
+    clear_histogram<THREADS>(s);
+    if (tid < 4) s.counters[tid] = 0u;
+    if (tid == 4) s.pooled = 0u, s.below = 0u;
+    __syncthreads();
+    uint32_t largest = 0u;
+#pragma unroll
+    for (int u = 0; u < QUADS; ++u) {
+        const int32_t quad = tid + u * THREADS;
+        if (row.inside(row.position(quad))) {
+            atomicAdd(&s.hist[coarse_bin(v[u].x)], 1u);
+            const uint32_t key = order_key(__float_as_uint(v[u].x));
+            largest = key > largest ? key : largest;
+        }
+    }
+    largest = __reduce_max_sync(0xffffffffu, largest);
+    if ((tid & 31) == 0) atomicMax(&s.counters[3], largest);
+    __syncthreads();
+    const int32_t size = row.quads - (row.lead > 0 ? 1 : 0);  // quads whose first value belongs to the row
+    const Floor f = floor_from_sample<THREADS>(s, k, size, len);
+    __syncthreads();
+    bool done = false;
+    if (p.sampled && f.value > -INFINITY) {
+        const Pool pool{dynamic, &s.pooled, p.capacity};
+        constexpr int kBatch = QUADS < kStreamBatch ? QUADS : kStreamBatch;
+#pragma unroll
+        for (int u = 0; u < QUADS; u += kBatch) {
+            float4 batch[kBatch];
+#pragma unroll
+            for (int w = 0; w < kBatch; ++w) batch[w] = v[u + w];
+            pool.take(batch, row.position(tid + u * THREADS), 4 * THREADS, f.value);
+        }
+        __syncthreads();
+        done = select<THREADS>(s, dynamic, s.pooled, p.capacity, static_cast<uint32_t>(k), f, out);
+    }
+    if (!done) select_from_histogram<THREADS>(s, dynamic, p.capacity, row, k, out);
+}
+
+template <bool DECODE, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(const TopkParams p) {
+    __shared__ Shared s;
+    extern __shared__ uint2 dynamic[];  // the candidate pool
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t ctas = cluster.num_blocks(), rank = cluster.block_rank();  // the CTAs of a cluster share one row
+    const int tid = threadIdx.x;
+    const int r = blockIdx.x >> (31 - __clz(ctas));  // a power of two
+    int64_t first;
+    const int32_t len = row_range<DECODE>(p, r, &first);
+    const int32_t k = len < p.top_k ? len : p.top_k;
+    int32_t* out = p.indices + static_cast<int64_t>(r) * p.top_k;
+    // Everything up to the first cluster barrier depends on the row only, so the CTAs of a cluster leave together.
+    if (rank == 0)
+        for (int i = k + tid; i < p.top_k; i += THREADS) out[i] = -1;
+    if (len <= p.top_k) {  // everything is selected
+        if (rank == 0)
+            for (int i = tid; i < len; i += THREADS) out[i] = i;
+        return;
+    }
+    const Row row(p.logits + static_cast<int64_t>(r) * p.stride0 + first * p.stride1, p.stride1, len);
+    if (!p.sampled) {
+        if (rank == 0) select_from_histogram<THREADS>(s, dynamic, p.capacity, row, k, out);
+        return;
+    }
+    // this CTA's share of the whole quads; its first batch is on its way while the sample is evaluated
+    const int32_t begin = row.first_whole(), end = row.end_whole();
+    const int32_t share = end > begin ? (end - begin + static_cast<int32_t>(ctas) - 1) / static_cast<int32_t>(ctas) : 0;
+    const int32_t from = begin + static_cast<int32_t>(rank) * share, to = from + share < end ? from + share : end;
+    const float4 none = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    int32_t left = to - from - tid;  // quads from this thread's next one to the end of the share
+    int32_t position = row.position(from + tid);
+    const float* next = row.x + position;
+    float4 v[kStreamBatch];
+    const auto load_batch = [&]() {
+#pragma unroll
+        for (int u = 0; u < kStreamBatch; ++u) v[u] = u * THREADS < left ? load_quad(next + 4 * u * THREADS) : none;
+    };
+    load_batch();
+    clear_histogram<THREADS>(s);
+    if (tid < 4) s.counters[tid] = 0u;
+    if (tid == 4) s.pooled = 0u, s.below = 0u;
+    __syncthreads();
+    // every CTA of the cluster takes the same sample: runs of 8 consecutive quads (one 128-byte line each, where the row is
+    // so aligned) spread evenly over the row
+    const int32_t base = row.stride == 1 ? begin : 0, span = row.stride == 1 ? end - begin : row.quads;
+    const int32_t step = span > kSampleQuads ? span / (kSampleQuads / 8) : 8;
+    uint32_t largest = 0u;
+    float peak = -INFINITY;
+    {
+        constexpr int kMine = kSampleQuads / THREADS;
+        float4 sample[kMine];
+#pragma unroll
+        for (int u = 0; u < kMine; ++u) {
+            const int32_t j = tid + u * THREADS, quad = (j >> 3) * step + (j & 7);
+            sample[u] = quad < span ? row.load(base + quad) : none;
+        }
+#pragma unroll
+        for (int u = 0; u < kMine; ++u) {
+            const int32_t j = tid + u * THREADS;
+            if ((j >> 3) * step + (j & 7) >= span) continue;
+            const float value[4] = {sample[u].x, sample[u].y, sample[u].z, sample[u].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                atomicAdd(&s.hist[coarse_bin(value[e])], 1u);
+                peak = fmaxf(peak, value[e]);
+            }
+        }
+    }
+    largest = order_key(__float_as_uint(peak));
+    largest = __reduce_max_sync(0xffffffffu, largest);
+    if ((tid & 31) == 0) atomicMax(&s.counters[3], largest);
+    __syncthreads();
+    const Floor f = floor_from_sample<THREADS>(s, k, 4 * (span < kSampleQuads ? span : kSampleQuads), len);
+    if (!(f.value > -INFINITY)) {
+        __syncthreads();
+        if (rank == 0) select_from_histogram<THREADS>(s, dynamic, p.capacity, row, k, out);
+        return;
+    }
+    if (ctas > 1) cluster.sync();  // the first CTA's counters are zero before anybody reserves room in its pool
+    else __syncthreads();
+    const Pool pool{dynamic, &s.pooled, p.capacity};
+    // full batches, then what is left of the share, then the quads that are not whole
+    constexpr int kBatch = kStreamBatch * THREADS;
+    while (left + tid >= kBatch) {
+        pool.take(v, position, 4 * THREADS, f.value);
+        left -= kBatch, position += 4 * kBatch, next += 4 * kBatch;
+        if (left + tid >= kBatch) {
+#pragma unroll
+            for (int u = 0; u < kStreamBatch; ++u) v[u] = load_quad(next + 4 * u * THREADS);
+        } else {
+            load_batch();
+        }
+    }
+    if (left + tid > 0) pool.take(v, position, 4 * THREADS, f.value);
+    float4 edge[1];
+    if (row.stride != 1) {
+        for (int32_t e = static_cast<int32_t>(rank) * THREADS + tid; e - (tid & 31) < row.quads; e += static_cast<int32_t>(ctas) * THREADS) {
+            edge[0] = e < row.quads ? row.load(e) : none;
+            pool.take(edge, row.position(e), 0, f.value);
+        }
+    } else if (rank == 0 && tid < 32) {
+        if (begin > 0) {
+            edge[0] = tid == 0 ? row.load(0) : none;
+            pool.take(edge, row.position(0), 0, f.value);
+        }
+        if (end < row.quads && end >= begin) {
+            edge[0] = tid == 0 ? row.load(end) : none;
+            pool.take(edge, row.position(end), 0, f.value);
+        }
+    }
+    __syncthreads();
+    if (ctas > 1) {
+        if (rank != 0) {
+            // hand the candidates over to the first CTA through distributed shared memory
+            const uint32_t mine = s.pooled;
+            if (tid == 0) s.result[3] = atomicAdd(cluster.map_shared_rank(&s.pooled, 0), mine);
+            __syncthreads();
+            const uint32_t at = s.result[3];
+            if (mine <= p.capacity && at + mine <= p.capacity) {
+                uint2* remote = cluster.map_shared_rank(dynamic, 0);
+                for (uint32_t i = tid; i < mine; i += THREADS) remote[at + i] = dynamic[i];
+            }
+        }
+        cluster.sync();  // all candidates have arrived
+        if (rank != 0) return;
+    }
+    if (!select<THREADS>(s, dynamic, s.pooled, p.capacity, static_cast<uint32_t>(k), f, out))
+        select_from_histogram<THREADS>(s, dynamic, p.capacity, row, k, out);
+}
+
+// Candidates to expect when the sample holds `size` of `len` values (see floor_from_sample): their number, and its spread.
+struct Expected {
+    double count, deviation;
+    Expected(double k, double size, double len) {
+        const double mean = k * size / len, rank = mean + 4.0 * std::sqrt(mean) + 3.0;
+        count = rank * len / size, deviation = count / std::sqrt(rank);
+    }
+};
+
+// Room for them with six standard deviations on top.
+uint32_t pool_capacity(const Expected& e) { return static_cast<uint32_t>(std::min(e.count + 6.0 * e.deviation + 64.0, 8192.0)); }
+
+constexpr size_t kMaxDynamicBytes = sizeof(uint2) * 8192;
+
+template <typename Kernel>
+cudaError_t launch(Kernel kernel, const TopkParams& p, int threads, unsigned ctas, cudaStream_t stream) {
+    if (p.num_rows * static_cast<int64_t>(ctas) > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(static_cast<unsigned>(p.num_rows) * ctas), config.blockDim = dim3(static_cast<unsigned>(threads));
+    config.dynamicSmemBytes = sizeof(uint2) * p.capacity, config.stream = stream;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = ctas, attribute[0].val.clusterDim.y = 1, attribute[0].val.clusterDim.z = 1;
+    config.attrs = attribute, config.numAttrs = ctas > 1 ? 1 : 0;
+    const cudaError_t err = cudaLaunchKernelEx(&config, kernel, p);
+    if (err != cudaSuccess) return err;
+    count_launch();
+    return cudaGetLastError();
+}
+
+// Per-device set-up, once per device however many host threads make their first call at the same time.
+struct DeviceSetup {
+    std::once_flag once;
+    cudaError_t status = cudaSuccess;
+    int sms = 0;
+};
+
+template <bool DECODE>
+cudaError_t set_up(DeviceSetup** result) {
+    static DeviceSetup setups[64];
+    int dev = 0;
+    const cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    DeviceSetup& setup = setups[dev];
+    std::call_once(setup.once, [&]() {
+        const auto allow = [&](auto* kernel) {
+            if (setup.status == cudaSuccess)
+                setup.status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxDynamicBytes));
+        };
+        allow(topk_stream_kernel<DECODE, 512>), allow(topk_stream_kernel<DECODE, 256>);
+        allow(topk_registers_kernel<DECODE, 512, 4>), allow(topk_registers_kernel<DECODE, 512, 8>), allow(topk_registers_kernel<DECODE, 256, 8>);
+        if (setup.status == cudaSuccess) setup.status = cudaDeviceGetAttribute(&setup.sms, cudaDevAttrMultiProcessorCount, dev);
+    });
+    *result = &setup;
+    return setup.status;
+}
+
+template <bool DECODE>
+cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
+    DeviceSetup* setup = nullptr;
+    const cudaError_t err = set_up<DECODE>(&setup);
+    if (err != cudaSuccess) return err;
+    const int sms = setup->sms;
+    const bool aligned = p.stride1 == 1 && (reinterpret_cast<uintptr_t>(p.logits) & 15u) == 0 && p.stride0 % 4 == 0 && !p.row_starts;
+    const int64_t quads = (static_cast<int64_t>(p.vocab) + (aligned ? 0 : 3) + 3) / 4;
+    const auto registers = [&](auto* kernel, int threads) {
+        p.capacity = pool_capacity(Expected(p.top_k, 1.0, 4.0));
+        return launch(kernel, p, threads, 1, stream);
+    };
+    const auto whole = [&](auto* kernel, int threads) {
+        p.capacity = kCountingMax;  // of the histogram route
+        return launch(kernel, p, threads, 1, stream);
+    };
+    const auto stream_rows = [&](auto* kernel, int threads, unsigned ctas) {
+        p.capacity = pool_capacity(Expected(p.top_k, std::min(p.vocab, 4 * kSampleQuads), p.vocab));
+        return launch(kernel, p, threads, ctas, stream);
+    };
+    // Few rows: the time of one row counts, so it gets many threads, or a cluster.  Many rows: small CTAs, of which more are
+    // resident and cover each other's barriers.  Where the lines lie was measured: 61 x 4096, k 512: 5.1 us with 512 threads, 6.0 with
+    // 256, 8.4 with 128; 4096 x 2048: 57 / 29 / 23 us.  Rows of up to 4096 values need no sample (1531 x 4096, k 512: 17 us,
+    // 23 us with one), longer ones do (4096 x 8192: 49 us, 67 us without).
+    const int64_t rows = p.num_rows;
+    if (rows < 2 * sms) {
+        if (quads <= 512 * 2) return whole(topk_short_kernel<DECODE, 512, 2>, 512);
+        if (quads <= 512 * 4) return registers(topk_registers_kernel<DECODE, 512, 4>, 512);
+        if (quads <= 512 * 8) return registers(topk_registers_kernel<DECODE, 512, 8>, 512);
+        unsigned ctas = 1;  // up to two CTAs per SM, and 8192 values for each (61 x 65536: 10.6 us with 4, 15 with 1 or 8)
+        while (ctas < 8 && rows * ctas * 2 <= 2 * sms && static_cast<int64_t>(p.vocab) >= 8192LL * ctas * 2) ctas *= 2;
+        return stream_rows(topk_stream_kernel<DECODE, 512>, 512, ctas);
+    }
+    if (quads <= 128 * 4) return whole(topk_short_kernel<DECODE, 128, 4>, 128);
+    if (quads <= 256 * 4) return whole(topk_short_kernel<DECODE, 256, 4>, 256);
+    if (quads <= 256 * 8) return registers(topk_registers_kernel<DECODE, 256, 8>, 256);
+    if (p.vocab <= 65536) return stream_rows(topk_stream_kernel<DECODE, 256>, 256, 1);
+    // long rows: two CTAs each while there are few waves of them (496 rows of up to 262144: 74.5 us, 77.5 with one)
+    return stream_rows(topk_stream_kernel<DECODE, 512>, 512, p.vocab >= 131072 && rows < 8LL * sms ? 2 : 1);
 }
 
 }  // namespace
@@ -448,48 +946,8 @@ cudaError_t launch_topk_per_row(const float* logits, int64_t stride0, int64_t st
     p.logits = logits, p.stride0 = stride0, p.stride1 = stride1, p.indices = indices;
     p.num_rows = static_cast<int32_t>(num_rows), p.vocab = vocab, p.top_k = top_k;
     p.seq_lens = seq_lens, p.next_n = next_n, p.row_starts = row_starts, p.row_ends = row_ends;
-    constexpr size_t kDynamicBytes = sizeof(uint2) * kCandidateCap;
-    // rows that fit into the buffer as a whole keep 4-byte keys only: more CTAs per SM for the many-short-rows case
-    const size_t dynamic_bytes = vocab <= kCandidateCap ? sizeof(uint32_t) * static_cast<size_t>(vocab > 256 ? vocab : 256) : kDynamicBytes;
-    // per-device set-up, once per device however many host threads make their first call at the same time
-    struct DeviceSetup {
-        std::once_flag once;
-        cudaError_t status = cudaSuccess;
-        int sms = 0;
-    };
-    static DeviceSetup setups[64];
-    int dev = 0;
-    cudaError_t err = cudaGetDevice(&dev);
-    if (err != cudaSuccess) return err;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    DeviceSetup& setup = setups[dev];
-    std::call_once(setup.once, [&]() {
-        setup.status = cudaFuncSetAttribute(topk_per_row_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDynamicBytes));
-        if (setup.status == cudaSuccess)
-            setup.status = cudaFuncSetAttribute(topk_per_row_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDynamicBytes));
-        if (setup.status == cudaSuccess) setup.status = cudaDeviceGetAttribute(&setup.sms, cudaDevAttrMultiProcessorCount, dev);
-    });
-    if (setup.status != cudaSuccess) return setup.status;
-    // CTAs per row: long rows are shared by a cluster (shorter streaming time per row, no straggling rows at the
-    // end of the grid); the candidates meet in the first CTA's shared memory.
-    // Only while the grid would not fill the GPU otherwise (about 3 CTAs per SM are resident): with many rows the
-    // repeated sample and the barriers cost more than the shorter rows win.
-    const int sms = setup.sms;
-    unsigned ctas = vocab >= 131072 ? 8u : vocab >= 65536 ? 4u : vocab >= 32768 ? 2u : 1u;
-    while (ctas > 1 && num_rows * ctas > 3LL * sms) ctas >>= 1;
-    if (num_rows * ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(static_cast<unsigned>(num_rows * ctas)), config.blockDim = dim3(kTopkThreads);
-    config.dynamicSmemBytes = dynamic_bytes, config.stream = stream;
-    p.pair_capacity = static_cast<uint32_t>(dynamic_bytes / sizeof(uint2));
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeClusterDimension;
-    attribute[0].val.clusterDim.x = ctas, attribute[0].val.clusterDim.y = 1, attribute[0].val.clusterDim.z = 1;
-    config.attrs = attribute, config.numAttrs = 1;
-    err = seq_lens ? cudaLaunchKernelEx(&config, topk_per_row_kernel<true>, p) : cudaLaunchKernelEx(&config, topk_per_row_kernel<false>, p);
-    if (err != cudaSuccess) return err;
-    count_launch();
-    return cudaGetLastError();
+    p.sampled = 2 * static_cast<int64_t>(top_k) + 512 <= 8192;
+    return seq_lens ? launch_topk<true>(p, stream) : launch_topk<false>(p, stream);
 }
 
 }  // namespace dsv4

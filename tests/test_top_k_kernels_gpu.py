@@ -1,0 +1,60 @@
+"""The selection kernels at the widths, row counts and lengths where one hands over to the next, and on rows that mislead
+the sample: selected values against torch.topk, positions distinct and inside the row."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+import flaggems_vllm as fg
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def check(logits, starts, ends, k):
+    rows, width = logits.shape
+    out = torch.full((rows, k), -7, dtype=torch.int32, device=DEV)
+    fg.top_k_per_row_prefill(logits, starts, ends, out, rows, logits.stride(0), logits.stride(1), k)
+    got = out.cpu()
+    for r in range(rows):
+        a, b = int(starts[r]), int(ends[r])
+        n = min(k, b - a)
+        assert bool((got[r, n:] == -1).all())
+        chosen = got[r, :n].long()
+        assert chosen.unique().numel() == n and (n == 0 or (int(chosen.min()) >= 0 and int(chosen.max()) < b - a))
+        row = logits[r, a:b].cpu()
+        assert torch.equal(row[chosen].sort().values, row.topk(n).values.sort().values), (r, a, b)
+
+
+@pytest.mark.parametrize("rows", [3, 320])  # few rows: wide CTAs and clusters; many: small ones
+@pytest.mark.parametrize("width", [2048, 2049, 4096, 4100, 8192, 8196, 16384, 16388, 33000])
+def test_widths_where_the_kernel_changes(rows, width):
+    g = torch.Generator(device=DEV).manual_seed(width + rows)
+    logits = torch.randn(rows, width, generator=g, device=DEV)
+    starts = torch.randint(0, 9, (rows,), generator=g, device=DEV, dtype=torch.int32)
+    lengths = torch.randint(400, width - 16, (rows,), generator=g, device=DEV, dtype=torch.int32)
+    lengths[0], lengths[1], lengths[2] = 512, 513, width - 16
+    check(logits, starts, starts + lengths, 512)
+
+
+@pytest.mark.parametrize("k", [1, 64, 2048, 3839, 3841, 6000])
+def test_numbers_selected(k):
+    logits = torch.randn(5, 20000, generator=torch.Generator(device=DEV).manual_seed(k), device=DEV)
+    ends = torch.tensor([20000, 6001, 19999, 8191, 3], dtype=torch.int32, device=DEV)
+    check(logits, torch.zeros(5, dtype=torch.int32, device=DEV), ends, k)
+
+
+@pytest.mark.parametrize("width", [3000, 8000, 15000, 70000])
+def test_rows_that_mislead_the_sample(width):
+    g = torch.Generator(device=DEV).manual_seed(7)
+    x = torch.randn(8, width, generator=g, device=DEV)
+    x[0, 1000:1700] += 8.0  # all of the top k in one run
+    x[1] = x[1].sort().values
+    x[2] = x[2].sort(descending=True).values
+    x[3] = (x[3] * 4).round() / 4  # few distinct values
+    x[4, 600:] = -float("inf")  # masked
+    x[5, ::4] += 6.0  # what a sample of every fourth value sees
+    x[6] = -x[6].abs() * 1e-30
+    x[7, 5::2] = float("inf")
+    ends = torch.full((8,), width, dtype=torch.int32, device=DEV)
+    check(x, torch.zeros_like(ends), ends, 512)
