@@ -113,6 +113,7 @@ PrologueParams make_params(void* q, const void* kv, void* k_cache, const int64_t
 }
 }  // namespace
 
+int launch_mode() { return current_pdl(); }
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 }  // namespace dsv4
 

@@ -56,6 +56,7 @@ __device__ __forceinline__ bool locate(const CpGatherParams& p, int32_t t, int32
 // side by side); the lane groups then fetch block and position of their tokens with shuffles.
 template <int WARPS, int LANES, int U>
 __global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_vec_kernel(const CpGatherParams p) {
+    begin_dependent_kernel();
     constexpr int kGroups = 32 / LANES;
     static_assert(kGroups * U <= 32, "a warp locates one token per lane");
     const int lane = threadIdx.x & 31;
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_vec_kernel(const
 // Any head_dim and any alignment: one warp per token, byte by byte.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_bytes_kernel(const CpGatherParams p) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (t >= p.num_tokens) return;
@@ -155,7 +157,7 @@ cudaError_t launch_cp_gather_indexer(const void* cache, int64_t block_stride, vo
     if (!vec) {
         const int64_t grid = (num_tokens + WARPS - 1) / WARPS;
         if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-        cp_gather_indexer_bytes_kernel<WARPS><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p);
+        launch_dependent(cp_gather_indexer_bytes_kernel<WARPS>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
     } else {
         constexpr int U = 4;
         const int chunks = head_dim / 16;
@@ -164,7 +166,7 @@ cudaError_t launch_cp_gather_indexer(const void* cache, int64_t block_stride, vo
         const int64_t per_cta = static_cast<int64_t>(WARPS) * (32 / LANES) * U;                                           \
         const int64_t grid = (num_tokens + per_cta - 1) / per_cta;                                                        \
         if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;                                                    \
-        cp_gather_indexer_vec_kernel<WARPS, LANES, U><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p);          \
+        launch_dependent(cp_gather_indexer_vec_kernel<WARPS, LANES, U>, static_cast<unsigned>(grid), WARPS * 32, stream, p);          \
     } while (0)
         if (chunks <= 4) DSV4_CP_GATHER(4);
         else if (chunks <= 8) DSV4_CP_GATHER(8);

@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(WARPS * 32)
 gather_dequant_kernel(const uint8_t* __restrict__ k_cache, const int64_t* __restrict__ slots, int64_t num_slots,
                       uint8_t* __restrict__ out, int64_t out_row_bytes, int64_t block_size, int64_t block_stride,
                       int aligned16) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t i = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (i >= num_slots) return;
@@ -98,6 +99,7 @@ __device__ __forceinline__ int64_t load_index(const void* p, int64_t i, int is64
 
 template <int WARPS, bool FAST>
 __global__ void __launch_bounds__(WARPS * 32) gather_dequant_requests_kernel(const GatherParams g) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t req = blockIdx.y;
     const int64_t seq_len = load_index(g.seq_lens, req, g.index64);
@@ -188,7 +190,7 @@ cudaError_t launch_gather_dequant(const uint8_t* k_cache, const int64_t* slots, 
     const int64_t grid = (num_slots + WARPS - 1) / WARPS;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const int aligned16 = ((reinterpret_cast<uintptr_t>(k_cache) | static_cast<uintptr_t>(block_stride)) & 15u) == 0;
-    gather_dequant_kernel<WARPS><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(
+    launch_dependent(gather_dequant_kernel<WARPS>, static_cast<unsigned>(grid), WARPS * 32, stream,
         k_cache, slots, num_slots, out, out_row_stride * 2, block_size, block_stride, aligned16);
     count_launch();
     return cudaGetLastError();
@@ -217,8 +219,8 @@ cudaError_t launch_gather_dequant_requests(uint8_t* out, int64_t out_stride0, in
                       ((addr(k_cache) | static_cast<uintptr_t>(block_stride)) & 15u) == 0 && (addr(out) & 15u) == 0 &&
                       out_stride0 % 8 == 0 && out_stride1 % 8 == 0 && (block_size * kTokenDataBytes) % 8 == 0;
     const dim3 grid(static_cast<unsigned>(ctas), static_cast<unsigned>(num_reqs));
-    if (fast) gather_dequant_requests_kernel<WARPS, true><<<grid, WARPS * 32, 0, stream>>>(g);
-    else gather_dequant_requests_kernel<WARPS, false><<<grid, WARPS * 32, 0, stream>>>(g);
+    if (fast) launch_dependent(gather_dequant_requests_kernel<WARPS, true>, grid, WARPS * 32, stream, g);
+    else launch_dependent(gather_dequant_requests_kernel<WARPS, false>, grid, WARPS * 32, stream, g);
     count_launch();
     return cudaGetLastError();
 }

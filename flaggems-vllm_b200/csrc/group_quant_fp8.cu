@@ -32,6 +32,7 @@ struct GroupQuantParams {
 // (IEEE division, the verified reciprocal-and-correct division for the default eps, or x * (1/scale) for `act_quant`).
 template <int WARPS, int LANES, int CHUNKS, int U, bool UE8M0, int DIVISION>
 __global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_kernel(const GroupQuantParams p) {
+    begin_dependent_kernel();
     constexpr int kGroups = 32 / LANES;
     const int lane = threadIdx.x & 31;
     const int sub = lane % LANES;
@@ -96,6 +97,7 @@ __global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_kernel(const Group
 // Any group size and alignment: one warp per group, element by element.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_scalar_kernel(const GroupQuantParams p, const int ue8m0, const int reciprocal) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t g = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (g >= p.num_groups) return;
@@ -120,10 +122,10 @@ void launch_vector(const GroupQuantParams& p, bool ue8m0, int division, cudaStre
     constexpr int WARPS = 4, U = CHUNKS == 1 ? 4 : 2;
     const int64_t per_cta = static_cast<int64_t>(WARPS) * (32 / LANES) * U;
     const unsigned grid = static_cast<unsigned>((p.num_groups + per_cta - 1) / per_cta);
-    if (ue8m0) group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, true, kDivideIeee><<<grid, WARPS * 32, 0, stream>>>(p);
-    else if (division == kDivideFast) group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, false, kDivideFast><<<grid, WARPS * 32, 0, stream>>>(p);
-    else if (division == kMultiplyReciprocal) group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, false, kMultiplyReciprocal><<<grid, WARPS * 32, 0, stream>>>(p);
-    else group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, false, kDivideIeee><<<grid, WARPS * 32, 0, stream>>>(p);
+    if (ue8m0) launch_dependent(group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, true, kDivideIeee>, grid, WARPS * 32, stream, p);
+    else if (division == kDivideFast) launch_dependent(group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, false, kDivideFast>, grid, WARPS * 32, stream, p);
+    else if (division == kMultiplyReciprocal) launch_dependent(group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, false, kMultiplyReciprocal>, grid, WARPS * 32, stream, p);
+    else launch_dependent(group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, false, kDivideIeee>, grid, WARPS * 32, stream, p);
 }
 
 }  // namespace
@@ -153,7 +155,7 @@ cudaError_t launch_group_quant_fp8(const void* x, int64_t x_stride, void* out, f
     const int division = act_quant_rules ? kMultiplyReciprocal : (eps == 1e-10f ? kDivideFast : kDivideIeee);
     if (!vec) {
         constexpr int WARPS = 4;
-        group_quant_fp8_scalar_kernel<WARPS><<<static_cast<unsigned>((num_groups + WARPS - 1) / WARPS), WARPS * 32, 0, stream>>>(p, ue8m0, act_quant_rules);
+        launch_dependent(group_quant_fp8_scalar_kernel<WARPS>, static_cast<unsigned>((num_groups + WARPS - 1) / WARPS), WARPS * 32, stream, p, ue8m0, act_quant_rules);
     } else if (group_size == 64) {
         launch_vector<8, 1>(p, ue8m0 != 0, division, stream);
     } else if (group_size == 128) {

@@ -50,6 +50,7 @@ __device__ __forceinline__ float group_scale(float amax, bool ue8m0) {
 
 template <int WARPS, bool FP16>
 __global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_kernel(const IndexerParams p) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (t >= p.num_tokens) return;
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_kernel(const Index
 // moves 32/G tokens, and U passes are loaded (slot and row) before any is used.
 template <int WARPS, int G, int U, bool FP16>
 __global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_rows_kernel(const IndexerParams p) {
+    begin_dependent_kernel();
     constexpr int TOKENS = 32 / G;
     const int lane = threadIdx.x & 31, sub = lane % G, which = lane / G;
     const int64_t base = (static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5)) * (U * TOKENS) + which;
@@ -157,6 +159,7 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_rows_kernel(const 
 // UE8M0 (power-of-two scales): bf16 keys stay packed - group maximum and scaling on the bf16x2 words, as in quant8_pow2.
 template <int WARPS, int U, bool FP16, bool UE8M0>
 __global__ void __launch_bounds__(WARPS * 32, DSV4_INDEXER_K_CTAS) indexer_k_quant_128_kernel(const IndexerParams p) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31, sub = lane & 7, which = lane >> 3;
     const int64_t base = (static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5)) * (U * 4) + which;
     uint4 lo[U], hi[U];
@@ -228,7 +231,7 @@ template <int G, bool FP16>
 void launch_rows(const IndexerParams& p, cudaStream_t stream) {
     constexpr int WARPS = 4, U = 2, PER_CTA = WARPS * U * (32 / G);
     const unsigned grid = static_cast<unsigned>((p.num_tokens + PER_CTA - 1) / PER_CTA);
-    indexer_k_quant_rows_kernel<WARPS, G, U, FP16><<<grid, WARPS * 32, 0, stream>>>(p);
+    launch_dependent(indexer_k_quant_rows_kernel<WARPS, G, U, FP16>, grid, WARPS * 32, stream, p);
 }
 
 }  // namespace
@@ -255,10 +258,10 @@ cudaError_t launch_indexer_k_quant(const void* k, int64_t k_stride, int is_fp16,
 #endif
         constexpr int W = 4, U = DSV4_INDEXER_K_U;
         const unsigned g128 = static_cast<unsigned>((num_tokens + W * U * 4 - 1) / (W * U * 4));
-        if (is_fp16) ue8m0 ? indexer_k_quant_128_kernel<W, U, true, true><<<g128, W * 32, 0, stream>>>(p)
-                           : indexer_k_quant_128_kernel<W, U, true, false><<<g128, W * 32, 0, stream>>>(p);
-        else ue8m0 ? indexer_k_quant_128_kernel<W, U, false, true><<<g128, W * 32, 0, stream>>>(p)
-                   : indexer_k_quant_128_kernel<W, U, false, false><<<g128, W * 32, 0, stream>>>(p);
+        if (is_fp16) ue8m0 ? launch_dependent(indexer_k_quant_128_kernel<W, U, true, true>, g128, W * 32, stream, p)
+                           : launch_dependent(indexer_k_quant_128_kernel<W, U, true, false>, g128, W * 32, stream, p);
+        else ue8m0 ? launch_dependent(indexer_k_quant_128_kernel<W, U, false, true>, g128, W * 32, stream, p)
+                   : launch_dependent(indexer_k_quant_128_kernel<W, U, false, false>, g128, W * 32, stream, p);
         count_launch();
         return cudaGetLastError();
     }
@@ -269,8 +272,8 @@ cudaError_t launch_indexer_k_quant(const void* k, int64_t k_stride, int is_fp16,
         count_launch();
         return cudaGetLastError();
     }
-    if (is_fp16) indexer_k_quant_kernel<WARPS, true><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p);
-    else indexer_k_quant_kernel<WARPS, false><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p);
+    if (is_fp16) launch_dependent(indexer_k_quant_kernel<WARPS, true>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
+    else launch_dependent(indexer_k_quant_kernel<WARPS, false>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
     count_launch();
     return cudaGetLastError();
 }

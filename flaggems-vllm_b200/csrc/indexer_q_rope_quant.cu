@@ -102,6 +102,7 @@ __device__ __forceinline__ void load_row(const uint8_t* p, float (&x)[E]) {
 
 template <int WARPS, int E, bool FP4>
 __global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_kernel(const IndexerQParams p) {
+    begin_dependent_kernel();
     constexpr int D = 32 * E;
     const int lane = threadIdx.x & 31;
     const uint32_t row = blockIdx.x * WARPS + (threadIdx.x >> 5);
@@ -177,6 +178,7 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_kernel(const 
 // on a multiple of 8 values.
 template <int WARPS, int G, int U, bool FP4>
 __global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_rows_kernel(const IndexerQParams p, const int cs_vec4) {
+    begin_dependent_kernel();
     constexpr int D = 8 * G, ROWS = 32 / G;
     const int lane = threadIdx.x & 31, sub = lane % G, slot = lane / G;
     const uint32_t total = static_cast<uint32_t>(p.num_tokens) * static_cast<uint32_t>(p.num_heads);
@@ -268,8 +270,8 @@ template <int G>
 cudaError_t launch_rows(const IndexerQParams& p, bool fp4, int64_t rows, int cs_vec4, cudaStream_t stream) {
     constexpr int WARPS = 4, U = 2, PER_CTA = WARPS * U * (32 / G);
     const unsigned grid = static_cast<unsigned>((rows + PER_CTA - 1) / PER_CTA);
-    if (fp4) indexer_q_rope_quant_rows_kernel<WARPS, G, U, true><<<grid, WARPS * 32, 0, stream>>>(p, cs_vec4);
-    else indexer_q_rope_quant_rows_kernel<WARPS, G, U, false><<<grid, WARPS * 32, 0, stream>>>(p, cs_vec4);
+    if (fp4) launch_dependent(indexer_q_rope_quant_rows_kernel<WARPS, G, U, true>, grid, WARPS * 32, stream, p, cs_vec4);
+    else launch_dependent(indexer_q_rope_quant_rows_kernel<WARPS, G, U, false>, grid, WARPS * 32, stream, p, cs_vec4);
     return cudaGetLastError();
 }
 
@@ -280,6 +282,7 @@ cudaError_t launch_rows(const IndexerQParams& p, bool fp4, int64_t rows, int cs_
 // 4 lanes.
 template <int WARPS, bool FP4>
 __global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_token_kernel(const IndexerQParams p) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31, sub = lane & 7, which = lane >> 3;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (t >= p.num_tokens) return;
@@ -399,8 +402,8 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_token_kernel(
 template <int E>
 cudaError_t launch_e(const IndexerQParams& p, bool fp4, unsigned grid, cudaStream_t stream) {
     constexpr int WARPS = 8;
-    if (fp4) indexer_q_rope_quant_kernel<WARPS, E, true><<<grid, WARPS * 32, 0, stream>>>(p);
-    else indexer_q_rope_quant_kernel<WARPS, E, false><<<grid, WARPS * 32, 0, stream>>>(p);
+    if (fp4) launch_dependent(indexer_q_rope_quant_kernel<WARPS, E, true>, grid, WARPS * 32, stream, p);
+    else launch_dependent(indexer_q_rope_quant_kernel<WARPS, E, false>, grid, WARPS * 32, stream, p);
     return cudaGetLastError();
 }
 
@@ -436,8 +439,8 @@ cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q,
     if (token_shape) {
         constexpr int WARPS = 4;
         const unsigned grid = static_cast<unsigned>((num_tokens + WARPS - 1) / WARPS);
-        if (fp4) indexer_q_rope_quant_token_kernel<WARPS, true><<<grid, WARPS * 32, 0, stream>>>(p);
-        else indexer_q_rope_quant_token_kernel<WARPS, false><<<grid, WARPS * 32, 0, stream>>>(p);
+        if (fp4) launch_dependent(indexer_q_rope_quant_token_kernel<WARPS, true>, grid, WARPS * 32, stream, p);
+        else launch_dependent(indexer_q_rope_quant_token_kernel<WARPS, false>, grid, WARPS * 32, stream, p);
         count_launch();
         return cudaGetLastError();
     }

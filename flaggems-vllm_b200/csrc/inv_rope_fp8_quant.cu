@@ -47,6 +47,7 @@ constexpr int kHeadsPerTask = 16;
 template <int WARPS, bool PACKED, bool FASTDIV, int U, int MIN_CTAS, bool PREFETCH>
 __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kernel(const InvRopeParams p, const uint32_t tasks_per_token,
                                                                       const uint32_t tpt_mul, const uint32_t tpt_shift) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const uint32_t task = blockIdx.x * WARPS + (threadIdx.x >> 5);
     if (task >= static_cast<uint32_t>(p.padded_tokens) * tasks_per_token) return;
@@ -178,6 +179,7 @@ struct InvRopeGeometry {
 
 template <int WARPS, bool PACKED>
 __global__ void __launch_bounds__(WARPS * 32) inv_rope_fp8_quant_any_kernel(const InvRopeParams p, const InvRopeGeometry geo) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t row = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (row >= p.padded_tokens * p.num_heads) return;
@@ -259,8 +261,8 @@ cudaError_t launch_inv_rope_fp8_quant_any(const void* o, int64_t o_stride_token,
     p.num_tokens = num_tokens, p.padded_tokens = padded_tokens, p.num_heads = num_heads, p.heads_per_group = heads_per_group;
     p.eps = eps;
     const InvRopeGeometry geo{nope_dim, rope_dim, group_size, (nope_dim + rope_dim) / group_size};
-    if (packed) inv_rope_fp8_quant_any_kernel<WARPS, true><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p, geo);
-    else inv_rope_fp8_quant_any_kernel<WARPS, false><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p, geo);
+    if (packed) launch_dependent(inv_rope_fp8_quant_any_kernel<WARPS, true>, static_cast<unsigned>(grid), WARPS * 32, stream, p, geo);
+    else launch_dependent(inv_rope_fp8_quant_any_kernel<WARPS, false>, static_cast<unsigned>(grid), WARPS * 32, stream, p, geo);
     count_launch();
     return cudaGetLastError();
 }
@@ -292,9 +294,9 @@ cudaError_t launch_inv_rope_fp8_quant(const void* o, int64_t o_stride_token, int
     // (72 registers) 256 us, 8 CTAs (64 registers, 8 bytes spilled) 257 us, 6 CTAs 262 us; one pass in flight at 10 CTAs
     // 265-282 us.  fp32-scale mode: two passes at 8 CTAs (64 registers) 269 us, at 7 CTAs 270 us; one pass at 10 CTAs
     // (48 registers) 272 us, at 9 CTAs 274 us, at 11 CTAs 301 us.
-    if (packed) inv_rope_fp8_quant_kernel<WARPS, true, false, 2, DSV4_INVROPE_UE8M0_CTAS, true><<<g, WARPS * 32, 0, stream>>>(p, tpt, tpt_mul, tpt_shift);
-    else if (eps == 1e-10f) inv_rope_fp8_quant_kernel<WARPS, false, true, 2, DSV4_INVROPE_FP32_CTAS, true><<<g, WARPS * 32, 0, stream>>>(p, tpt, tpt_mul, tpt_shift);
-    else inv_rope_fp8_quant_kernel<WARPS, false, false, 2, 8, false><<<g, WARPS * 32, 0, stream>>>(p, tpt, tpt_mul, tpt_shift);
+    if (packed) launch_dependent(inv_rope_fp8_quant_kernel<WARPS, true, false, 2, DSV4_INVROPE_UE8M0_CTAS, true>, g, WARPS * 32, stream, p, tpt, tpt_mul, tpt_shift);
+    else if (eps == 1e-10f) launch_dependent(inv_rope_fp8_quant_kernel<WARPS, false, true, 2, DSV4_INVROPE_FP32_CTAS, true>, g, WARPS * 32, stream, p, tpt, tpt_mul, tpt_shift);
+    else launch_dependent(inv_rope_fp8_quant_kernel<WARPS, false, false, 2, 8, false>, g, WARPS * 32, stream, p, tpt, tpt_mul, tpt_shift);
     count_launch();
     return cudaGetLastError();
 }

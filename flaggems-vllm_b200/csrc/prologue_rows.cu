@@ -18,12 +18,6 @@ namespace {
 
 // PADDED: out-of-place form (vLLM >= 0.22 calls the operator that way): rows go to p.q_out with out_heads heads per
 // token and the CTAs after the q tiles zero-fill the extra heads.
-// Programmatic dependent launch (sm_90+): the kernel may start while the preceding kernel of the stream still runs;
-// `wait` returns once that kernel has completed and its writes are visible (a no-op for an ordinary launch), and
-// `launch_dependents` lets the next kernel of the stream start its own independent part.
-__device__ __forceinline__ void wait_for_preceding_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // STAGED: the cos|sin rows of the tile's tokens go through shared memory (one fetch per CTA, one barrier).  Without
 // it every warp fetches position and table row of its own rows straight into registers (lane i holds cosine i and
 // sine i): 256 more bytes from L2 per row, but no barrier and no shared-memory round trip in the dependent chain

@@ -33,6 +33,7 @@ __device__ __forceinline__ float inv_rms_of(float sum, int size, float eps) {
 template <int WARPS, int CH>
 __global__ void __launch_bounds__(WARPS * 32, CH <= 2 ? 16 : (CH <= 6 ? 8 : 6)) q_kv_rmsnorm_kernel(const NormRows q, const NormRows kv, int64_t num_tokens,
                                                                  float eps) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (r >= 2 * num_tokens) return;
@@ -118,6 +119,7 @@ __device__ __forceinline__ void store_any(uint8_t* base, int64_t i, int dtype, f
 
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) q_kv_rmsnorm_any_kernel(const AnyRows q, const AnyRows kv, int64_t num_tokens, float eps) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (r >= 2 * num_tokens) return;
@@ -161,10 +163,10 @@ cudaError_t launch_q_kv_rmsnorm(const void* q, void* q_out, const void* q_weight
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const int64_t longest = (a.vec_ok ? q_size : 0) > (b.vec_ok ? kv_size : 0) ? (a.vec_ok ? q_size : 0) : (b.vec_ok ? kv_size : 0);
     const unsigned g = static_cast<unsigned>(grid);
-    if (longest <= 512) q_kv_rmsnorm_kernel<WARPS, 2><<<g, WARPS * 32, 0, stream>>>(a, b, num_tokens, eps);
-    else if (longest <= 1024) q_kv_rmsnorm_kernel<WARPS, 4><<<g, WARPS * 32, 0, stream>>>(a, b, num_tokens, eps);
-    else if (longest <= 1536) q_kv_rmsnorm_kernel<WARPS, 6><<<g, WARPS * 32, 0, stream>>>(a, b, num_tokens, eps);
-    else q_kv_rmsnorm_kernel<WARPS, 8><<<g, WARPS * 32, 0, stream>>>(a, b, num_tokens, eps);
+    if (longest <= 512) launch_dependent(q_kv_rmsnorm_kernel<WARPS, 2>, g, WARPS * 32, stream, a, b, num_tokens, eps);
+    else if (longest <= 1024) launch_dependent(q_kv_rmsnorm_kernel<WARPS, 4>, g, WARPS * 32, stream, a, b, num_tokens, eps);
+    else if (longest <= 1536) launch_dependent(q_kv_rmsnorm_kernel<WARPS, 6>, g, WARPS * 32, stream, a, b, num_tokens, eps);
+    else launch_dependent(q_kv_rmsnorm_kernel<WARPS, 8>, g, WARPS * 32, stream, a, b, num_tokens, eps);
     count_launch();
     return cudaGetLastError();
 }
@@ -181,7 +183,7 @@ cudaError_t launch_q_kv_rmsnorm_any(const void* q, void* q_out, const void* q_we
                     kv_in_stride, kv_out_stride, static_cast<int32_t>(kv_size), kv_dtype, kv_weight_dtype};
     const int64_t grid = (2 * num_tokens + WARPS - 1) / WARPS;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    q_kv_rmsnorm_any_kernel<WARPS><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(a, b, num_tokens, eps);
+    launch_dependent(q_kv_rmsnorm_any_kernel<WARPS>, static_cast<unsigned>(grid), WARPS * 32, stream, a, b, num_tokens, eps);
     count_launch();
     return cudaGetLastError();
 }

@@ -44,6 +44,7 @@ __device__ __forceinline__ int32_t to_slot(const GlobalTopkParams& p, const int3
 // One warp per token.  VEC: rows are 16-byte aligned and topk is a multiple of 4, so a lane moves 4 entries at a time.
 template <int WARPS, bool VEC>
 __global__ void __launch_bounds__(WARPS * 32) global_topk_kernel(const GlobalTopkParams p) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (t >= p.num_tokens) return;
@@ -94,6 +95,7 @@ struct CombineParams {
 // One warp per query token.  VEC: rows 16-byte aligned and widths multiples of 4.
 template <int WARPS, bool VEC>
 __global__ void __launch_bounds__(WARPS * 32) combine_topk_swa_kernel(const CombineParams p) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int32_t token = static_cast<int32_t>(blockIdx.x * WARPS + (threadIdx.x >> 5));
     if (token >= p.num_tokens) return;
@@ -159,8 +161,8 @@ cudaError_t launch_global_topk(const int32_t* local, int64_t local_stride, const
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const auto addr = [](const void* q) { return reinterpret_cast<uintptr_t>(q); };
     const bool vec = topk % 4 == 0 && local_stride % 4 == 0 && global_stride % 4 == 0 && addr(local) % 16 == 0 && addr(global) % 16 == 0;
-    if (vec) global_topk_kernel<WARPS, true><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p);
-    else global_topk_kernel<WARPS, false><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p);
+    if (vec) launch_dependent(global_topk_kernel<WARPS, true>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
+    else launch_dependent(global_topk_kernel<WARPS, false>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
     count_launch();
     return cudaGetLastError();
 }
@@ -185,8 +187,8 @@ cudaError_t launch_combine_topk_swa(const int32_t* topk_indices, int64_t topk_st
     const auto addr = [](const void* q) { return reinterpret_cast<uintptr_t>(q); };
     const bool vec = topk_width % 4 == 0 && combined_width % 4 == 0 && topk_stride % 4 == 0 && combined_stride % 4 == 0 &&
                      addr(topk_indices) % 16 == 0 && addr(combined) % 16 == 0;
-    if (vec) combine_topk_swa_kernel<WARPS, true><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p);
-    else combine_topk_swa_kernel<WARPS, false><<<static_cast<unsigned>(grid), WARPS * 32, 0, stream>>>(p);
+    if (vec) launch_dependent(combine_topk_swa_kernel<WARPS, true>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
+    else launch_dependent(combine_topk_swa_kernel<WARPS, false>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
     count_launch();
     return cudaGetLastError();
 }

@@ -566,6 +566,7 @@ __device__ __forceinline__ int32_t row_range(const TopkParams& p, int r, int64_t
 // a large part is selected: fewer phases, and about 25 instructions per value.
 template <bool DECODE, int THREADS, int QUADS>
 __global__ void __launch_bounds__(THREADS) topk_short_kernel(const TopkParams p) {
+    begin_dependent_kernel();
     __shared__ Shared s;
     extern __shared__ uint2 dynamic[];
     const int tid = threadIdx.x, lane = tid & 31;
@@ -649,6 +650,7 @@ __global__ void __launch_bounds__(THREADS) topk_short_kernel(const TopkParams p)
 // One CTA per row, the row in registers: QUADS x 4 values per thread.  The sample is the first value of every quad.
 template <bool DECODE, int THREADS, int QUADS>
 __global__ void __launch_bounds__(THREADS) topk_registers_kernel(const TopkParams p) {
+    begin_dependent_kernel();
     __shared__ Shared s;
     extern __shared__ uint2 dynamic[];
     const int tid = threadIdx.x;
@@ -708,6 +710,7 @@ __global__ void __launch_bounds__(THREADS) topk_registers_kernel(const TopkParam
 
 template <bool DECODE, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(const TopkParams p) {
+    begin_dependent_kernel();
     __shared__ Shared s;
     extern __shared__ uint2 dynamic[];  // the candidate pool
     cg::cluster_group cluster = cg::this_cluster();
@@ -854,14 +857,8 @@ constexpr size_t kMaxDynamicBytes = sizeof(uint2) * 8192;
 template <typename Kernel>
 cudaError_t launch(Kernel kernel, const TopkParams& p, int threads, unsigned ctas, cudaStream_t stream) {
     if (p.num_rows * static_cast<int64_t>(ctas) > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(static_cast<unsigned>(p.num_rows) * ctas), config.blockDim = dim3(static_cast<unsigned>(threads));
-    config.dynamicSmemBytes = sizeof(uint2) * p.capacity, config.stream = stream;
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeClusterDimension;
-    attribute[0].val.clusterDim.x = ctas, attribute[0].val.clusterDim.y = 1, attribute[0].val.clusterDim.z = 1;
-    config.attrs = attribute, config.numAttrs = ctas > 1 ? 1 : 0;
-    const cudaError_t err = cudaLaunchKernelEx(&config, kernel, p);
+    const cudaError_t err = launch_dependent_cluster(kernel, static_cast<unsigned>(p.num_rows) * ctas, static_cast<unsigned>(threads), ctas,
+                                                     sizeof(uint2) * p.capacity, stream, p);
     if (err != cudaSuccess) return err;
     count_launch();
     return cudaGetLastError();

@@ -366,6 +366,7 @@ int dsv4_bulk_wait_selftest(void* q, const void* kv, void* k_cache, const int64_
  *   mode 1: the kernel also fetches position_ids, slot_mapping and the cos/sin rows at once and waits for the
  *           preceding kernel only before it touches q, kv and the cache.  The caller promises that position_ids,
  *           slot_mapping and cos_sin_cache are not written by the kernel that precedes the call in the stream.
+ * The other operators of this library are launched the way of mode 2 in both modes, and plainly in mode 0.
  * Returns the previous mode. */
 int dsv4_set_pdl(int mode);
 
