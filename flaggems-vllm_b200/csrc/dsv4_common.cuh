@@ -166,6 +166,23 @@ __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     return v;
 }
 
+// The same for 32 bytes (p 32-byte aligned): one instruction, 1 KiB per warp.
+struct Bytes32 {
+    uint4 lo, hi;
+};
+__device__ __forceinline__ Bytes32 ld_stream32(const void* p) {
+    Bytes32 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v.lo.x), "=r"(v.lo.y), "=r"(v.lo.z), "=r"(v.lo.w), "=r"(v.hi.x), "=r"(v.hi.y), "=r"(v.hi.z), "=r"(v.hi.w)
+                 : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void st_stream32(void* p, const Bytes32& v) {
+    asm volatile("st.global.L1::no_allocate.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v.lo.x), "r"(v.lo.y), "r"(v.lo.z),
+                 "r"(v.lo.w), "r"(v.hi.x), "r"(v.hi.y), "r"(v.hi.z), "r"(v.hi.w)
+                 : "memory");
+}
+
 __device__ __forceinline__ void st_stream16(void* p, uint4 v) {
     asm volatile("st.global.L1::no_allocate.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z),
                  "r"(v.w)

@@ -27,42 +27,40 @@ struct GroupQuantParams {
     uint32_t gpr_mul, gpr_shift;  // fast division of a group index by groups_per_row
 };
 
-// LANES adjacent lanes per group, CHUNKS x 8 values per lane (group_size = LANES * CHUNKS * 8), U groups per lane
-// group in flight.  UE8M0: power-of-two scales (exact reciprocal multiply); DIVISION: how x / scale is formed otherwise
+// LANES adjacent lanes per group, 16 values per lane (group_size = 16 * LANES), U groups per lane group in flight.  WIDE: one
+// 32-byte load and one 16-byte store per lane and group; otherwise (rows on 16-byte boundaries only) two loads and two stores.
+// UE8M0: power-of-two scales (exact reciprocal multiply); DIVISION: how x / scale is formed otherwise
 // (IEEE division, the verified reciprocal-and-correct division for the default eps, or x * (1/scale) for `act_quant`).
-template <int WARPS, int LANES, int CHUNKS, int U, bool UE8M0, int DIVISION>
+template <int WARPS, int LANES, int U, bool WIDE, bool UE8M0, int DIVISION>
 __global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_kernel(const GroupQuantParams p) {
     begin_dependent_kernel();
     constexpr int kGroups = 32 / LANES;
     const int lane = threadIdx.x & 31;
     const int sub = lane % LANES;
     const int64_t first = (static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5)) * (kGroups * U) + lane / LANES;
-    uint4 v[U][CHUNKS];
+    Bytes32 v[U];
     int64_t row[U];
     int32_t col[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const int64_t g = first + u * kGroups;
         row[u] = 0, col[u] = 0;
-#pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) v[u][c] = make_uint4(0u, 0u, 0u, 0u);
+        v[u].lo = v[u].hi = make_uint4(0u, 0u, 0u, 0u);
         if (g < p.num_groups) {
             row[u] = fast_div(static_cast<uint32_t>(g), p.gpr_mul, p.gpr_shift);
             col[u] = static_cast<int32_t>(g - row[u] * p.groups_per_row);
-            const uint8_t* src = p.x + (row[u] * p.x_stride + static_cast<int64_t>(col[u]) * p.group_size) * 2;
-#pragma unroll
-            for (int c = 0; c < CHUNKS; ++c) v[u][c] = ld_stream16(src + 16 * (sub + c * LANES));
+            const uint8_t* src = p.x + (row[u] * p.x_stride + static_cast<int64_t>(col[u]) * p.group_size) * 2 + 32 * sub;
+            if (WIDE) v[u] = ld_stream32(src);
+            else v[u].lo = ld_stream16(src), v[u].hi = ld_stream16(src + 16);
         }
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const int64_t g = first + u * kGroups;
         // |.| maximum on the packed words (even and odd elements side by side), then across the group's lanes
-        uint32_t pk = max_abs_bf16x2(max_abs_bf16x2(v[u][0].x, v[u][0].y), max_abs_bf16x2(v[u][0].z, v[u][0].w));
-#pragma unroll
-        for (int c = 1; c < CHUNKS; ++c)
-            pk = max_abs_bf16x2(pk, max_abs_bf16x2(max_abs_bf16x2(v[u][c].x, v[u][c].y), max_abs_bf16x2(v[u][c].z, v[u][c].w)));
-        pk &= 0x7fff7fffu;
+        const uint4 &a = v[u].lo, &b = v[u].hi;
+        uint32_t pk = max_abs_bf16x2(max_abs_bf16x2(max_abs_bf16x2(a.x, a.y), max_abs_bf16x2(a.z, a.w)),
+                                     max_abs_bf16x2(max_abs_bf16x2(b.x, b.y), max_abs_bf16x2(b.z, b.w))) & 0x7fff7fffu;
 #pragma unroll
         for (int m = 1; m < LANES; m <<= 1) pk = max_bf16x2(pk, __shfl_xor_sync(0xffffffffu, pk, m));
         const float amax = fmaxf(bf16_lo(pk), bf16_hi(pk));
@@ -74,22 +72,19 @@ __global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_kernel(const Group
         }
         const bool two_term = !UE8M0 && DIVISION == kDivideFast && __all_sync(0xffffffffu, scale <= kTwoTermMaxScale);
         if (g >= p.num_groups) continue;
-        uint8_t* dst = p.out + g * p.group_size;
+        uint2 qa, qb;
         if (UE8M0) {
-#pragma unroll
-            for (int c = 0; c < CHUNKS; ++c) st_global8(dst + 8 * (sub + c * LANES), quant8_pow2(v[u][c], code));
+            qa = quant8_pow2(a, code), qb = quant8_pow2(b, code);
         } else {
             // one warp-uniform choice of the division form per pass (see ScaleDivider); lanes past the last group
             // have left the loop body above only after the vote, so every lane takes part in it
             const ScaleDivider<DIVISION> by_scale(scale);
-            if (two_term) {
-#pragma unroll
-                for (int c = 0; c < CHUNKS; ++c) st_global8(dst + 8 * (sub + c * LANES), quant8_by<DIVISION, true>(v[u][c], by_scale));
-            } else {
-#pragma unroll
-                for (int c = 0; c < CHUNKS; ++c) st_global8(dst + 8 * (sub + c * LANES), quant8_by<DIVISION, false>(v[u][c], by_scale));
-            }
+            if (two_term) qa = quant8_by<DIVISION, true>(a, by_scale), qb = quant8_by<DIVISION, true>(b, by_scale);
+            else qa = quant8_by<DIVISION, false>(a, by_scale), qb = quant8_by<DIVISION, false>(b, by_scale);
         }
+        uint8_t* dst = p.out + g * p.group_size + 16 * sub;
+        if (WIDE) st_stream16(dst, make_uint4(qa.x, qa.y, qb.x, qb.y));
+        else st_global8(dst, qa), st_global8(dst + 8, qb);
         if (sub == 0) p.scales[row[u] * p.scale_stride_row + col[u] * p.scale_stride_group] = scale;
     }
 }
@@ -117,15 +112,29 @@ __global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_scalar_kernel(cons
     if (lane == 0) p.scales[row * p.scale_stride_row + col * p.scale_stride_group] = scale;
 }
 
-template <int LANES, int CHUNKS>
+template <int LANES, int U, bool WIDE>
 void launch_vector(const GroupQuantParams& p, bool ue8m0, int division, cudaStream_t stream) {
-    constexpr int WARPS = 4, U = CHUNKS == 1 ? 4 : 2;
+    constexpr int WARPS = 4;
     const int64_t per_cta = static_cast<int64_t>(WARPS) * (32 / LANES) * U;
     const unsigned grid = static_cast<unsigned>((p.num_groups + per_cta - 1) / per_cta);
-    if (ue8m0) launch_dependent(group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, true, kDivideIeee>, grid, WARPS * 32, stream, p);
-    else if (division == kDivideFast) launch_dependent(group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, false, kDivideFast>, grid, WARPS * 32, stream, p);
-    else if (division == kMultiplyReciprocal) launch_dependent(group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, false, kMultiplyReciprocal>, grid, WARPS * 32, stream, p);
-    else launch_dependent(group_quant_fp8_kernel<WARPS, LANES, CHUNKS, U, false, kDivideIeee>, grid, WARPS * 32, stream, p);
+    const auto run = [&](auto* kernel) { launch_dependent(kernel, grid, WARPS * 32, stream, p); };
+    if (ue8m0) run(group_quant_fp8_kernel<WARPS, LANES, U, WIDE, true, kDivideIeee>);
+    else if (division == kDivideFast) run(group_quant_fp8_kernel<WARPS, LANES, U, WIDE, false, kDivideFast>);
+    else if (division == kMultiplyReciprocal) run(group_quant_fp8_kernel<WARPS, LANES, U, WIDE, false, kMultiplyReciprocal>);
+    else run(group_quant_fp8_kernel<WARPS, LANES, U, WIDE, false, kDivideIeee>);
+}
+
+// HBM-bound once a lane moves 32 bytes at a time: 32768 x 7168, groups of 128, 121 -> 102 us with power-of-two scales and
+// 132 -> 102 us with fp32 scales (7.0 TB/s, the 2-read-1-write ceiling of the probe) against 16-byte loads; 4097 x 7168 16.5 /
+// 18.1 -> 12.0 / 13.4 us.  Two groups in flight per lane group: one gives 119 us and four 103 us there.  Few groups want
+// as many warps as there are (1531 x 1536: 2.0 us with one, 2.3 with two; 4097 x 1536: 3.9 and 3.4 us).
+constexpr int64_t kFewGroups = 32768;
+
+template <int LANES>
+void launch_vector(const GroupQuantParams& p, bool wide, bool ue8m0, int division, cudaStream_t stream) {
+    if (!wide) launch_vector<LANES, 2, false>(p, ue8m0, division, stream);
+    else if (p.num_groups <= kFewGroups) launch_vector<LANES, 1, true>(p, ue8m0, division, stream);
+    else launch_vector<LANES, 2, true>(p, ue8m0, division, stream);
 }
 
 }  // namespace
@@ -152,18 +161,19 @@ cudaError_t launch_group_quant_fp8(const void* x, int64_t x_stride, void* out, f
     const auto addr = [](const void* q) { return reinterpret_cast<uintptr_t>(q); };
     const bool vec = addr(x) % 16 == 0 && x_stride % 8 == 0 && addr(out) % 8 == 0 &&
                      (group_size == 64 || group_size == 128 || group_size == 256 || group_size == 512);
+    const bool wide = addr(x) % 32 == 0 && x_stride % 16 == 0 && addr(out) % 16 == 0;
     const int division = act_quant_rules ? kMultiplyReciprocal : (eps == 1e-10f ? kDivideFast : kDivideIeee);
     if (!vec) {
         constexpr int WARPS = 4;
         launch_dependent(group_quant_fp8_scalar_kernel<WARPS>, static_cast<unsigned>((num_groups + WARPS - 1) / WARPS), WARPS * 32, stream, p, ue8m0, act_quant_rules);
     } else if (group_size == 64) {
-        launch_vector<8, 1>(p, ue8m0 != 0, division, stream);
+        launch_vector<4>(p, wide, ue8m0 != 0, division, stream);
     } else if (group_size == 128) {
-        launch_vector<16, 1>(p, ue8m0 != 0, division, stream);
+        launch_vector<8>(p, wide, ue8m0 != 0, division, stream);
     } else if (group_size == 256) {
-        launch_vector<32, 1>(p, ue8m0 != 0, division, stream);
+        launch_vector<16>(p, wide, ue8m0 != 0, division, stream);
     } else {
-        launch_vector<32, 2>(p, ue8m0 != 0, division, stream);
+        launch_vector<32>(p, wide, ue8m0 != 0, division, stream);
     }
     count_launch();
     return cudaGetLastError();
