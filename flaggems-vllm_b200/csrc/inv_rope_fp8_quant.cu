@@ -27,33 +27,32 @@ struct InvRopeParams {
     uint32_t hpg_mul, hpg_shift;      // fast division of a head index by heads_per_group
 };
 
+// A warp owns `heads_per_task` consecutive heads of one token and walks them U at a time.  Of a head, lane l < 28 holds the
+// un-rotated values [16l, 16l + 16) and every lane the 4-byte rotary pair 448+2l, 449+2l, so every lane rotates exactly one
+// pair with a cosine and sine it loaded once for the whole task.  The quantisation groups of 128 are the lanes 0-7, 8-15,
+// 16-23, and 24-27 together with all rotary pairs.
 // PACKED: power-of-two scales, the 4 UE8M0 bytes of a head packed into one int32.
-// A warp owns kHeadsPerTask consecutive heads of one token and walks them U at a time.  Rows are held in the
-// A/B/T layout (A: 16 B per lane, B: 16 B in lanes 0-23, T: the 4-byte rotary pair 448+2l, 449+2l of lane l), so
-// every lane rotates exactly one pair with a cosine and sine it loaded once for the whole task.  The four
-// quantisation groups of 128 are: A lanes 0-15, A lanes 16-31, B lanes 0-15, and B lanes 16-23 together with T.
-constexpr int kHeadsPerTask = 16;
-#ifndef DSV4_INVROPE_UE8M0_CTAS
-#define DSV4_INVROPE_UE8M0_CTAS 7  // CTAs per SM of the UE8M0-scale instantiation (72 registers with two passes in flight)
-#endif
-#ifndef DSV4_INVROPE_FP32_CTAS
-#define DSV4_INVROPE_FP32_CTAS 8  // CTAs per SM of the fp32-scale instantiation (64 registers with two passes in flight)
-#endif
-
 // FASTDIV (fp32-scale mode only): see ScaleDivider.
-// PREFETCH: two passes of U heads in flight - the loads of the next pass go out before the current one is worked on, so
-// a warp always has rows on their way while it computes (UE8M0 scales: 267 -> 256 us on 1 Mi rows; fp32 scales, once the
-// per-head address arithmetic was reduced to increments: 272 -> 269 us).
-template <int WARPS, bool PACKED, bool FASTDIV, int U, int MIN_CTAS, bool PREFETCH>
-__global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kernel(const InvRopeParams p, const uint32_t tasks_per_token,
+// WIDE: one 32-byte load and one 16-byte store per lane and head; otherwise (rows on 16-byte boundaries only) two of half the
+// size.
+// Two passes of U heads are in flight: the loads of the next pass go out before the current one is worked on (8192 x 128 rows:
+// 241 us, 253 us with one pass of four heads).
+// Bound by instruction issue before HBM in 16-byte pieces (253 us, fp32 scales 265 us); with 32-byte loads, 16-byte stores
+// and 6 shuffles a head 241 us = 6.7 TB/s and 247 us.  CTAs per SM: 6 247 us, 7 241 us, 8 306 us (spills).
+constexpr int kMainLanes = 28;
+constexpr int kHeadsInFlight = 2;  // per pass
+constexpr int kCtasPerSm = 7;      // 72 registers
+
+template <int WARPS, bool PACKED, bool FASTDIV, int U, int MIN_CTAS, bool WIDE>
+__global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kernel(const InvRopeParams p, const int heads_per_task, const uint32_t tasks_per_token,
                                                                       const uint32_t tpt_mul, const uint32_t tpt_shift) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const uint32_t task = blockIdx.x * WARPS + (threadIdx.x >> 5);
     if (task >= static_cast<uint32_t>(p.padded_tokens) * tasks_per_token) return;
     const uint32_t token = fast_div(task, tpt_mul, tpt_shift);
-    const int head_begin = static_cast<int>(task - token * tasks_per_token) * kHeadsPerTask;
-    const int head_end = head_begin + kHeadsPerTask < p.num_heads ? head_begin + kHeadsPerTask : p.num_heads;
+    const int head_begin = static_cast<int>(task - token * tasks_per_token) * heads_per_task;
+    const int head_end = head_begin + heads_per_task < p.num_heads ? head_begin + heads_per_task : p.num_heads;
     if (token >= p.num_tokens) {
         // token padding of the scale storage (a multiple of 4 tokens): zero scales
         for (int head = head_begin; head < head_end; ++head) {
@@ -68,39 +67,41 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kerne
         }
         return;
     }
-    const float* cs = p.cos_sin + p.positions[token] * p.cos_sin_stride;
-    const float c = cs[lane], sn = cs[32 + lane];
     const uint8_t* in_token = p.o + static_cast<int64_t>(token) * p.o_stride_token * 2;
-    uint4 a[U], b[U], a_next[U], b_next[U];
+    Bytes32 v[U], v_next[U];
     uint32_t tail[U], tail_next[U];
-    const auto load_pass = [&](int h0, uint4 (&ra)[U], uint4 (&rb)[U], uint32_t (&rt)[U]) {
+    const auto load_pass = [&](int h0, Bytes32 (&rv)[U], uint32_t (&rt)[U]) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            ra[u] = rb[u] = make_uint4(0u, 0u, 0u, 0u);
+            rv[u].lo = rv[u].hi = make_uint4(0u, 0u, 0u, 0u);
             rt[u] = 0u;
             if (h0 + u < head_end) {
                 const uint8_t* in = in_token + (h0 + u) * p.o_stride_head * 2;
-                ra[u] = ld_stream16(in + 16 * lane);
-                if (lane < kFirstRopeLane) rb[u] = ld_stream16(in + 512 + 16 * lane);
+                if (lane < kMainLanes) {
+                    if (WIDE) rv[u] = ld_stream32(in + 32 * lane);
+                    else rv[u].lo = ld_stream16(in + 32 * lane), rv[u].hi = ld_stream16(in + 32 * lane + 16);
+                }
                 rt[u] = ld_stream4(in + 2 * kNopeDim + 4 * lane);
             }
         }
     };
+    load_pass(head_begin, v, tail);
+    const float* cs = p.cos_sin + p.positions[token] * p.cos_sin_stride;
+    const float c = cs[lane], sn = cs[32 + lane];
     // Output addresses advance by constants from one head to the next and are recomputed only where a new group of heads
-    // begins: `out` = the head's 512 e4m3 bytes, `scale_at` = its first scale (this lane's half of the four in fp32 mode).
+    // begins: `out` = the head's 512 e4m3 bytes, `scale_at` = its scales (fp32: this lane group's of the four).
     int group = static_cast<int>(fast_div(static_cast<uint32_t>(head_begin), p.hpg_mul, p.hpg_shift));
     int head_in_group = head_begin - group * p.heads_per_group;
     const int64_t group_bytes = static_cast<int64_t>(p.heads_per_group) * (kRowBytes / 2);
     const int64_t scale_column = p.padded_tokens * 4;                       // bytes between scale columns of one token
     const int64_t scale_step = PACKED ? scale_column : 4 * scale_column;    // ... between consecutive heads
-    const int64_t lane_scale = PACKED ? 0 : (lane >> 4) * scale_column;     // fp32: lanes 0 / 16 store groups 0,2 / 1,3
+    const int64_t lane_scale = PACKED ? 0 : (lane >> 3) * scale_column;     // fp32: lanes 0 / 8 / 16 / 24 store one each
     const auto group_out = [&](int g) { return p.fp8 + (static_cast<int64_t>(g) * p.num_tokens + token) * group_bytes; };
     const auto group_scale = [&](int g) { return p.scale + (g * p.scale_stride_group + token) * 4 + lane_scale; };
     uint8_t* out = group_out(group) + static_cast<int64_t>(head_in_group) * (kRowBytes / 2);
     uint8_t* scale_at = group_scale(group) + head_in_group * scale_step;
-    load_pass(head_begin, a, b, tail);
     for (int h0 = head_begin; h0 < head_end; h0 += U) {
-        if (PREFETCH) load_pass(h0 + U, a_next, b_next, tail_next);  // past the last head of the task: nothing is loaded
+        load_pass(h0 + U, v_next, tail_next);  // past the last head of the task: nothing is loaded
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int head = h0 + u;
@@ -109,48 +110,45 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kerne
             const float e = bf16_lo(tail[u]), o = bf16_hi(tail[u]);
             const uint32_t rot = pack_bf16x2(__fadd_rn(__fmul_rn(e, c), __fmul_rn(o, sn)), __fsub_rn(__fmul_rn(o, c), __fmul_rn(e, sn)));
             const float te = bf16_lo(rot), to = bf16_hi(rot);
-            // Group maxima on the packed words: |.| maxima of the even and the odd elements side by side (the sign
-            // bits of the intermediate words are meaningless and cleared at the end).
-            const uint32_t pa = max_abs_bf16x2(max_abs_bf16x2(a[u].x, a[u].y), max_abs_bf16x2(a[u].z, a[u].w));
-            uint32_t pb = max_abs_bf16x2(max_abs_bf16x2(b[u].x, b[u].y), max_abs_bf16x2(b[u].z, b[u].w));
-            // Group 3 = B of lanes 16-23 and all of T: the upper half-warp folds its own pair and the pair of the
-            // lane 16 below into its B maximum, so that one packed reduction over 16 lanes serves all four groups.
-            const uint32_t rot_other = __shfl_xor_sync(0xffffffffu, rot, 16);
-            if (lane >= 16) pb = max_abs_bf16x2(max_abs_bf16x2(pb, rot), rot_other);
-            // (A even | B even) against (A odd | B odd): the A maximum in the low half, the B maximum in the high half
-            uint32_t both = max_abs_bf16x2(__byte_perm(pa, pb, 0x5410), __byte_perm(pa, pb, 0x7632)) & 0x7fff7fffu;
+            // Group maxima on the packed words: |.| maxima of the even and the odd elements side by side (the sign bits of
+            // the intermediate words are meaningless and cleared at the end), then the maximum of the lane's 16 values in
+            // the low half and that of its pair in the high half of one word.
+            const uint4 &a = v[u].lo, &b = v[u].hi;
+            const uint32_t pm = max_abs_bf16x2(max_abs_bf16x2(max_abs_bf16x2(a.x, a.y), max_abs_bf16x2(a.z, a.w)),
+                                               max_abs_bf16x2(max_abs_bf16x2(b.x, b.y), max_abs_bf16x2(b.z, b.w)));
+            uint32_t both = max_abs_bf16x2(__byte_perm(pm, rot, 0x5410), __byte_perm(pm, rot, 0x7632)) & 0x7fff7fffu;
 #pragma unroll
-            for (int m = 1; m <= 8; m <<= 1) both = max_bf16x2(both, __shfl_xor_sync(0xffffffffu, both, m));
-            const uint32_t both_other = __shfl_xor_sync(0xffffffffu, both, 16);
-            const float ma = bf16_lo(both), mb = bf16_hi(both);
-            const float m3 = lane >= 16 ? mb : bf16_hi(both_other);
-            const float sa = __fmul_rn(fmaxf(ma, p.eps), 1.0f / 448.0f), sb = __fmul_rn(fmaxf(mb, p.eps), 1.0f / 448.0f);
-            const float s3 = __fmul_rn(fmaxf(m3, p.eps), 1.0f / 448.0f);
+            for (int m = 1; m <= 4; m <<= 1) both = max_bf16x2(both, __shfl_xor_sync(0xffffffffu, both, m));
+            const uint32_t of_eight = both;  // low half: the group's maximum (without the pairs in lanes 24-31)
+#pragma unroll
+            for (int m = 8; m <= 16; m <<= 1) both = max_bf16x2(both, __shfl_xor_sync(0xffffffffu, both, m));
+            const float m3 = fmaxf(bf16_hi(both), bf16_lo(__shfl_sync(0xffffffffu, of_eight, 24)));
+            const float mm = lane >= 24 ? m3 : bf16_lo(of_eight);
+            const float sm = __fmul_rn(fmaxf(mm, p.eps), 1.0f / 448.0f), s3 = __fmul_rn(fmaxf(m3, p.eps), 1.0f / 448.0f);
+            uint2 qa, qb;
+            uint32_t qt;
             if (PACKED) {
-                const uint32_t code_a = pow2_ceil_code(sa), code_b = pow2_ceil_code(sb), code_3 = pow2_ceil_code(s3);
-                st_global8(out + 8 * lane, quant8_pow2(a[u], code_a));
-                if (lane < kFirstRopeLane) st_global8(out + 256 + 8 * lane, quant8_pow2(b[u], code_b));
+                const uint32_t code_m = pow2_ceil_code(sm), code_3 = pow2_ceil_code(s3);
+                qa = quant8_pow2(a, code_m), qb = quant8_pow2(b, code_m);
                 const float inv3 = __uint_as_float((254u - code_3) << 23);
-                *reinterpret_cast<uint16_t*>(out + kNopeDim + 2 * lane) =
-                    static_cast<uint16_t>(pack_e4m3x4(__fmul_rn(te, inv3), __fmul_rn(to, inv3), 0.f, 0.f));
-                // chunk k of the head in byte k: lane 0 holds the codes of groups 0 and 2, lane 16 those of 1 and 3
-                const uint32_t mine = code_a | (code_b << 16);
-                const uint32_t word = mine | (__shfl_xor_sync(0xffffffffu, mine, 16) << 8);
+                qt = pack_e4m3x4(__fmul_rn(te, inv3), __fmul_rn(to, inv3), 0.f, 0.f);
+                // chunk k of the head in byte k
+                const uint32_t word = __reduce_or_sync(0xffffffffu, code_m << (8 * (lane >> 3)));
                 if (lane == 0) *reinterpret_cast<uint32_t*>(scale_at) = word;
             } else {
-                // the three-instruction form of the fast division for every scale: measured here, a warp-uniform choice
-                // between it and the two-instruction form was no faster (296 us against 294 us on 1 Mi rows)
+                // the three-instruction form of the fast division for every scale: a warp-uniform choice between it and the
+                // two-instruction form was no faster
                 constexpr int kDivision = FASTDIV ? kDivideFast : kDivideIeee;
-                const ScaleDivider<kDivision> by_a(sa), by_b(sb), by_3(s3);
-                st_global8(out + 8 * lane, quant8_by<kDivision, false>(a[u], by_a));
-                if (lane < kFirstRopeLane) st_global8(out + 256 + 8 * lane, quant8_by<kDivision, false>(b[u], by_b));
-                *reinterpret_cast<uint16_t*>(out + kNopeDim + 2 * lane) = static_cast<uint16_t>(
-                    pack_e4m3x4(by_3.template quotient<false>(te), by_3.template quotient<false>(to), 0.f, 0.f));
-                if ((lane & 15) == 0) {
-                    *reinterpret_cast<float*>(scale_at) = sa;
-                    *reinterpret_cast<float*>(scale_at + 2 * scale_column) = sb;  // lane 16: sb is s3
-                }
+                const ScaleDivider<kDivision> by_m(sm), by_3(s3);
+                qa = quant8_by<kDivision, false>(a, by_m), qb = quant8_by<kDivision, false>(b, by_m);
+                qt = pack_e4m3x4(by_3.template quotient<false>(te), by_3.template quotient<false>(to), 0.f, 0.f);
+                if ((lane & 7) == 0) *reinterpret_cast<float*>(scale_at) = sm;
             }
+            if (lane < kMainLanes) {
+                if (WIDE) st_stream16(out + 16 * lane, make_uint4(qa.x, qa.y, qb.x, qb.y));
+                else st_global8(out + 16 * lane, qa), st_global8(out + 16 * lane + 8, qb);
+            }
+            *reinterpret_cast<uint16_t*>(out + kNopeDim + 2 * lane) = static_cast<uint16_t>(qt);
             // on to the next head
             out += kRowBytes / 2, scale_at += scale_step;
             if (++head_in_group == p.heads_per_group) {
@@ -158,12 +156,8 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kerne
                 out = group_out(group), scale_at = group_scale(group);
             }
         }
-        if (PREFETCH) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) a[u] = a_next[u], b[u] = b_next[u], tail[u] = tail_next[u];
-        } else {
-            load_pass(h0 + U, a, b, tail);
-        }
+        for (int u = 0; u < U; ++u) v[u] = v_next[u], tail[u] = tail_next[u];
     }
 }
 
@@ -274,7 +268,12 @@ cudaError_t launch_inv_rope_fp8_quant(const void* o, int64_t o_stride_token, int
     constexpr int WARPS = 4;
     const int64_t rows = padded_tokens * num_heads;
     if (rows == 0) return cudaSuccess;
-    const int64_t tasks_per_token = (num_heads + kHeadsPerTask - 1) / kHeadsPerTask;
+    // The longest task that still leaves about 4096 of them (the GPU holds 148 x 28 warps): its set-up is shared by more heads,
+    // and two passes are in flight.  61 x 128 rows: 3.7 us with 2 heads per task, 7.2 with 16; 256 x 128: 9.9 us with 8, 11.3 with
+    // 2 or 16; 4096 x 128: 123 us with 16, 162 with 2.
+    int heads_per_task = 2;
+    while (heads_per_task < 16 && rows >= 8192LL * heads_per_task) heads_per_task *= 2;
+    const int64_t tasks_per_token = (num_heads + heads_per_task - 1) / heads_per_task;
     const int64_t tasks = padded_tokens * tasks_per_token;
     const int64_t grid = (tasks + WARPS - 1) / WARPS;
     if (grid > 0x7fffffffLL || tasks >= (1LL << 31)) return cudaErrorInvalidConfiguration;
@@ -290,13 +289,13 @@ cudaError_t launch_inv_rope_fp8_quant(const void* o, int64_t o_stride_token, int
     make_fast_divisor(static_cast<uint32_t>(tasks_per_token), &tpt_mul, &tpt_shift);
     const unsigned g = static_cast<unsigned>(grid);
     const uint32_t tpt = static_cast<uint32_t>(tasks_per_token);
-    // Heads in flight per warp and CTAs per SM, measured on 1 Mi rows.  UE8M0 mode, two passes of 2 heads in flight: 7 CTAs
-    // (72 registers) 256 us, 8 CTAs (64 registers, 8 bytes spilled) 257 us, 6 CTAs 262 us; one pass in flight at 10 CTAs
-    // 265-282 us.  fp32-scale mode: two passes at 8 CTAs (64 registers) 269 us, at 7 CTAs 270 us; one pass at 10 CTAs
-    // (48 registers) 272 us, at 9 CTAs 274 us, at 11 CTAs 301 us.
-    if (packed) launch_dependent(inv_rope_fp8_quant_kernel<WARPS, true, false, 2, DSV4_INVROPE_UE8M0_CTAS, true>, g, WARPS * 32, stream, p, tpt, tpt_mul, tpt_shift);
-    else if (eps == 1e-10f) launch_dependent(inv_rope_fp8_quant_kernel<WARPS, false, true, 2, DSV4_INVROPE_FP32_CTAS, true>, g, WARPS * 32, stream, p, tpt, tpt_mul, tpt_shift);
-    else launch_dependent(inv_rope_fp8_quant_kernel<WARPS, false, false, 2, 8, false>, g, WARPS * 32, stream, p, tpt, tpt_mul, tpt_shift);
+    const auto addr = [](const void* q) { return reinterpret_cast<uintptr_t>(q); };
+    const bool wide = addr(o) % 32 == 0 && o_stride_token % 16 == 0 && o_stride_head % 16 == 0 && addr(fp8) % 16 == 0;
+    const auto run = [&](auto* kernel) { launch_dependent(kernel, g, WARPS * 32, stream, p, heads_per_task, tpt, tpt_mul, tpt_shift); };
+    constexpr int U = kHeadsInFlight, C = kCtasPerSm;
+    if (packed) wide ? run(inv_rope_fp8_quant_kernel<WARPS, true, false, U, C, true>) : run(inv_rope_fp8_quant_kernel<WARPS, true, false, U, C, false>);
+    else if (eps == 1e-10f) wide ? run(inv_rope_fp8_quant_kernel<WARPS, false, true, U, C, true>) : run(inv_rope_fp8_quant_kernel<WARPS, false, true, U, C, false>);
+    else wide ? run(inv_rope_fp8_quant_kernel<WARPS, false, false, U, C, true>) : run(inv_rope_fp8_quant_kernel<WARPS, false, false, U, C, false>);
     count_launch();
     return cudaGetLastError();
 }
