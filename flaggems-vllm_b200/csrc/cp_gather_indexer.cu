@@ -116,6 +116,45 @@ __global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_vec_kernel(const
     }
 }
 
+// The DeepSeek-V4 indexer shape (128 values, one scale) with 32-byte aligned rows: a warp owns 32 consecutive tokens.  It finds the
+// request of the first one together (few requests: a vote instead of a bisection, three dependent loads to the data instead
+// of about eight), every lane moves on from there to its own token, copies that token's scale, and four lanes copy the 128
+// bytes of a token with 32-byte accesses (16 sequences of up to 16384 tokens: 10.8 -> 9.7 us; 32 of up to 4096: 6.3 -> 4.1 us).
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_128_kernel(const CpGatherParams p) {
+    begin_dependent_kernel();
+    const int lane = threadIdx.x & 31;
+    const int32_t first = static_cast<int32_t>((static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5)) * 32);
+    if (first >= p.num_tokens) return;
+    const int32_t t = first + lane;
+    int32_t b = count_not_above(p.cu_seqlen, p.batch + 1, 0, first) - 1;
+    int32_t block = -1, in_block = 0;
+    if (t < p.num_tokens) {
+        while (b < p.batch && __ldg(p.cu_seqlen + b + 1) <= t) ++b;  // b + 1 <= batch
+        if (b >= 0 && b < p.batch) {
+            const int32_t off = t - __ldg(p.cu_seqlen + b);
+            const int32_t idx = p.bs_shift >= 0 ? off >> p.bs_shift : off / p.block_size;
+            in_block = off - idx * p.block_size;
+            block = __ldg(p.block_table + static_cast<int64_t>(b) * p.block_table_stride + idx);
+        }
+    }
+    const uint8_t* src[4];
+    Bytes32 v[4];
+    uint32_t scale = 0u;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int from = u * 8 + (lane >> 2);
+        const int32_t its_block = __shfl_sync(0xffffffffu, block, from), its_place = __shfl_sync(0xffffffffu, in_block, from);
+        src[u] = its_block < 0 ? nullptr : p.cache + its_block * p.block_stride + its_place * 128 + 32 * (lane & 3);
+        if (src[u]) v[u] = ld_stream32(src[u]);
+    }
+    if (block >= 0) scale = ld_stream4(p.cache + block * p.block_stride + p.block_size * 128 + in_block * 4);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (src[u]) st_stream32(p.k_out + static_cast<int64_t>(first + u * 8 + (lane >> 2)) * p.k_out_stride + 32 * (lane & 3), v[u]);
+    if (block >= 0) st_stream4(p.scale_out + static_cast<int64_t>(t) * p.scale_out_stride, scale);
+}
+
 // Any head_dim and any alignment: one warp per token, byte by byte.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_bytes_kernel(const CpGatherParams p) {
@@ -158,6 +197,9 @@ cudaError_t launch_cp_gather_indexer(const void* cache, int64_t block_stride, vo
         const int64_t grid = (num_tokens + WARPS - 1) / WARPS;
         if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
         launch_dependent(cp_gather_indexer_bytes_kernel<WARPS>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
+    } else if (head_dim == 128 && num_quant_blocks == 1 && batch <= 255 && block_size <= (1 << 20) && addr(cache) % 32 == 0 &&
+               block_stride % 32 == 0 && addr(k_out) % 32 == 0 && k_out_stride % 32 == 0) {
+        launch_dependent(cp_gather_indexer_128_kernel<WARPS>, static_cast<unsigned>((num_tokens + WARPS * 32 - 1) / (WARPS * 32)), WARPS * 32, stream, p);
     } else {
         constexpr int U = 4;
         const int chunks = head_dim / 16;

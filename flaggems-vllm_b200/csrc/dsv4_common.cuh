@@ -71,6 +71,19 @@ __device__ __forceinline__ uint32_t fast_div(uint32_t n, uint32_t mul, uint32_t 
     return static_cast<uint32_t>((static_cast<uint64_t>(n) * mul) >> shift);
 }
 
+// How many of the n non-decreasing entries of `list`, less `base`, are <= t.  Whole warps call it with the same arguments: one
+// coalesced load and one vote per 32 entries, where a bisection is a chain of dependent loads.
+__device__ __forceinline__ int32_t count_not_above(const int32_t* list, int32_t n, int32_t base, int32_t t) {
+    int32_t count = 0;
+    for (int32_t i = 0; i < n; i += 32) {
+        const int32_t at = i + static_cast<int32_t>(threadIdx.x & 31);
+        const uint32_t votes = __ballot_sync(0xffffffffu, at < n && __ldg(list + at) - base <= t);
+        count += __popc(votes);
+        if (votes != 0xffffffffu) break;
+    }
+    return count;
+}
+
 // slot -> (block, offset in block); block sizes are powers of two in practice (16, 64): shift and mask then,
 // a 64-bit division otherwise.  `shift` < 0 means "not a power of two".
 __device__ __forceinline__ void split_slot(int64_t slot, int64_t block_size, int shift, int64_t* block, int64_t* in_block) {
