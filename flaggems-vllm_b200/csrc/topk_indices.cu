@@ -41,39 +41,60 @@ __device__ __forceinline__ int32_t to_slot(const GlobalTopkParams& p, const int3
     return __ldg(table_row + block) * p.block_size + in_block;
 }
 
-// One warp per token.  VEC: rows are 16-byte aligned and topk is a multiple of 4, so a lane moves 4 entries at a time.
-template <int WARPS, bool VEC>
+// W consecutive int32 of a lane as one 32-byte (W = 8) or 16-byte (W = 4) access.
+template <int W>
+struct Entries {
+    int32_t v[W];
+    __device__ __forceinline__ void load(const int32_t* p) {
+        if constexpr (W == 8) {
+            const Bytes32 b = ld_stream32(p);
+            v[0] = b.lo.x, v[1] = b.lo.y, v[2] = b.lo.z, v[3] = b.lo.w, v[4] = b.hi.x, v[5] = b.hi.y, v[6] = b.hi.z, v[7] = b.hi.w;
+        } else {
+            const uint4 b = ld_stream16(p);
+            v[0] = b.x, v[1] = b.y, v[2] = b.z, v[3] = b.w;
+        }
+    }
+    __device__ __forceinline__ void store(int32_t* p) const {
+        const auto u = [&](int i) { return static_cast<uint32_t>(v[i]); };
+        if constexpr (W == 8) st_stream32(p, Bytes32{make_uint4(u(0), u(1), u(2), u(3)), make_uint4(u(4), u(5), u(6), u(7))});
+        else st_stream16(p, make_uint4(u(0), u(1), u(2), u(3)));
+    }
+};
+
+// One warp per token.  W: entries a lane moves at a time (rows aligned and topk a multiple of it), or 1.  Two accesses per lane are
+// in flight: 512 entries of a row in one pass where W is 8 (a decode batch of 61 rows 3.7 -> 3.1 us, bound by its three dependent
+// loads; 32768 x 2048: 86.8 -> 85.4 us, 6.3 TB/s).
+template <int WARPS, int W>
 __global__ void __launch_bounds__(WARPS * 32) global_topk_kernel(const GlobalTopkParams p) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (t >= p.num_tokens) return;
     const int32_t* table_row = p.block_table + static_cast<int64_t>(__ldg(p.token_to_req + t)) * p.block_table_stride;
+    const bool valid = p.is_valid == nullptr || __ldg(p.is_valid + t) != 0;
     const int32_t* in = p.local + t * p.local_stride;
     int32_t* out = p.global + t * p.global_stride;
     int32_t count = 0;
-    if (VEC) {
-        for (int c = 4 * lane; c < p.topk; c += 256) {
-            // two chunks of 4 in flight per lane
-            const bool second = c + 128 < p.topk;
-            const uint4 a = ld_stream16(in + c);
-            const uint4 b = second ? ld_stream16(in + c + 128) : make_uint4(0u, 0u, 0u, 0u);
-            uint4 ra, rb;
-            ra.x = to_slot(p, table_row, a.x, &count), ra.y = to_slot(p, table_row, a.y, &count);
-            ra.z = to_slot(p, table_row, a.z, &count), ra.w = to_slot(p, table_row, a.w, &count);
-            st_stream16(out + c, ra);
-            if (second) {
-                rb.x = to_slot(p, table_row, b.x, &count), rb.y = to_slot(p, table_row, b.y, &count);
-                rb.z = to_slot(p, table_row, b.z, &count), rb.w = to_slot(p, table_row, b.w, &count);
-                st_stream16(out + c + 128, rb);
+    if constexpr (W > 1) {
+        constexpr int U = 2;
+        for (int c = W * lane; c < p.topk; c += U * 32 * W) {
+            Entries<W> e[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c + u * 32 * W < p.topk) e[u].load(in + c + u * 32 * W);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (c + u * 32 * W >= p.topk) continue;
+#pragma unroll
+                for (int i = 0; i < W; ++i) e[u].v[i] = to_slot(p, table_row, e[u].v[i], &count);
+                e[u].store(out + c + u * 32 * W);
             }
         }
     } else {
         for (int c = lane; c < p.topk; c += 32) out[c] = to_slot(p, table_row, in[c], &count);
     }
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) count += __shfl_xor_sync(0xffffffffu, count, m);
-    if (lane == 0) p.lens[t] = (p.is_valid == nullptr || __ldg(p.is_valid + t) != 0) ? count : 0;
+    count = __reduce_add_sync(0xffffffffu, count);
+    if (lane == 0) p.lens[t] = valid ? count : 0;
 }
 
 struct CombineParams {
@@ -92,8 +113,10 @@ struct CombineParams {
     uint32_t cr_mul, cr_shift;
 };
 
-// One warp per query token.  VEC: rows 16-byte aligned and widths multiples of 4.
-template <int WARPS, bool VEC>
+// One warp per query token.  W as above; three accesses per lane in flight, so that a row of 512 + 128 entries is one pass where
+// W is 8.  Few requests: the token's is found by a vote instead of a bisection (1531 rows of 640: 3.2 -> 2.6 us,
+// 8192: 7.1 -> 5.7 us).
+template <int WARPS, int W>
 __global__ void __launch_bounds__(WARPS * 32) combine_topk_swa_kernel(const CombineParams p) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
@@ -101,14 +124,19 @@ __global__ void __launch_bounds__(WARPS * 32) combine_topk_swa_kernel(const Comb
     if (token >= p.num_tokens) return;
     // request of the token: the last b with query_start_loc[b] - query_start_loc[0] <= token
     const int32_t base = __ldg(p.query_start_loc);
-    int32_t left = 0, right = p.num_reqs + 1;
-    for (int32_t s = 0; s < p.search_steps; ++s) {
-        const int32_t mid = (left + right) >> 1;
-        const bool before = mid <= p.num_reqs && __ldg(p.query_start_loc + mid) - base <= token;
-        left = before ? mid + 1 : left;
-        right = before ? right : mid;
+    int32_t b;
+    if (p.num_reqs < 256) {
+        b = count_not_above(p.query_start_loc, p.num_reqs + 1, base, token) - 1;
+    } else {
+        int32_t left = 0, right = p.num_reqs + 1;
+        for (int32_t s = 0; s < p.search_steps; ++s) {
+            const int32_t mid = (left + right) >> 1;
+            const bool before = mid <= p.num_reqs && __ldg(p.query_start_loc + mid) - base <= token;
+            left = before ? mid + 1 : left;
+            right = before ? right : mid;
+        }
+        b = left - 1;
     }
-    const int32_t b = left - 1;
     if (b < 0 || b >= p.num_reqs) return;  // a row no request covers: not written, as in the reference
     const int32_t query_start = __ldg(p.query_start_loc + b) - base, query_end = __ldg(p.query_start_loc + b + 1) - base;
     if (token >= query_end) return;
@@ -130,13 +158,24 @@ __global__ void __launch_bounds__(WARPS * 32) combine_topk_swa_kernel(const Comb
     const auto entry = [&](int32_t c, int32_t loaded) -> int32_t {
         return c < topk_len ? loaded + shift : (c < valid_len ? swa_first + c : -1);
     };
-    if (VEC) {
-        for (int32_t c = 4 * lane; c < p.combined_width; c += 128) {
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (c < topk_len) v = ld_stream16(in + c);  // stays inside the row: c + 4 <= topk_width because topk_len <= topk_width
-            uint4 r;
-            r.x = entry(c, v.x), r.y = entry(c + 1, v.y), r.z = entry(c + 2, v.z), r.w = entry(c + 3, v.w);
-            st_stream16(out + c, r);
+    if constexpr (W > 1) {
+        constexpr int U = 3;
+        for (int32_t c = W * lane; c < p.combined_width; c += U * 32 * W) {
+            Entries<W> e[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int32_t at = c + u * 32 * W;
+                // stays inside the row: at + W <= topk_width because topk_len <= topk_width
+                if (at < topk_len) e[u].load(in + at);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int32_t at = c + u * 32 * W;
+                if (at >= p.combined_width) continue;
+#pragma unroll
+                for (int i = 0; i < W; ++i) e[u].v[i] = entry(at + i, e[u].v[i]);
+                e[u].store(out + at);
+            }
         }
     } else {
         for (int32_t c = lane; c < p.combined_width; c += 32) out[c] = entry(c, c < topk_len ? in[c] : 0);
@@ -160,9 +199,11 @@ cudaError_t launch_global_topk(const int32_t* local, int64_t local_stride, const
     const int64_t grid = (num_tokens + WARPS - 1) / WARPS;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const auto addr = [](const void* q) { return reinterpret_cast<uintptr_t>(q); };
-    const bool vec = topk % 4 == 0 && local_stride % 4 == 0 && global_stride % 4 == 0 && addr(local) % 16 == 0 && addr(global) % 16 == 0;
-    if (vec) launch_dependent(global_topk_kernel<WARPS, true>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
-    else launch_dependent(global_topk_kernel<WARPS, false>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
+    const auto rows_of = [&](unsigned w) { return topk % w == 0 && local_stride % w == 0 && global_stride % w == 0 && addr(local) % (4 * w) == 0 && addr(global) % (4 * w) == 0; };
+    const dim3 blocks(static_cast<unsigned>(grid));
+    if (rows_of(8)) launch_dependent(global_topk_kernel<WARPS, 8>, blocks, WARPS * 32, stream, p);
+    else if (rows_of(4)) launch_dependent(global_topk_kernel<WARPS, 4>, blocks, WARPS * 32, stream, p);
+    else launch_dependent(global_topk_kernel<WARPS, 1>, blocks, WARPS * 32, stream, p);
     count_launch();
     return cudaGetLastError();
 }
@@ -185,10 +226,14 @@ cudaError_t launch_combine_topk_swa(const int32_t* topk_indices, int64_t topk_st
     const int64_t grid = (num_tokens + WARPS - 1) / WARPS;
     if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     const auto addr = [](const void* q) { return reinterpret_cast<uintptr_t>(q); };
-    const bool vec = topk_width % 4 == 0 && combined_width % 4 == 0 && topk_stride % 4 == 0 && combined_stride % 4 == 0 &&
-                     addr(topk_indices) % 16 == 0 && addr(combined) % 16 == 0;
-    if (vec) launch_dependent(combine_topk_swa_kernel<WARPS, true>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
-    else launch_dependent(combine_topk_swa_kernel<WARPS, false>, static_cast<unsigned>(grid), WARPS * 32, stream, p);
+    const auto rows_of = [&](unsigned w) {
+        return topk_width % w == 0 && combined_width % w == 0 && topk_stride % w == 0 && combined_stride % w == 0 && addr(topk_indices) % (4 * w) == 0 &&
+               addr(combined) % (4 * w) == 0;
+    };
+    const dim3 blocks(static_cast<unsigned>(grid));
+    if (rows_of(8)) launch_dependent(combine_topk_swa_kernel<WARPS, 8>, blocks, WARPS * 32, stream, p);
+    else if (rows_of(4)) launch_dependent(combine_topk_swa_kernel<WARPS, 4>, blocks, WARPS * 32, stream, p);
+    else launch_dependent(combine_topk_swa_kernel<WARPS, 1>, blocks, WARPS * 32, stream, p);
     count_launch();
     return cudaGetLastError();
 }
