@@ -5,6 +5,8 @@
 // One warp per row; a row of up to 2048 elements stays in registers between the reduction and
 // the scaling (one read, one write per element); longer or unaligned rows take a two-pass
 // scalar path.  Row 2t is the q row of token t, row 2t+1 its kv row.
+#include <algorithm>
+
 #include <cuda_fp16.h>
 
 #include "dsv4_common.cuh"
@@ -18,10 +20,10 @@ struct NormRows {
     const uint8_t* weight;
     int64_t in_stride, out_stride;  // elements
     int32_t size;
-    int32_t vec_ok;                 // 16-byte path usable for this tensor
+    int32_t vec_ok;                 // vectorised path usable for this tensor
 };
 
-constexpr int kMaxChunks = 8;  // at most 8 16-byte chunks per lane are held in registers: 8 * 32 * 8 = 2048 elements
+constexpr int kMaxChunks = 4;  // at most 4 32-byte chunks per lane are held in registers: 4 * 32 * 16 = 2048 elements
 
 __device__ __forceinline__ float inv_rms_of(float sum, int size, float eps) {
     const float v = __fadd_rn(__fdiv_rn(sum, static_cast<float>(size)), eps);
@@ -29,10 +31,11 @@ __device__ __forceinline__ float inv_rms_of(float sum, int size, float eps) {
     return fmaf(r0, fmaf(-0.5f * v * r0, r0, 0.5f), r0);
 }
 
-// CH = chunks per lane the launch needs (2, 4, 6 or 8): fewer live registers for the common 1536 / 512 rows.
-template <int WARPS, int CH>
-__global__ void __launch_bounds__(WARPS * 32, CH <= 2 ? 16 : (CH <= 6 ? 8 : 6)) q_kv_rmsnorm_kernel(const NormRows q, const NormRows kv, int64_t num_tokens,
-                                                                 float eps) {
+// CH = 32-byte chunks per lane the launch needs (1 to 4): fewer live registers for the common 1536 / 512 rows.  WIDE: one 32-byte
+// access per chunk, otherwise (rows on 16-byte boundaries only) two.  EARLY: the weights are fetched before the reduction.
+template <int WARPS, int CH, bool WIDE, bool EARLY>
+__global__ void __launch_bounds__(WARPS * 32, EARLY ? 1 : CH == 1 ? 16 : CH == 2 ? 10 : CH == 3 ? 7 : 6)
+q_kv_rmsnorm_kernel(const NormRows q, const NormRows kv, int64_t num_tokens, float eps) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
@@ -44,35 +47,55 @@ __global__ void __launch_bounds__(WARPS * 32, CH <= 2 ? 16 : (CH <= 6 ? 8 : 6)) 
     uint8_t* out = t.out + token * t.out_stride * 2;
     const int size = t.size;
     if (t.vec_ok) {
-        const int chunks = size >> 3;
-        uint4 x[CH];
+        const int chunks = size >> 4;
+        Bytes32 x[CH], w[CH];
+        const auto load_weights = [&](int j) {
+            const int c = lane + 32 * j;
+            const uint4* from = reinterpret_cast<const uint4*>(t.weight + 32 * c);
+            w[j].lo = w[j].hi = make_uint4(0u, 0u, 0u, 0u);
+            if (c < chunks) w[j].lo = __ldg(from), w[j].hi = __ldg(from + 1);
+        };
         float acc = 0.0f;
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
             const int c = lane + 32 * j;
-            x[j] = make_uint4(0u, 0u, 0u, 0u);
-            if (c < chunks) x[j] = ld_stream16(in + 16 * c);
+            x[j].lo = x[j].hi = make_uint4(0u, 0u, 0u, 0u);
+            if (c < chunks) {
+                if (WIDE) x[j] = ld_stream32(in + 32 * c);
+                else x[j].lo = ld_stream16(in + 32 * c), x[j].hi = ld_stream16(in + 32 * c + 16);
+            }
+        }
+        if (EARLY) {
+#pragma unroll
+            for (int j = 0; j < CH; ++j) load_weights(j);
         }
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
-            float f[8];
-            unpack8(x[j], f);
+            float f[8], g[8];
+            unpack8(x[j].lo, f), unpack8(x[j].hi, g);
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc = fmaf(f[i], f[i], acc);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc = fmaf(g[i], g[i], acc);
         }
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
         const float rr = inv_rms_of(acc, size, eps);
+        const auto apply = [&](const uint4& xv, const uint4& wv) {
+            float f[8], g[8];
+            unpack8(xv, f), unpack8(wv, g);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = __fmul_rn(__fmul_rn(f[i], rr), g[i]);
+            return pack8(f);
+        };
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
             const int c = lane + 32 * j;
+            if (!EARLY) load_weights(j);
             if (c < chunks) {
-                float f[8], w[8];
-                unpack8(x[j], f);
-                unpack8(__ldg(reinterpret_cast<const uint4*>(t.weight + 16 * c)), w);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) f[i] = __fmul_rn(__fmul_rn(f[i], rr), w[i]);
-                st_stream16(out + 16 * c, pack8(f));
+                const Bytes32 y{apply(x[j].lo, w[j].lo), apply(x[j].hi, w[j].hi)};
+                if (WIDE) st_stream32(out + 32 * c, y);
+                else st_stream16(out + 32 * c, y.lo), st_stream16(out + 32 * c + 16, y.hi);
             }
         }
     } else {
@@ -140,10 +163,29 @@ __global__ void __launch_bounds__(WARPS * 32) q_kv_rmsnorm_any_kernel(const AnyR
         store_any(out, i, t.dtype, __fmul_rn(__fmul_rn(load_any(in, i, t.dtype), rr), load_any(t.weight, i, t.weight_dtype)));
 }
 
-bool vec_ok(const void* in, const void* out, const void* w, int64_t in_stride, int64_t out_stride, int64_t size) {
-    const auto a = [](const void* p) { return reinterpret_cast<uintptr_t>(p) & 15u; };
-    return a(in) == 0 && a(out) == 0 && a(w) == 0 && in_stride % 8 == 0 && out_stride % 8 == 0 && size % 8 == 0 &&
-           size <= kMaxChunks * 256;
+// Rows and weights on boundaries of `bytes` (16 or 32), 16 values per lane and chunk.
+bool on_boundaries(uintptr_t bytes, const NormRows& t) {
+    const auto off = [&](const void* p) { return reinterpret_cast<uintptr_t>(p) % bytes; };
+    const int64_t elements = static_cast<int64_t>(bytes / 2);
+    return off(t.in) == 0 && off(t.out) == 0 && reinterpret_cast<uintptr_t>(t.weight) % 16 == 0 && t.in_stride % elements == 0 &&
+           t.out_stride % elements == 0 && t.size % 16 == 0 && t.size <= kMaxChunks * 512;
+}
+
+// Up to here the weights are fetched before the reduction (90 registers for rows of 1536: the launch is over before occupancy
+// counts; 61 tokens 1.8 us against 2.4), above it afterwards (7 CTAs per SM: 65536 tokens 80 us = 6.7 TB/s against 91; with 16-byte
+// accesses 85.5).
+constexpr int64_t kEarlyWeightTokens = 4096;
+
+template <bool WIDE, bool EARLY>
+void launch_rows(const NormRows& q, const NormRows& kv, int64_t num_tokens, float eps, cudaStream_t stream) {
+    constexpr int WARPS = 4;
+    const dim3 grid(static_cast<unsigned>((2 * num_tokens + WARPS - 1) / WARPS));
+    const int32_t longest = std::max(q.vec_ok ? q.size : 0, kv.vec_ok ? kv.size : 0);
+    const auto run = [&](auto* kernel) { launch_dependent(kernel, grid, WARPS * 32, stream, q, kv, num_tokens, eps); };
+    if (longest <= 512) run(q_kv_rmsnorm_kernel<WARPS, 1, WIDE, EARLY>);
+    else if (longest <= 1024) run(q_kv_rmsnorm_kernel<WARPS, 2, WIDE, EARLY>);
+    else if (longest <= 1536) run(q_kv_rmsnorm_kernel<WARPS, 3, WIDE, EARLY>);
+    else run(q_kv_rmsnorm_kernel<WARPS, 4, WIDE, EARLY>);
 }
 
 }  // namespace
@@ -151,22 +193,17 @@ bool vec_ok(const void* in, const void* out, const void* w, int64_t in_stride, i
 cudaError_t launch_q_kv_rmsnorm(const void* q, void* q_out, const void* q_weight, int64_t q_in_stride, int64_t q_out_stride,
                                 int64_t q_size, const void* kv, void* kv_out, const void* kv_weight, int64_t kv_in_stride,
                                 int64_t kv_out_stride, int64_t kv_size, int64_t num_tokens, float eps, cudaStream_t stream) {
-    constexpr int WARPS = 4;
     if (num_tokens == 0) return cudaSuccess;
+    if ((2 * num_tokens + 3) / 4 > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
     NormRows a{static_cast<const uint8_t*>(q), static_cast<uint8_t*>(q_out), static_cast<const uint8_t*>(q_weight),
-               q_in_stride, q_out_stride, static_cast<int32_t>(q_size),
-               vec_ok(q, q_out, q_weight, q_in_stride, q_out_stride, q_size) ? 1 : 0};
+               q_in_stride, q_out_stride, static_cast<int32_t>(q_size), 0};
     NormRows b{static_cast<const uint8_t*>(kv), static_cast<uint8_t*>(kv_out), static_cast<const uint8_t*>(kv_weight),
-               kv_in_stride, kv_out_stride, static_cast<int32_t>(kv_size),
-               vec_ok(kv, kv_out, kv_weight, kv_in_stride, kv_out_stride, kv_size) ? 1 : 0};
-    const int64_t grid = (2 * num_tokens + WARPS - 1) / WARPS;
-    if (grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    const int64_t longest = (a.vec_ok ? q_size : 0) > (b.vec_ok ? kv_size : 0) ? (a.vec_ok ? q_size : 0) : (b.vec_ok ? kv_size : 0);
-    const unsigned g = static_cast<unsigned>(grid);
-    if (longest <= 512) launch_dependent(q_kv_rmsnorm_kernel<WARPS, 2>, g, WARPS * 32, stream, a, b, num_tokens, eps);
-    else if (longest <= 1024) launch_dependent(q_kv_rmsnorm_kernel<WARPS, 4>, g, WARPS * 32, stream, a, b, num_tokens, eps);
-    else if (longest <= 1536) launch_dependent(q_kv_rmsnorm_kernel<WARPS, 6>, g, WARPS * 32, stream, a, b, num_tokens, eps);
-    else launch_dependent(q_kv_rmsnorm_kernel<WARPS, 8>, g, WARPS * 32, stream, a, b, num_tokens, eps);
+               kv_in_stride, kv_out_stride, static_cast<int32_t>(kv_size), 0};
+    a.vec_ok = on_boundaries(16, a) ? 1 : 0, b.vec_ok = on_boundaries(16, b) ? 1 : 0;
+    const bool wide = (!a.vec_ok || on_boundaries(32, a)) && (!b.vec_ok || on_boundaries(32, b));
+    if (!wide) launch_rows<false, false>(a, b, num_tokens, eps, stream);
+    else if (num_tokens <= kEarlyWeightTokens) launch_rows<true, true>(a, b, num_tokens, eps, stream);
+    else launch_rows<true, false>(a, b, num_tokens, eps, stream);
     count_launch();
     return cudaGetLastError();
 }
