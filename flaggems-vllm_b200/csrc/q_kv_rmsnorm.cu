@@ -47,13 +47,17 @@ q_kv_rmsnorm_kernel(const NormRows q, const NormRows kv, int64_t num_tokens, flo
     uint8_t* out = t.out + token * t.out_stride * 2;
     const int size = t.size;
     if (t.vec_ok) {
-        const int chunks = size >> 4;
+        const int chunks = (size + 15) >> 4;
+        const int half = WIDE ? -1 : (size & 8 ? chunks - 1 : -1);  // the chunk whose second 8 values lie outside the row
         Bytes32 x[CH], w[CH];
         const auto load_weights = [&](int j) {
             const int c = lane + 32 * j;
             const uint4* from = reinterpret_cast<const uint4*>(t.weight + 32 * c);
             w[j].lo = w[j].hi = make_uint4(0u, 0u, 0u, 0u);
-            if (c < chunks) w[j].lo = __ldg(from), w[j].hi = __ldg(from + 1);
+            if (c < chunks) {
+                w[j].lo = __ldg(from);
+                if (c != half) w[j].hi = __ldg(from + 1);
+            }
         };
         float acc = 0.0f;
 #pragma unroll
@@ -62,7 +66,8 @@ q_kv_rmsnorm_kernel(const NormRows q, const NormRows kv, int64_t num_tokens, flo
             x[j].lo = x[j].hi = make_uint4(0u, 0u, 0u, 0u);
             if (c < chunks) {
                 if (WIDE) x[j] = ld_stream32(in + 32 * c);
-                else x[j].lo = ld_stream16(in + 32 * c), x[j].hi = ld_stream16(in + 32 * c + 16);
+                else x[j].lo = ld_stream16(in + 32 * c);
+                if (!WIDE && c != half) x[j].hi = ld_stream16(in + 32 * c + 16);
             }
         }
         if (EARLY) {
@@ -95,7 +100,8 @@ q_kv_rmsnorm_kernel(const NormRows q, const NormRows kv, int64_t num_tokens, flo
             if (c < chunks) {
                 const Bytes32 y{apply(x[j].lo, w[j].lo), apply(x[j].hi, w[j].hi)};
                 if (WIDE) st_stream32(out + 32 * c, y);
-                else st_stream16(out + 32 * c, y.lo), st_stream16(out + 32 * c + 16, y.hi);
+                else st_stream16(out + 32 * c, y.lo);
+                if (!WIDE && c != half) st_stream16(out + 32 * c + 16, y.hi);
             }
         }
     } else {
@@ -168,7 +174,7 @@ bool on_boundaries(uintptr_t bytes, const NormRows& t) {
     const auto off = [&](const void* p) { return reinterpret_cast<uintptr_t>(p) % bytes; };
     const int64_t elements = static_cast<int64_t>(bytes / 2);
     return off(t.in) == 0 && off(t.out) == 0 && reinterpret_cast<uintptr_t>(t.weight) % 16 == 0 && t.in_stride % elements == 0 &&
-           t.out_stride % elements == 0 && t.size % 16 == 0 && t.size <= kMaxChunks * 512;
+           t.out_stride % elements == 0 && t.size % elements == 0 && t.size <= kMaxChunks * 512;
 }
 
 // Up to here the weights are fetched before the reduction (90 registers for rows of 1536: the launch is over before occupancy

@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("q_size,kv_size", [(16, 512), (512, 512), (528, 16), (1024, 500), (1536, 512), (1552, 512), (2048, 1536), (2064, 512)])
+@pytest.mark.parametrize("q_size,kv_size", [(16, 512), (512, 512), (528, 16), (1024, 500), (1000, 504), (8, 1544), (1536, 512), (1552, 512), (2048, 1536), (2064, 512)])
 @pytest.mark.parametrize("offset", [0, 8])  # rows on 32-byte and on 16-byte boundaries
 @pytest.mark.parametrize("tokens", [1, 5, 4099])
 def test_row_sizes(q_size, kv_size, offset, tokens):
