@@ -179,7 +179,13 @@ __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     return v;
 }
 
-// The same for 32 bytes (p 32-byte aligned): one instruction, 1 KiB per warp.
+// Fetches `bytes` (a multiple of 16) from p (16-byte aligned) into L2, one instruction by one thread: the loads that follow then
+// wait for L2 instead of HBM, without registers holding what is in flight.
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// ld_stream16 / st_stream16 for 32 bytes (p 32-byte aligned): one instruction, 1 KiB per warp.
 struct Bytes32 {
     uint4 lo, hi;
 };

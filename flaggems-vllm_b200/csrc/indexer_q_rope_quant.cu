@@ -35,13 +35,16 @@ struct IndexerQParams {
     int32_t scales_word_aligned;  // fp4: every head's group of scale bytes starts on a 4-byte boundary
 };
 
-__device__ __forceinline__ float load_weight(const uint8_t* base, int64_t idx, int dtype) {
-    if (dtype == 2) return reinterpret_cast<const float*>(base)[idx];
-    const uint16_t h = reinterpret_cast<const uint16_t*>(base)[idx];
-    if (dtype == 0) return bf16_lo(h);
+__device__ __forceinline__ float weight_value(uint32_t bits, int dtype) {
+    if (dtype == 2) return __uint_as_float(bits);
+    if (dtype == 0) return bf16_lo(bits);
     float f;
-    asm("{.reg .f16 t; mov.b16 t, %1; cvt.f32.f16 %0, t;}" : "=f"(f) : "h"(h));
+    asm("{.reg .f16 t; mov.b16 t, %1; cvt.f32.f16 %0, t;}" : "=f"(f) : "h"(static_cast<uint16_t>(bits)));
     return f;
+}
+
+__device__ __forceinline__ float load_weight(const uint8_t* base, int64_t idx, int dtype) {
+    return weight_value(dtype == 2 ? reinterpret_cast<const uint32_t*>(base)[idx] : reinterpret_cast<const uint16_t*>(base)[idx], dtype);
 }
 
 // UE8M0 byte of an MXFP4 block whose absolute maximum is `amax`: ceil(log2(max(amax, 6*2^-126) / 6)) + 127 clamped to
@@ -275,127 +278,126 @@ cudaError_t launch_rows(const IndexerQParams& p, bool fp4, int64_t rows, int cs_
     return cudaGetLastError();
 }
 
-// Large batches of the DeepSeek-V4 geometry (head_dim 128 = 64 un-rotated + 64 rotary): one warp per TOKEN.
-// A head is 8 lanes; lane s keeps un-rotated values [8s, 8s+8) and rotary values [64+8s, 64+8s+8) (four pairs), so
-// every lane rotates (no divergence), the lane's four cosines and sines are loaded once per token and reused for
-// every head, and pointers advance by constants from one group of four heads to the next.  MXFP4 blocks of 32 are
-// 4 lanes.
-template <int WARPS, bool FP4>
-__global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_token_kernel(const IndexerQParams p) {
+// The DeepSeek-V4 geometry (head_dim 128 = 64 un-rotated + 64 rotary): a warp owns `heads_per_task` consecutive heads of one token,
+// eight at a time.  A head is 4 lanes; lane s keeps the un-rotated values [16s, 16s+16) and the rotary values [64+16s, 64+16s+16)
+// (eight pairs), so every lane rotates (no divergence) and its eight cosines and sines are loaded once per task.  MXFP4 blocks of
+// 32 are 2 lanes.  WIDE: 32-byte loads, otherwise (rows on 16-byte boundaries only) two of half the size.  Two passes are in
+// flight: the loads of the next one go out before the current one is worked on.  PREFETCH: one instruction sends the rest of the
+// task's rows to L2 at its start (6 CTAs per SM; without it 7).
+// Bound by instruction issue (0.7 per cycle; rotation, conversions) and DRAM together; the rotation on packed f32x2 instructions was
+// faster by 2 % and not bit for bit the same, an even split of the passes over resident warps no faster.
+template <int WARPS, bool FP4, bool WIDE, bool PREFETCH>
+__global__ void __launch_bounds__(WARPS * 32, PREFETCH ? 6 : 7) indexer_q_rope_quant_heads_kernel(const IndexerQParams p, const int heads_per_task, const uint32_t tasks_per_token,
+                                                                                const uint32_t tpt_mul, const uint32_t tpt_shift) {
     begin_dependent_kernel();
-    const int lane = threadIdx.x & 31, sub = lane & 7, which = lane >> 3;
-    const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31, sub = lane & 3, which = lane >> 2;
+    const uint32_t task = blockIdx.x * WARPS + (threadIdx.x >> 5);
+    const int64_t t = fast_div(task, tpt_mul, tpt_shift);
     if (t >= p.num_tokens) return;
-    const int64_t pos = p.positions[t];
-    float c[4], sn[4];
-    if (p.cos_sin_bf16) {
-        const uint16_t* cs = reinterpret_cast<const uint16_t*>(p.cos_sin) + pos * p.cos_sin_stride + 4 * sub;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) c[j] = bf16_lo(cs[j]), sn[j] = bf16_lo(cs[32 + j]);
-    } else {
-        const float* cs = reinterpret_cast<const float*>(p.cos_sin) + pos * p.cos_sin_stride + 4 * sub;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) c[j] = cs[j], sn[j] = cs[32 + j];
-    }
-    const uint8_t* q_tok = p.q + t * p.q_stride0 * 2 + 16 * sub;
-    uint8_t* out_tok = p.out + t * p.out_stride0;
-#ifndef DSV4_INDEXER_Q_U
-#define DSV4_INDEXER_Q_U 2
-#endif
-    constexpr int U = DSV4_INDEXER_Q_U;  // groups of four heads per pass
-    // Two passes are in flight: the loads of the next pass go out before the current one is worked on, so a warp
-    // always has rows on their way while it computes.
-    uint4 nope[U], rope[U], nope_next[U], rope_next[U];
-    const auto load_pass = [&](int h0, uint4 (&n)[U], uint4 (&r)[U]) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int h = h0 + 4 * u + which;
-            n[u] = r[u] = make_uint4(0u, 0u, 0u, 0u);
-            if (h < p.num_heads) {
-                const uint8_t* row = q_tok + h * p.q_stride1 * 2;
-                n[u] = ld_stream16(row);
-                r[u] = ld_stream16(row + 128);
-            }
-        }
+    const int head_begin = static_cast<int>(task - static_cast<uint32_t>(t) * tasks_per_token) * heads_per_task;
+    const int head_end = head_begin + heads_per_task < p.num_heads ? head_begin + heads_per_task : p.num_heads;
+    const int64_t head_bytes = p.q_stride1 * 2;
+    const uint8_t* row = p.q + t * p.q_stride0 * 2 + (head_begin + which) * head_bytes + 32 * sub;
+    const auto load32 = [](const uint8_t* from) {
+        if (WIDE) return ld_stream32(from);
+        Bytes32 v;
+        v.lo = ld_stream16(from), v.hi = ld_stream16(from + 16);
+        return v;
     };
-    load_pass(0, nope, rope);
-    for (int h0 = 0; h0 < p.num_heads; h0 += 4 * U) {
-        load_pass(h0 + 4 * U, nope_next, rope_next);  // past the last head: zeros, nothing is loaded
+    Bytes32 nope, rope, nope_next, rope_next;
+    nope.lo = nope.hi = rope.lo = rope.hi = make_uint4(0u, 0u, 0u, 0u);
+    nope_next = nope, rope_next = rope;
+    // The head's weight travels with its row: fetched in the pass that uses it, its latency would show in every pass (its bits
+    // only: a conversion would wait for them).
+    const auto weight_of = [&](int h) -> uint32_t {
+        const int64_t at = t * p.weights_stride + h;
+        if (sub != 0) return 0u;
+        return p.weights_dtype == 2 ? __ldg(reinterpret_cast<const uint32_t*>(p.weights) + at) : __ldg(reinterpret_cast<const uint16_t*>(p.weights) + at);
+    };
+    uint32_t weight_bits = 0u, weight_next = 0u;
+    if (head_begin + which < head_end) nope = load32(row), rope = load32(row + 128), weight_bits = weight_of(head_begin + which);
+    if (PREFETCH && lane == 0 && head_bytes == 256 && head_end > head_begin + 16)
+        prefetch_l2(p.q + t * p.q_stride0 * 2 + (head_begin + 16) * 256, static_cast<uint32_t>(head_end - head_begin - 16) * 256u);
+    const int64_t pos = p.positions[t];
+    float c[8], sn[8];
+    if (p.cos_sin_bf16) {
+        const uint16_t* cs = reinterpret_cast<const uint16_t*>(p.cos_sin) + pos * p.cos_sin_stride + 8 * sub;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int h = h0 + 4 * u + which;
-            const bool live = h < p.num_heads;
-            float y[8];
-            unpack8(rope[u], y);
-            uint32_t rot[4];  // the rotated pairs, rounded to bf16 as the reference does before quantising
+        for (int j = 0; j < 8; ++j) c[j] = bf16_lo(cs[j]), sn[j] = bf16_lo(cs[32 + j]);
+    } else {
+        const float* cs = reinterpret_cast<const float*>(p.cos_sin) + pos * p.cos_sin_stride + 8 * sub;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float e = y[2 * j], o = y[2 * j + 1];
-                // separately rounded products
-                rot[j] = pack_bf16x2(__fsub_rn(__fmul_rn(e, c[j]), __fmul_rn(o, sn[j])),
-                                     __fadd_rn(__fmul_rn(o, c[j]), __fmul_rn(e, sn[j])));
-            }
-            uint8_t* out = out_tok + h * p.out_stride1;
-            float weight_factor = 1.0f;
-            if (FP4) {
-                // everything on the packed words: |.| maxima of the un-rotated half (low 16 bits of `both`) and of the
-                // rotated half (high 16 bits) reduced together over the 4 lanes of a block of 32
-                const uint32_t plain[4] = {nope[u].x, nope[u].y, nope[u].z, nope[u].w};
-                const uint32_t pn = max_abs_bf16x2(max_abs_bf16x2(plain[0], plain[1]), max_abs_bf16x2(plain[2], plain[3]));
-                const uint32_t pr = max_abs_bf16x2(max_abs_bf16x2(rot[0], rot[1]), max_abs_bf16x2(rot[2], rot[3]));
-                uint32_t both = max_abs_bf16x2(__byte_perm(pn, pr, 0x5410), __byte_perm(pn, pr, 0x7632)) & 0x7fff7fffu;
+        for (int j = 0; j < 8; ++j) c[j] = __ldg(cs + j), sn[j] = __ldg(cs + 32 + j);
+    }
+    uint8_t* out = p.out + t * p.out_stride0 + (head_begin + which) * p.out_stride1;
+    for (int h = head_begin + which; h - which < head_end; h += 8) {
+        const bool live = h < head_end;
+        row += 8 * head_bytes;
+        if (h + 8 < head_end) nope_next = load32(row), rope_next = load32(row + 128), weight_next = weight_of(h + 8);
+        float weight_factor = 1.0f;
+        uint32_t rot[8];  // the rotated pairs, rounded to bf16 as the reference does before quantising
+        const uint32_t raw[8] = {rope.lo.x, rope.lo.y, rope.lo.z, rope.lo.w, rope.hi.x, rope.hi.y, rope.hi.z, rope.hi.w};
 #pragma unroll
-                for (int m = 1; m < 4; m <<= 1) both = max_bf16x2(both, __shfl_xor_sync(0xffffffffu, both, m));
-                const uint32_t code_n = mxfp4_code(bf16_lo(both)), code_r = mxfp4_code(bf16_hi(both));
-                uint32_t wn[4], wr[4];
-                scale_pow2_bf16x2(plain, code_n, wn);
-                scale_pow2_bf16x2(rot, code_r, wr);
-                const uint32_t bn = pack_e2m1x8(wn), br = pack_e2m1x8(wr);
-                // the head's four scale bytes in one word: blocks (un-rotated 0-31, 32-63, rotated 0-31, 32-63)
-                const uint32_t mine = code_n | (code_r << 16);
-                const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 4);
-                if (live) {
-                    *reinterpret_cast<uint32_t*>(out + 4 * sub) = bn;
-                    *reinterpret_cast<uint32_t*>(out + 32 + 4 * sub) = br;
-                    if (sub == 0) {
-                        uint8_t* sc = p.scales + t * p.scale_stride0 + h * p.scale_stride1;
-                        const uint32_t word = (mine & 0xffu) | ((other & 0xffu) << 8) | (mine & 0xff0000u) | ((other & 0xff0000u) << 8);
-                        if (p.scales_word_aligned) {
-                            *reinterpret_cast<uint32_t*>(sc) = word;
-                        } else {
-                            sc[0] = static_cast<uint8_t>(word), sc[1] = static_cast<uint8_t>(word >> 8);
-                            sc[2] = static_cast<uint8_t>(word >> 16), sc[3] = static_cast<uint8_t>(word >> 24);
-                        }
+        for (int j = 0; j < 8; ++j) {
+            const float e = bf16_lo(raw[j]), o = bf16_hi(raw[j]);
+            // separately rounded products
+            rot[j] = pack_bf16x2(__fsub_rn(__fmul_rn(e, c[j]), __fmul_rn(o, sn[j])), __fadd_rn(__fmul_rn(o, c[j]), __fmul_rn(e, sn[j])));
+        }
+        const uint4 ra = make_uint4(rot[0], rot[1], rot[2], rot[3]), rb = make_uint4(rot[4], rot[5], rot[6], rot[7]);
+        // |.| maxima on the packed words: of the un-rotated values in `pn`, of the rotated ones in `pr`
+        const auto max16 = [](const uint4& a, const uint4& b) {
+            return max_abs_bf16x2(max_abs_bf16x2(max_abs_bf16x2(a.x, a.y), max_abs_bf16x2(a.z, a.w)),
+                                  max_abs_bf16x2(max_abs_bf16x2(b.x, b.y), max_abs_bf16x2(b.z, b.w)));
+        };
+        const uint32_t pn = max16(nope.lo, nope.hi), pr = max16(ra, rb);
+        if (FP4) {
+            // the two maxima side by side in one word, reduced over the 2 lanes of a block
+            uint32_t both = max_abs_bf16x2(__byte_perm(pn, pr, 0x5410), __byte_perm(pn, pr, 0x7632)) & 0x7fff7fffu;
+            both = max_bf16x2(both, __shfl_xor_sync(0xffffffffu, both, 1));
+            const uint32_t code_n = mxfp4_code(bf16_lo(both)), code_r = mxfp4_code(bf16_hi(both));
+            const auto pack = [](const uint4& v, uint32_t code) {
+                const uint32_t in[4] = {v.x, v.y, v.z, v.w};
+                uint32_t w[4];
+                scale_pow2_bf16x2(in, code, w);
+                return pack_e2m1x8(w);
+            };
+            const uint2 bn = make_uint2(pack(nope.lo, code_n), pack(nope.hi, code_n)), br = make_uint2(pack(ra, code_r), pack(rb, code_r));
+            // the head's four scale bytes in one word: blocks (un-rotated 0-31, 32-63, rotated 0-31, 32-63)
+            const uint32_t mine = code_n | (code_r << 16);
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 2);
+            if (live) {
+                st_global8(out + 8 * sub, bn);
+                st_global8(out + 32 + 8 * sub, br);
+                if (sub == 0) {
+                    uint8_t* sc = p.scales + t * p.scale_stride0 + h * p.scale_stride1;
+                    const uint32_t word = mine | (other << 8);
+                    if (p.scales_word_aligned) {
+                        *reinterpret_cast<uint32_t*>(sc) = word;
+                    } else {
+                        sc[0] = static_cast<uint8_t>(word), sc[1] = static_cast<uint8_t>(word >> 8);
+                        sc[2] = static_cast<uint8_t>(word >> 16), sc[3] = static_cast<uint8_t>(word >> 24);
                     }
                 }
-            } else {
-                float x[8];
-                unpack8(nope[u], x);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) y[2 * j] = bf16_lo(rot[j]), y[2 * j + 1] = bf16_hi(rot[j]);
-                float amax = 0.0f;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fmaxf(fabsf(x[i]), fabsf(y[i])));
-#pragma unroll
-                for (int m = 1; m < 8; m <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
-                const uint32_t code = ue8m0_code(amax);
-                const float inv = __uint_as_float((254u - code) << 23);
-                weight_factor = __uint_as_float(code << 23);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) x[i] = __fmul_rn(x[i], inv), y[i] = __fmul_rn(y[i], inv);
-                if (live) {
-                    st_global8(out + 8 * sub, make_uint2(pack_e4m3x4(x[0], x[1], x[2], x[3]), pack_e4m3x4(x[4], x[5], x[6], x[7])));
-                    st_global8(out + 64 + 8 * sub, make_uint2(pack_e4m3x4(y[0], y[1], y[2], y[3]), pack_e4m3x4(y[4], y[5], y[6], y[7])));
-                }
             }
-            if (live && sub == 0) {
-                float w = load_weight(p.weights, t * p.weights_stride + h, p.weights_dtype);
-                if (!FP4) w = __fmul_rn(w, weight_factor);
-                p.weights_out[t * p.weights_out_stride + h] = __fmul_rn(__fmul_rn(w, p.softmax_scale), p.head_scale);
+        } else {
+            uint32_t pk = max_abs_bf16x2(pn, pr) & 0x7fff7fffu;
+            pk = max_bf16x2(pk, __shfl_xor_sync(0xffffffffu, pk, 1));
+            pk = max_bf16x2(pk, __shfl_xor_sync(0xffffffffu, pk, 2));
+            const uint32_t code = ue8m0_code(fmaxf(bf16_lo(pk), bf16_hi(pk)));
+            weight_factor = __uint_as_float(code << 23);
+            const uint2 n0 = quant8_pow2(nope.lo, code), n1 = quant8_pow2(nope.hi, code), r0 = quant8_pow2(ra, code), r1 = quant8_pow2(rb, code);
+            if (live) {
+                st_stream16(out + 16 * sub, make_uint4(n0.x, n0.y, n1.x, n1.y));
+                st_stream16(out + 64 + 16 * sub, make_uint4(r0.x, r0.y, r1.x, r1.y));
             }
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) nope[u] = nope_next[u], rope[u] = rope_next[u];
+        if (live && sub == 0) {
+            float w = weight_value(weight_bits, p.weights_dtype);
+            if (!FP4) w = __fmul_rn(w, weight_factor);
+            p.weights_out[t * p.weights_out_stride + h] = __fmul_rn(__fmul_rn(w, p.softmax_scale), p.head_scale);
+        }
+        out += 8 * p.out_stride1;
+        nope = nope_next, rope = rope_next, weight_bits = weight_next;
     }
 }
 
@@ -432,15 +434,25 @@ cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q,
     const int nope = head_dim - rot_dim;
     const bool rows_shape = nope % 8 == 0 && rot_dim % 8 == 0 && addr(q) % 16 == 0 && q_stride0 % 8 == 0 && q_stride1 % 8 == 0 &&
                             addr(out) % 8 == 0 && out_stride0 % 8 == 0 && out_stride1 % 8 == 0;
-    // one warp per token pays off once there are enough tokens to fill the GPU with warps
-    const bool token_shape = head_dim == 128 && rot_dim == 64 && num_tokens >= 8192 && addr(q) % 16 == 0 && q_stride0 % 8 == 0 &&
-                             q_stride1 % 8 == 0 && addr(out) % 8 == 0 && out_stride0 % 8 == 0 && out_stride1 % 8 == 0 &&
-                             (cos_sin_bf16 || addr(cos_sin) % 4 == 0);
-    if (token_shape) {
+    const bool heads_shape = head_dim == 128 && rot_dim == 64 && rows_shape &&
+                             (fp4 || (addr(out) % 16 == 0 && out_stride0 % 16 == 0 && out_stride1 % 16 == 0));
+    if (heads_shape) {
         constexpr int WARPS = 4;
-        const unsigned grid = static_cast<unsigned>((num_tokens + WARPS - 1) / WARPS);
-        if (fp4) launch_dependent(indexer_q_rope_quant_token_kernel<WARPS, true>, grid, WARPS * 32, stream, p);
-        else launch_dependent(indexer_q_rope_quant_token_kernel<WARPS, false>, grid, WARPS * 32, stream, p);
+        // Heads per warp: few rows, short tasks, so that there are enough of them (61 tokens x 64 heads: 2.0 us with 8, 3.6 with 32);
+        // from 65536 rows on 16 (1531 tokens: 6.9 us; 12.6 on the rows kernel), from 196608 on 64 (4096 tokens: 17.7 us; 29).  The
+        // largest batches take 32 and the prefetch: 16384 tokens 71.6 -> 65.2 us (FP8) and 64.9 -> 62.3 us (MXFP4), 65536 tokens
+        // 262 -> 239 us and 242 -> 227 us; 8192 tokens are as fast with 64 (35.3 / 33.6 us) as the one-warp-per-token form was.
+        const bool prefetch = rows >= 786432;
+        const int heads_per_task = prefetch ? 32 : rows >= 196608 ? 64 : rows >= 65536 ? 16 : 8;
+        const int64_t tasks_per_token = (num_heads + heads_per_task - 1) / heads_per_task;
+        const dim3 grid(static_cast<unsigned>((num_tokens * tasks_per_token + WARPS - 1) / WARPS));
+        uint32_t mul, shift;
+        make_fast_divisor(static_cast<uint32_t>(tasks_per_token), &mul, &shift);
+        const bool wide = addr(q) % 32 == 0 && q_stride0 % 16 == 0 && q_stride1 % 16 == 0;
+        const auto run = [&](auto* kernel) { launch_dependent(kernel, grid, WARPS * 32, stream, p, heads_per_task, static_cast<uint32_t>(tasks_per_token), mul, shift); };
+        if (!wide) fp4 ? run(indexer_q_rope_quant_heads_kernel<WARPS, true, false, false>) : run(indexer_q_rope_quant_heads_kernel<WARPS, false, false, false>);
+        else if (!prefetch) fp4 ? run(indexer_q_rope_quant_heads_kernel<WARPS, true, true, false>) : run(indexer_q_rope_quant_heads_kernel<WARPS, false, true, false>);
+        else fp4 ? run(indexer_q_rope_quant_heads_kernel<WARPS, true, true, true>) : run(indexer_q_rope_quant_heads_kernel<WARPS, false, true, true>);
         count_launch();
         return cudaGetLastError();
     }
