@@ -58,6 +58,7 @@ struct TopkParams {
     int32_t num_rows, vocab, top_k;
     uint32_t capacity;  // of the candidate pool
     bool sampled;       // top_k is small enough for it
+    bool ahead;         // the streaming kernel sends batches to L2 ahead of their loads
     // decode
     const int32_t* seq_lens;
     int32_t next_n;
@@ -748,6 +749,13 @@ __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(co
         for (int u = 0; u < kStreamBatch; ++u) v[u] = u * THREADS < left ? load_quad(next + 4 * u * THREADS) : none;
     };
     load_batch();
+    // With many rows, the batch after that one to L2, by one instruction of one thread; from then on always the batch after the next.
+    constexpr int kBatch = kStreamBatch * THREADS;
+    const auto send_to_l2 = [&](int32_t quads_ahead) {  // (thread 0's `left` is what remains of the share)
+        const int32_t room = left - quads_ahead;
+        if (tid == 0 && p.ahead && room > 0) prefetch_l2(next + 4 * quads_ahead, 16u * static_cast<uint32_t>(room < kBatch ? room : kBatch));
+    };
+    send_to_l2(kBatch);
     clear_histogram<THREADS>(s);
     if (tid < 4) s.counters[tid] = 0u;
     if (tid == 4) s.pooled = 0u, s.below = 0u;
@@ -792,8 +800,8 @@ __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(co
     else __syncthreads();
     const Pool pool{dynamic, &s.pooled, p.capacity};
     // full batches, then what is left of the share, then the quads that are not whole
-    constexpr int kBatch = kStreamBatch * THREADS;
     while (left + tid >= kBatch) {
+        send_to_l2(2 * kBatch);
         pool.take(v, position, 4 * THREADS, f.value);
         left -= kBatch, position += 4 * kBatch, next += 4 * kBatch;
         if (left + tid >= kBatch) {
@@ -910,6 +918,9 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
     };
     const auto stream_rows = [&](auto* kernel, int threads, unsigned ctas) {
         p.capacity = pool_capacity(Expected(p.top_k, std::min(p.vocab, 4 * kSampleQuads), p.vocab));
+        // pays once the GPU is full (4096 x 32768, k 2048: 145 -> 137 us; 1000 x 40000: 59 -> 53 us; 496 x 262144: 107 -> 100 us),
+        // costs 1-2 % below; more than one batch ahead is slower again
+        p.ahead = p.num_rows * static_cast<int64_t>(ctas) >= 6LL * sms;
         return launch(kernel, p, threads, ctas, stream);
     };
     // Few rows: the time of one row counts, so it gets many threads, or a cluster.  Many rows: small CTAs, of which more are
