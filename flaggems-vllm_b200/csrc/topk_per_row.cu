@@ -920,7 +920,7 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
         p.capacity = pool_capacity(Expected(p.top_k, std::min(p.vocab, 4 * kSampleQuads), p.vocab));
         // pays once the GPU is full (4096 x 32768, k 2048: 145 -> 137 us; 1000 x 40000: 59 -> 53 us; 496 x 262144: 107 -> 100 us),
         // costs 1-2 % below; more than one batch ahead is slower again
-        p.ahead = p.num_rows * static_cast<int64_t>(ctas) >= 6LL * sms;
+        p.ahead = p.num_rows * static_cast<int64_t>(ctas) * threads >= 1536LL * sms;
         return launch(kernel, p, threads, ctas, stream);
     };
     // Few rows: the time of one row counts, so it gets many threads, or a cluster.  Many rows: small CTAs, of which more are
@@ -940,8 +940,9 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
     if (quads <= 256 * 4) return whole(topk_short_kernel<DECODE, 256, 4>, 256);
     if (quads <= 256 * 8) return registers(topk_registers_kernel<DECODE, 256, 8>, 256);
     if (p.vocab <= 65536) return stream_rows(topk_stream_kernel<DECODE, 256>, 256, 1);
-    // long rows: two CTAs each while there are few waves of them (496 rows of up to 262144: 74.5 us, 77.5 with one)
-    return stream_rows(topk_stream_kernel<DECODE, 512>, 512, p.vocab >= 131072 && rows < 8LL * sms ? 2 : 1);
+    // very long rows: two CTAs each while there are few waves of them (496 rows of up to 262144: 72 us, 75 with one; 320 rows 57
+    // and 62 us), otherwise one (800 rows of up to 200000: 87 us, 95 with two; 400 of up to 140000: 42 and 48 us)
+    return stream_rows(topk_stream_kernel<DECODE, 512>, 512, p.vocab >= 196608 && rows < 4LL * sms ? 2 : 1);
 }
 
 }  // namespace
