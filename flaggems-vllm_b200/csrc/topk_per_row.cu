@@ -67,13 +67,16 @@ struct TopkParams {
     const int32_t* row_ends;
 };
 
-// Unsigned key with the order of the float values (negative values below positive ones, -0 below +0).
+// Unsigned key with the order of the float values (negative values below positive ones, -0 below +0, a NaN above +inf or, with
+// its sign bit set, below -inf).
 __device__ __forceinline__ uint32_t order_key(uint32_t bits) { return (bits & 0x80000000u) ? ~bits : bits | 0x80000000u; }
 
-// Coarse monotone code: the top 11 bits of the order key of the value rounded to fp16.
+// Coarse monotone code: the top 11 bits of the order key of the value rounded to fp16.  The sign is the value's own: the
+// conversion drops that of a NaN, and the code has to order NaNs as order_key() does (the top one or the bottom one).
 __device__ __forceinline__ uint32_t coarse_bin(float x) {
-    const int32_t h = __half_as_short(__float2half_rn(x));  // sign-extended
-    return static_cast<uint32_t>((h ^ ((h >> 15) | 0x8000)) & 0xffff) >> 5;
+    const uint32_t sign = static_cast<uint32_t>(__float_as_int(x) >> 31);  // all ones or zero
+    const uint32_t h = __half_as_ushort(__float2half_rn(fabsf(x)));
+    return ((h ^ sign ^ 0x8000u) & 0xffffu) >> 5;
 }
 
 // A value whose coarse code is `bin`, the lowest one up to the rounding to fp16; -inf for the codes below it.
@@ -331,8 +334,8 @@ struct Pool {
     uint32_t capacity;
 
     // Takes the values of N quads per lane that reach `floor` (> -inf); quad u holds the positions from p + u * step on, and what
-    // is no part of the row is -inf.  NaNs of either sign pass the comparison, as the largest values should.  Whole warps call
-    // it: a lane counts, the warp adds up and reserves room with one atomic, the lane writes; three instructions per value,
+    // is no part of the row is -inf.  NaNs of either sign pass the comparison: one with its sign bit clear is among the largest
+    // values, one with it set is sorted out by select().  Whole warps call it: a lane counts, the warp adds up and reserves room with one atomic, the lane writes; three instructions per value,
     // the writes predicated, no branches.
     template <int N>
     __device__ __forceinline__ void take(const float4 (&v)[N], int32_t p, int32_t step, float floor) const {

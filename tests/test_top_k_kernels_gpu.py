@@ -58,3 +58,32 @@ def test_rows_that_mislead_the_sample(width):
     x[7, 5::2] = float("inf")
     ends = torch.full((8,), width, dtype=torch.int32, device=DEV)
     check(x, torch.zeros_like(ends), ends, 512)
+
+
+@pytest.mark.parametrize("rows", [8, 320])
+@pytest.mark.parametrize("width", [1500, 3000, 8000, 15000, 20000, 70000])
+def test_nans_rank_by_their_sign(width, rows):
+    """A NaN is above +inf, one with its sign bit set below -inf, in every kernel and on every route (a pool full of NaNs
+    takes the histogram route): the selected bit patterns are those of the largest integer keys of the rows."""
+    g = torch.Generator(device=DEV).manual_seed(width)
+    x = torch.randn(rows, width, generator=g, device=DEV)
+    bits = x.view(torch.int32)
+    up, down = 0x7FC00000, -0x400000  # the quiet NaNs
+    scattered = torch.rand(rows, width, generator=g, device=DEV)
+    bits[0, 7::211] = up
+    bits[1, 7::211] = down
+    bits[2, 3::97], bits[2, 5::89] = up, down
+    bits[3, ::2] = down
+    bits[4, 1::2] = up
+    bits[5][scattered[5] > 100.0 / width] = down  # fewer numbers than are selected
+    bits[6] = torch.where(scattered[6] < 0.5, up, down)
+    bits[7, 11::13] = down + torch.arange(len(bits[7, 11::13]), device=DEV, dtype=torch.int32) % 64
+    bits[7, 12::130] = -0x800000  # -inf
+    k = 512
+    out = torch.full((rows, k), -7, dtype=torch.int32, device=DEV)
+    zeros, ends = torch.zeros(rows, dtype=torch.int32, device=DEV), torch.full((rows,), width, dtype=torch.int32, device=DEV)
+    fg.top_k_per_row_prefill(x, zeros, ends, out, rows, x.stride(0), x.stride(1), k)
+    key = torch.where(bits < 0, -0x80000000 - (bits.long() + 1), bits.long())
+    chosen = out.long().sort(dim=1).values
+    assert bool((chosen[:, 0] >= 0).all()) and bool((chosen[:, -1] < width).all()) and bool((chosen[:, 1:] > chosen[:, :-1]).all())
+    assert torch.equal(key.gather(1, chosen).sort(dim=1).values, key.topk(k, dim=1).values.sort(dim=1).values)
