@@ -56,6 +56,10 @@ int current_table_staging() {
 // microseconds; 2e8 cycles are about a tenth of a second at B200 clocks.
 std::atomic<long long> g_bulk_wait_cycles{200000000LL};
 
+// total >= count * each for count > 0, each >= 0, without the product: sizes come from callers, and one that wraps would let a
+// kernel read far outside the cache.
+bool holds(int64_t total, int64_t count, int64_t each) { return each == 0 ? total >= 0 : total / each >= count; }
+
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // `any_alignment`: where given, q and kv only need their element's 2-byte alignment and the table its 4 bytes, and
@@ -71,7 +75,7 @@ int validate(const void* q, const void* kv, const void* k_cache, const int64_t* 
     if (num_heads > 0 && !q) return DSV4_ERR_NULL_POINTER;
     if (num_tokens_insert > 0) {
         if (!kv || !k_cache || !slot_mapping) return DSV4_ERR_NULL_POINTER;
-        if (cache_block_size <= 0 || kv_block_stride_bytes < cache_block_size * (kTokenDataBytes + kScaleBytes))
+        if (cache_block_size <= 0 || !holds(kv_block_stride_bytes, cache_block_size, kTokenDataBytes + kScaleBytes))
             return DSV4_ERR_BAD_SIZE;
     }
     if (!aligned16(q) || !aligned16(kv) || !aligned16(cos_sin_cache)) {
@@ -182,7 +186,7 @@ int dsv4_gather_dequant_k_cache(const void* k_cache, const int64_t* slots, int64
     if (num_slots < 0 || out_row_stride < kHeadDim) return DSV4_ERR_BAD_SIZE;
     if (num_slots == 0) return DSV4_OK;
     if (!k_cache || !slots || !out) return DSV4_ERR_NULL_POINTER;
-    if (cache_block_size <= 0 || kv_block_stride_bytes < cache_block_size * (kTokenDataBytes + kScaleBytes))
+    if (cache_block_size <= 0 || !holds(kv_block_stride_bytes, cache_block_size, kTokenDataBytes + kScaleBytes))
         return DSV4_ERR_BAD_SIZE;
     if (!aligned16(out) || (out_row_stride % 8) != 0) return DSV4_ERR_MISALIGNED;
     return static_cast<int>(launch_gather_dequant(static_cast<const uint8_t*>(k_cache), slots, num_slots,
@@ -200,8 +204,8 @@ int dsv4_dequantize_and_gather_k_cache(void* out, int64_t out_stride0, int64_t o
         return DSV4_ERR_BAD_SIZE;
     if (num_reqs == 0 || out_tokens == 0) return DSV4_OK;
     if (!out || !k_cache || !seq_lens || !block_table) return DSV4_ERR_NULL_POINTER;
-    if (cache_block_size <= 0 || max_blocks_per_seq <= 0 || scale_slots * 64 < nope_dim) return DSV4_ERR_BAD_SIZE;
-    if (kv_block_stride_bytes < cache_block_size * (nope_dim + 2 * rope_dim + scale_slots)) return DSV4_ERR_BAD_SIZE;
+    if (cache_block_size <= 0 || max_blocks_per_seq <= 0 || int64_t{64} * scale_slots < nope_dim) return DSV4_ERR_BAD_SIZE;
+    if (!holds(kv_block_stride_bytes, cache_block_size, int64_t{2} * rope_dim + nope_dim + scale_slots)) return DSV4_ERR_BAD_SIZE;
     if (num_reqs > 65535) return DSV4_ERR_TOO_LARGE;
     if ((reinterpret_cast<uintptr_t>(out) & 1u) != 0) return DSV4_ERR_MISALIGNED;
     return static_cast<int>(launch_gather_dequant_requests(
@@ -307,7 +311,7 @@ int dsv4_indexer_k_quant_and_cache(const void* k, int64_t k_row_stride, int32_t 
         return DSV4_ERR_BAD_SIZE;
     if (num_tokens == 0) return DSV4_OK;
     if (!k || !kv_cache || !slot_mapping) return DSV4_ERR_NULL_POINTER;
-    if (cache_block_stride_bytes < cache_block_size * (head_dim + 4 * (head_dim / quant_block_size))) return DSV4_ERR_BAD_SIZE;
+    if (!holds(cache_block_stride_bytes, cache_block_size, head_dim + 4 * (head_dim / quant_block_size))) return DSV4_ERR_BAD_SIZE;
     // the fp32 scale region of every block must be 4-byte aligned
     if ((reinterpret_cast<uintptr_t>(k) & 1u) != 0 || (reinterpret_cast<uintptr_t>(kv_cache) & 3u) != 0 ||
         cache_block_stride_bytes % 4 != 0 || (cache_block_size * head_dim) % 4 != 0)
@@ -329,7 +333,7 @@ int dsv4_cp_gather_indexer_k_quant_cache(const void* k_cache, int64_t cache_bloc
         return DSV4_ERR_BAD_SIZE;
     if (num_tokens == 0 || batch == 0) return DSV4_OK;
     if (!k_cache || !k_out || !scale_out || !block_table || !cu_seqlen) return DSV4_ERR_NULL_POINTER;
-    if (cache_block_stride_bytes < cache_block_size * (head_dim + 4 * num_quant_blocks) || k_out_stride_bytes < head_dim ||
+    if (!holds(cache_block_stride_bytes, cache_block_size, head_dim + 4 * num_quant_blocks) || k_out_stride_bytes < head_dim ||
         scale_out_stride_bytes < 4 * num_quant_blocks)
         return DSV4_ERR_BAD_SIZE;
     return static_cast<int>(launch_cp_gather_indexer(k_cache, cache_block_stride_bytes, k_out, k_out_stride_bytes, scale_out,
@@ -359,7 +363,7 @@ int dsv4_combine_topk_swa_indices(const int32_t* topk_indices, int64_t topk_stri
                                   int64_t M, int64_t N, void* cuda_stream) {
     const int64_t lim = 1LL << 31;
     if (num_tokens < 0 || num_tokens >= lim || num_reqs < 0 || num_reqs >= lim - 1 || topk < 0 || topk > topk_width ||
-        topk_width >= lim || window_size < 0 || compress_ratio <= 0 || compress_ratio >= lim || combined_width >= lim ||
+        topk_width >= lim || window_size < 0 || window_size >= lim || compress_ratio <= 0 || compress_ratio >= lim || combined_width >= lim ||
         topk + window_size > combined_width || topk_stride < topk_width || combined_stride < combined_width || M <= -lim ||
         M >= lim || N <= -lim || N >= lim)
         return DSV4_ERR_BAD_SIZE;

@@ -78,6 +78,26 @@ def test_rejections_happen_before_any_launch():
     assert _native.launch_count() == before
 
 
+@pytest.mark.parametrize("block_size", [1 << 61, (1 << 61) + 1, 1 << 62, (1 << 63) - 1])
+def test_sizes_whose_product_wraps_are_rejected(block_size):
+    """block_size times a token's bytes, or the sum of its parts, beyond 64 (32) bits: refused, not wrapped to a small or
+    negative number.  Without a GPU an accepted call would return a CUDA error instead of -2."""
+    lib = _native.lib()
+    vp, i64, i32 = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int
+    reader, keys, combine = (getattr(lib, f) for f in (
+        "dsv4_dequantize_and_gather_k_cache", "dsv4_indexer_k_quant_and_cache", "dsv4_combine_topk_swa_indices"))
+    reader.argtypes = [vp, i64, i64, i64, vp, vp, vp, vp, i64, i64, i64, i64, i64, i32, i32, i32, i32, vp]
+    keys.argtypes = [vp, i64, i32, vp, i64, vp, i64, i64, i64, i64, i32, vp]
+    combine.argtypes = [vp, i64, i64, vp, vp, vp, vp, i64, i64, vp, i64, i64, i64, i64, i64, i64, i64, vp]
+    a = 0x1000
+    assert lib.dsv4_qnorm_rope_kv_insert(a, a, a, a, a, a, 1e-6, 4, 8, 4, block_size, 64 * 584, None) == -2
+    assert lib.dsv4_gather_dequant_k_cache(a, a, 3, a, 512, block_size, 64 * 584, None) == -2
+    assert reader(a, 512, 512, 8, a, a, None, a, 1, 4, block_size, 64 * 584, 0, 448, 64, 8, 0, None) == -2
+    assert reader(a, 512, 512, 8, a, a, None, a, 1, 4, 64, 64 * 584, 0, 448, 1 << 30, 8, 0, None) == -2
+    assert keys(a, 128, 0, a, 64 * 132, a, 4, block_size, 128, 128, 1, None) == -2
+    assert combine(a, 8, 8, a, a, a, a, 128, 128, a, 1, 1, (1 << 63) - 1, 4, 8, 0, 0, None) == -2
+
+
 def test_variant_selection_round_trip():
     prev = _native.set_variant(_native.VARIANT_ROWS)
     assert _native.lib().dsv4_get_variant() == _native.VARIANT_ROWS
