@@ -575,7 +575,8 @@ PyMethodDef kMethods[] = {
     {"bind", bind, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
-PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host_calls", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+// The build records in the module's docstring which interpreter and torch it is for, and builds anew where they have changed.
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_host_calls", DSV4_BUILT_FOR, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 

@@ -44,6 +44,13 @@ def command(extra_flags=(), out: Path = OUT, sources=SOURCES) -> list[str]:
     ]
 
 
+def built_for() -> str:
+    """What the extension module depends on besides its sources: the interpreter and torch, whose C++ interface it calls."""
+    import torch
+
+    return f"dsv4-built-for:{sys.implementation.cache_tag}:torch-{torch.__version__};"
+
+
 def host_command(out: Path = HOST_OUT) -> list[str]:
     """g++ command of the extension module: linked against the operator library beside it (found at load time through
     $ORIGIN) and against torch's libraries, which the interpreter has loaded by then."""
@@ -53,7 +60,7 @@ def host_command(out: Path = HOST_OUT) -> list[str]:
     cuda = Path(nvcc_path()).resolve().parent.parent
     includes = (root / "include", root / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"])
     return [
-        shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+        shutil.which("g++") or "g++", f'-DDSV4_BUILT_FOR="{built_for()}"', "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
         *[f"-I{i}" for i in includes], *[str(CSRC / s) for s in HOST_SOURCES], "-o", str(out),
         f"-L{OUT.parent}", f"-l:{OUT.name}", f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",
         "-Wl,-rpath,$ORIGIN",
@@ -63,6 +70,8 @@ def host_command(out: Path = HOST_OUT) -> list[str]:
 def up_to_date(out: Path = OUT, sources=SOURCES) -> bool:
     if not out.exists():
         return False
+    if out == HOST_OUT and built_for().encode() not in out.read_bytes():
+        return False  # built for another torch: its symbols need not be there any more
     newest = max((CSRC / f).resolve().stat().st_mtime for f in tuple(sources) + HEADERS)
     return out.stat().st_mtime >= newest
 

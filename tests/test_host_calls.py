@@ -5,7 +5,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from flaggems_vllm import _native
+from flaggems_vllm import _native, build
 
 FRONT_ENDS = [n for n in dir(_native.host_calls()) if not n.startswith("_") and n != "bind"]
 
@@ -15,3 +15,12 @@ FRONT_ENDS = [n for n in dir(_native.host_calls()) if not n.startswith("_") and 
                                   (1 << 80,) * 10, (float("nan"),) * 10])
 def test_refuses_without_raising(name, args):
     assert getattr(_native.host_calls(), name)(*args) is None
+
+
+def test_another_torch_makes_the_build_stale(monkeypatch):
+    """The module calls torch's C++ interface: built for another version, it may not even load."""
+    assert _native.host_calls().__doc__ == build.built_for()
+    assert build.up_to_date(build.HOST_OUT, build.HOST_SOURCES)
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + "1")
+    assert not build.up_to_date(build.HOST_OUT, build.HOST_SOURCES)
+    assert build.up_to_date(build.OUT, build.SOURCES)  # the operator library knows nothing of torch
