@@ -8,7 +8,9 @@
 //
 // Contract with the Python wrappers: a function returns its result (True for operators that fill their arguments) or None
 // when an argument is not acceptable; the wrapper then runs its own assertions, which name the argument.  The checks below
-// are those assertions, one for one.  A non-zero code of the C ABI is handed to the callable given to bind(), which raises.
+// are those assertions, one for one (tests/test_host_checks_agree.py compares the two), and a few limits of the C ABI: the text of
+// the first check that failed is what _refusal() returns, for arguments that the assertions let pass.  A non-zero code of the C
+// ABI is handed to the callable given to bind(), which raises.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -16,6 +18,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
+
+#include <cstdio>
 
 #include "../../include/dsv4_prologue.h"
 
@@ -25,6 +29,7 @@ using at::ScalarType;
 using at::Tensor;
 
 PyObject* g_check = nullptr;  // raises for a non-zero code of the C ABI
+thread_local char t_refusal[256] = "";  // why the thread's last refused call was refused
 
 // Argument list of one call.  `ok` turns false at the first argument that is not acceptable.
 struct Arguments {
@@ -32,50 +37,66 @@ struct Arguments {
     Py_ssize_t count;
     bool ok = true;
 
-    void require(bool condition) { ok = ok && condition; }
+    void require(bool condition, const char* text) {
+        if (ok && !condition) refuse("%s", text);
+    }
+    template <typename... Values>
+    void refuse(const char* format, Values... what) {
+        ok = false;
+        std::snprintf(t_refusal, sizeof t_refusal, format, what...);
+    }
 
     // A tensor with storage of its own (wrapper subclasses that dispatch to Python have none), or null.
     const Tensor* tensor(Py_ssize_t i) {
         if (!ok) return nullptr;
-        if (i >= count || !THPVariable_Check(values[i])) return reject();
-        const Tensor& t = THPVariable_Unpack(values[i]);
-        if (!t.defined() || t.unsafeGetTensorImpl()->is_python_dispatch()) return reject();
-        return &t;
+        if (i < count && THPVariable_Check(values[i])) {
+            const Tensor& t = THPVariable_Unpack(values[i]);
+            if (t.defined() && !t.unsafeGetTensorImpl()->is_python_dispatch()) return &t;
+        }
+        refuse("argument %d is not a tensor with storage of its own", static_cast<int>(i));
+        return nullptr;
     }
     bool is_none(Py_ssize_t i) const { return i >= count || values[i] == Py_None; }
-    int64_t integer(Py_ssize_t i) {
+    // Whatever int() takes.
+    int64_t integer_of(Py_ssize_t i) {
         if (!ok) return 0;
-        if (i >= count) return ok = false, 0;
-        if (PyLong_CheckExact(values[i])) {
-            const long long v = PyLong_AsLongLong(values[i]);
-            if (v == -1 && PyErr_Occurred()) return PyErr_Clear(), ok = false, 0;
-            return v;
+        if (i < count) {
+            PyObject* number = PyLong_CheckExact(values[i]) ? Py_NewRef(values[i]) : PyNumber_Long(values[i]);
+            const long long v = number ? PyLong_AsLongLong(number) : -1;
+            Py_XDECREF(number);
+            if (v != -1 || !PyErr_Occurred()) return v;
+            PyErr_Clear();
         }
-        PyObject* number = PyNumber_Long(values[i]);
-        if (!number) return PyErr_Clear(), ok = false, 0;
-        const long long v = PyLong_AsLongLong(number);
-        Py_DECREF(number);
-        if (v == -1 && PyErr_Occurred()) return PyErr_Clear(), ok = false, 0;
-        return v;
+        refuse("argument %d is not an integer of 64 bits", static_cast<int>(i));
+        return 0;
+    }
+    // The same without text, for the sizes that the assertions compare or compute with.
+    int64_t integer(Py_ssize_t i) {
+        if (ok && i < count && (PyUnicode_Check(values[i]) || PyBytes_Check(values[i]) || PyByteArray_Check(values[i])))
+            refuse("argument %d is not a number", static_cast<int>(i));
+        return integer_of(i);
     }
     float real(Py_ssize_t i) {
         if (!ok) return 0.0f;
-        if (i >= count) return ok = false, 0.0f;
-        const double v = PyFloat_AsDouble(values[i]);
-        if (v == -1.0 && PyErr_Occurred()) return PyErr_Clear(), ok = false, 0.0f;
-        return static_cast<float>(v);
+        if (i < count) {
+            const double v = PyFloat_AsDouble(values[i]);
+            if (v != -1.0 || !PyErr_Occurred()) return static_cast<float>(v);
+            PyErr_Clear();
+        }
+        refuse("argument %d is not a number", static_cast<int>(i));
+        return 0.0f;
     }
     bool truth(Py_ssize_t i) {
         if (!ok || i >= count) return false;
         const int v = PyObject_IsTrue(values[i]);
-        if (v < 0) return PyErr_Clear(), ok = false, false;
-        return v != 0;
-    }
-    const Tensor* reject() {
-        ok = false;
-        return nullptr;
+        if (v >= 0) return v != 0;
+        PyErr_Clear();
+        refuse("argument %d has no truth value", static_cast<int>(i));
+        return false;
     }
 };
+
+#define REQUIRE(...) a.require((__VA_ARGS__), #__VA_ARGS__)
 
 bool is(const Tensor& t, ScalarType type) { return t.scalar_type() == type; }
 bool on(const Tensor& t, const Tensor& first) { return t.is_cuda() && t.get_device() == first.get_device(); }
@@ -147,16 +168,16 @@ PyObject* prologue(Arguments& a) {
     const float eps = a.real(6);
     const int64_t block = a.integer(7);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(q->is_cuda() && q->is_contiguous() && kv->is_contiguous() && q->dim() == 3 && q->size(2) == 512);
+    REQUIRE(q->is_cuda() && q->is_contiguous() && kv->is_contiguous() && q->dim() == 3 && q->size(2) == 512);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t tokens = q->size(0), heads = q->size(1);
-    a.require(kv->dim() == 2 && kv->size(0) == tokens && kv->size(1) == 512);
-    a.require(is(*q, at::kBFloat16) && is(*kv, at::kBFloat16) && is(*cache, at::kByte));
-    a.require(slots->dim() == 1 && is(*slots, at::kLong) && slots->is_contiguous() && slots->size(0) <= tokens);
-    a.require(pos->dim() == 1 && is(*pos, at::kLong) && pos->is_contiguous() && pos->size(0) == tokens);
-    a.require(cs->dim() == 2 && cs->size(1) == 64 && is(*cs, at::kFloat) && cs->is_contiguous());
-    a.require(cache->dim() == 2 && cache->stride(1) == 1 && block > 0 && cache->size(1) / 584 >= block);
-    a.require(on(*kv, *q) && on(*cache, *q) && on(*slots, *q) && on(*pos, *q) && on(*cs, *q));
+    REQUIRE(kv->dim() == 2 && kv->size(0) == tokens && kv->size(1) == 512);
+    REQUIRE(is(*q, at::kBFloat16) && is(*kv, at::kBFloat16) && is(*cache, at::kByte));
+    REQUIRE(slots->dim() == 1 && is(*slots, at::kLong) && slots->is_contiguous() && slots->size(0) <= tokens);
+    REQUIRE(pos->dim() == 1 && is(*pos, at::kLong) && pos->is_contiguous() && pos->size(0) == tokens);
+    REQUIRE(cs->dim() == 2 && cs->size(1) == 64 && is(*cs, at::kFloat) && cs->is_contiguous());
+    REQUIRE(cache->dim() == 2 && cache->stride(1) == 1 && block > 0 && cache->size(1) / 584 >= block);
+    REQUIRE(on(*kv, *q) && on(*cache, *q) && on(*slots, *q) && on(*pos, *q) && on(*cs, *q));
     if (!a.ok) Py_RETURN_NONE;
     if (tokens == 0) Py_RETURN_TRUE;
     if (!launch_on(*q, [&](void* stream) {
@@ -183,12 +204,12 @@ PyObject* q_kv_rmsnorm(Arguments& a) {
     const Tensor *qr = a.tensor(0), *kv = a.tensor(1), *qw = a.tensor(2), *kw = a.tensor(3);
     const float eps = a.real(4);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(qr->is_cuda() && qr->dim() == 2 && kv->dim() == 2 && qr->size(0) == kv->size(0));
+    REQUIRE(qr->is_cuda() && qr->dim() == 2 && kv->dim() == 2 && qr->size(0) == kv->size(0));
     if (!a.ok) Py_RETURN_NONE;
-    a.require(qr->stride(1) == 1 && kv->stride(1) == 1 && qw->is_contiguous() && kw->is_contiguous());
-    a.require(dtype_code(*qr) >= 0 && dtype_code(*kv) >= 0 && dtype_code(*qw) >= 0 && dtype_code(*kw) >= 0);
-    a.require(on(*kv, *qr) && on(*qw, *qr) && on(*kw, *qr));
-    a.require(qw->dim() == 1 && qw->size(0) == qr->size(1) && kw->dim() == 1 && kw->size(0) == kv->size(1));
+    REQUIRE(qr->stride(1) == 1 && kv->stride(1) == 1 && qw->is_contiguous() && kw->is_contiguous());
+    REQUIRE(dtype_code(*qr) >= 0 && dtype_code(*kv) >= 0 && dtype_code(*qw) >= 0 && dtype_code(*kw) >= 0);
+    REQUIRE(on(*kv, *qr) && on(*qw, *qr) && on(*kw, *qr));
+    REQUIRE(qw->dim() == 1 && qw->size(0) == qr->size(1) && kw->dim() == 1 && kw->size(0) == kv->size(1));
     if (!a.ok) Py_RETURN_NONE;
     const int64_t tokens = qr->size(0);
     Tensor qo = make_empty(qr->sizes(), qr->scalar_type(), *qr), ko = make_empty(kv->sizes(), kv->scalar_type(), *qr);
@@ -208,10 +229,10 @@ PyObject* group_quant(Arguments& a) {
     const float eps = a.real(2);
     const bool column_major = a.truth(3), ue8m0 = a.truth(4);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(x->is_cuda() && is(*x, at::kBFloat16) && x->dim() >= 2 && group > 0);
+    REQUIRE(x->is_cuda() && is(*x, at::kBFloat16) && x->dim() >= 2 && group > 0);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t cols = x->size(-1);
-    a.require(cols % group == 0 && x->stride(-1) == 1 && (x->dim() == 2 || (x->is_contiguous() && !column_major)));
+    REQUIRE(cols % group == 0 && x->stride(-1) == 1 && (x->dim() == 2 || (x->is_contiguous() && !column_major)));
     if (!a.ok) Py_RETURN_NONE;
     const int64_t rows = cols > 0 ? x->numel() / cols : 0, groups = cols / group;
     Tensor xq = make_empty(x->sizes(), at::kFloat8_e4m3fn, *x), xs;
@@ -239,7 +260,7 @@ PyObject* act_quant(Arguments& a) {
     const int64_t block = a.integer(1);
     const bool round_scale = a.truth(2);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(x->is_cuda() && is(*x, at::kBFloat16) && x->dim() >= 1 && x->is_contiguous() && block > 0 && x->size(-1) % block == 0);
+    REQUIRE(x->is_cuda() && is(*x, at::kBFloat16) && x->dim() >= 1 && x->is_contiguous() && block > 0 && x->size(-1) % block == 0);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t cols = x->size(-1), rows = cols > 0 ? x->numel() / cols : 0;
     Tensor y = make_empty(x->sizes(), at::kFloat8_e4m3fn, *x);
@@ -262,15 +283,15 @@ PyObject* inv_rope_fp8_quant(Arguments& a) {
     const float eps = a.real(8);
     const bool packed = a.truth(9);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(o->is_cuda() && o->dim() == 3 && pos->dim() == 1 && cs->dim() == 2 && n_groups > 0 && per_group > 0 && group > 0);
+    REQUIRE(o->is_cuda() && o->dim() == 3 && pos->dim() == 1 && cs->dim() == 2 && n_groups > 0 && per_group > 0 && group > 0);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t tokens = o->size(0), heads = o->size(1), head_dim = o->size(2);
-    a.require(o->stride(2) == 1 && pos->size(0) == tokens && heads == n_groups * per_group && nope >= 0 && rope >= 0);
-    a.require(head_dim == nope + rope && head_dim % group == 0 && nope % group == group - rope && rope % 2 == 0 && group % 2 == 0);
-    a.require(cs->size(1) == rope && is(*cs, at::kFloat) && cs->stride(1) == 1);
-    a.require(is(*o, at::kBFloat16) && is(*pos, at::kLong) && pos->is_contiguous() && on(*pos, *o) && on(*cs, *o));
+    REQUIRE(o->stride(2) == 1 && pos->size(0) == tokens && heads == n_groups * per_group && nope >= 0 && rope >= 0);
+    REQUIRE(head_dim == nope + rope && head_dim % group == 0 && nope % group == group - rope && rope % 2 == 0 && group % 2 == 0);
+    REQUIRE(cs->size(1) == rope && is(*cs, at::kFloat) && cs->stride(1) == 1);
+    REQUIRE(is(*o, at::kBFloat16) && is(*pos, at::kLong) && pos->is_contiguous() && on(*pos, *o) && on(*cs, *o));
     const int64_t per_head = group > 0 ? head_dim / group : 0;
-    a.require(!packed || per_head == 4);
+    REQUIRE(!packed || per_head == 4);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t d = per_group * head_dim, padded = (tokens + 3) / 4 * 4;
     const int64_t inner = packed ? (d / group + 3) / 4 : d / group;
@@ -294,14 +315,14 @@ PyObject* indexer_q_rope_quant(Arguments& a) {
     const float softmax_scale = a.real(4), head_scale = a.real(5);
     const bool fp4 = a.truth(6);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(q->is_cuda() && pos->dim() == 1 && q->dim() == 3 && cs->dim() == 2 && w->dim() == 2);
+    REQUIRE(q->is_cuda() && pos->dim() == 1 && q->dim() == 3 && cs->dim() == 2 && w->dim() == 2);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t tokens = pos->size(0), heads = q->size(1), dim = q->size(2), rot = cs->size(1);
-    a.require(is(*q, at::kBFloat16) && q->stride(2) == 1 && q->size(0) == tokens && is(*pos, at::kLong) && pos->is_contiguous());
-    a.require((is(*cs, at::kFloat) || is(*cs, at::kBFloat16)) && cs->stride(1) == 1);
-    a.require(dtype_code(*w) >= 0 && w->size(0) == tokens && w->size(1) == heads && w->stride(1) == 1);
-    a.require((dim == 64 || dim == 128 || dim == 256) && rot % 2 == 0 && rot <= dim && (dim - rot) % (dim / 32) == 0);
-    a.require(on(*pos, *q) && on(*cs, *q) && on(*w, *q));
+    REQUIRE(is(*q, at::kBFloat16) && q->stride(2) == 1 && q->size(0) == tokens && is(*pos, at::kLong) && pos->is_contiguous());
+    REQUIRE((is(*cs, at::kFloat) || is(*cs, at::kBFloat16)) && cs->stride(1) == 1);
+    REQUIRE(dtype_code(*w) >= 0 && w->size(0) == tokens && w->size(1) == heads && w->stride(1) == 1);
+    REQUIRE((dim == 64 || dim == 128 || dim == 256) && rot % 2 == 0 && rot <= dim && (dim - rot) % (dim / 32) == 0);
+    REQUIRE(on(*pos, *q) && on(*cs, *q) && on(*w, *q));
     if (!a.ok) Py_RETURN_NONE;
     Tensor w_out = make_empty({tokens, heads}, at::kFloat, *q), q_out, scale;
     void* scale_ptr = nullptr;
@@ -317,7 +338,7 @@ PyObject* indexer_q_rope_quant(Arguments& a) {
         q_out = make_empty(q->sizes(), at::kFloat8_e4m3fn, *q);
     } else {  // keeps the order of dimensions in memory that a dense, permuted q has
         q_out = at::empty_like(*q, q->options().dtype(at::kFloat8_e4m3fn));
-        a.require(q_out.stride(2) == 1);
+        REQUIRE(q_out.stride(2) == 1);
         if (!a.ok) Py_RETURN_NONE;
     }
     if (tokens > 0 && !launch_on(*q, [&](void* stream) {
@@ -347,13 +368,13 @@ PyObject* indexer_k_quant(Arguments& a) {
     const int64_t group = a.integer(3);
     const bool ue8m0 = a.truth(4);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(k->is_cuda() && k->dim() == 2 && cache->dim() == 3 && slots->dim() == 1 && group > 0);
+    REQUIRE(k->is_cuda() && k->dim() == 2 && cache->dim() == 3 && slots->dim() == 1 && group > 0);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t dim = k->size(1), tokens = slots->size(0), block = cache->size(1), row = cache->size(2);
-    a.require(dim % group == 0 && k->stride(1) == 1 && (is(*k, at::kBFloat16) || is(*k, at::kHalf)) && k->size(0) >= tokens);
-    a.require(is(*slots, at::kLong) && slots->is_contiguous() && is(*cache, at::kByte));
-    a.require(row == dim + 4 * (dim / group) && (cache->is_contiguous() || (cache->stride(2) == 1 && (block == 1 || cache->stride(1) == row))));
-    a.require(on(*cache, *k) && on(*slots, *k));
+    REQUIRE(dim % group == 0 && k->stride(1) == 1 && (is(*k, at::kBFloat16) || is(*k, at::kHalf)) && k->size(0) >= tokens);
+    REQUIRE(is(*slots, at::kLong) && slots->is_contiguous() && is(*cache, at::kByte));
+    REQUIRE(row == dim + 4 * (dim / group) && (cache->is_contiguous() || (cache->stride(2) == 1 && (block == 1 || cache->stride(1) == row))));
+    REQUIRE(on(*cache, *k) && on(*slots, *k));
     if (!a.ok) Py_RETURN_NONE;
     if (tokens == 0 || cache->size(0) == 0) Py_RETURN_TRUE;
     if (!launch_on(*k, [&](void* stream) {
@@ -368,20 +389,20 @@ PyObject* indexer_k_quant(Arguments& a) {
 PyObject* cp_gather_indexer(Arguments& a) {
     const Tensor *cache = a.tensor(0), *k = a.tensor(1), *scale = a.tensor(2), *table = a.tensor(3), *cu = a.tensor(4);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(cache->is_cuda() && cache->dim() == 3 && k->dim() == 2 && scale->dim() == 2 && table->dim() == 2 && cu->dim() == 1);
+    REQUIRE(cache->is_cuda() && cache->dim() == 3 && k->dim() == 2 && scale->dim() == 2 && table->dim() == 2 && cu->dim() == 1);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t tokens = k->size(0), dim = k->size(1), block = cache->size(1), batch = table->size(0);
     const int64_t scale_bytes = scale->size(1) * static_cast<int64_t>(scale->element_size());
-    a.require(scale_bytes > 0);
+    REQUIRE(scale_bytes > 0);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t group = dim * 4 / scale_bytes;
-    a.require(group > 0 && dim % group == 0);
+    REQUIRE(group > 0 && dim % group == 0);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t groups = dim / group;
-    a.require(is(*cache, at::kByte) && cache->is_contiguous() && cache->size(2) == dim + 4 * groups);
-    a.require(k->element_size() == 1 && k->stride(1) == 1 && scale->size(0) >= tokens && scale->stride(1) == 1 && scale_bytes == 4 * groups);
-    a.require(is(*table, at::kInt) && table->stride(1) == 1 && is(*cu, at::kInt) && cu->is_contiguous() && cu->size(0) == batch + 1);
-    a.require(on(*k, *cache) && on(*scale, *cache) && on(*table, *cache) && on(*cu, *cache));
+    REQUIRE(is(*cache, at::kByte) && cache->is_contiguous() && cache->size(2) == dim + 4 * groups);
+    REQUIRE(k->element_size() == 1 && k->stride(1) == 1 && scale->size(0) >= tokens && scale->stride(1) == 1 && scale_bytes == 4 * groups);
+    REQUIRE(is(*table, at::kInt) && table->stride(1) == 1 && is(*cu, at::kInt) && cu->is_contiguous() && cu->size(0) == batch + 1);
+    REQUIRE(on(*k, *cache) && on(*scale, *cache) && on(*table, *cache) && on(*cu, *cache));
     if (!a.ok) Py_RETURN_NONE;
     if (tokens == 0 || batch == 0 || cache->size(0) == 0) Py_RETURN_TRUE;
     if (!launch_on(*cache, [&](void* stream) {
@@ -397,16 +418,16 @@ PyObject* cp_gather_indexer(Arguments& a) {
 // topk_indices, token_to_req_indices, block_table, block_size, is_valid_token or None -> (global_indices, lens)
 PyObject* global_topk(Arguments& a) {
     const Tensor *topk = a.tensor(0), *request = a.tensor(1), *table = a.tensor(2);
-    const int64_t block = a.integer(3);
+    const int64_t block = a.integer_of(3);
     const Tensor* valid = a.is_none(4) ? nullptr : a.tensor(4);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(topk->is_cuda() && topk->dim() == 2 && table->dim() == 2 && request->dim() == 1 && block > 0);
+    REQUIRE(topk->is_cuda() && topk->dim() == 2 && table->dim() == 2 && request->dim() == 1 && block > 0);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t tokens = topk->size(0), width = topk->size(1);
-    a.require(is(*topk, at::kInt) && topk->stride(1) == 1 && is(*table, at::kInt) && table->stride(1) == 1);
-    a.require(is(*request, at::kInt) && request->is_contiguous() && request->size(0) == tokens);
-    a.require(!valid || (is(*valid, at::kInt) && valid->is_contiguous() && valid->dim() == 1 && valid->size(0) == tokens && on(*valid, *topk)));
-    a.require(on(*request, *topk) && on(*table, *topk));
+    REQUIRE(is(*topk, at::kInt) && topk->stride(1) == 1 && is(*table, at::kInt) && table->stride(1) == 1);
+    REQUIRE(is(*request, at::kInt) && request->is_contiguous() && request->size(0) == tokens);
+    REQUIRE(!valid || (is(*valid, at::kInt) && valid->is_contiguous() && valid->dim() == 1 && valid->size(0) == tokens && on(*valid, *topk)));
+    REQUIRE(on(*request, *topk) && on(*table, *topk));
     if (!a.ok) Py_RETURN_NONE;
     Tensor out = topk->is_contiguous() ? make_empty(topk->sizes(), at::kInt, *topk) : at::empty_like(*topk);
     Tensor lens = make_empty({tokens}, at::kInt, *topk);
@@ -424,14 +445,14 @@ PyObject* global_topk(Arguments& a) {
 PyObject* combine_topk_swa(Arguments& a) {
     constexpr int64_t kAlignment = 128;  // of a row of the result, in entries
     const Tensor *topk = a.tensor(0), *start = a.tensor(1), *seq = a.tensor(2), *gather = a.tensor(3);
-    const int64_t window = a.integer(4), ratio = a.integer(5), k = a.integer(6), m = a.integer(7), n = a.integer(8);
+    const int64_t window = a.integer(4), ratio = a.integer_of(5), k = a.integer(6), m = a.integer_of(7), n = a.integer_of(8);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(topk->is_cuda() && topk->dim() == 2 && start->dim() == 1 && seq->dim() == 1 && gather->dim() == 1);
+    REQUIRE(topk->is_cuda() && topk->dim() == 2 && start->dim() == 1 && seq->dim() == 1 && gather->dim() == 1);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t tokens = topk->size(0), requests = seq->size(0);
-    a.require(is(*topk, at::kInt) && topk->stride(1) == 1 && k <= topk->size(1) && k + window >= 0);
-    for (const Tensor* t : {start, seq, gather}) a.require(is(*t, at::kInt) && t->is_contiguous() && on(*t, *topk));
-    a.require(start->size(0) >= requests + 1 && gather->size(0) >= requests);
+    REQUIRE(is(*topk, at::kInt) && topk->stride(1) == 1 && k <= topk->size(1) && k + window >= 0);
+    for (const Tensor* t : {start, seq, gather}) REQUIRE(is(*t, at::kInt) && t->is_contiguous() && on(*t, *topk));
+    REQUIRE(start->size(0) >= requests + 1 && gather->size(0) >= requests);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t width = (k + window + kAlignment - 1) / kAlignment * kAlignment;
     Tensor combined = make_empty({tokens, width}, at::kInt, *topk), lens = make_empty({tokens}, at::kInt, *topk);
@@ -451,22 +472,22 @@ PyObject* dequantize_and_gather(Arguments& a) {
     const Tensor *out = a.tensor(0), *cache = a.tensor(1), *seq = a.tensor(2);
     const Tensor* gather = a.is_none(3) ? nullptr : a.tensor(3);
     const Tensor* table = a.tensor(4);
-    const int64_t block = a.integer(5), offset = a.integer(6), rope = a.integer(7);
+    const int64_t block = a.integer_of(5), offset = a.integer_of(6), rope = a.integer(7);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(out->is_cuda() && out->dim() == 3 && seq->dim() == 1 && table->dim() == 2);
+    REQUIRE(out->is_cuda() && out->dim() == 3 && seq->dim() == 1 && table->dim() == 2);
     // a 3-D cache with gaps between its rows is copied by the wrapper first
-    a.require(cache->dim() == 2 || (cache->dim() == 3 && cache->is_contiguous()));
+    REQUIRE(cache->dim() == 2 || (cache->dim() == 3 && cache->is_contiguous()));
     if (!a.ok) Py_RETURN_NONE;
     const int64_t width = out->size(2), nope = a.is_none(8) ? width - rope : a.integer(8);
     const int64_t slots = a.is_none(9) ? (nope + 63) / 64 + (nope % 64 == 0 ? 1 : 0) : a.integer(9);
     const int64_t requests = seq->size(0);
-    a.require(is(*out, at::kBFloat16) && out->stride(2) == 1 && table->size(0) == requests && requests <= out->size(0));
-    a.require(nope >= 0 && rope >= 0 && nope + rope <= width && nope <= INT32_MAX && rope <= INT32_MAX && slots <= INT32_MAX);
-    a.require(is(*cache, at::kByte) && cache->stride(-1) == 1);
+    REQUIRE(is(*out, at::kBFloat16) && out->stride(2) == 1 && table->size(0) == requests && requests <= out->size(0));
+    REQUIRE(nope >= 0 && rope >= 0 && nope + rope <= width && nope <= INT32_MAX && rope <= INT32_MAX && slots <= INT32_MAX);
+    REQUIRE(is(*cache, at::kByte) && cache->stride(-1) == 1);
     const ScalarType index = seq->scalar_type();
-    a.require((index == at::kInt || index == at::kLong) && is(*table, index) && seq->is_contiguous() && table->is_contiguous());
-    a.require(!gather || (is(*gather, index) && gather->is_contiguous() && gather->dim() == 1 && gather->size(0) == requests && on(*gather, *out)));
-    a.require(on(*cache, *out) && on(*seq, *out) && on(*table, *out));
+    REQUIRE((index == at::kInt || index == at::kLong) && is(*table, index) && seq->is_contiguous() && table->is_contiguous());
+    REQUIRE(!gather || (is(*gather, index) && gather->is_contiguous() && gather->dim() == 1 && gather->size(0) == requests && on(*gather, *out)));
+    REQUIRE(on(*cache, *out) && on(*seq, *out) && on(*table, *out));
     if (!a.ok) Py_RETURN_NONE;
     if (requests == 0 || out->size(1) == 0) Py_RETURN_TRUE;
     const int64_t pitch = cache->dim() == 3 ? cache->size(1) * cache->size(2) : cache->stride(0);
@@ -482,10 +503,10 @@ PyObject* dequantize_and_gather(Arguments& a) {
 
 // The arguments all selection operators share.
 void require_topk(Arguments& a, const Tensor& logits, const Tensor& indices, int64_t rows, int64_t stride0, int64_t stride1, int64_t k) {
-    a.require(logits.is_cuda() && logits.dim() == 2 && is(logits, at::kFloat) && indices.dim() == 2);
+    REQUIRE(logits.is_cuda() && logits.dim() == 2 && is(logits, at::kFloat) && indices.dim() == 2);
     if (!a.ok) return;
-    a.require(rows == logits.size(0) && stride0 == logits.stride(0) && stride1 == logits.stride(1));
-    a.require(is(indices, at::kInt) && indices.is_contiguous() && indices.size(0) >= rows && indices.size(1) == k && on(indices, logits));
+    REQUIRE(rows == logits.size(0) && stride0 == logits.stride(0) && stride1 == logits.stride(1));
+    REQUIRE(is(indices, at::kInt) && indices.is_contiguous() && indices.size(0) >= rows && indices.size(1) == k && on(indices, logits));
 }
 
 // logits, next_n, seq_lens, indices, num_rows, stride0, stride1, top_k
@@ -494,10 +515,10 @@ PyObject* top_k_decode(Arguments& a) {
     const int64_t next_n = a.integer(1), rows = a.integer(4), stride0 = a.integer(5), stride1 = a.integer(6), k = a.integer(7);
     if (!a.ok) Py_RETURN_NONE;
     require_topk(a, *logits, *indices, rows, stride0, stride1, k);
-    a.require(is(*seq, at::kInt) && seq->dim() == 1 && seq->is_contiguous() && on(*seq, *logits));
-    a.require(next_n >= 1 && next_n < (int64_t{1} << 31));
+    REQUIRE(is(*seq, at::kInt) && seq->dim() == 1 && seq->is_contiguous() && on(*seq, *logits));
+    REQUIRE(next_n >= 1 && next_n < (int64_t{1} << 31));
     if (!a.ok) Py_RETURN_NONE;
-    a.require(seq->size(0) * next_n >= rows);
+    REQUIRE(seq->size(0) * next_n >= rows);
     if (!a.ok) Py_RETURN_NONE;
     if (rows == 0 || k == 0) Py_RETURN_TRUE;
     if (!launch_on(*logits, [&](void* stream) {
@@ -516,7 +537,7 @@ PyObject* top_k_prefill(Arguments& a) {
     if (!a.ok) Py_RETURN_NONE;
     require_topk(a, *logits, *indices, rows, stride0, stride1, k);
     for (const Tensor* t : {starts, ends})
-        a.require(is(*t, at::kInt) && t->dim() == 1 && t->is_contiguous() && t->size(0) >= rows && on(*t, *logits));
+        REQUIRE(is(*t, at::kInt) && t->dim() == 1 && t->is_contiguous() && t->size(0) >= rows && on(*t, *logits));
     if (!a.ok) Py_RETURN_NONE;
     if (rows == 0 || k == 0) Py_RETURN_TRUE;
     if (!launch_on(*logits, [&](void* stream) {
@@ -531,14 +552,14 @@ PyObject* top_k_prefill(Arguments& a) {
 // logits, lengths, output, k, max_seq_len or None
 PyObject* persistent_topk(Arguments& a) {
     const Tensor *logits = a.tensor(0), *lengths = a.tensor(1), *output = a.tensor(2);
-    const int64_t k = a.integer(3), longest = a.is_none(4) ? INT64_MAX : a.integer(4);
+    const int64_t k = a.integer(3), longest = a.is_none(4) ? INT64_MAX : a.integer_of(4);
     if (!a.ok) Py_RETURN_NONE;
-    a.require(logits->is_cuda() && logits->dim() == 2 && output->dim() == 2 && (lengths->dim() == 1 || lengths->dim() == 2));
+    REQUIRE(logits->is_cuda() && logits->dim() == 2 && output->dim() == 2 && (lengths->dim() == 1 || lengths->dim() == 2));
     if (!a.ok) Py_RETURN_NONE;
     const int64_t rows = logits->size(0);
-    a.require(is(*logits, at::kFloat) && is(*lengths, at::kInt) && is(*output, at::kInt) && lengths->is_contiguous() && output->is_contiguous());
-    a.require(lengths->numel() == rows && output->size(0) == rows && output->size(1) == k && (k == 512 || k == 1024 || k == 2048));
-    a.require(on(*lengths, *logits) && on(*output, *logits));
+    REQUIRE(is(*logits, at::kFloat) && is(*lengths, at::kInt) && is(*output, at::kInt) && lengths->is_contiguous() && output->is_contiguous());
+    REQUIRE(lengths->numel() == rows && output->size(0) == rows && output->size(1) == k && (k == 512 || k == 1024 || k == 2048));
+    REQUIRE(on(*lengths, *logits) && on(*output, *logits));
     if (!a.ok) Py_RETURN_NONE;
     if (rows == 0) Py_RETURN_TRUE;
     if (!launch_on(*logits, [&](void* stream) {
@@ -555,6 +576,8 @@ PyObject* bind(PyObject*, PyObject* check) {
     g_check = Py_NewRef(check);
     Py_RETURN_NONE;
 }
+
+PyObject* refusal(PyObject*, PyObject*) { return PyUnicode_FromString(t_refusal); }
 
 #define DSV4_ENTRY(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<name>)), METH_FASTCALL, nullptr}
 PyMethodDef kMethods[] = {
@@ -573,6 +596,7 @@ PyMethodDef kMethods[] = {
     DSV4_ENTRY(top_k_prefill),
     DSV4_ENTRY(persistent_topk),
     {"bind", bind, METH_O, nullptr},
+    {"_refusal", refusal, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 // The build records in the module's docstring which interpreter and torch it is for, and builds anew where they have changed.

@@ -154,8 +154,8 @@ def host_calls():
 
 def refuse():
     """Raised by an operator whose native front end refused arguments that its own assertions let pass (a size the
-    library rejects, a tensor without storage)."""
-    raise Dsv4Error(-2, lib().dsv4_error_string(-2).decode())
+    library rejects, a number that is none, a tensor without storage): names the check that failed."""
+    raise Dsv4Error(-2, f"the call was refused ({host_calls()._refusal()})")
 
 
 def device_error() -> int:

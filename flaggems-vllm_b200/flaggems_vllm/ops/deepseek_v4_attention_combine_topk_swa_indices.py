@@ -42,6 +42,7 @@ def combine_topk_swa_indices(
     num_reqs = seq_lens.shape[0]
     assert topk_indices.dtype == torch.int32 and topk_indices.stride(1) == 1, "int32 indices with unit inner stride"
     assert topk <= topk_indices.shape[1], "topk entries are read from every row"
+    assert topk + window_size >= 0, "a row of the result holds topk + window_size entries"
     for t in (query_start_loc, seq_lens, gather_lens):
         assert t.dtype == torch.int32 and t.dim() == 1 and t.is_contiguous() and t.device == dev
     assert query_start_loc.shape[0] >= num_reqs + 1 and gather_lens.shape[0] >= num_reqs

@@ -32,7 +32,8 @@ def indexer_k_quant_and_cache(k: torch.Tensor, kv_cache: torch.Tensor, slot_mapp
     assert k.dim() == 2 and k.stride(1) == 1 and k.dtype in (torch.bfloat16, torch.float16)
     assert k.shape[0] >= num_tokens
     assert slot_mapping.dtype == torch.int64 and slot_mapping.dim() == 1 and slot_mapping.is_contiguous()
-    assert kv_cache.dtype == torch.uint8 and kv_cache.dim() == 3 and kv_cache[0].is_contiguous()
+    assert kv_cache.dtype == torch.uint8 and kv_cache.dim() == 3 and kv_cache.stride(2) == 1, "[blocks, block_size, row] bytes"
+    assert kv_cache.shape[1] == 1 or kv_cache.stride(1) == kv_cache.shape[2], "a block's bytes must be adjacent"
     assert kv_cache.shape[2] == head_dim + 4 * (head_dim // quant_block_size), "cache row = values + fp32 scales"
     assert kv_cache.device == k.device and slot_mapping.device == k.device
     _native.refuse()
