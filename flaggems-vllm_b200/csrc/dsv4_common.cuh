@@ -208,12 +208,6 @@ __device__ __forceinline__ void st_stream16(void* p, uint4 v) {
                  : "memory");
 }
 
-__device__ __forceinline__ uint2 ld_stream8(const void* p) {
-    uint2 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-    return v;
-}
-
 __device__ __forceinline__ uint32_t ld_stream4(const void* p) {
     uint32_t v;
     asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));
@@ -237,7 +231,6 @@ __device__ __forceinline__ float4 ld_readonly_f4(const float* p) {
 __device__ __forceinline__ float bf16_lo(uint32_t u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
-// Two floats -> packed bf16 pair, round to nearest even (lo in bits 0-15).
 // Element-wise maximum of two bf16 pairs (one instruction).
 __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
     uint32_t d;
@@ -253,6 +246,7 @@ __device__ __forceinline__ uint32_t max_abs_bf16x2(uint32_t a, uint32_t b) {
     return d;
 }
 
+// Two floats -> packed bf16 pair, round to nearest even (lo in bits 0-15).
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));

@@ -23,7 +23,6 @@ struct InvRopeParams {
     int64_t num_tokens, padded_tokens;
     int32_t num_heads, heads_per_group;
     float eps;
-    uint32_t heads_mul, heads_shift;  // fast division of a row index by num_heads (rows < 2^31)
     uint32_t hpg_mul, hpg_shift;      // fast division of a head index by heads_per_group
 };
 
@@ -283,7 +282,6 @@ cudaError_t launch_inv_rope_fp8_quant(const void* o, int64_t o_stride_token, int
     p.fp8 = static_cast<uint8_t*>(fp8), p.scale = static_cast<uint8_t*>(scale), p.scale_stride_group = scale_stride_group;
     p.num_tokens = num_tokens, p.padded_tokens = padded_tokens, p.num_heads = num_heads, p.heads_per_group = heads_per_group;
     p.eps = eps;
-    make_fast_divisor(static_cast<uint32_t>(num_heads), &p.heads_mul, &p.heads_shift);
     make_fast_divisor(static_cast<uint32_t>(heads_per_group), &p.hpg_mul, &p.hpg_shift);
     uint32_t tpt_mul, tpt_shift;
     make_fast_divisor(static_cast<uint32_t>(tasks_per_token), &tpt_mul, &tpt_shift);

@@ -81,36 +81,7 @@ def lib() -> ctypes.CDLL:
     L.dsv4_qnorm_rope_kv_insert_padded.restype = i32
     L.dsv4_gather_dequant_k_cache.argtypes = [vp, vp, i64, vp, i64, i64, i64, vp]
     L.dsv4_gather_dequant_k_cache.restype = i32
-    L.dsv4_dequantize_and_gather_k_cache.argtypes = [vp, i64, i64, i64, vp, vp, vp, vp, i64, i64, i64, i64, i64,
-                                                     i32, i32, i32, i32, vp]
-    L.dsv4_dequantize_and_gather_k_cache.restype = i32
-    L.dsv4_fused_q_kv_rmsnorm.argtypes = [vp, vp, vp, i64, i64, i64, vp, vp, vp, i64, i64, i64, i64, f32, vp]
-    L.dsv4_fused_q_kv_rmsnorm.restype = i32
-    L.dsv4_fused_q_kv_rmsnorm_dtypes.argtypes = [vp, vp, vp, i64, i64, i64, i32, i32, vp, vp, vp, i64, i64, i64, i32, i32, i64, f32, vp]
-    L.dsv4_fused_q_kv_rmsnorm_dtypes.restype = i32
-    L.dsv4_fused_inv_rope_fp8_quant.argtypes = [vp, i64, i64, vp, vp, i64, vp, vp, i64, i64, i64, i64, i64, f32, i32, vp]
-    L.dsv4_fused_inv_rope_fp8_quant.restype = i32
-    L.dsv4_fused_inv_rope_fp8_quant_geometry.argtypes = [vp, i64, i64, vp, vp, i64, vp, vp, i64, i64, i64, i64, i64, i64, i64, i64, f32, i32, vp]
-    L.dsv4_fused_inv_rope_fp8_quant_geometry.restype = i32
-    L.dsv4_indexer_k_quant_and_cache.argtypes = [vp, i64, i32, vp, i64, vp, i64, i64, i64, i64, i32, vp]
-    L.dsv4_indexer_k_quant_and_cache.restype = i32
-    L.dsv4_cp_gather_indexer_k_quant_cache.argtypes = [vp, i64, vp, i64, vp, i64, vp, i64, vp, i64, i64, i64, i64, i64, vp]
-    L.dsv4_cp_gather_indexer_k_quant_cache.restype = i32
-    L.dsv4_compute_global_topk_indices_and_lens.argtypes = [vp, i64, vp, vp, i64, vp, vp, i64, vp, i64, i64, i64, vp]
-    L.dsv4_compute_global_topk_indices_and_lens.restype = i32
-    L.dsv4_combine_topk_swa_indices.argtypes = [vp, i64, i64, vp, vp, vp, vp, i64, i64, vp, i64, i64, i64, i64, i64, i64, i64, vp]
-    L.dsv4_combine_topk_swa_indices.restype = i32
-    L.dsv4_per_token_group_quant_fp8.argtypes = [vp, i64, vp, vp, i64, i64, i64, i64, i64, f32, i32, vp]
-    L.dsv4_per_token_group_quant_fp8.restype = i32
-    L.dsv4_act_quant.argtypes = [vp, i64, vp, vp, i64, i64, i64, i32, vp]
-    L.dsv4_act_quant.restype = i32
-    L.dsv4_top_k_per_row_decode.argtypes = [vp, i64, i64, i64, vp, vp, i64, i64, i64, vp]
-    L.dsv4_top_k_per_row_decode.restype = i32
-    L.dsv4_top_k_per_row_prefill.argtypes = [vp, i64, i64, vp, vp, vp, i64, i64, i64, vp]
-    L.dsv4_top_k_per_row_prefill.restype = i32
-    L.dsv4_fused_indexer_q_rope_quant.argtypes = [vp, vp, i64, i64, vp, i64, i32, i64, vp, i64, i64, vp, i64, i64, vp, i64, i32,
-                                                  vp, i64, f32, f32, i64, i64, i64, i32, vp]
-    L.dsv4_fused_indexer_q_rope_quant.restype = i32
+    # the other operators are called from host_calls.cpp, which is compiled against the header
     L.dsv4_device_error.argtypes = [vp]
     L.dsv4_device_error.restype = i32
     L.dsv4_set_pdl.argtypes = [i32]
