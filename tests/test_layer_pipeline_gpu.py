@@ -10,6 +10,7 @@ import pytest
 import torch
 
 import flaggems_vllm as fg
+from flaggems_vllm import _native
 from flaggems_vllm.testing import compare, workloads
 from oracle import c_oracle
 
@@ -159,3 +160,52 @@ def test_chain_replays_from_a_cuda_graph():
         assert torch.equal(unordered(k, raw(captured[k])), unordered(k, raw(eager[k]))), k
     for k in buffers:
         assert torch.equal(unordered(k, buffers[k]), unordered(k, eager_buffers[k])), k
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("mode", [0, 1, 2])
+def test_chain_in_every_launch_mode(mode, graph):
+    """Every operator reads what the one in front of it wrote, launched dependently or not: two chains with different inputs take
+    turns, so that memory of the allocator holds the other chain's values and an early read shows."""
+    data = [to_device(make_inputs(seed)) for seed in (2, 3)]
+    raw = lambda t: t.view(torch.uint8) if t.dtype.itemsize == 1 else t
+    ordered = lambda k, t: t.sort(dim=1).values if k in ("slots_topk", "topk") else raw(t).clone()
+    previous = _native.set_pdl(0)
+    try:
+        want = []
+        for d in data:
+            buffers = fresh_buffers(d)
+            out = run_chain(d, buffers)
+            torch.cuda.synchronize()
+            want.append({k: ordered(k, t) for k, t in {**out, **buffers}.items()})
+        _native.set_pdl(mode)
+        buffers = [fresh_buffers(d) for d in data]
+        seen = []
+
+        def turns():
+            for turn in range(6):
+                i = turn % 2
+                for b in buffers[i].values():
+                    b.zero_()
+                out = run_chain(data[i], buffers[i])
+                seen.append((i, {k: ordered(k, t) for k, t in {**out, **buffers[i]}.items()}))
+
+        if graph:
+            s = torch.cuda.Stream()
+            s.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(s):
+                run_chain(data[0], buffers[0])
+                captured = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(captured, stream=s):
+                    turns()
+                captured.replay()
+            s.synchronize()
+        else:
+            turns()
+            torch.cuda.synchronize()
+        assert len(seen) == 6
+        for i, got in seen:
+            for k in want[i]:
+                assert torch.equal(got[k], want[i][k]), (k, i)
+    finally:
+        _native.set_pdl(previous)

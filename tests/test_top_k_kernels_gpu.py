@@ -87,3 +87,24 @@ def test_nans_rank_by_their_sign(width, rows):
     chosen = out.long().sort(dim=1).values
     assert bool((chosen[:, 0] >= 0).all()) and bool((chosen[:, -1] < width).all()) and bool((chosen[:, 1:] > chosen[:, :-1]).all())
     assert torch.equal(key.gather(1, chosen).sort(dim=1).values, key.topk(k, dim=1).values.sort(dim=1).values)
+
+
+@pytest.mark.parametrize("rows,width", [(900, 33000), (450, 70001), (450, 140000), (700, 65540), (450, 196608), (600, 196612)])
+@pytest.mark.parametrize("k", [512, 2048])
+def test_rows_that_fill_the_gpu(rows, width, k):
+    """The streaming kernel with batches sent to L2 ahead of their loads: small CTAs, wide ones, and pairs of wide ones.  Ranges of
+    every length, most of them starting off a 16-byte boundary, ties included."""
+    g = torch.Generator(device=DEV).manual_seed(rows + width)
+    x = torch.randn(rows, width, generator=g, device=DEV)
+    x[::3] = (x[::3] * 64).round() / 64
+    starts = torch.randint(0, 9, (rows,), generator=g, device=DEV, dtype=torch.int32)
+    lengths = torch.randint(k, width - 9, (rows,), generator=g, device=DEV, dtype=torch.int32)
+    lengths[:4] = torch.tensor([k, k + 1, width - 9, 4097], dtype=torch.int32, device=DEV)
+    out = torch.full((rows, k), -7, dtype=torch.int32, device=DEV)
+    fg.top_k_per_row_prefill(x, starts, starts + lengths, out, rows, x.stride(0), x.stride(1), k)
+    chosen = out.long().sort(dim=1).values
+    assert bool((chosen[:, 0] >= 0).all()) and bool((chosen[:, -1] < lengths).all()) and bool((chosen[:, 1:] > chosen[:, :-1]).all())
+    got = x.gather(1, chosen + starts[:, None]).sort(dim=1).values
+    for r in range(rows):
+        a, n = int(starts[r]), int(lengths[r])
+        assert torch.equal(got[r], x[r, a : a + n].topk(k).values.sort().values), (r, a, n)
