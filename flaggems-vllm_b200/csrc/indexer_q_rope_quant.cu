@@ -5,8 +5,9 @@
 //          an sm_100 instruction), weights scaled by softmax_scale*head_scale only.
 // Reference: src/flaggems_vllm/ops/fused_indexer_q_rope_quant.py:69-410 and its torch statement
 // tests/test_fused_indexer_q_rope_quant.py:48-113.
-// Fast shape: head_dim/8 lanes per (token, head) row, 16 bytes per lane, several rows per warp instruction.
-// General shape: one warp per row; lane l keeps E = head_dim/32 consecutive values (E/2 rotary pairs).
+// Three kernels: of the DeepSeek-V4 geometry (128 = 64 + 64) a warp walks several heads of one token, 4 lanes a head; other
+// geometries with a rotary tail on a multiple of 8 values take head_dim/8 lanes per (token, head) row, 16 bytes per lane; any
+// other takes one warp per row, where lane l keeps E = head_dim/32 consecutive values (E/2 rotary pairs).
 #include "dsv4_common.cuh"
 
 namespace dsv4 {
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_kernel(const 
     }
 }
 
-// Fast shape: a row is D/8 lanes holding 8 values (16 bytes) each, so one warp instruction moves 32/G rows;
+// Rows of 16-byte pieces: a row is D/8 lanes holding 8 values (16 bytes) each, so one warp instruction moves 32/G rows;
 // U passes per warp are loaded before any is used.  Needs 16-byte aligned rows and a rotary tail that starts
 // on a multiple of 8 values.
 template <int WARPS, int G, int U, bool FP4>
@@ -438,12 +439,14 @@ cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q,
                              (fp4 || (addr(out) % 16 == 0 && out_stride0 % 16 == 0 && out_stride1 % 16 == 0));
     if (heads_shape) {
         constexpr int WARPS = 4;
-        // Heads per warp: few rows, short tasks, so that there are enough of them (61 tokens x 64 heads: 2.0 us with 8, 3.6 with 32);
-        // from 65536 rows on 16 (1531 tokens: 6.9 us; 12.6 on the rows kernel), from 196608 on 64 (4096 tokens: 17.7 us; 29).  The
-        // largest batches take 32 and the prefetch: 16384 tokens 71.6 -> 65.2 us (FP8) and 64.9 -> 62.3 us (MXFP4), 65536 tokens
-        // 262 -> 239 us and 242 -> 227 us; 8192 tokens are as fast with 64 (35.3 / 33.6 us) as the one-warp-per-token form was.
-        const bool prefetch = rows >= 786432;
-        const int heads_per_task = prefetch ? 32 : rows >= 196608 ? 64 : rows >= 65536 ? 16 : 8;
+        // Heads per warp: few rows, short tasks, so that there are enough of them; many rows, long ones, whose set-up more heads
+        // share.  Both sides of each line, FP8 / MXFP4, us a launch of 64 heads a token, rows from HBM:
+        //   8 | 16            832 tokens  6.2 / 6.4 | 6.0 / 6.2 (rows in L2: 5.0 / 5.0 | 5.0 / 5.1)   1023 tokens  7.2 / 7.3 | 6.5 / 6.6
+        //   16 | 64          3072 tokens 15.4 / 15.5 | 16.9 / 16.9                                    4096 tokens 20.4 / 20.5 | 19.2 / 18.4
+        //   64 | prefetch    8192 tokens 36.1 / 34.5 | 37.2 / 35.3     9216 tokens 43.3 / 41.4 | 41.1 / 39.5     65536 tokens 257 / 240 | 240 / 231
+        // Tasks of 64 heads fill the GPU with 4144 tokens at a time: 4608 tokens would be 11 % faster with 32, 8192 are 3 % slower.
+        const bool prefetch = rows >= 589824;
+        const int heads_per_task = prefetch ? 32 : rows >= 212992 ? 64 : rows >= 57344 ? 16 : 8;
         const int64_t tasks_per_token = (num_heads + heads_per_task - 1) / heads_per_task;
         const dim3 grid(static_cast<unsigned>((num_tokens * tasks_per_token + WARPS - 1) / WARPS));
         uint32_t mul, shift;

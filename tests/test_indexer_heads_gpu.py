@@ -14,7 +14,7 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("fp4", [False, True])
-@pytest.mark.parametrize("tokens,heads", [(1, 1), (3, 9), (5, 64), (1023, 64), (1025, 64), (3075, 64), (12289, 64), (11000, 75)])
+@pytest.mark.parametrize("tokens,heads", [(1, 1), (3, 9), (5, 64), (895, 64), (897, 64), (1023, 64), (1025, 64), (3075, 64), (3327, 64), (3329, 64), (9217, 64), (12289, 64), (11000, 75)])
 @pytest.mark.parametrize("offset", [0, 8])  # rows on 32-byte and on 16-byte boundaries
 def test_heads_per_task(tokens, heads, fp4, offset):
     if tokens > 4000 and offset:
