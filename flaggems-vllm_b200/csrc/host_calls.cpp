@@ -61,9 +61,9 @@ struct Arguments {
     int64_t integer_of(Py_ssize_t i) {
         if (!ok) return 0;
         if (i < count) {
-            PyObject* number = PyLong_CheckExact(values[i]) ? Py_NewRef(values[i]) : PyNumber_Long(values[i]);
+            PyObject* number = PyLong_CheckExact(values[i]) ? values[i] : PyNumber_Long(values[i]);
             const long long v = number ? PyLong_AsLongLong(number) : -1;
-            Py_XDECREF(number);
+            if (number != values[i]) Py_XDECREF(number);
             if (v != -1 || !PyErr_Occurred()) return v;
             PyErr_Clear();
         }

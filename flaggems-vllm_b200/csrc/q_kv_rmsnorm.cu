@@ -2,6 +2,8 @@
 // activations [N, Q] and of the latent KV [N, KV] in one launch.
 // Reference: src/flaggems_vllm/ops/deepseek_v4_attention_fused_q_kv_rmsnorm.py:24-103
 //   y = (x * rsqrt(mean(x^2) + eps)) * w, fp32 arithmetic, bf16 in and out.
+// The order of the sum of squares is this kernel's own (a lane adds up runs of 16 neighbouring values, then the warp its lanes),
+// as the reference leaves it open; other orders move about one output in 10^5 by one bf16 step.
 // One warp per row; a row of up to 2048 elements stays in registers between the reduction and
 // the scaling (one read, one write per element); longer or unaligned rows take a two-pass
 // scalar path.  Row 2t is the q row of token t, row 2t+1 its kv row.
@@ -177,9 +179,11 @@ bool on_boundaries(uintptr_t bytes, const NormRows& t) {
            t.out_stride % elements == 0 && t.size % elements == 0 && t.size <= kMaxChunks * 512;
 }
 
-// Up to here the weights are fetched before the reduction (90 registers for rows of 1536: the launch is over before occupancy
-// counts; 61 tokens 1.8 us against 2.4), above it afterwards (7 CTAs per SM: 65536 tokens 80 us = 6.7 TB/s against 91; with 16-byte
-// accesses 85.5).
+// Up to here the weights are fetched before the reduction (90 registers for rows of 1536), above it afterwards (72, 7 CTAs per
+// SM).  Before | after, us a launch of rows of 1536 and 512: 61 tokens 1.6 | 2.1, 1100 tokens 3.2 | 3.6, 65536 tokens 91 | 80 (6.7 TB/s;
+// 85.5 with 16-byte accesses).  In between it depends on where the rows come from.  Out of L2, as a projection has just written
+// them: 1531 tokens 3.5 | 3.8, 3072 tokens 5.0 | 5.5, 4096 tokens 6.1 | 6.1, 8192 tokens 10.5 | 9.3, which is where the line lies.
+// From HBM: 1531 tokens 4.5 | 4.0, 3072 tokens 6.8 | 6.4, 4096 tokens 8.6 | 7.6.
 constexpr int64_t kEarlyWeightTokens = 4096;
 
 template <bool WIDE, bool EARLY>

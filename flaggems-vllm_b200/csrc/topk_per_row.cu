@@ -29,9 +29,9 @@
 // for the pool, a histogram route reads the row twice more; thousands of near-equal values take a radix selection over the
 // row.  The result does not depend on the route; the sample only decides how fast it is reached.
 // HBM traffic on the normal route: the row once (4 bytes per value); top_k * 4 bytes written.
-// Measured (rows of ragged length, a quarter to the whole of the width; before -> after the pool, the scans by one warp and the
-// choice of CTA sizes): 4096 x 32768, k 2048: 236 -> 123 us; k 512: 192 -> 95 us (3.5 TB/s); 496 x 262144, k 512: 98 -> 74 us;
-// 4096 x 65536, k 1024: 290 -> 150 us (4.5 TB/s); 61 x 16384: 12.8 -> 7.0 us; 1 x 32768: 11.8 -> 7.5 us.
+// Measured (rows of ragged length, a quarter to the whole of the width; before -> after the pool, the scans by one warp, the
+// choice of CTA sizes and the batches sent to L2 ahead): 4096 x 32768, k 2048: 236 -> 124 us; k 512: 192 -> 96 us (3.5 TB/s);
+// 496 x 262144, k 512: 98 -> 74 us; 4096 x 65536, k 1024: 290 -> 147 us (4.6 TB/s); 61 x 16384: 12.8 -> 6.5 us; 1 x 32768: 11.8 -> 6.5 us.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
@@ -335,8 +335,9 @@ struct Pool {
 
     // Takes the values of N quads per lane that reach `floor` (> -inf); quad u holds the positions from p + u * step on, and what
     // is no part of the row is -inf.  NaNs of either sign pass the comparison: one with its sign bit clear is among the largest
-    // values, one with it set is sorted out by select().  Whole warps call it: a lane counts, the warp adds up and reserves room with one atomic, the lane writes; three instructions per value,
-    // the writes predicated, no branches.
+    // values, one with it set is sorted out by select().  Whole warps call it: a lane counts, the warp adds up and reserves room
+    // with one atomic, the lane writes; predicated, without branches.  A value costs two instructions to count, four to write
+    // (executed or not) and its position; the whole kernel executes about 27 per 32 values (rows of 32768 values with k 2048).
     template <int N>
     __device__ __forceinline__ void take(const float4 (&v)[N], int32_t p, int32_t step, float floor) const {
         const int lane = threadIdx.x & 31;
@@ -943,8 +944,13 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
     if (quads <= 256 * 4) return whole(topk_short_kernel<DECODE, 256, 4>, 256);
     if (quads <= 256 * 8) return registers(topk_registers_kernel<DECODE, 256, 8>, 256);
     if (p.vocab <= 65536) return stream_rows(topk_stream_kernel<DECODE, 256>, 256, 1);
-    // very long rows: two CTAs each while there are few waves of them (496 rows of up to 262144: 72 us, 75 with one; 320 rows 57
-    // and 62 us), otherwise one (800 rows of up to 200000: 87 us, 95 with two; 400 of up to 140000: 42 and 48 us)
+    // Very long rows: two CTAs each for up to 1.33 waves of single ones (444 fit the GPU), where the second wave would be mostly
+    // empty.  One | two, us, k 512, rows of ragged and of full length:
+    //   262144 wide   320 rows 62 | 57, 69 | 73    400 rows 64 | 64, 73 | 81   496 rows 76 | 74, 111 | 102   560 rows 88 | 83, 117 | 110
+    //                 640 rows 94 | 91, 132 | 119  800 rows 107 | 110, 139 | 147
+    //   200000 wide   320 rows 50 | 48, 57 | 58    496 rows 64 | 64, 87 | 82    640 rows 75 | 75, 98 | 98     800 rows 89 | 94, 112 | 118
+    //   150000 wide   320 rows 40 | 41, 62 | 64    496 rows 51 | 53, 82 | 82    800 rows 69 | 77, 103 | 112
+    // With k 2048 the pairs are 2-6 % behind that: 200000 wide, 496 rows 69 | 71, 92 | 90; 640 rows 80 | 84, 103 | 108.
     return stream_rows(topk_stream_kernel<DECODE, 512>, 512, p.vocab >= 196608 && rows < 4LL * sms ? 2 : 1);
 }
 
