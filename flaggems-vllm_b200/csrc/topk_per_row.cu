@@ -949,7 +949,7 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
     //   262144 wide   320 rows 62 | 57, 69 | 73    400 rows 64 | 64, 73 | 81   496 rows 76 | 74, 111 | 102   560 rows 88 | 83, 117 | 110
     //                 640 rows 94 | 91, 132 | 119  800 rows 107 | 110, 139 | 147
     //   200000 wide   320 rows 50 | 48, 57 | 58    496 rows 64 | 64, 87 | 82    640 rows 75 | 75, 98 | 98     800 rows 89 | 94, 112 | 118
-    //   150000 wide   320 rows 40 | 41, 62 | 64    496 rows 51 | 53, 82 | 82    800 rows 69 | 77, 103 | 112
+    //   140000 wide   320 rows 38 | 39, 43 | 47    496 rows 48 | 51, 64 | 68    800 rows 64 | 73, 84 | 97
     // With k 2048 the pairs are 2-6 % behind that: 200000 wide, 496 rows 69 | 71, 92 | 90; 640 rows 80 | 84, 103 | 108.
     return stream_rows(topk_stream_kernel<DECODE, 512>, 512, p.vocab >= 196608 && rows < 4LL * sms ? 2 : 1);
 }

@@ -148,8 +148,8 @@ def set_variant(variant: int) -> int:
 
 
 def set_pdl(mode) -> int:
-    """Programmatic dependent launch of the prologue (see dsv4_set_pdl): 0 / False off, 1 / True with early index
-    reads, 2 with ordinary stream semantics; returns the previous mode."""
+    """Programmatic dependent launch of the operators (see dsv4_set_pdl): 0 / False off, 1 / True with early index
+    reads by the prologue, 2 with ordinary stream semantics; returns the previous mode."""
     return int(lib().dsv4_set_pdl(int(mode)))
 
 

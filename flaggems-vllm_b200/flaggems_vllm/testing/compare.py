@@ -56,7 +56,7 @@ def q_stats(q: torch.Tensor, q_ref: torch.Tensor, chunk_tokens: int = 2048) -> d
     max_ulp: worst distance over the 448 un-rotated values and over the rotated values that did
     not cancel; tail_cancellations: rotated values more than 1 own-ulp apart yet within one ulp
     of their pair's magnitude; tail_violations: rotated values outside even that."""
-    worst, differ, total, cancel, violate = 0, 0, 0, 0, 0
+    worst, differ, total, cancel, violate, rows, tail = 0, 0, 0, 0, 0, 0, 0
     has_nan = False
     for s in range(0, q.shape[0], chunk_tokens):
         a, b = q[s : s + chunk_tokens], q_ref[s : s + chunk_tokens]
@@ -64,6 +64,8 @@ def q_stats(q: torch.Tensor, q_ref: torch.Tensor, chunk_tokens: int = 2048) -> d
             continue
         d = bf16_ulp_distance(a, b)
         differ += int((d != 0).sum().item())
+        rows += int((d != 0).any(dim=-1).sum().item())
+        tail += int((d[..., NOPE_DIM:] != 0).sum().item())
         total += d.numel()
         has_nan = has_nan or bool(torch.isnan(a.float()).any().item())
         worst = max(worst, int(d[..., :NOPE_DIM].max().item()))
@@ -75,7 +77,7 @@ def q_stats(q: torch.Tensor, q_ref: torch.Tensor, chunk_tokens: int = 2048) -> d
             violate += int((far & ~within).sum().item())
             tail_d = torch.where(far & within, torch.ones_like(tail_d), tail_d)
         worst = max(worst, int(tail_d.max().item()))
-    return {"max_ulp": worst, "mismatch_fraction": differ / max(total, 1), "elements": total, "nan": has_nan,
+    return {"max_ulp": worst, "mismatch_fraction": differ / max(total, 1), "elements": total, "rows_that_differ": rows, "tail_mismatches": tail, "nan": has_nan,
             "tail_cancellations": cancel, "tail_violations": violate}
 
 
@@ -84,7 +86,8 @@ def assert_q_close(q, q_ref, max_ulp: int = 1, max_fraction: float = 1e-3) -> di
     assert not s["nan"], "NaN in q"
     assert s["tail_violations"] == 0, f"{s['tail_violations']} rotated values off by more than a pair-magnitude ulp"
     assert s["max_ulp"] <= max_ulp, f"q differs by {s['max_ulp']} bf16 ulp (allowed {max_ulp})"
-    assert s["mismatch_fraction"] <= max_fraction, f"q mismatch fraction {s['mismatch_fraction']:.3e}"
+    assert s["mismatch_fraction"] <= max_fraction, (
+        f"q mismatch fraction {s['mismatch_fraction']:.3e}, in {s['rows_that_differ']} rows, {s['tail_mismatches']} of them rotated values")
     return s
 
 
