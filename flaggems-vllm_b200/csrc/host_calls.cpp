@@ -38,12 +38,12 @@ struct Arguments {
     bool ok = true;
 
     void require(bool condition, const char* text) {
-        if (ok && !condition) refuse("%s", text);
+        if (ok && !condition) refuse(text);
     }
-    template <typename... Values>
-    void refuse(const char* format, Values... what) {
+    __attribute__((noinline, cold)) void refuse(const char* text, Py_ssize_t argument = -1) {
         ok = false;
-        std::snprintf(t_refusal, sizeof t_refusal, format, what...);
+        if (argument < 0) std::snprintf(t_refusal, sizeof t_refusal, "%s", text);
+        else std::snprintf(t_refusal, sizeof t_refusal, "argument %d %s", static_cast<int>(argument), text);
     }
 
     // A tensor with storage of its own (wrapper subclasses that dispatch to Python have none), or null.
@@ -53,7 +53,7 @@ struct Arguments {
             const Tensor& t = THPVariable_Unpack(values[i]);
             if (t.defined() && !t.unsafeGetTensorImpl()->is_python_dispatch()) return &t;
         }
-        refuse("argument %d is not a tensor with storage of its own", static_cast<int>(i));
+        refuse("is not a tensor with storage of its own", i);
         return nullptr;
     }
     bool is_none(Py_ssize_t i) const { return i >= count || values[i] == Py_None; }
@@ -67,13 +67,13 @@ struct Arguments {
             if (v != -1 || !PyErr_Occurred()) return v;
             PyErr_Clear();
         }
-        refuse("argument %d is not an integer of 64 bits", static_cast<int>(i));
+        refuse("is not an integer of 64 bits", i);
         return 0;
     }
     // The same without text, for the sizes that the assertions compare or compute with.
     int64_t integer(Py_ssize_t i) {
-        if (ok && i < count && (PyUnicode_Check(values[i]) || PyBytes_Check(values[i]) || PyByteArray_Check(values[i])))
-            refuse("argument %d is not a number", static_cast<int>(i));
+        if (ok && i < count && !PyLong_CheckExact(values[i]) && (PyUnicode_Check(values[i]) || PyBytes_Check(values[i]) || PyByteArray_Check(values[i])))
+            refuse("is not a number", i);
         return integer_of(i);
     }
     float real(Py_ssize_t i) {
@@ -83,7 +83,7 @@ struct Arguments {
             if (v != -1.0 || !PyErr_Occurred()) return static_cast<float>(v);
             PyErr_Clear();
         }
-        refuse("argument %d is not a number", static_cast<int>(i));
+        refuse("is not a number", i);
         return 0.0f;
     }
     bool truth(Py_ssize_t i) {
@@ -91,7 +91,7 @@ struct Arguments {
         const int v = PyObject_IsTrue(values[i]);
         if (v >= 0) return v != 0;
         PyErr_Clear();
-        refuse("argument %d has no truth value", static_cast<int>(i));
+        refuse("has no truth value", i);
         return false;
     }
 };
