@@ -1,4 +1,4 @@
-"""Where the upstream source tree is present (the build container; not the GPU box), run its own torch reference
+"""Where the upstream source tree is present, run its own torch reference
 functions on fresh seeded inputs - larger than the committed fixtures - and compare the oracles with them directly.
 Skipped elsewhere.  No GPU."""
 from __future__ import annotations
