@@ -39,7 +39,10 @@ int current_pdl() {
 // Where the rows variant takes the cos|sin rows from: -1 = by launch size (per-warp fetch up to kPerWarpTableRows rows
 // of q, shared-memory staging above), 0 = always per warp, 1 = always staged.
 std::atomic<int> g_table_staging{-2};  // -2: not initialised from the environment yet
-constexpr int64_t kPerWarpTableRows = 65536;
+// The line between them, per warp (with its rows sent to L2 ahead) | staged, us a launch behind another one:
+//   256 x 128 rows 10.7 | 12.0   1024 x 128  39.7 | 41.4   4096 x 128  157.4 | 158.8   16384 x 128  627 | 631   32768 x 64  643.6 | 644.3
+//   32768 x 128  1261-1268 | 1256
+constexpr int64_t kPerWarpTableRows = 2097152;
 
 int current_table_staging() {
     int v = g_table_staging.load(std::memory_order_relaxed);

@@ -119,7 +119,21 @@ inline void make_fast_divisor(uint32_t d, uint32_t* mul, uint32_t* shift) {
 // completed before it touches memory.  Back-to-back launches of a few microseconds lose about 2 us each without it.
 __device__ __forceinline__ void wait_for_preceding_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// First statement of such a kernel.
+// Tells L2 to fetch `bytes` (a multiple of 16) from p (16-byte aligned), one instruction by one thread.  A hint: it moves no value
+// into the kernel, so it may come before wait_for_preceding_kernel() even where the kernel in front still writes that memory
+// (L2 is where both kernels' accesses meet, so the fetched line is the one those writes go to).  The address must not depend on
+// device memory.
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+// The same for the line that holds p, whatever its alignment.
+__device__ __forceinline__ void prefetch_line_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Whether this CTA (of a one-dimensional grid) is among those that can be resident while the kernel in front drains, and so has
+// time to fill with prefetches before wait_for_preceding_kernel() returns.  Later CTAs find that kernel complete.
+__device__ __forceinline__ bool starts_early() { return blockIdx.x * blockDim.x < 148u * 1536u; }
+
+// First statement of such a kernel, or the first after its prefetches.
 __device__ __forceinline__ void begin_dependent_kernel() {
     wait_for_preceding_kernel();
     let_next_kernel_start();
@@ -177,12 +191,6 @@ __device__ __forceinline__ uint4 ld_stream16(const void* p) {
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;
-}
-
-// Fetches `bytes` (a multiple of 16) from p (16-byte aligned) into L2, one instruction by one thread: the loads that follow then
-// wait for L2 instead of HBM, without registers holding what is in flight.
-__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
 // ld_stream16 / st_stream16 for 32 bytes (p 32-byte aligned): one instruction, 1 KiB per warp.
