@@ -33,11 +33,18 @@ struct GroupQuantParams {
 // (IEEE division, the verified reciprocal-and-correct division for the default eps, or x * (1/scale) for `act_quant`).
 template <int WARPS, int LANES, int U, bool WIDE, bool UE8M0, int DIVISION>
 __global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_kernel(const GroupQuantParams p) {
-    begin_dependent_kernel();
     constexpr int kGroups = 32 / LANES;
     const int lane = threadIdx.x & 31;
     const int sub = lane % LANES;
     const int64_t first = (static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5)) * (kGroups * U) + lane / LANES;
+    if (starts_early() && lane < kGroups * U) {  // one group per lane
+        const int64_t g = first - lane / LANES + lane;
+        if (g < p.num_groups) {
+            const int64_t r = fast_div(static_cast<uint32_t>(g), p.gpr_mul, p.gpr_shift);
+            prefetch_l2(p.x + (r * p.x_stride + (g - r * p.groups_per_row) * p.group_size) * 2, 32u * LANES);
+        }
+    }
+    begin_dependent_kernel();
     Bytes32 v[U];
     int64_t row[U];
     int32_t col[U];

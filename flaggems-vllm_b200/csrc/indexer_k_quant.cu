@@ -159,9 +159,15 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_rows_kernel(const 
 // UE8M0 (power-of-two scales): bf16 keys stay packed - group maximum and scaling on the bf16x2 words, as in quant8_pow2.
 template <int WARPS, int U, bool FP16, bool UE8M0>
 __global__ void __launch_bounds__(WARPS * 32, DSV4_INDEXER_K_CTAS) indexer_k_quant_128_kernel(const IndexerParams p) {
-    begin_dependent_kernel();
     const int lane = threadIdx.x & 31, sub = lane & 7, which = lane >> 3;
     const int64_t base = (static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5)) * (U * 4) + which;
+    if (starts_early() && sub == 0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (base + u * 4 < p.num_tokens) prefetch_l2(p.k + (base + u * 4) * p.k_stride * 2, 256u);
+        if (which == 0 && base < p.num_tokens) prefetch_line_l2(p.slot_mapping + base);
+    }
+    begin_dependent_kernel();
     uint4 lo[U], hi[U];
     int64_t slot[U];
 #pragma unroll

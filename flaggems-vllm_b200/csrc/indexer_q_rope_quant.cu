@@ -290,7 +290,6 @@ cudaError_t launch_rows(const IndexerQParams& p, bool fp4, int64_t rows, int cs_
 template <int WARPS, bool FP4, bool WIDE, bool PREFETCH>
 __global__ void __launch_bounds__(WARPS * 32, PREFETCH ? 6 : 7) indexer_q_rope_quant_heads_kernel(const IndexerQParams p, const int heads_per_task, const uint32_t tasks_per_token,
                                                                                 const uint32_t tpt_mul, const uint32_t tpt_shift) {
-    begin_dependent_kernel();
     const int lane = threadIdx.x & 31, sub = lane & 3, which = lane >> 2;
     const uint32_t task = blockIdx.x * WARPS + (threadIdx.x >> 5);
     const int64_t t = fast_div(task, tpt_mul, tpt_shift);
@@ -299,6 +298,12 @@ __global__ void __launch_bounds__(WARPS * 32, PREFETCH ? 6 : 7) indexer_q_rope_q
     const int head_end = head_begin + heads_per_task < p.num_heads ? head_begin + heads_per_task : p.num_heads;
     const int64_t head_bytes = p.q_stride1 * 2;
     const uint8_t* row = p.q + t * p.q_stride0 * 2 + (head_begin + which) * head_bytes + 32 * sub;
+    if (starts_early()) {
+        // the lines of the first pass, one per lane
+        if (lane < 16 && head_begin + (lane >> 1) < head_end) prefetch_line_l2(p.q + t * p.q_stride0 * 2 + (head_begin + (lane >> 1)) * head_bytes + 128 * (lane & 1));
+        if (lane == 31) prefetch_line_l2(p.positions + t);
+    }
+    begin_dependent_kernel();
     const auto load32 = [](const uint8_t* from) {
         if (WIDE) return ld_stream32(from);
         Bytes32 v;

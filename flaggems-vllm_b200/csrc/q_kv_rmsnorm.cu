@@ -39,7 +39,6 @@ __device__ __forceinline__ float inv_rms_of(float sum, int size, float eps) {
 template <int WARPS, int CH, bool WIDE, bool EARLY>
 __global__ void __launch_bounds__(WARPS * 32, EARLY ? 1 : CH == 1 ? 16 : CH == 2 ? 10 : CH == 3 ? 7 : 6)
 q_kv_rmsnorm_kernel(const NormRows q, const NormRows kv, int64_t num_tokens, float eps) {
-    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (r >= 2 * num_tokens) return;
@@ -49,6 +48,8 @@ q_kv_rmsnorm_kernel(const NormRows q, const NormRows kv, int64_t num_tokens, flo
     const uint8_t* in = t.in + token * t.in_stride * 2;
     uint8_t* out = t.out + token * t.out_stride * 2;
     const int size = t.size;
+    if (t.vec_ok && lane == 0 && starts_early()) prefetch_l2(in, 2u * static_cast<uint32_t>(size));
+    begin_dependent_kernel();
     if (t.vec_ok) {
         const int chunks = (size + 15) >> 4;
         const int half = WIDE ? -1 : (size & 8 ? chunks - 1 : -1);  // the chunk whose second 8 values lie outside the row
