@@ -29,9 +29,12 @@
 // for the pool, a histogram route reads the row twice more; thousands of near-equal values take a radix selection over the
 // row.  The result does not depend on the route; the sample only decides how fast it is reached.
 // HBM traffic on the normal route: the row once (4 bytes per value); top_k * 4 bytes written.
-// Measured (rows of ragged length, a quarter to the whole of the width; before -> after the pool, the scans by one warp, the
-// choice of CTA sizes and the batches sent to L2 ahead): 4096 x 32768, k 2048: 236 -> 124 us; k 512: 192 -> 96 us (3.5 TB/s);
-// 496 x 262144, k 512: 98 -> 74 us; 4096 x 65536, k 1024: 290 -> 147 us (4.6 TB/s); 61 x 16384: 12.8 -> 6.5 us; 1 x 32768: 11.8 -> 6.5 us.
+// Bound by instruction issue and by the phases between barriers before HBM: a row of 32768 values takes 20.5 k warp instructions with
+// k 2048 and 17.6 k with k 512 (27.6 k and 22.8 k before signs were shifted into a word instead of counted by comparisons, the
+// sample was halved, and places in the result were reserved for four candidates per thread at a time).  Measured before -> after
+// that: rows of full length, 4096 x 32768, k 2048 137 -> 121 us, k 512 111 -> 100 us (5.4 TB/s); a causal chunk of 4096 rows,
+// k 2048 145 -> 121 us (its sample is now taken in whole lines, the ends of its rows are loaded early); ragged rows, 496 x 262144,
+// k 512 74 -> 70 us; 4096 x 65536, k 1024 147 -> 130 us; 1000 x 40000, k 512 37 -> 30 us.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
@@ -49,7 +52,11 @@ namespace cg = cooperative_groups;
 constexpr int kBins = 2048;
 constexpr int kCountingMax = kBins / 2;  // candidates of one bin ranked by counting (they are kept where the histogram was)
 constexpr int kStreamBatch = 4;          // quads (of 4 consecutive values) per thread in flight
-constexpr int kSampleQuads = 1024;       // of the streaming kernel
+constexpr int kSelectBatch = 4;          // candidates per thread that share one reservation of places in the result
+// Quads in the sample of the streaming kernel with CTAs of that size.  A larger sample leaves fewer candidates to rank, a smaller one
+// is sooner done: rows of 32768 to 65536 values with CTAs of 256 threads, 512 | 1024 quads, 4096 x 32768, k 2048 121 | 128 us,
+// k 512 100 | 111 us; 4096 x 65536, k 1024 132 | 142 us.
+__host__ __device__ constexpr int sample_quads(int threads) { return threads >= 512 ? 1024 : 512; }
 
 struct TopkParams {
     const float* logits;
@@ -69,7 +76,7 @@ struct TopkParams {
 
 // Unsigned key with the order of the float values (negative values below positive ones, -0 below +0, a NaN above +inf or, with
 // its sign bit set, below -inf).
-__device__ __forceinline__ uint32_t order_key(uint32_t bits) { return (bits & 0x80000000u) ? ~bits : bits | 0x80000000u; }
+__device__ __forceinline__ uint32_t order_key(uint32_t bits) { return bits ^ (static_cast<uint32_t>(static_cast<int32_t>(bits) >> 31) | 0x80000000u); }
 
 // Coarse monotone code: the top 11 bits of the order key of the value rounded to fp16.  The sign is the value's own: the
 // conversion drops that of a NaN, and the code has to order NaNs as order_key() does (the top one or the bottom one).
@@ -94,7 +101,7 @@ struct Shared {
     uint32_t scratch[32];
     uint32_t result[4];
     uint32_t counters[4];  // 0: emitted, 1: collected, 2: ties taken / dense candidates, 3: largest key of the sample
-    uint32_t pooled, below;  // candidates in the pool; those of them below the floor
+    uint32_t pooled;  // candidates in the pool
 };
 
 struct Threshold {
@@ -334,16 +341,27 @@ struct Pool {
     uint32_t capacity;
 
     // Takes the values of N quads per lane that reach `floor` (> -inf); quad u holds the positions from p + u * step on, and what
-    // is no part of the row is -inf.  NaNs of either sign pass the comparison: one with its sign bit clear is among the largest
-    // values, one with it set is sorted out by select().  Whole warps call it: a lane counts, the warp adds up and reserves room
-    // with one atomic, the lane writes; predicated, without branches.  A value costs two instructions to count, four to write
-    // (executed or not) and its position; the whole kernel executes about 27 per 32 values (rows of 32768 values with k 2048).
+    // is no part of the row is -inf.  NaNs of either sign are taken: one with its sign bit clear is among the largest values, one
+    // with it set is sorted out by select().  Whole warps call it: a lane marks its candidates, the warp adds up their numbers and
+    // reserves room with one atomic, the lane writes them.
     template <int N>
     __device__ __forceinline__ void take(const float4 (&v)[N], int32_t p, int32_t step, float floor) const {
+        static_assert(N <= 4, "one bit per value");
         const int lane = threadIdx.x & 31;
-        uint32_t mine = 0u;
+        // Bit 4N - 1 - i: value i is below the floor, by the sign of their difference (of a NaN it is +).  Two differences an
+        // instruction and one instruction a value to shift the sign in, where a comparison and a predicated addition were two.
+        uint64_t minus_floor;
+        asm("{.reg .f32 n; neg.f32 n, %1; mov.b64 %0, {n, n};}" : "=l"(minus_floor) : "f"(floor));
+        uint32_t below = 0u;
+        const auto push = [&](float a, float b) {
+            uint64_t d;
+            asm("{.reg .b64 t; mov.b64 t, {%1, %2}; add.rn.f32x2 %0, t, %3;}" : "=l"(d) : "f"(a), "f"(b), "l"(minus_floor));
+            below = __funnelshift_l(static_cast<uint32_t>(d), below, 1);
+            below = __funnelshift_l(static_cast<uint32_t>(d >> 32), below, 1);
+        };
 #pragma unroll
-        for (int u = 0; u < N; ++u) count(mine, v[u].x, floor), count(mine, v[u].y, floor), count(mine, v[u].z, floor), count(mine, v[u].w, floor);
+        for (int u = 0; u < N; ++u) push(v[u].x, v[u].y), push(v[u].z, v[u].w);
+        const uint32_t marks = ~below & ((1u << (4 * N)) - 1u), mine = __popc(marks);
         uint32_t upto = mine;
 #pragma unroll
         for (int m = 1; m < 32; m <<= 1)
@@ -362,36 +380,20 @@ struct Pool {
         uint32_t address = static_cast<uint32_t>(__cvta_generic_to_shared(entries + (end - total + upto - mine)));
 #pragma unroll
         for (int u = 0; u < N; ++u) {
-            const int32_t q = p + u * step;
-            put(address, v[u].x, q, floor), put(address, v[u].y, q + 1, floor), put(address, v[u].z, q + 2, floor), put(address, v[u].w, q + 3, floor);
+            const float e[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (marks & (1u << (4 * (N - u) - 1 - j))) {
+                    asm volatile("st.shared.f32 [%0], %1; st.shared.u32 [%0+4], %2;" ::"r"(address), "f"(e[j]), "r"(p + u * step + j) : "memory");
+                    address += sizeof(uint2);
+                }
         }
-    }
-
-private:
-    static __device__ __forceinline__ void count(uint32_t& n, float v, float floor) {
-        asm("{.reg .pred t;\n"
-            "setp.geu.f32 t, %1, %2;\n"
-            "@t add.u32 %0, %0, 1;}"
-            : "+r"(n)
-            : "f"(v), "f"(floor));
-    }
-    static __device__ __forceinline__ void put(uint32_t& address, float v, int32_t p, float floor) {
-        asm volatile(
-            "{.reg .pred t;\n"
-            "setp.geu.f32 t, %1, %2;\n"
-            "@t st.shared.f32 [%0], %1;\n"
-            "@t st.shared.u32 [%0+4], %3;\n"
-            "@t add.u32 %0, %0, 8;}"
-            : "+r"(address)
-            : "f"(v), "f"(floor), "r"(p)
-            : "memory");
     }
 };
 
 // Bin of a candidate in the histogram that ranks them: linear in the key from `anchor` on, the first and the last bin open.
 __device__ __forceinline__ uint32_t fine_bin(uint32_t key, uint32_t anchor, int shift) {
-    const uint32_t bin = key > anchor ? (key - anchor) >> shift : 0u;
-    return bin < kBins - 1u ? bin : kBins - 1u;
+    return min((max(key, anchor) - anchor) >> shift, kBins - 1u);
 }
 // 2048 bins between the key candidates start at and one near the top of the row (the largest of the sample) leave a handful
 // of candidates in the bin of the k-th largest.
@@ -506,41 +508,72 @@ __device__ __noinline__ void select_from_histogram(Shared& s, uint2* cand, uint3
 }
 
 // Ranks the `size` candidates and emits the k largest; false (in every thread) when the pool does not hold them.  hist and the
-// counters are zero on entry, a barrier ago or more.  A negative NaN, the smallest key, may be among the candidates: keys
-// below the floor do not count.
+// counters are zero on entry, a barrier ago or more.  A negative NaN, the smallest key, may be among the candidates: where the
+// k-th largest is so near the floor that it could count, the pool does not do.
 template <int THREADS>
 __device__ __forceinline__ bool select(Shared& s, const uint2* pool, uint32_t size, uint32_t capacity, uint32_t k, const Floor& f, int32_t* out) {
     const int tid = threadIdx.x;
     const uint32_t floor_key = f.key;
     if (size < k || size > capacity) return false;
-    for (uint32_t i = tid; i < size; i += THREADS) {
-        const uint32_t key = order_key(pool[i].x);
-        if (key >= floor_key) atomicAdd(&s.hist[fine_bin(key, f.anchor, f.shift)], 1u);
-        else atomicAdd(&s.below, 1u);
-    }
+#pragma unroll 4
+    for (uint32_t i = tid; i < size; i += THREADS) atomicAdd(&s.hist[fine_bin(order_key(pool[i].x), f.anchor, f.shift)], 1u);
     __syncthreads();
-    if (size - s.below < k) return false;
     Threshold t;
     if (f.shift > 16) {  // the bins cover many octaves: the candidates reach down to values near zero
         t = find_threshold<THREADS>(s, k);
     } else {
         if (tid < 32) {
-            t = scan_up(s.hist, size - s.below - k);
+            t = scan_up(s.hist, size - k);
             if (tid == 0) s.result[0] = t.bin, s.result[1] = t.need, s.result[2] = t.count;
         }
         __syncthreads();
         t.bin = s.result[0], t.need = s.result[1], t.count = s.result[2];
     }
+    if (t.bin == 0u) {  // where keys below the floor would be, and are not told apart
+        bool strays = false;
+        for (uint32_t i = tid; i < size; i += THREADS) strays |= order_key(pool[i].x) < floor_key;
+        if (__syncthreads_or(strays)) return false;
+    }
     const bool take_all = t.need == t.count;
     if (!take_all && t.count > kCountingMax) return false;
-    const uint32_t lowest = take_all ? t.bin : t.bin + 1u;  // of the bins taken whole
+    // The bins as ranges of keys: above `untaken` a candidate is selected, above `below` (and not above `untaken`) it is in the
+    // bin of the k-th largest.  The first bin begins at the floor, the last one has no end.
+    const auto last_before = [&](uint32_t bin) {
+        if (bin >= kBins) return 0xffffffffu;
+        const uint32_t start = f.anchor + (bin << f.shift);
+        if (start < f.anchor) return 0xffffffffu;  // past the largest key there is
+        return (bin == 0u || start < floor_key ? floor_key : start) - 1u;
+    };
+    const uint32_t untaken = last_before(take_all ? t.bin : t.bin + 1u), below = last_before(t.bin);
     uint2* dense = reinterpret_cast<uint2*>(s.hist);  // the histogram is no longer needed
-    for (uint32_t i = tid; i - (tid & 31) < size; i += THREADS) {  // whole warps stay together for append()
-        const uint2 e = i < size ? pool[i] : make_uint2(0u, 0u);
-        const uint32_t key = order_key(e.x), bin = fine_bin(key, f.anchor, f.shift);
-        const bool in = i < size && key >= floor_key;
-        append(out, &s.counters[0], in && bin >= lowest, static_cast<int32_t>(e.y));
-        if (in && !take_all && bin == t.bin) dense[atomicAdd(&s.counters[2], 1u)] = make_uint2(key, e.y);
+    const int lane = tid & 31;
+    for (uint32_t i0 = tid; i0 - lane < size; i0 += kSelectBatch * THREADS) {  // whole warps stay together
+        uint32_t key[kSelectBatch], at = 0u;
+        int32_t position[kSelectBatch];
+#pragma unroll
+        for (int u = 0; u < kSelectBatch; ++u) {
+            const uint32_t i = i0 + u * THREADS;
+            key[u] = 0u, position[u] = 0;
+            if (i < size) {
+                const uint2 e = pool[i];
+                key[u] = order_key(e.x), position[u] = static_cast<int32_t>(e.y);
+            }
+            if (key[u] > untaken) ++at;
+        }
+        const uint32_t mine = at;
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, at, m);
+            if (lane >= m) at += up;
+        }
+        uint32_t base = 0u;
+        if (lane == 31 && at > 0u) base = atomicAdd(&s.counters[0], at);
+        int32_t* to = out + (__shfl_sync(0xffffffffu, base, 31) + at - mine);
+#pragma unroll
+        for (int u = 0; u < kSelectBatch; ++u) {
+            if (key[u] > untaken) *to++ = position[u];
+            else if (key[u] > below) dense[atomicAdd(&s.counters[2], 1u)] = make_uint2(key[u], static_cast<uint32_t>(position[u]));
+        }
     }
     if (take_all) return true;
     __syncthreads();
@@ -678,7 +711,7 @@ __global__ void __launch_bounds__(THREADS) topk_registers_kernel(const TopkParam
     }
     clear_histogram<THREADS>(s);
     if (tid < 4) s.counters[tid] = 0u;
-    if (tid == 4) s.pooled = 0u, s.below = 0u;
+    if (tid == 4) s.pooled = 0u;
     __syncthreads();
     uint32_t largest = 0u;
 #pragma unroll
@@ -715,6 +748,7 @@ __global__ void __launch_bounds__(THREADS) topk_registers_kernel(const TopkParam
 
 template <bool DECODE, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(const TopkParams p) {
+    constexpr int kSampleQuads = sample_quads(THREADS);
     begin_dependent_kernel();
     __shared__ Shared s;
     extern __shared__ uint2 dynamic[];  // the candidate pool
@@ -753,6 +787,14 @@ __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(co
         for (int u = 0; u < kStreamBatch; ++u) v[u] = u * THREADS < left ? load_quad(next + 4 * u * THREADS) : none;
     };
     load_batch();
+    // The up to three values in front of the first whole quad and behind the last one, one per lane of the first CTA's first warp.
+    float edge_value = -INFINITY;
+    int32_t edge_position = -1;
+    if (row.stride == 1 && rank == 0 && tid < 6) {
+        edge_position = tid < 3 ? (tid < row.position(begin) ? tid : -1) : (end >= begin ? row.position(end) + tid - 3 : -1);
+        if (begin == 0 && tid < 3) edge_position = -1;
+        edge_value = row.edge(edge_position);
+    }
     // With many rows, the batch after that one to L2, by one instruction of one thread; from then on always the batch after the next.
     constexpr int kBatch = kStreamBatch * THREADS;
     const auto send_to_l2 = [&](int32_t quads_ahead) {  // (thread 0's `left` is what remains of the share)
@@ -762,12 +804,16 @@ __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(co
     send_to_l2(kBatch);
     clear_histogram<THREADS>(s);
     if (tid < 4) s.counters[tid] = 0u;
-    if (tid == 4) s.pooled = 0u, s.below = 0u;
+    if (tid == 4) s.pooled = 0u;
     __syncthreads();
     // every CTA of the cluster takes the same sample: runs of 8 consecutive quads (one 128-byte line each, where the row is
     // so aligned) spread evenly over the row
     const int32_t base = row.stride == 1 ? begin : 0, span = row.stride == 1 ? end - begin : row.quads;
-    const int32_t step = span > kSampleQuads ? span / (kSampleQuads / 8) : 8;
+    const auto sampled_quad = [&](int32_t j) {  // runs of 8, each on a multiple of 8
+        const int32_t run = j >> 3;
+        const int32_t at = span > kSampleQuads ? static_cast<int32_t>(static_cast<uint32_t>((static_cast<uint64_t>(run) * static_cast<uint32_t>(span)) / (kSampleQuads / 8)) & ~7u) : 8 * run;
+        return at + (j & 7);
+    };
     uint32_t largest = 0u;
     float peak = -INFINITY;
     {
@@ -775,13 +821,12 @@ __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(co
         float4 sample[kMine];
 #pragma unroll
         for (int u = 0; u < kMine; ++u) {
-            const int32_t j = tid + u * THREADS, quad = (j >> 3) * step + (j & 7);
-            sample[u] = quad < span ? row.load(base + quad) : none;
+            const int32_t quad = sampled_quad(tid + u * THREADS);
+            sample[u] = quad >= span ? none : row.stride == 1 ? load_quad(row.x + row.position(base + quad)) : row.load(base + quad);
         }
 #pragma unroll
         for (int u = 0; u < kMine; ++u) {
-            const int32_t j = tid + u * THREADS;
-            if ((j >> 3) * step + (j & 7) >= span) continue;
+            if (sampled_quad(tid + u * THREADS) >= span) continue;
             const float value[4] = {sample[u].x, sample[u].y, sample[u].z, sample[u].w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -823,14 +868,8 @@ __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(co
             pool.take(edge, row.position(e), 0, f.value);
         }
     } else if (rank == 0 && tid < 32) {
-        if (begin > 0) {
-            edge[0] = tid == 0 ? row.load(0) : none;
-            pool.take(edge, row.position(0), 0, f.value);
-        }
-        if (end < row.quads && end >= begin) {
-            edge[0] = tid == 0 ? row.load(end) : none;
-            pool.take(edge, row.position(end), 0, f.value);
-        }
+        edge[0] = make_float4(edge_value, -INFINITY, -INFINITY, -INFINITY);
+        pool.take(edge, edge_position, 0, f.value);
     }
     __syncthreads();
     if (ctas > 1) {
@@ -921,7 +960,7 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
         return launch(kernel, p, threads, 1, stream);
     };
     const auto stream_rows = [&](auto* kernel, int threads, unsigned ctas) {
-        p.capacity = pool_capacity(Expected(p.top_k, std::min(p.vocab, 4 * kSampleQuads), p.vocab));
+        p.capacity = pool_capacity(Expected(p.top_k, std::min(p.vocab, 4 * sample_quads(threads)), p.vocab));
         // pays once the GPU is full (4096 x 32768, k 2048: 145 -> 137 us; 1000 x 40000: 59 -> 53 us; 496 x 262144: 107 -> 100 us),
         // costs 1-2 % below; more than one batch ahead is slower again
         p.ahead = p.num_rows * static_cast<int64_t>(ctas) * threads >= 1536LL * sms;
