@@ -34,7 +34,7 @@
 // sample was halved, and places in the result were reserved for four candidates per thread at a time).  Measured before -> after
 // that: rows of full length, 4096 x 32768, k 2048 137 -> 121 us, k 512 111 -> 100 us (5.4 TB/s); a causal chunk of 4096 rows,
 // k 2048 145 -> 121 us (its sample is now taken in whole lines, the ends of its rows are loaded early); ragged rows, 496 x 262144,
-// k 512 74 -> 70 us; 4096 x 65536, k 1024 147 -> 130 us; 1000 x 40000, k 512 37 -> 30 us.
+// k 512 74 -> 70 us (and 67 us with two batches in flight); 4096 x 65536, k 1024 147 -> 130 us; 1000 x 40000, k 512 37 -> 30 us.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
@@ -746,8 +746,11 @@ __global__ void __launch_bounds__(THREADS) topk_registers_kernel(const TopkParam
     if (!done) select_from_histogram<THREADS>(s, dynamic, p.capacity, row, k, out);
 }
 
-template <bool DECODE, int THREADS>
-__global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(const TopkParams p) {
+// TWO: two batches in flight per thread, the next one asked for before this one is looked through: 64 registers, so two CTAs of 512
+// threads per SM instead of three, but a CTA by itself runs at about twice the rate (30 x 262144 in clusters of 8: 14.3 -> 11.7 us,
+// 60 x 50000, k 1024: 11.4 -> 9.1 us, 100 x 262144, k 2048: 29.5 -> 25.8 us).
+template <bool DECODE, int THREADS, bool TWO>
+__global__ void __launch_bounds__(THREADS, TWO ? 1024 / THREADS : 1536 / THREADS) topk_stream_kernel(const TopkParams p) {
     constexpr int kSampleQuads = sample_quads(THREADS);
     begin_dependent_kernel();
     __shared__ Shared s;
@@ -849,18 +852,33 @@ __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_stream_kernel(co
     else __syncthreads();
     const Pool pool{dynamic, &s.pooled, p.capacity};
     // full batches, then what is left of the share, then the quads that are not whole
-    while (left + tid >= kBatch) {
-        send_to_l2(2 * kBatch);
-        pool.take(v, position, 4 * THREADS, f.value);
-        left -= kBatch, position += 4 * kBatch, next += 4 * kBatch;
+    const auto load_next = [&](float4(&to)[kStreamBatch]) {
         if (left + tid >= kBatch) {
 #pragma unroll
-            for (int u = 0; u < kStreamBatch; ++u) v[u] = load_quad(next + 4 * u * THREADS);
+            for (int u = 0; u < kStreamBatch; ++u) to[u] = load_quad(next + 4 * u * THREADS);
         } else {
-            load_batch();
+#pragma unroll
+            for (int u = 0; u < kStreamBatch; ++u) to[u] = u * THREADS < left ? load_quad(next + 4 * u * THREADS) : none;
+        }
+    };
+    // looks through the batch in `now` while the next one is on its way to `then`, and says whether there is one
+    const auto step = [&](float4(&now)[kStreamBatch], float4(&then)[kStreamBatch]) {
+        send_to_l2(2 * kBatch);
+        left -= kBatch, next += 4 * kBatch;
+        if (TWO) load_next(then);
+        pool.take(now, position, 4 * THREADS, f.value);
+        if (!TWO) load_next(then);
+        position += 4 * kBatch;
+        return left + tid > 0;
+    };
+    if (left + tid > 0) {
+        if constexpr (TWO) {
+            float4 w[kStreamBatch];
+            while (step(v, w) && step(w, v)) {}
+        } else {
+            while (step(v, v)) {}
         }
     }
-    if (left + tid > 0) pool.take(v, position, 4 * THREADS, f.value);
     float4 edge[1];
     if (row.stride != 1) {
         for (int32_t e = static_cast<int32_t>(rank) * THREADS + tid; e - (tid & 31) < row.quads; e += static_cast<int32_t>(ctas) * THREADS) {
@@ -935,7 +953,7 @@ cudaError_t set_up(DeviceSetup** result) {
             if (setup.status == cudaSuccess)
                 setup.status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxDynamicBytes));
         };
-        allow(topk_stream_kernel<DECODE, 512>), allow(topk_stream_kernel<DECODE, 256>);
+        allow(topk_stream_kernel<DECODE, 512, true>), allow(topk_stream_kernel<DECODE, 512, false>), allow(topk_stream_kernel<DECODE, 256, false>);
         allow(topk_registers_kernel<DECODE, 512, 4>), allow(topk_registers_kernel<DECODE, 512, 8>), allow(topk_registers_kernel<DECODE, 256, 8>);
         if (setup.status == cudaSuccess) setup.status = cudaDeviceGetAttribute(&setup.sms, cudaDevAttrMultiProcessorCount, dev);
     });
@@ -977,20 +995,19 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
         if (quads <= 512 * 8) return registers(topk_registers_kernel<DECODE, 512, 8>, 512);
         unsigned ctas = 1;  // up to two CTAs per SM, and 8192 values for each (61 x 65536: 10.6 us with 4, 15 with 1 or 8)
         while (ctas < 8 && rows * ctas * 2 <= 2 * sms && static_cast<int64_t>(p.vocab) >= 8192LL * ctas * 2) ctas *= 2;
-        return stream_rows(topk_stream_kernel<DECODE, 512>, 512, ctas);
+        return stream_rows(topk_stream_kernel<DECODE, 512, true>, 512, ctas);
     }
     if (quads <= 128 * 4) return whole(topk_short_kernel<DECODE, 128, 4>, 128);
     if (quads <= 256 * 4) return whole(topk_short_kernel<DECODE, 256, 4>, 256);
     if (quads <= 256 * 8) return registers(topk_registers_kernel<DECODE, 256, 8>, 256);
-    if (p.vocab <= 65536) return stream_rows(topk_stream_kernel<DECODE, 256>, 256, 1);
-    // Very long rows: two CTAs each for up to 1.33 waves of single ones (444 fit the GPU), where the second wave would be mostly
-    // empty.  One | two, us, k 512, rows of ragged and of full length:
-    //   262144 wide   320 rows 62 | 57, 69 | 73    400 rows 64 | 64, 73 | 81   496 rows 76 | 74, 111 | 102   560 rows 88 | 83, 117 | 110
-    //                 640 rows 94 | 91, 132 | 119  800 rows 107 | 110, 139 | 147
-    //   200000 wide   320 rows 50 | 48, 57 | 58    496 rows 64 | 64, 87 | 82    640 rows 75 | 75, 98 | 98     800 rows 89 | 94, 112 | 118
-    //   140000 wide   320 rows 38 | 39, 43 | 47    496 rows 48 | 51, 64 | 68    800 rows 64 | 73, 84 | 97
-    // With k 2048 the pairs are 2-6 % behind that: 200000 wide, 496 rows 69 | 71, 92 | 90; 640 rows 80 | 84, 103 | 108.
-    return stream_rows(topk_stream_kernel<DECODE, 512>, 512, p.vocab >= 196608 && rows < 4LL * sms ? 2 : 1);
+    if (p.vocab <= 65536) return stream_rows(topk_stream_kernel<DECODE, 256, false>, 256, 1);
+    // Longer rows: three CTAs per SM while that makes one wave, then two with two batches in flight each.  Three | two per SM, us,
+    // k 512 unless said otherwise, rows of ragged and of full length:
+    //   320 x 200000  43 | 43, 50 | 64        310 x 140000, k 2048  35 | 37        444 x 262144, full 79 | 86
+    //   496 x 262144  73 | 67, 108 | 88       496 x 100000  35 | 33, 47 | 44       800 x 262144  98 | 97, 134 | 134
+    // (A pair of CTAs per row: 496 x 262144 70, 100; 320 x 200000 45, 56; 800 x 262144 99, 138.)
+    if (rows <= 3LL * sms) return stream_rows(topk_stream_kernel<DECODE, 512, false>, 512, 1);
+    return stream_rows(topk_stream_kernel<DECODE, 512, true>, 512, 1);
 }
 
 }  // namespace
