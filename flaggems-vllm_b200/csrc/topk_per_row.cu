@@ -34,7 +34,7 @@
 // sample was halved, and places in the result were reserved for four candidates per thread at a time).  Measured before -> after
 // that: rows of full length, 4096 x 32768, k 2048 137 -> 121 us, k 512 111 -> 100 us (5.4 TB/s); a causal chunk of 4096 rows,
 // k 2048 145 -> 121 us (its sample is now taken in whole lines, the ends of its rows are loaded early); ragged rows, 496 x 262144,
-// k 512 74 -> 70 us (and 67 us with two batches in flight); 4096 x 65536, k 1024 147 -> 130 us; 1000 x 40000, k 512 37 -> 30 us.
+// k 512 74 -> 70 us (67 us with two batches in flight, 60 us with the longest rows first); 4096 x 65536, k 1024 147 -> 130 us; 1000 x 40000, k 512 37 -> 30 us.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
@@ -66,6 +66,7 @@ struct TopkParams {
     uint32_t capacity;  // of the candidate pool
     bool sampled;       // top_k is small enough for it
     bool ahead;         // the streaming kernel sends batches to L2 ahead of their loads
+    int32_t length_shift;  // where it takes the rows in the order of their lengths: which brings the width below 64
     // decode
     const int32_t* seq_lens;
     int32_t next_n;
@@ -746,10 +747,73 @@ __global__ void __launch_bounds__(THREADS) topk_registers_kernel(const TopkParam
     if (!done) select_from_histogram<THREADS>(s, dynamic, p.capacity, row, k, out);
 }
 
+// The row at `place` in the order of lengths, the longest first: by 64 classes of length and, inside a class, by index, so that every
+// CTA finds the same order.  All threads call it; at most kOrderedRows rows.
+constexpr int kOrderedRows = 1024;
+template <bool DECODE, int THREADS>
+__device__ __forceinline__ int row_at_place(Shared& s, const TopkParams& p, uint32_t place) {
+    constexpr int kPer = kOrderedRows / THREADS, kWarps = THREADS / 32;
+    const int tid = threadIdx.x, lane = tid & 31;
+    uint32_t* const classes = s.hist;       // rows per class
+    uint32_t* const cells = s.hist + 64;    // rows of the class looked for, by 32 rows
+    if (tid < 128) s.hist[tid] = 0u;
+    __syncthreads();
+    uint32_t mine[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const int r = i * THREADS + tid;
+        mine[i] = 64u;
+        if (r < p.num_rows) {
+            int64_t first;
+            mine[i] = 63u - min(static_cast<uint32_t>(row_range<DECODE>(p, r, &first)) >> p.length_shift, 63u);
+            atomicAdd(&classes[mine[i]], 1u);
+        }
+    }
+    __syncthreads();
+    // the class in which the count reaches the place, and the place inside it
+    const auto scan = [&](uint32_t a) {
+#pragma unroll
+        for (int m = 1; m < 32; m <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, a, m);
+            if (lane >= m) a += up;
+        }
+        return a;
+    };
+    const auto find = [&](const uint32_t* counts, uint32_t want, uint32_t* inside) {  // of 64 counts
+        const uint32_t a = counts[2 * lane], b = counts[2 * lane + 1], upto = scan(a + b), before = upto - a - b;
+        const int at = __ffs(__ballot_sync(0xffffffffu, upto > want)) - 1;
+        const uint32_t left = want - __shfl_sync(0xffffffffu, before, at), first = __shfl_sync(0xffffffffu, a, at);
+        *inside = left < first ? left : left - first;
+        return static_cast<uint32_t>(2 * at) + (left < first ? 0u : 1u);
+    };
+    uint32_t inside;
+    const uint32_t wanted = find(classes, place, &inside);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+        const uint32_t votes = __ballot_sync(0xffffffffu, mine[i] == wanted);
+        if (lane == 0) cells[i * kWarps + (tid >> 5)] = __popc(votes);
+    }
+    __syncthreads();
+    uint32_t nth;
+    const uint32_t cell = find(cells, inside, &nth);
+    if (static_cast<int>(cell % kWarps) == (tid >> 5)) {
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const uint32_t votes = __ballot_sync(0xffffffffu, mine[i] == wanted);
+            if (i == static_cast<int>(cell / kWarps) && mine[i] == wanted && __popc(votes & ((1u << lane) - 1u)) == nth) s.result[0] = i * THREADS + tid;
+        }
+    }
+    __syncthreads();
+    const int r = static_cast<int>(s.result[0]);
+    __syncthreads();
+    return r;
+}
+
 // TWO: two batches in flight per thread, the next one asked for before this one is looked through: 64 registers, so two CTAs of 512
 // threads per SM instead of three, but a CTA by itself runs at about twice the rate (30 x 262144 in clusters of 8: 14.3 -> 11.7 us,
-// 60 x 50000, k 1024: 11.4 -> 9.1 us, 100 x 262144, k 2048: 29.5 -> 25.8 us).
-template <bool DECODE, int THREADS, bool TWO>
+// 60 x 50000, k 1024: 11.4 -> 9.1 us, 100 x 262144, k 2048: 29.5 -> 25.8 us).  LONGEST_FIRST: the CTAs (one per row) take the rows in the
+// order of their lengths.
+template <bool DECODE, int THREADS, bool TWO, bool LONGEST_FIRST = false>
 __global__ void __launch_bounds__(THREADS, TWO ? 1024 / THREADS : 1536 / THREADS) topk_stream_kernel(const TopkParams p) {
     constexpr int kSampleQuads = sample_quads(THREADS);
     begin_dependent_kernel();
@@ -758,7 +822,7 @@ __global__ void __launch_bounds__(THREADS, TWO ? 1024 / THREADS : 1536 / THREADS
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t ctas = cluster.num_blocks(), rank = cluster.block_rank();  // the CTAs of a cluster share one row
     const int tid = threadIdx.x;
-    const int r = blockIdx.x >> (31 - __clz(ctas));  // a power of two
+    const int r = LONGEST_FIRST ? row_at_place<DECODE, THREADS>(s, p, blockIdx.x) : static_cast<int>(blockIdx.x >> (31 - __clz(ctas)));  // a power of two
     int64_t first;
     const int32_t len = row_range<DECODE>(p, r, &first);
     const int32_t k = len < p.top_k ? len : p.top_k;
@@ -953,7 +1017,7 @@ cudaError_t set_up(DeviceSetup** result) {
             if (setup.status == cudaSuccess)
                 setup.status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxDynamicBytes));
         };
-        allow(topk_stream_kernel<DECODE, 512, true>), allow(topk_stream_kernel<DECODE, 512, false>), allow(topk_stream_kernel<DECODE, 256, false>);
+        allow(topk_stream_kernel<DECODE, 512, true>), allow(topk_stream_kernel<DECODE, 512, true, true>), allow(topk_stream_kernel<DECODE, 512, false>), allow(topk_stream_kernel<DECODE, 256, false>);
         allow(topk_registers_kernel<DECODE, 512, 4>), allow(topk_registers_kernel<DECODE, 512, 8>), allow(topk_registers_kernel<DECODE, 256, 8>);
         if (setup.status == cudaSuccess) setup.status = cudaDeviceGetAttribute(&setup.sms, cudaDevAttrMultiProcessorCount, dev);
     });
@@ -1007,6 +1071,15 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
     //   496 x 262144  73 | 67, 108 | 88       496 x 100000  35 | 33, 47 | 44       800 x 262144  98 | 97, 134 | 134
     // (A pair of CTAs per row: 496 x 262144 70, 100; 320 x 200000 45, 56; 800 x 262144 99, 138.)
     if (rows <= 3LL * sms) return stream_rows(topk_stream_kernel<DECODE, 512, false>, 512, 1);
+    // Up to two waves of them, the longest rows first: what runs at the end, on a GPU that is no longer full, is then short.  Finding
+    // the order costs a CTA about 1 us, which pays for very long rows of different length only.  By index | longest first, us:
+    //   460 x 131072  39 | 36, full length 50 | 52    460 x 200000  54 | 47, 70 | 73    592 x 200000  60 | 56, 81 | 85
+    //   496 x 262144  67 | 60, full length 90 | 94    592 x 262144, k 1024  76 | 70, 102 | 105
+    //   740 x 131072  54 | 56    740 x 262144  91 | 91, full length 133 | 137    496 x 100000  33 | 33, full length 44 | 46
+    if (rows <= 4LL * sms && rows <= kOrderedRows && p.vocab >= 131072) {
+        while ((p.vocab >> p.length_shift) >= 64) ++p.length_shift;
+        return stream_rows(topk_stream_kernel<DECODE, 512, true, true>, 512, 1);
+    }
     return stream_rows(topk_stream_kernel<DECODE, 512, true>, 512, 1);
 }
 

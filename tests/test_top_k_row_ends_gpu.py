@@ -9,8 +9,9 @@ import flaggems_vllm as fg
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
-# rows, width: clusters of CTAs with two batches in flight, CTAs of 256 threads, CTAs of 512 threads in one wave, and in more
-SHAPES = [(3, 40003), (320, 17000), (320, 70001), (460, 140002)]
+# rows, width: clusters of CTAs with two batches in flight, CTAs of 256 threads, CTAs of 512 threads in one wave, in more, and in more
+# with the longest rows first
+SHAPES = [(3, 40003), (320, 17000), (320, 70001), (460, 70001), (460, 140002), (592, 131072)]
 
 
 def rows_of(rows, width, seed):
