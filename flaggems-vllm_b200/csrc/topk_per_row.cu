@@ -18,8 +18,8 @@
 //   3. the candidates (about 1.1 to 3 k of them) are ranked by a histogram of (key - key(t)), whose bins are fine where
 //      the k-th largest is to be expected; the few candidates of its bin are ranked by counting.
 // Three kernels:
-//   topk_short_kernel       one CTA per row, the row in registers; short rows, of which a large part is selected, go without a
-//                           sample: a coarse histogram of all values, then straight to the ranking
+//   topk_short_kernel       one CTA per row, the row's coarse codes in registers; short rows, of which a large part is selected, go
+//                           without a sample: a coarse histogram of all values, then straight to the ranking
 //   topk_registers_kernel   one CTA per row, the row in registers, its sample taken from them
 //   topk_stream_kernel      longer rows: one CTA, or a thread-block cluster of 2 / 4 / 8 CTAs, streams the row past t; the
 //                           first 64 bytes of every thread are on their way while the sample is evaluated.  In a
@@ -86,6 +86,21 @@ __device__ __forceinline__ uint32_t coarse_bin(float x) {
     const uint32_t h = __half_as_ushort(__float2half_rn(fabsf(x)));
     return ((h ^ sign ^ 0x8000u) & 0xffffu) >> 5;
 }
+
+// The same for two values, x in the low half of the result.
+__device__ __forceinline__ uint32_t coarse_bins(float x, float y) {
+    uint32_t magnitudes, signs, bins;
+    asm("{.reg .f32 a, b;\n"
+        "abs.f32 a, %1;\n"
+        "abs.f32 b, %2;\n"
+        "cvt.rn.f16x2.f32 %0, b, a;}"
+        : "=r"(magnitudes)
+        : "f"(x), "f"(y));
+    asm("prmt.b32 %0, %1, %2, 0xffbb;" : "=r"(signs) : "r"(__float_as_uint(x)), "r"(__float_as_uint(y)));  // each sign 16 times
+    bins = ((magnitudes ^ signs ^ 0x80008000u) >> 5) & 0x07ff07ffu;
+    return bins;
+}
+constexpr uint32_t kBinOfMinusInfinity = 31;  // below it lie the NaNs with their sign bit set only
 
 // A value whose coarse code is `bin`, the lowest one up to the rounding to fp16; -inf for the codes below it.
 __device__ __forceinline__ float value_of_bin(uint32_t bin) {
@@ -600,14 +615,19 @@ __device__ __forceinline__ int32_t row_range(const TopkParams& p, int r, int64_t
     return end > start ? static_cast<int32_t>(end - start) : 0;
 }
 
-// One CTA per row, the row in registers, no sample: the coarse histogram of all values gives the bin of the k-th largest,
-// what lies above it is emitted from the registers, and the values of the bin are ranked by counting.  For short rows, of which
-// a large part is selected: fewer phases, and about 25 instructions per value.
+// One CTA per row, no sample: the coarse histogram of all values gives the bin of the k-th largest, what lies above it is emitted, and
+// the values of the bin are ranked by counting.  For short rows, of which a large part is selected.  Bound by instruction issue, so
+// two values travel in one register from the conversion to fp16 on: their codes are compared by an addition that carries into
+// bit 15 and bit 31, and the values themselves are not kept (the few that are ranked are read once more).
+// 4096 x 4096, k 512: 9.4 k -> 6.2 k warp instructions a row, 45.6 -> 29.9 us; 4096 x 2048 27.1 -> 18.9 us; 1531 x 2600 14.6 -> 10.8 us;
+// 61 x 4096 4.2 -> 3.8 us.  Values beside the row count as -inf, which only matters where the k-th largest is that small: such rows take the histogram route.
 template <bool DECODE, int THREADS, int QUADS>
-__global__ void __launch_bounds__(THREADS) topk_short_kernel(const TopkParams p) {
+__global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_short_kernel(const TopkParams p) {
     begin_dependent_kernel();
     __shared__ Shared s;
     extern __shared__ uint2 dynamic[];
+    constexpr int kPairs = 2 * QUADS;
+    static_assert(kPairs <= 8, "a pair has one bit in either half of a word, from bits 15 and 31 down");
     const int tid = threadIdx.x, lane = tid & 31;
     const int r = blockIdx.x;
     int64_t first;
@@ -620,29 +640,29 @@ __global__ void __launch_bounds__(THREADS) topk_short_kernel(const TopkParams p)
         return;
     }
     const Row row(p.logits + static_cast<int64_t>(r) * p.stride0 + first * p.stride1, p.stride1, len);
+    const int32_t begin = row.first_whole(), whole = row.end_whole() - begin;
     float4 v[QUADS];
 #pragma unroll
-    for (int u = 0; u < QUADS; ++u)
-        if (tid + u * THREADS < row.quads) v[u] = row.load(tid + u * THREADS);
+    for (int u = 0; u < QUADS; ++u) {
+        const int32_t quad = tid + u * THREADS;
+        if (static_cast<uint32_t>(quad - begin) < static_cast<uint32_t>(whole)) v[u] = load_quad(row.x + row.position(quad));
+        else if (quad < row.quads) v[u] = row.load(quad);
+        else v[u] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    }
     clear_histogram<THREADS>(s);
     if (tid < 4) s.counters[tid] = 0u;
     __syncthreads();
-    uint32_t largest = 0u;
-    const auto for_each = [&](auto&& visit) {  // visit(number of the value in the thread, value, position)
+    const auto beyond = [&](int pair) { return (tid & ~31) + (pair >> 1) * THREADS >= row.quads; };  // nothing of it for the warp
+    uint32_t bins[kPairs], largest = 0u;
 #pragma unroll
-        for (int u = 0; u < QUADS; ++u) {
-            if ((tid & ~31) + u * THREADS >= row.quads) break;  // nothing left for the warp
-            const int32_t i = tid + u * THREADS < row.quads ? row.position(tid + u * THREADS) : -8;
-            visit(4 * u, v[u].x, i), visit(4 * u + 1, v[u].y, i + 1), visit(4 * u + 2, v[u].z, i + 2), visit(4 * u + 3, v[u].w, i + 3);
-        }
-    };
-    for_each([&](int, float x, int32_t i) {
-        if (!row.inside(i)) return;
-        const uint32_t bin = coarse_bin(x);
-        atomicAdd(&s.hist[bin], 1u);
-        largest = bin > largest ? bin : largest;
-    });
-    largest = __reduce_max_sync(0xffffffffu, largest);
+    for (int j = 0; j < kPairs; ++j) {
+        bins[j] = 0u;
+        if (beyond(j)) continue;
+        bins[j] = j & 1 ? coarse_bins(v[j >> 1].z, v[j >> 1].w) : coarse_bins(v[j >> 1].x, v[j >> 1].y);
+        atomicAdd(&s.hist[bins[j] & 0xffffu], 1u), atomicAdd(&s.hist[bins[j] >> 16], 1u);
+        asm("max.u16x2 %0, %0, %1;" : "+r"(largest) : "r"(bins[j]));
+    }
+    largest = __reduce_max_sync(0xffffffffu, max(largest & 0xffffu, largest >> 16));
     if (lane == 0) atomicMax(&s.counters[3], largest);
     __syncthreads();
     Threshold t;
@@ -657,19 +677,21 @@ __global__ void __launch_bounds__(THREADS) topk_short_kernel(const TopkParams p)
         t.bin = s.result[0], t.need = s.result[1], t.count = s.result[2];
     }
     const bool take_all = t.need == t.count;
-    if (!take_all && t.count > kCountingMax) {
+    if (t.bin <= kBinOfMinusInfinity || (!take_all && t.count > kCountingMax)) {
         select_from_histogram<THREADS>(s, dynamic, p.capacity, row, k, out);
         return;
     }
-    const uint32_t lowest = take_all ? t.bin : t.bin + 1u;  // of the bins taken whole
+    // pair j: bit 15 - j for its first value, bit 31 - j for its second
+    const auto at_least = [&](uint32_t bin) {
+        const uint32_t up = (0x8000u - bin) * 0x10001u;
+        uint32_t marks = 0u;
+#pragma unroll
+        for (int j = 0; j < kPairs; ++j) marks |= ((bins[j] + up) >> j) & (0x80008000u >> j);
+        return marks;
+    };
     uint2* dense = reinterpret_cast<uint2*>(s.hist);  // the histogram is no longer needed
-    uint32_t mask = 0u;
-    for_each([&](int n, float x, int32_t i) {
-        const uint32_t bin = row.inside(i) ? coarse_bin(x) : 0u;
-        if (row.inside(i) && bin >= lowest) mask |= 1u << n;
-        else if (row.inside(i) && bin == t.bin) dense[atomicAdd(&s.counters[2], 1u)] = make_uint2(order_key(__float_as_uint(x)), static_cast<uint32_t>(i));
-    });
-    uint32_t at = __popc(mask);
+    const uint32_t reach = at_least(t.bin), taken = take_all ? reach : at_least(t.bin + 1u);  // of the bins taken whole
+    uint32_t at = __popc(taken);
 #pragma unroll
     for (int m = 1; m < 32; m <<= 1) {
         const uint32_t up = __shfl_up_sync(0xffffffffu, at, m);
@@ -677,11 +699,21 @@ __global__ void __launch_bounds__(THREADS) topk_short_kernel(const TopkParams p)
     }
     uint32_t base = 0u;
     if (lane == 31 && at > 0u) base = atomicAdd(&s.counters[0], at);
-    at += __shfl_sync(0xffffffffu, base, 31) - __popc(mask);
-    for_each([&](int n, float, int32_t i) {
-        if (mask & (1u << n)) out[at++] = i;
-    });
+    at += __shfl_sync(0xffffffffu, base, 31) - __popc(taken);
+    const auto position = [&](int pair) { return row.position(tid + (pair >> 1) * THREADS) + 2 * (pair & 1); };
+#pragma unroll
+    for (int j = 0; j < kPairs; ++j) {
+        if (beyond(j)) continue;
+        if (taken & (0x8000u >> j)) out[at++] = position(j);
+        if (taken & (0x80000000u >> j)) out[at++] = position(j) + 1;
+    }
     if (take_all) return;
+    for (uint32_t left = reach & ~taken; left;) {
+        const int bit = 31 - __clz(left);
+        left ^= 1u << bit;
+        const int32_t i = position(15 - (bit & 15)) + (bit >> 4);
+        dense[atomicAdd(&s.counters[2], 1u)] = make_uint2(order_key(__float_as_uint(row.value(i))), static_cast<uint32_t>(i));
+    }
     __syncthreads();
     rank_by_counting<THREADS>(s, dense, t.count, t.need, out);
 }
@@ -1050,8 +1082,8 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
     };
     // Few rows: the time of one row counts, so it gets many threads, or a cluster.  Many rows: small CTAs, of which more are
     // resident and cover each other's barriers.  Where the lines lie was measured: 61 x 4096, k 512: 5.1 us with 512 threads, 6.0 with
-    // 256, 8.4 with 128; 4096 x 2048: 57 / 29 / 23 us.  Rows of up to 4096 values need no sample (1531 x 4096, k 512: 17 us,
-    // 23 us with one), longer ones do (4096 x 8192: 49 us, 67 us without).
+    // 256, 8.4 with 128; 4096 x 2048: 57 / 29 / 23 us (both before the codes of two values shared a register: 3.8 and 19 us now).  Rows
+    // of up to 4096 values need no sample (1531 x 4096, k 512: 17 us, 23 us with one), longer ones do (4096 x 8192: 49 us, 67 us without).
     const int64_t rows = p.num_rows;
     if (rows < 2 * sms) {
         if (quads <= 512 * 2) return whole(topk_short_kernel<DECODE, 512, 2>, 512);
