@@ -844,9 +844,10 @@ __device__ __forceinline__ int row_at_place(Shared& s, const TopkParams& p, uint
 // TWO: two batches in flight per thread, the next one asked for before this one is looked through: 64 registers, so two CTAs of 512
 // threads per SM instead of three, but a CTA by itself runs at about twice the rate (30 x 262144 in clusters of 8: 14.3 -> 11.7 us,
 // 60 x 50000, k 1024: 11.4 -> 9.1 us, 100 x 262144, k 2048: 29.5 -> 25.8 us).  LONGEST_FIRST: the CTAs (one per row) take the rows in the
-// order of their lengths.
+// order of their lengths.  CTAs of 256 threads: five per SM with 48 registers; six with 40 were up to 3 % slower (a causal chunk of
+// 4096 x 32768, k 2048 122.5 | 119 us, 1000 x 40000 30.2 | 29.6 us; the pool for k 2048 leaves room for five anyway).
 template <bool DECODE, int THREADS, bool TWO, bool LONGEST_FIRST = false>
-__global__ void __launch_bounds__(THREADS, TWO ? 1024 / THREADS : 1536 / THREADS) topk_stream_kernel(const TopkParams p) {
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 5 : TWO ? 2 : 3) topk_stream_kernel(const TopkParams p) {
     constexpr int kSampleQuads = sample_quads(THREADS);
     begin_dependent_kernel();
     __shared__ Shared s;
