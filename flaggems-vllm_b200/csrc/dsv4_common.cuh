@@ -129,12 +129,13 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
 // The same for the line that holds p, whatever its alignment.
 __device__ __forceinline__ void prefetch_line_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// Whether this CTA (of a one-dimensional grid) is among those that can be resident while the kernel in front drains, and so has
-// time to fill with prefetches before wait_for_preceding_kernel() returns.  Later CTAs find that kernel complete.
+// Whether this CTA (of 128 threads, in a one-dimensional grid) is among those that can be resident while the kernel in front drains,
+// and so has time to fill with prefetches before wait_for_preceding_kernel() returns.  Later CTAs find that kernel complete.
 // Measured in chains of launches, inputs from HBM: norms and quantisers of 2462 tokens 18.9 -> 17.9 us, the indexer's query and key
 // kernels of 2500 tokens 15.8 -> 15.2 us, a prefill layer of 1531 tokens 213 -> 209.4 us.  A warp asks for what it loads first
-// and no more: twice that cost more L2 requests than it saved (15.8 -> 16.2 us).
-__device__ __forceinline__ bool starts_early() { return blockIdx.x * blockDim.x < 148u * 1536u; }
+// and no more: twice that cost more L2 requests than it saved (15.8 -> 16.2 us).  Not in the epilogue's quantiser: no gain at 8192
+// tokens, and 61 tokens out of L2 took 4.1 us instead of 3.5.
+__device__ __forceinline__ bool starts_early() { return blockIdx.x < 148u * 12u; }
 
 // First statement of such a kernel, or the first after its prefetches.
 __device__ __forceinline__ void begin_dependent_kernel() {

@@ -45,19 +45,13 @@ constexpr int kCtasPerSm = 7;      // 72 registers
 template <int WARPS, bool PACKED, bool FASTDIV, int U, int MIN_CTAS, bool WIDE>
 __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kernel(const InvRopeParams p, const int heads_per_task, const uint32_t tasks_per_token,
                                                                       const uint32_t tpt_mul, const uint32_t tpt_shift) {
+    begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const uint32_t task = blockIdx.x * WARPS + (threadIdx.x >> 5);
     if (task >= static_cast<uint32_t>(p.padded_tokens) * tasks_per_token) return;
     const uint32_t token = fast_div(task, tpt_mul, tpt_shift);
     const int head_begin = static_cast<int>(task - token * tasks_per_token) * heads_per_task;
     const int head_end = head_begin + heads_per_task < p.num_heads ? head_begin + heads_per_task : p.num_heads;
-    const uint8_t* in_token = p.o + static_cast<int64_t>(token) * p.o_stride_token * 2;
-    if (token < p.num_tokens && starts_early()) {
-        // the lines of the first pass, one per lane
-        if (lane < 8 * U && head_begin + (lane >> 3) < head_end) prefetch_line_l2(in_token + (head_begin + (lane >> 3)) * p.o_stride_head * 2 + 128 * (lane & 7));
-        if (lane == 31) prefetch_line_l2(p.positions + token);
-    }
-    begin_dependent_kernel();
     if (token >= p.num_tokens) {
         // token padding of the scale storage (a multiple of 4 tokens): zero scales
         for (int head = head_begin; head < head_end; ++head) {
@@ -72,6 +66,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kerne
         }
         return;
     }
+    const uint8_t* in_token = p.o + static_cast<int64_t>(token) * p.o_stride_token * 2;
     Bytes32 v[U], v_next[U];
     uint32_t tail[U], tail_next[U];
     const auto load_pass = [&](int h0, Bytes32 (&rv)[U], uint32_t (&rt)[U]) {
