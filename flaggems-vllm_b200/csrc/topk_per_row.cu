@@ -1090,7 +1090,7 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
         if (quads <= 512 * 2) return whole(topk_short_kernel<DECODE, 512, 2>, 512);
         if (quads <= 512 * 4) return registers(topk_registers_kernel<DECODE, 512, 4>, 512);
         if (quads <= 512 * 8) return registers(topk_registers_kernel<DECODE, 512, 8>, 512);
-        unsigned ctas = 1;  // up to two CTAs per SM, and 8192 values for each (61 x 65536: 10.6 us with 4, 15 with 1 or 8)
+        unsigned ctas = 1;  // up to two CTAs per SM, and 8192 values for each (61 x 65536: 10.6 us with 4, 15 with 1 or 8; 8.9 us with 4 since two batches are in flight)
         while (ctas < 8 && rows * ctas * 2 <= 2 * sms && static_cast<int64_t>(p.vocab) >= 8192LL * ctas * 2) ctas *= 2;
         return stream_rows(topk_stream_kernel<DECODE, 512, true>, 512, ctas);
     }
