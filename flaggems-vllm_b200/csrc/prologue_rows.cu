@@ -55,9 +55,13 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) prologue_rows_kernel(con
     if (static_cast<int64_t>(blockIdx.x) < kv_ctas) {
         // ---- latent KV: RoPE tail + UE8M0/e4m3 quantisation + scatter through slot_mapping
         const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + warp;
-        if (t >= p.num_tokens_insert) return;
-        const int64_t slot = p.slot_mapping[t];
-        if (slot < 0) return;
+        const int64_t slot = t < p.num_tokens_insert ? p.slot_mapping[t] : -1;
+        if (slot < 0) {
+            // A launch must not end before the kernel in front of it: the next one in the stream waits for this one only.  (One of
+            // nothing but skipped tokens and no heads would.)
+            if (PDL == 1) wait_for_preceding_kernel();
+            return;
+        }
         const int64_t pos = p.position_ids[t];
         if (CHECKED) {
             const bool bad_pos = pos < 0 || pos >= p.max_pos, bad_slot = slot >= p.num_slots;

@@ -556,6 +556,32 @@ def test_programmatic_dependent_launch_gives_the_same_result(mode):
     assert _native.set_pdl(previous) == previous
 
 
+@pytest.mark.parametrize("mode", [1, 2])
+def test_a_call_without_work_keeps_the_order_of_its_neighbours(mode):
+    """No heads and only skipped tokens: nothing to do, but the kernel behind the call waits for the call alone, so the call may
+    not end before the kernel in front of it.  A long producer, the empty call, a consumer of what the producer writes last."""
+    g = torch.Generator(device=DEV).manual_seed(5)
+    n, act = 65536, lambda *shape: torch.empty(shape, dtype=torch.bfloat16, device=DEV).normal_(generator=g)
+    weights = act(1536), act(512)
+    kc, cs = torch.zeros(1, 64 * 584, dtype=torch.uint8, device=DEV), torch.zeros(4, 64, device=DEV)
+    empty_q, kv = torch.empty(8, 0, 512, dtype=torch.bfloat16, device=DEV), torch.zeros(8, 512, dtype=torch.bfloat16, device=DEV)
+    slots, pos = torch.full((8,), -1, dtype=torch.int64, device=DEV), torch.zeros(8, dtype=torch.int64, device=DEV)
+    previous = _native.set_pdl(mode)
+    try:
+        for _ in range(8):
+            qr, latent = act(n, 1536), act(n, 512)  # other values every time: memory of an earlier pass does not help
+            torch.cuda.synchronize()
+            normed, _ = flaggems_vllm.fused_q_kv_rmsnorm(qr, latent, *weights, 1e-6)
+            op(empty_q, kv, kc, slots, pos, cs, 1e-6, 64)
+            codes, scales = flaggems_vllm.per_token_group_quant_fp8(normed, 128)
+            torch.cuda.synchronize()
+            want_codes, want_scales = flaggems_vllm.per_token_group_quant_fp8(normed, 128)
+            assert torch.equal(codes.view(torch.uint8), want_codes.view(torch.uint8)) and torch.equal(scales, want_scales)
+    finally:
+        _native.set_pdl(previous)
+    assert not kc.any()
+
+
 @pytest.mark.parametrize("staging", [0, 1])
 @pytest.mark.parametrize("pdl", [0, 1, 2])
 @pytest.mark.parametrize("n,h", [(37, 9), (600, 128)])
