@@ -39,9 +39,16 @@ int current_pdl() {
 // Where the rows variant takes the cos|sin rows from: -1 = by launch size (per-warp fetch up to kPerWarpTableRows rows
 // of q, shared-memory staging above), 0 = always per warp, 1 = always staged.
 std::atomic<int> g_table_staging{-2};  // -2: not initialised from the environment yet
-// The line between them, per warp (with its rows sent to L2 ahead) | staged, us a launch behind another one:
-//   256 x 128 rows 10.7 | 12.0   1024 x 128  39.7 | 41.4   4096 x 128  157.4 | 158.8   16384 x 128  627 | 631   32768 x 64  643.6 | 644.3
-//   32768 x 128  1261-1268 | 1256
+// The line between them.  Per warp | staged, us a launch (tokens x heads), from a graph one behind another in launch modes 0, 1 and 2,
+// and in mode 2 with a small torch kernel in front of each, its 1.2 us included, the better of two runs:
+//   256 x 128     11.8 | 11.8     11.3 | 11.5     10.3 | 11.6     12.5 | 13.3
+//   1024 x 128    41.3 | 41.4     40.5 | 41.2     39.4 | 41.0     42.2 | 42.8
+//   4096 x 128     158 | 159       157 | 159       156 | 158       159 | 160
+//   16384 x 128    625 | 627       624 | 633       632 | 628       626 | 629
+//   32768 x 128   1244 | 1252     1254 | 1266     1271 | 1253     1271 | 1264
+// Modes 0 and 1 send nothing to L2 ahead; that the per-warp form is no slower there is for the barrier it does without.  From about
+// 20000 tokens on, up to the line, the two are level: medians of five processes of the default mode 26000 x 64 507.5 | 509.5,
+// 32768 x 64 641-652 | 641-643, 32768 x 48 486-494 | 488-489.
 constexpr int64_t kPerWarpTableRows = 2097152;
 
 int current_table_staging() {

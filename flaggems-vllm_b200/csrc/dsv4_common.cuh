@@ -57,7 +57,7 @@ struct PrologueParams {
     // stream has finished, wait for it only before touching q and kv (rows variant; 0 = ordinary launch)
     int pdl;
     // rows variant: 1 = the cos|sin rows of a tile go through shared memory (one fetch per CTA), 0 = every warp
-    // fetches the table row of its own rows into registers (no barrier; chosen for launches of a few waves)
+    // fetches the table row of its own rows into registers (no barrier; chosen except for the largest launches)
     int table_staging;
     // bulk variant: SM cycles after which a wait on a shared-memory barrier gives up (the kernel then sets the
     // device error word and returns), and a self-test hook: the tile whose loader announces bytes it never sends

@@ -39,8 +39,9 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) prologue_rows_kernel(con
     // that the preceding kernel does not write the former).
     if (PDL == 2) {
         // The tile's rows, positions and slots go to L2 while the kernel in front drains: a launch of a few waves spends a tenth
-        // of its time on the way from that kernel's end to its own full rate (256 x 128 heads: 12.0 -> 10.7 us; large launches,
-        // which are staged, have nothing to gain).
+        // of its time on the way from that kernel's end to its own full rate (256 x 128 heads behind a launch of its own kind 12.0 ->
+        // 10.7 us, behind a torch kernel, which lets it start only at its end, 12.1 -> 11.4 us, on an idle GPU no change; large
+        // launches, which are staged, have nothing to gain).
         if (!STAGED && starts_early()) {
             const bool is_kv = static_cast<int64_t>(blockIdx.x) < kv_ctas;
             const int64_t rows = is_kv ? WARPS : TILE;

@@ -587,8 +587,9 @@ def test_a_call_without_work_keeps_the_order_of_its_neighbours(mode):
 @pytest.mark.parametrize("n,h", [(37, 9), (600, 128)])
 def test_every_launch_mode_and_table_staging_gives_the_oracle_result(staging, pdl, n, h):
     """The rows kernel has two ways to fetch the cos/sin rows (per warp into registers, or once per CTA through shared
-    memory; chosen by launch size unless forced) and three launch modes; the result does not depend on either.  Both
-    sizes are run in both staging modes: a launch of a few CTAs and one above the size at which the library switches."""
+    memory; chosen by launch size unless forced) and three launch modes; the result does not depend on either.  Both ways are
+    forced here, for a launch of a few CTAs and for one of several waves; the size at which the library switches by itself
+    has a test of its own below."""
     q, kv, kc, slots, pos, cs = random_case(n, h, 64, n // 64 + 3, seed=1000 + n, minus_one=max(1, n // 10))
     previous_staging, previous_pdl = _native.set_table_staging(staging), _native.set_pdl(pdl)
     try:
@@ -597,6 +598,29 @@ def test_every_launch_mode_and_table_staging_gives_the_oracle_result(staging, pd
         _native.set_table_staging(previous_staging)
         _native.set_pdl(previous_pdl)
     assert _native.set_table_staging(previous_staging) == previous_staging
+
+
+@pytest.mark.parametrize("n,h", [(16384, 128), (16385, 128)])
+def test_the_choice_by_launch_size_gives_what_both_forms_give(n, h):
+    """The sizes at which the library hands over from one way of fetching the cos/sin rows to the other (2^21 rows).  Chosen by
+    size, forced either way: the same bytes."""
+    g = torch.Generator(device=DEV).manual_seed(n)
+    q0 = torch.empty(n, h, 512, dtype=torch.bfloat16, device=DEV).normal_(generator=g)
+    kv = torch.empty(n, 512, dtype=torch.bfloat16, device=DEV).normal_(generator=g)
+    cs, blocks = workloads.cos_sin_table(4096).to(DEV), -(-n // 64)
+    pos, slots = torch.randint(0, 4096, (n,), generator=g, device=DEV), torch.randperm(blocks * 64, generator=g, device=DEV)[:n].contiguous()
+    results = []
+    previous = _native.set_table_staging(-1)
+    try:
+        for staging in (-1, 0, 1):
+            _native.set_table_staging(staging)
+            q, kc = q0.clone(), torch.zeros(blocks, 64 * 584, dtype=torch.uint8, device=DEV)
+            op(q, kv, kc, slots, pos, cs, 1e-6, 64)
+            results.append((q, kc))
+    finally:
+        _native.set_table_staging(previous)
+    for q, kc in results[1:]:
+        assert torch.equal(q.view(torch.int16), results[0][0].view(torch.int16)) and torch.equal(kc, results[0][1])
 
 
 @pytest.mark.parametrize("q_off,kv_off,cs_off", [(1, 0, 0), (0, 3, 0), (0, 0, 1), (5, 7, 3), (4, 4, 2)])
