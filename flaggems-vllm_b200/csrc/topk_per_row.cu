@@ -56,6 +56,12 @@ constexpr int kSelectBatch = 4;          // candidates per thread that share one
 // Quads in the sample of the streaming kernel with CTAs of that size.  A larger sample leaves fewer candidates to rank, a smaller one
 // is sooner done: rows of 32768 to 65536 values with CTAs of 256 threads, 512 | 1024 quads, 4096 x 32768, k 2048 121 | 128 us,
 // k 512 100 | 111 us; 4096 x 65536, k 1024 132 | 142 us.
+// All that holds for values independent of their neighbours.  Where they vary smoothly along the row, the 32 values of a run count for
+// less, and a row is misjudged (and read twice more) oftener, with either size alike.  Share of such rows among moving sums of L
+// independent values, 32768 to 262144 wide, k 512 to 2048: none up to L 4, 0-2 % at 8, 4-8 % at 16, 10-20 % at 32, 18-31 % at 128.
+// L 1 | 8 | 32 | 128, us (in brackets with 1024 quads for all CTAs, in the kernel before):
+//   4096 x 32768, k 2048  117 | 152 | 193 | 210 (137 | 173 | 227 | 230)     k 512  98 | 127 | 166 | 191 (111 | 142 | 180 | 202)
+//   4096 x 65536, k 1024  182 | 242 | 303 | 352 (195 | 255 | 333 | 385)     496 x 262144, k 512  92 | 203 | 239 | 257 (101 | 227 | 313 | 361)
 __host__ __device__ constexpr int sample_quads(int threads) { return threads >= 512 ? 1024 : 512; }
 
 struct TopkParams {
@@ -620,7 +626,10 @@ __device__ __forceinline__ int32_t row_range(const TopkParams& p, int r, int64_t
 // two values travel in one register from the conversion to fp16 on: their codes are compared by an addition that carries into
 // bit 15 and bit 31, and the values themselves are not kept (the few that are ranked are read once more).
 // 4096 x 4096, k 512: 9.4 k -> 6.2 k warp instructions a row, 45.6 -> 29.9 us; 4096 x 2048 27.1 -> 18.9 us; 1531 x 2600 14.6 -> 10.8 us;
-// 61 x 4096 4.2 -> 3.8 us.  Values beside the row count as -inf, which only matters where the k-th largest is that small: such rows take the histogram route.
+// 61 x 4096 4.2 -> 3.8 us.  Values beside the row count as -inf, which only matters where the k-th largest is that small: such rows
+// take the histogram route.  4096 x 1400, k 512, 400 finite values a row and -inf or the lowest float behind them: 73 us, where rows of
+// finite values take 20 us (ranking the thousand equal values by counting took 1267 us); 61 x 1400 7.4 and 3.0 us; 4096 x 4096, where
+// they are too many for the pool, 201 and 30 us.
 template <bool DECODE, int THREADS, int QUADS>
 __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_short_kernel(const TopkParams p) {
     begin_dependent_kernel();
@@ -1076,8 +1085,12 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
     };
     const auto stream_rows = [&](auto* kernel, int threads, unsigned ctas) {
         p.capacity = pool_capacity(Expected(p.top_k, std::min(p.vocab, 4 * sample_quads(threads)), p.vocab));
-        // pays once the GPU is full (4096 x 32768, k 2048: 145 -> 137 us; 1000 x 40000: 59 -> 53 us; 496 x 262144: 107 -> 100 us),
-        // costs 1-2 % below; more than one batch ahead is slower again
+        // Pays once the GPU is full.  Without | with it, us, k 512 and rows of full length unless said otherwise: 4096 x 32768 106 | 98,
+        // causal with k 2048 130 | 117; 1531 x 32768 49.4 | 45.3; 1000 x 40000 40.7 | 38.6; 890 x 32768, k 2048 40.1 | 37.5; 496 x 262144
+        // 92.0 | 90.8, ragged 60.6 | 59.4; 444 x 100000 ragged 29.5 | 27.7.  Below the line small CTAs gain too (880 x 32768, k 2048
+        // 40.0 | 37.5; 600 x 32768 21.3 | 20.7; 296 x 65536 25.3 | 22.7), clusters hardly (61 x 65536 10.1 | 10.3; 140 x 65536 13.4 |
+        // 13.0; 290 x 40000 14.2 | 14.1).  Three wide CTAs per SM, which are past it only when all are there, gain up to 100000 values
+        // (320 x 100000 30.6 | 30.0) and lose beyond (400 x 140000 42.8 | 43.7; 440 x 262144 74.3 | 78.2; 444 x 262144 75.0 | 79.2).
         p.ahead = p.num_rows * static_cast<int64_t>(ctas) * threads >= 1536LL * sms;
         return launch(kernel, p, threads, ctas, stream);
     };
@@ -1090,7 +1103,11 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
         if (quads <= 512 * 2) return whole(topk_short_kernel<DECODE, 512, 2>, 512);
         if (quads <= 512 * 4) return registers(topk_registers_kernel<DECODE, 512, 4>, 512);
         if (quads <= 512 * 8) return registers(topk_registers_kernel<DECODE, 512, 8>, 512);
-        unsigned ctas = 1;  // up to two CTAs per SM, and 8192 values for each (61 x 65536: 10.6 us with 4, 15 with 1 or 8; 8.9 us with 4 since two batches are in flight)
+        // Up to two CTAs per SM, and 8192 values for each.  One | two | four CTAs a row, us: 61 x 17000 7.3 | 7.6 | 7.9; 61 x 40000 9.1 |
+        // 8.7 | 9.0; 100 x 20000 7.6 | 8.9 | 12.6; 140 x 20000 8.0 | 9.2 | 15.8; 140 x 40000 10.9 | 11.6 | 18.9; 148 x 65536 13.7 | 13.6 |
+        // 21.6; 120 x 262144 34.3 | 28.0 | 33.8.  (61 x 65536: 10.6 us with four, 15 with one or eight, before two batches were in flight;
+        // 10 us now with four.)  So from about 100 rows on a pair wants 32768 values or more for each, which the rule does not ask for.
+        unsigned ctas = 1;
         while (ctas < 8 && rows * ctas * 2 <= 2 * sms && static_cast<int64_t>(p.vocab) >= 8192LL * ctas * 2) ctas *= 2;
         return stream_rows(topk_stream_kernel<DECODE, 512, true>, 512, ctas);
     }
@@ -1102,7 +1119,12 @@ cudaError_t launch_topk(TopkParams& p, cudaStream_t stream) {
     // k 512 unless said otherwise, rows of ragged and of full length:
     //   320 x 200000  43 | 43, 50 | 64        310 x 140000, k 2048  35 | 37        444 x 262144, full 79 | 86
     //   496 x 262144  73 | 67, 108 | 88       496 x 100000  35 | 33, 47 | 44       800 x 262144  98 | 97, 134 | 134
-    // (A pair of CTAs per row: 496 x 262144 70, 100; 320 x 200000 45, 56; 800 x 262144 99, 138.)
+    //   320 x 262144  54 | 52, 62 | 80        400 x 262144  57 | 61, 70 | 86       444 x 262144  60 | 63, 79 | 86
+    //   320 x 262144, k 2048  57 | 54         400 x 262144, k 2048  60 | 64        400 x 131072  33 | 37
+    //   445 x 100000  27.6 | 31.6
+    // (A pair of CTAs per row: 496 x 262144 70, 100; 320 x 200000 45, 56; 320 x 262144 53, 69; 400 x 262144 60, 77; 800 x 262144 99, 138.)
+    // Up to 444 rows the longest first with two per SM (see below) would take 44, 51 and 56 us for 320, 400 and 444 ragged rows of 262144,
+    // but 83, 89 and 89 us for rows of full length, and the host does not know which they are.
     if (rows <= 3LL * sms) return stream_rows(topk_stream_kernel<DECODE, 512, false>, 512, 1);
     // Up to two waves of them, the longest rows first: what runs at the end, on a GPU that is no longer full, is then short.  Finding
     // the order costs a CTA about 1 us, which pays for very long rows of different length only.  By index | longest first, us:

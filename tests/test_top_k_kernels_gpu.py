@@ -60,6 +60,24 @@ def test_rows_that_mislead_the_sample(width):
     check(x, torch.zeros_like(ends), ends, 512)
 
 
+@pytest.mark.parametrize("rows,width", [(300, 8000), (300, 33000), (300, 70001), (450, 140000)])
+@pytest.mark.parametrize("length", [8, 128])
+def test_values_that_vary_smoothly_along_the_row(rows, width, length):
+    """Moving sums over `length` values: neighbours are alike, so the sample, which is taken in runs of neighbours, says less than
+    its size and misjudges up to a third of the rows, towards too few candidates as towards too many.  Every row against its
+    top k, with as many rows as take small CTAs, wide ones, and two batches in flight."""
+    g = torch.Generator(device=DEV).manual_seed(width + length)
+    steps = torch.randn(rows, width + length, generator=g, device=DEV).cumsum(dim=1, dtype=torch.float64)
+    x = ((steps[:, length:] - steps[:, :-length]) * length**-0.5).float()
+    for k in (512, 2048):
+        out = torch.full((rows, k), -7, dtype=torch.int32, device=DEV)
+        zeros, ends = torch.zeros(rows, dtype=torch.int32, device=DEV), torch.full((rows,), width, dtype=torch.int32, device=DEV)
+        fg.top_k_per_row_prefill(x, zeros, ends, out, rows, x.stride(0), x.stride(1), k)
+        chosen = out.long().sort(dim=1).values
+        assert bool((chosen[:, 0] >= 0).all()) and bool((chosen[:, -1] < width).all()) and bool((chosen[:, 1:] > chosen[:, :-1]).all())
+        assert torch.equal(x.gather(1, chosen).sort(dim=1).values, x.topk(k, dim=1).values.sort(dim=1).values)
+
+
 @pytest.mark.parametrize("rows", [8, 320])
 @pytest.mark.parametrize("width", [1500, 3000, 8000, 15000, 20000, 70000])
 def test_nans_rank_by_their_sign(width, rows):
@@ -89,11 +107,12 @@ def test_nans_rank_by_their_sign(width, rows):
     assert torch.equal(key.gather(1, chosen).sort(dim=1).values, key.topk(k, dim=1).values.sort(dim=1).values)
 
 
-@pytest.mark.parametrize("rows,width", [(900, 33000), (450, 70001), (450, 140000), (700, 65540), (450, 196608), (600, 196612)])
+@pytest.mark.parametrize("rows,width", [(900, 33000), (444, 70001), (450, 70001), (450, 140000), (700, 65540), (450, 196608), (600, 196612)])
 @pytest.mark.parametrize("k", [512, 2048])
 def test_rows_that_fill_the_gpu(rows, width, k):
-    """The streaming kernel with batches sent to L2 ahead of their loads: small CTAs, wide ones, and pairs of wide ones.  Ranges of
-    every length, most of them starting off a 16-byte boundary, ties included."""
+    """The streaming kernel with batches sent to L2 ahead of their loads: small CTAs, wide ones with one batch in flight (444 rows,
+    the most they take) and with two, and these with the longest rows first.  Ranges of every length, most of them starting off a
+    16-byte boundary, ties included."""
     g = torch.Generator(device=DEV).manual_seed(rows + width)
     x = torch.randn(rows, width, generator=g, device=DEV)
     x[::3] = (x[::3] * 64).round() / 64
