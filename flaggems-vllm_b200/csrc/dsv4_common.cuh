@@ -131,11 +131,14 @@ __device__ __forceinline__ void prefetch_line_l2(const void* p) { asm volatile("
 
 // Whether this CTA (of 128 threads, in a one-dimensional grid) is among those that can be resident while the kernel in front drains,
 // and so has time to fill with prefetches before wait_for_preceding_kernel() returns.  Later CTAs find that kernel complete.
-// Measured in chains of launches, inputs from HBM: norms and quantisers of 2462 tokens 18.9 -> 17.9 us, the indexer's query and key
-// kernels of 2500 tokens 15.8 -> 15.2 us, a prefill layer of 1531 tokens 213 -> 209.4 us.  A warp asks for what it loads first
-// and no more: twice that cost more L2 requests than it saved (15.8 -> 16.2 us).  Not in the epilogue's quantiser: no gain at 8192
-// tokens, and 61 tokens out of L2 took 4.1 us instead of 3.5.
-__device__ __forceinline__ bool starts_early() { return blockIdx.x < 148u * 12u; }
+// Measured in chains of this library's launches, which let the next one start early, inputs from HBM: norms and quantisers of 2462
+// tokens 18.9 -> 17.9 us, the indexer's query and key kernels of 2500 tokens 15.4 -> 14.7 us, 8192 tokens of norms 10.7 -> 10.4 us, a
+// prefill layer of 1531 tokens 213 -> 209 us.  Behind a torch kernel, which lets the next one start at its end only, there is little to
+// gain: the prologue of 256 x 128 heads 12.1 -> 11.4 us, the indexer 16.4 -> 16.0, norms 11.8 -> 11.9, the quantiser (2462 x 7168)
+// 8.9 -> 9.1; on an idle GPU nothing.  A warp asks for what it loads first and no more: twice that cost more L2 requests than it saved
+// (15.8 -> 16.2 us).  Not in the epilogue's quantiser: no gain at 8192 tokens, and 61 tokens out of L2 took 4.1 us instead of 3.5.
+constexpr unsigned kEarlyCtas = 148 * 12;  // a B200's SMs, CTAs on each: a hint, which any other number would leave correct
+__device__ __forceinline__ bool starts_early() { return blockIdx.x < kEarlyCtas; }
 
 // First statement of such a kernel, or the first after its prefetches.
 __device__ __forceinline__ void begin_dependent_kernel() {

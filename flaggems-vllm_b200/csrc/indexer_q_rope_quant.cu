@@ -445,10 +445,12 @@ cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q,
     if (heads_shape) {
         constexpr int WARPS = 4;
         // Heads per warp: few rows, short tasks, so that there are enough of them; many rows, long ones, whose set-up more heads
-        // share.  Both sides of each line, FP8 / MXFP4, us a launch of 64 heads a token, rows from HBM:
-        //   8 | 16            832 tokens  6.2 / 6.4 | 6.0 / 6.2 (rows in L2: 5.0 / 5.0 | 5.0 / 5.1)   1023 tokens  7.2 / 7.3 | 6.5 / 6.6
-        //   16 | 64          3072 tokens 15.4 / 15.5 | 16.9 / 16.9                                    4096 tokens 20.4 / 20.5 | 19.2 / 18.4
-        //   64 | prefetch    8192 tokens 36.1 / 34.5 | 37.2 / 35.3     9216 tokens 43.3 / 41.4 | 41.1 / 39.5     65536 tokens 257 / 240 | 240 / 231
+        // share.  Both sides of each line, FP8 / MXFP4, us a launch of 64 heads a token, from a graph with three inputs in rotation
+        // (from 3072 tokens on they come from HBM):
+        //   8 | 16            832 tokens  5.5 / 5.4 | 5.2 / 5.2          1023 tokens  6.1 / 6.1 | 5.3 / 5.4
+        //   16 | 64          3072 tokens 14.5 / 14.8 | 15.5 / 16.2       4096 tokens 19.6 / 19.8 | 17.7 / 17.3
+        //   64 | prefetch    8192 tokens 34.9 / 33.1 | 35.6 / 34.0       9216 tokens 42.2 / 39.9 | 39.2 / 37.3     65536 tokens 255 / 237 | 238 / 226-229
+        // The requests ahead of the wait change nothing for the last form (65536 tokens without them: 239 / 226-227).
         // Tasks of 64 heads fill the GPU with 4144 tokens at a time: 4608 tokens would be 11 % faster with 32, 8192 are 3 % slower.
         const bool prefetch = rows >= 589824;
         const int heads_per_task = prefetch ? 32 : rows >= 212992 ? 64 : rows >= 57344 ? 16 : 8;
