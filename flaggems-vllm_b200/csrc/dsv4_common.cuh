@@ -474,19 +474,25 @@ __device__ __forceinline__ uint2 quant8_by(const uint4& v, const ScaleDivider<MO
     return make_uint2(pack_e4m3x4(q[0], q[1], q[2], q[3]), pack_e4m3x4(q[4], q[5], q[6], q[7]));
 }
 
-// 8 bf16 values times the exact reciprocal of a power-of-two scale (same result as dividing by it).  The products are
-// formed on the packed words (`mul.rn.bf16x2`: a power-of-two factor only moves the exponent, so bf16 holds them
-// exactly; results below the bf16 range become zero with their sign, as their e4m3 bytes would anyway) and widened
-// afterwards: 4 multiplies instead of 8.  The reciprocal's exponent field 254 - code is in range for every bf16 maximum.
+// Both halves of a bf16 pair times a bf16 power of two, as fp32: exact, one instruction a value (the sum with -0 keeps the sign of
+// a zero).
+__device__ __forceinline__ float2 scaled_pair(uint32_t pair, uint16_t factor) {
+    float2 r;
+    asm("{.reg .b16 l, h;\n\t"
+        "mov.b32 {l, h}, %2;\n\t"
+        "fma.rn.f32.bf16 %0, l, %3, %4;\n\t"
+        "fma.rn.f32.bf16 %1, h, %3, %4;}"
+        : "=f"(r.x), "=f"(r.y)
+        : "r"(pair), "h"(factor), "f"(-0.0f));
+    return r;
+}
+
+// 8 bf16 values times the exact reciprocal of a power-of-two scale (same result as dividing by it).  The reciprocal's exponent field
+// 254 - code is in range for every bf16 maximum.
 __device__ __forceinline__ uint2 quant8_pow2(const uint4& v, uint32_t code) {
-    const uint32_t inv2 = ((254u - code) << 7) * 0x00010001u;  // 2^(127 - code) in both halves
-    uint32_t w[4];
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(w[0]) : "r"(v.x), "r"(inv2));
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(w[1]) : "r"(v.y), "r"(inv2));
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(w[2]) : "r"(v.z), "r"(inv2));
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(w[3]) : "r"(v.w), "r"(inv2));
-    return make_uint2(pack_e4m3x4(bf16_lo(w[0]), bf16_hi(w[0]), bf16_lo(w[1]), bf16_hi(w[1])),
-                      pack_e4m3x4(bf16_lo(w[2]), bf16_hi(w[2]), bf16_lo(w[3]), bf16_hi(w[3])));
+    const auto factor = static_cast<uint16_t>((254u - code) << 7);  // 2^(127 - code)
+    const float2 x0 = scaled_pair(v.x, factor), x1 = scaled_pair(v.y, factor), x2 = scaled_pair(v.z, factor), x3 = scaled_pair(v.w, factor);
+    return make_uint2(pack_e4m3x4(x0.x, x0.y, x1.x, x1.y), pack_e4m3x4(x2.x, x2.y, x3.x, x3.y));
 }
 
 // 8 bf16 -> 8 e4m3 bytes of value x / 2^(code-127) (division by a power of two: exact).

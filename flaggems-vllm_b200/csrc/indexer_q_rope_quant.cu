@@ -33,6 +33,7 @@ struct IndexerQParams {
     int64_t num_tokens;
     int32_t num_heads;
     uint32_t heads_mul, heads_shift;
+    float minus_zero;  // -0.0f: see rotate_two()
     int32_t scales_word_aligned;  // fp4: every head's group of scale bytes starts on a 4-byte boundary
 };
 
@@ -65,8 +66,10 @@ __device__ __forceinline__ uint32_t pack_e2m1x2(float lo, float hi) {
     return r;
 }
 
-// Four packed bf16 pairs -> one word of eight e2m1 codes (element 0 in bits 0-3), round to nearest even, saturating at +-6.
-__device__ __forceinline__ uint32_t pack_e2m1x8(const uint32_t (&w)[4]) {
+// Four packed bf16 pairs times 2^(127 - code), the factor given as bf16 -> one word of eight e2m1 codes (element 0 in bits 0-3),
+// round to nearest even, saturating at +-6.  Exact before the conversion (scaled_pair()).
+__device__ __forceinline__ uint32_t pack_e2m1x8(const uint4& v, uint16_t factor) {
+    const float2 x0 = scaled_pair(v.x, factor), x1 = scaled_pair(v.y, factor), x2 = scaled_pair(v.z, factor), x3 = scaled_pair(v.w, factor);
     uint32_t r;
     asm("{.reg .b8 t0, t1, t2, t3;\n\t"
         "cvt.rn.satfinite.e2m1x2.f32 t0, %2, %1;\n\t"
@@ -75,17 +78,43 @@ __device__ __forceinline__ uint32_t pack_e2m1x8(const uint32_t (&w)[4]) {
         "cvt.rn.satfinite.e2m1x2.f32 t3, %8, %7;\n\t"
         "mov.b32 %0, {t0, t1, t2, t3};}"
         : "=r"(r)
-        : "f"(bf16_lo(w[0])), "f"(bf16_hi(w[0])), "f"(bf16_lo(w[1])), "f"(bf16_hi(w[1])), "f"(bf16_lo(w[2])), "f"(bf16_hi(w[2])),
-          "f"(bf16_lo(w[3])), "f"(bf16_hi(w[3])));
+        : "f"(x0.x), "f"(x0.y), "f"(x1.x), "f"(x1.y), "f"(x2.x), "f"(x2.y), "f"(x3.x), "f"(x3.y));
     return r;
 }
 
-// Four packed bf16 pairs times 2^(127 - code): exact (a power-of-two factor only moves the exponent; products below the
-// bf16 range become zero with their sign, as their e2m1 codes would anyway).
-__device__ __forceinline__ void scale_pow2_bf16x2(const uint32_t (&v)[4], uint32_t code, uint32_t (&w)[4]) {
-    const uint32_t inv2 = ((254u - code) << 7) * 0x00010001u;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(w[j]) : "r"(v[j]), "r"(inv2));
+// mxfp4_code() of the two magnitudes in a bf16 pair, in 16-bit fields: a mantissa above 0x40 (1.5) is one that carries into the
+// exponent when 0x3f is added.  The floor of the maximum is a bf16 value, 0x01c0 (a NaN becomes it, as in fmaxf).
+__device__ __forceinline__ uint32_t mxfp4_codes(uint32_t magnitudes) {
+    return ((max_bf16x2(magnitudes, 0x01c001c0u) + 0x003f003fu) >> 7 & 0x01ff01ffu) - 0x00020002u;
+}
+
+// Rotation of two pairs: separately rounded products, then the sums, two values an instruction.  A product is fma(., ., -0) with a
+// -0 that comes from the launch's arguments: mul.rn.f32x2, or a -0 the assembler knows, it joins with the sum behind it, and a
+// few values in 10^6 then differ.
+__device__ __forceinline__ uint64_t f32x2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void rotate_two(uint32_t first, uint32_t second, uint64_t c, uint64_t s, uint64_t zero, uint32_t* to) {
+    const uint64_t e = f32x2(bf16_lo(first), bf16_lo(second)), o = f32x2(bf16_hi(first), bf16_hi(second));
+    uint64_t even, odd;
+    asm("{.reg .b64 a, b, d, f;\n\t"
+        "fma.rn.f32x2 a, %2, %4, %6;\n\t"
+        "fma.rn.f32x2 b, %3, %5, %6;\n\t"
+        "fma.rn.f32x2 d, %3, %4, %6;\n\t"
+        "fma.rn.f32x2 f, %2, %5, %6;\n\t"
+        "sub.rn.f32x2 %0, a, b;\n\t"
+        "add.rn.f32x2 %1, d, f;}"
+        : "=l"(even), "=l"(odd)
+        : "l"(e), "l"(o), "l"(c), "l"(s), "l"(zero));
+    asm("{.reg .f32 a, b, d, f;\n\t"
+        "mov.b64 {a, b}, %2;\n\t"
+        "mov.b64 {d, f}, %3;\n\t"
+        "cvt.rn.bf16x2.f32 %0, d, a;\n\t"
+        "cvt.rn.bf16x2.f32 %1, f, b;}"
+        : "=r"(to[0]), "=r"(to[1])
+        : "l"(even), "l"(odd));
 }
 
 template <int E>
@@ -284,11 +313,14 @@ cudaError_t launch_rows(const IndexerQParams& p, bool fp4, int64_t rows, int cs_
 // (eight pairs), so every lane rotates (no divergence) and its eight cosines and sines are loaded once per task.  MXFP4 blocks of
 // 32 are 2 lanes.  WIDE: 32-byte loads, otherwise (rows on 16-byte boundaries only) two of half the size.  Two passes are in
 // flight: the loads of the next one go out before the current one is worked on.  PREFETCH: one instruction sends the rest of the
-// task's rows to L2 at its start (6 CTAs per SM; without it 7).
-// Bound by instruction issue (0.7 per cycle; rotation, conversions) and DRAM together; the rotation on packed f32x2 instructions was
-// faster by 2 % and not bit for bit the same, an even split of the passes over resident warps no faster.
+// task's rows to L2 at its start.
+// Was bound by instruction issue: 345 warp instructions for a pass of eight heads with MXFP4, FP32 and conversion pipes apart.  Now
+// bf16 values are widened and scaled by one instruction each (scaled_pair()), two pairs rotated at a time (rotate_two()), two sets
+// of registers take turns instead of being copied, and weights and scale words are written for 32 heads at once.  64 heads a token,
+// before -> after: 16384 tokens, MXFP4 61.3 -> 57.2 us (6.1 TB/s), FP8 64.4 -> 62.8 us (6.7 TB/s); 65536 tokens 227.8 -> 214.0 and
+// 238.2 -> 236.6 us; 1531 tokens, out of L2, 8.0 -> 5.8 and 6.1 us; 61 tokens 2.1 -> 2.0 us.
 template <int WARPS, bool FP4, bool WIDE, bool PREFETCH>
-__global__ void __launch_bounds__(WARPS * 32, PREFETCH ? 6 : 7) indexer_q_rope_quant_heads_kernel(const IndexerQParams p, const int heads_per_task, const uint32_t tasks_per_token,
+__global__ void __launch_bounds__(WARPS * 32, 6) indexer_q_rope_quant_heads_kernel(const IndexerQParams p, const int heads_per_task, const uint32_t tasks_per_token,
                                                                                 const uint32_t tpt_mul, const uint32_t tpt_shift) {
     const int lane = threadIdx.x & 31, sub = lane & 3, which = lane >> 2;
     const uint32_t task = blockIdx.x * WARPS + (threadIdx.x >> 5);
@@ -310,101 +342,110 @@ __global__ void __launch_bounds__(WARPS * 32, PREFETCH ? 6 : 7) indexer_q_rope_q
         v.lo = ld_stream16(from), v.hi = ld_stream16(from + 16);
         return v;
     };
-    Bytes32 nope, rope, nope_next, rope_next;
-    nope.lo = nope.hi = rope.lo = rope.hi = make_uint4(0u, 0u, 0u, 0u);
-    nope_next = nope, rope_next = rope;
-    // The head's weight travels with its row: fetched in the pass that uses it, its latency would show in every pass (its bits
-    // only: a conversion would wait for them).
-    const auto weight_of = [&](int h) -> uint32_t {
+    // Of 32 heads (four passes) a lane writes the weight of head 8 * sub + which, and with MXFP4 the scales of that head: one load, one
+    // multiplication and one store for four passes instead of as many predicated ones, in every lane, in each.
+    const int own = head_begin + 8 * sub + which;
+    const auto weight_of = [&](int h) -> uint32_t {  // (its bits only: a conversion would wait for them)
         const int64_t at = t * p.weights_stride + h;
-        if (sub != 0) return 0u;
+        if (h >= head_end) return 0u;
         return p.weights_dtype == 2 ? __ldg(reinterpret_cast<const uint32_t*>(p.weights) + at) : __ldg(reinterpret_cast<const uint16_t*>(p.weights) + at);
     };
-    uint32_t weight_bits = 0u, weight_next = 0u;
-    if (head_begin + which < head_end) nope = load32(row), rope = load32(row + 128), weight_bits = weight_of(head_begin + which);
+    struct Rows {
+        Bytes32 nope, rope;
+    };
+    Rows a, b;
+    int h = head_begin + which;
+    a.nope.lo = a.nope.hi = a.rope.lo = a.rope.hi = make_uint4(0u, 0u, 0u, 0u);
+    if (h < head_end) a.nope = load32(row), a.rope = load32(row + 128);
+    b = a;
+    uint32_t weight_bits = weight_of(own);
     if (PREFETCH && lane == 0 && head_bytes == 256 && head_end > head_begin + 16)
         prefetch_l2(p.q + t * p.q_stride0 * 2 + (head_begin + 16) * 256, static_cast<uint32_t>(head_end - head_begin - 16) * 256u);
     const int64_t pos = p.positions[t];
-    float c[8], sn[8];
+    uint64_t c[4], sn[4];  // of two pairs each
+    const uint64_t zero = f32x2(p.minus_zero, p.minus_zero);
     if (p.cos_sin_bf16) {
         const uint16_t* cs = reinterpret_cast<const uint16_t*>(p.cos_sin) + pos * p.cos_sin_stride + 8 * sub;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) c[j] = bf16_lo(cs[j]), sn[j] = bf16_lo(cs[32 + j]);
+        for (int j = 0; j < 4; ++j) c[j] = f32x2(bf16_lo(cs[2 * j]), bf16_lo(cs[2 * j + 1])), sn[j] = f32x2(bf16_lo(cs[32 + 2 * j]), bf16_lo(cs[33 + 2 * j]));
     } else {
         const float* cs = reinterpret_cast<const float*>(p.cos_sin) + pos * p.cos_sin_stride + 8 * sub;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) c[j] = __ldg(cs + j), sn[j] = __ldg(cs + 32 + j);
+        for (int j = 0; j < 4; ++j) c[j] = f32x2(__ldg(cs + 2 * j), __ldg(cs + 2 * j + 1)), sn[j] = f32x2(__ldg(cs + 32 + 2 * j), __ldg(cs + 33 + 2 * j));
     }
     uint8_t* out = p.out + t * p.out_stride0 + (head_begin + which) * p.out_stride1;
-    for (int h = head_begin + which; h - which < head_end; h += 8) {
-        const bool live = h < head_end;
-        row += 8 * head_bytes;
-        if (h + 8 < head_end) nope_next = load32(row), rope_next = load32(row + 128), weight_next = weight_of(h + 8);
-        float weight_factor = 1.0f;
-        uint32_t rot[8];  // the rotated pairs, rounded to bf16 as the reference does before quantising
-        const uint32_t raw[8] = {rope.lo.x, rope.lo.y, rope.lo.z, rope.lo.w, rope.hi.x, rope.hi.y, rope.hi.z, rope.hi.w};
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float e = bf16_lo(raw[j]), o = bf16_hi(raw[j]);
-            // separately rounded products
-            rot[j] = pack_bf16x2(__fsub_rn(__fmul_rn(e, c[j]), __fmul_rn(o, sn[j])), __fadd_rn(__fmul_rn(o, c[j]), __fmul_rn(e, sn[j])));
+    uint32_t kept = 0u;  // of the head this lane writes weight and scales of: its scale word (MXFP4) or its scale code (FP8)
+    // What is written once for four passes, those up to `pass`.
+    const auto finish = [&](int pass) {
+        const int head = own + 8 * (pass & ~3);
+        if (head >= head_end || sub > (pass & 3)) return;
+        float w = weight_value(weight_bits, p.weights_dtype);
+        if (FP4) {
+            uint8_t* sc = p.scales + t * p.scale_stride0 + head * p.scale_stride1;
+            if (p.scales_word_aligned) {
+                *reinterpret_cast<uint32_t*>(sc) = kept;
+            } else {
+                sc[0] = static_cast<uint8_t>(kept), sc[1] = static_cast<uint8_t>(kept >> 8);
+                sc[2] = static_cast<uint8_t>(kept >> 16), sc[3] = static_cast<uint8_t>(kept >> 24);
+            }
+        } else {
+            w = __fmul_rn(w, __uint_as_float(kept << 23));
         }
+        p.weights_out[t * p.weights_out_stride + head] = __fmul_rn(__fmul_rn(w, p.softmax_scale), p.head_scale);
+    };
+    // Pass `pass` on the rows in `now`, while the next ones are on their way to `then`; says whether there is another.
+    const auto step = [&](int pass, const Rows& now, Rows& then) {
+        row += 8 * head_bytes;
+        if (h + 8 < head_end) then.nope = load32(row), then.rope = load32(row + 128);
+        const Bytes32 &nope = now.nope, &rope = now.rope;
+        uint32_t rot[8];  // the rotated pairs, rounded to bf16 as the reference does before quantising
+        rotate_two(rope.lo.x, rope.lo.y, c[0], sn[0], zero, rot), rotate_two(rope.lo.z, rope.lo.w, c[1], sn[1], zero, rot + 2);
+        rotate_two(rope.hi.x, rope.hi.y, c[2], sn[2], zero, rot + 4), rotate_two(rope.hi.z, rope.hi.w, c[3], sn[3], zero, rot + 6);
         const uint4 ra = make_uint4(rot[0], rot[1], rot[2], rot[3]), rb = make_uint4(rot[4], rot[5], rot[6], rot[7]);
         // |.| maxima on the packed words: of the un-rotated values in `pn`, of the rotated ones in `pr`
-        const auto max16 = [](const uint4& a, const uint4& b) {
-            return max_abs_bf16x2(max_abs_bf16x2(max_abs_bf16x2(a.x, a.y), max_abs_bf16x2(a.z, a.w)),
-                                  max_abs_bf16x2(max_abs_bf16x2(b.x, b.y), max_abs_bf16x2(b.z, b.w)));
+        const auto max16 = [](const uint4& x, const uint4& y) {
+            return max_abs_bf16x2(max_abs_bf16x2(max_abs_bf16x2(x.x, x.y), max_abs_bf16x2(x.z, x.w)),
+                                  max_abs_bf16x2(max_abs_bf16x2(y.x, y.y), max_abs_bf16x2(y.z, y.w)));
         };
         const uint32_t pn = max16(nope.lo, nope.hi), pr = max16(ra, rb);
         if (FP4) {
             // the two maxima side by side in one word, reduced over the 2 lanes of a block
             uint32_t both = max_abs_bf16x2(__byte_perm(pn, pr, 0x5410), __byte_perm(pn, pr, 0x7632)) & 0x7fff7fffu;
             both = max_bf16x2(both, __shfl_xor_sync(0xffffffffu, both, 1));
-            const uint32_t code_n = mxfp4_code(bf16_lo(both)), code_r = mxfp4_code(bf16_hi(both));
-            const auto pack = [](const uint4& v, uint32_t code) {
-                const uint32_t in[4] = {v.x, v.y, v.z, v.w};
-                uint32_t w[4];
-                scale_pow2_bf16x2(in, code, w);
-                return pack_e2m1x8(w);
-            };
-            const uint2 bn = make_uint2(pack(nope.lo, code_n), pack(nope.hi, code_n)), br = make_uint2(pack(ra, code_r), pack(rb, code_r));
+            const uint32_t codes = mxfp4_codes(both), factors = (0x00fe00feu - codes) << 7;  // 2^(127 - code) as bf16
+            const auto fn = static_cast<uint16_t>(factors), fr = static_cast<uint16_t>(factors >> 16);
+            const uint2 bn = make_uint2(pack_e2m1x8(nope.lo, fn), pack_e2m1x8(nope.hi, fn)), br = make_uint2(pack_e2m1x8(ra, fr), pack_e2m1x8(rb, fr));
             // the head's four scale bytes in one word: blocks (un-rotated 0-31, 32-63, rotated 0-31, 32-63)
-            const uint32_t mine = code_n | (code_r << 16);
-            const uint32_t other = __shfl_xor_sync(0xffffffffu, mine, 2);
-            if (live) {
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, codes, 2);
+            if (sub == (pass & 3)) kept = sub & 2 ? other | (codes << 8) : codes | (other << 8);
+            if (h < head_end) {
                 st_global8(out + 8 * sub, bn);
                 st_global8(out + 32 + 8 * sub, br);
-                if (sub == 0) {
-                    uint8_t* sc = p.scales + t * p.scale_stride0 + h * p.scale_stride1;
-                    const uint32_t word = mine | (other << 8);
-                    if (p.scales_word_aligned) {
-                        *reinterpret_cast<uint32_t*>(sc) = word;
-                    } else {
-                        sc[0] = static_cast<uint8_t>(word), sc[1] = static_cast<uint8_t>(word >> 8);
-                        sc[2] = static_cast<uint8_t>(word >> 16), sc[3] = static_cast<uint8_t>(word >> 24);
-                    }
-                }
             }
         } else {
             uint32_t pk = max_abs_bf16x2(pn, pr) & 0x7fff7fffu;
             pk = max_bf16x2(pk, __shfl_xor_sync(0xffffffffu, pk, 1));
             pk = max_bf16x2(pk, __shfl_xor_sync(0xffffffffu, pk, 2));
             const uint32_t code = ue8m0_code(fmaxf(bf16_lo(pk), bf16_hi(pk)));
-            weight_factor = __uint_as_float(code << 23);
+            if (sub == (pass & 3)) kept = code;
             const uint2 n0 = quant8_pow2(nope.lo, code), n1 = quant8_pow2(nope.hi, code), r0 = quant8_pow2(ra, code), r1 = quant8_pow2(rb, code);
-            if (live) {
+            if (h < head_end) {
                 st_stream16(out + 16 * sub, make_uint4(n0.x, n0.y, n1.x, n1.y));
                 st_stream16(out + 64 + 16 * sub, make_uint4(r0.x, r0.y, r1.x, r1.y));
             }
         }
-        if (live && sub == 0) {
-            float w = weight_value(weight_bits, p.weights_dtype);
-            if (!FP4) w = __fmul_rn(w, weight_factor);
-            p.weights_out[t * p.weights_out_stride + h] = __fmul_rn(__fmul_rn(w, p.softmax_scale), p.head_scale);
-        }
-        out += 8 * p.out_stride1;
-        nope = nope_next, rope = rope_next, weight_bits = weight_next;
+        out += 8 * p.out_stride1, h += 8;
+        return h - which < head_end;
+    };
+    int pass = 0;
+    while (step(pass, a, b)) {
+        const bool more = step(pass + 1, b, a);
+        if (!more || (pass & 2)) finish(pass + 1);
+        if (!more) return;
+        pass += 2;
+        if (!(pass & 2)) weight_bits = weight_of(own + 8 * pass);
     }
+    finish(pass);
 }
 
 template <int E>
@@ -433,7 +474,7 @@ cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q,
     p.scales = static_cast<uint8_t*>(scales), p.scale_stride0 = scale_stride0, p.scale_stride1 = scale_stride1;
     p.weights = static_cast<const uint8_t*>(weights), p.weights_stride = weights_stride, p.weights_dtype = weights_dtype;
     p.weights_out = weights_out, p.weights_out_stride = weights_out_stride;
-    p.softmax_scale = softmax_scale, p.head_scale = head_scale, p.num_tokens = num_tokens, p.num_heads = num_heads;
+    p.softmax_scale = softmax_scale, p.head_scale = head_scale, p.num_tokens = num_tokens, p.num_heads = num_heads, p.minus_zero = -0.0f;
     make_fast_divisor(static_cast<uint32_t>(num_heads), &p.heads_mul, &p.heads_shift);
     const auto addr = [](const void* q_) { return reinterpret_cast<uintptr_t>(q_); };
     p.scales_word_aligned = addr(scales) % 4 == 0 && scale_stride0 % 4 == 0 && scale_stride1 % 4 == 0;
@@ -445,15 +486,19 @@ cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q,
     if (heads_shape) {
         constexpr int WARPS = 4;
         // Heads per warp: few rows, short tasks, so that there are enough of them; many rows, long ones, whose set-up more heads
-        // share.  Both sides of each line, FP8 / MXFP4, us a launch of 64 heads a token, from a graph with three inputs in rotation
-        // (from 3072 tokens on they come from HBM):
-        //   8 | 16            832 tokens  5.5 / 5.4 | 5.2 / 5.2          1023 tokens  6.1 / 6.1 | 5.3 / 5.4
-        //   16 | 64          3072 tokens 14.5 / 14.8 | 15.5 / 16.2       4096 tokens 19.6 / 19.8 | 17.7 / 17.3
-        //   64 | prefetch    8192 tokens 34.9 / 33.1 | 35.6 / 34.0       9216 tokens 42.2 / 39.9 | 39.2 / 37.3     65536 tokens 255 / 237 | 238 / 226-229
-        // The requests ahead of the wait change nothing for the last form (65536 tokens without them: 239 / 226-227).
-        // Tasks of 64 heads fill the GPU with 4144 tokens at a time: 4608 tokens would be 11 % faster with 32, 8192 are 3 % slower.
+        // share; and where 64 or 32 heads make one wave that is nearly full, those.  FP8 / MXFP4, us a launch of 64 heads a token,
+        // from a graph with three inputs in rotation (from 3072 tokens on they come from HBM):
+        //   8 | 16           200 tokens  2.4 / 2.4 | 2.5 / 2.4         256 tokens  2.7 / 2.7 | 2.5 / 2.5
+        //   16 | 32 | 64      832 tokens  3.7 / 3.7 | 3.9 / 3.5 | 5.1 / 4.7        1280 tokens  5.7 / 5.6 | 5.8 / 5.5 | 6.1 / 6.0
+        //                    1536 tokens  6.8 / 6.2 | 6.1 / 5.8 | 7.5 / 6.9        1800 tokens  8.8 / 8.4 | 8.9 / 8.1 | 9.0 / 8.7
+        //                    2500 tokens 10.7 / 10.3 | 11.5 / 11.1 | 10.7 / 10.5   3072 tokens 13.4 / 12.9 | 12.6 / 12.2 | 12.0 / 11.7
+        //                    4096 tokens 18.1 / 17.0 | 18.2 / 17.0 | 19.9 / 18.4   8192 tokens 36.2 / 33.1 | 34.5 / 31.0 | 35.4 / 31.9
+        //   32 | prefetch    8192 tokens 34.5 / 31.0 | 34.0 / 31.4       9216 tokens 39.0 / 34.9 | 37.4 / 34.3     32768 tokens 127 / 113 | 121 / 109
+        // (With 64 at 5500 to 6500 tokens, nearly two waves of them, 3 % less than with 32.)
+        constexpr int64_t kWave = 148 * 6 * WARPS;  // warps of a B200
+        const auto fills_a_wave = [&](int64_t heads) { return rows <= kWave * heads && 9 * rows >= 7 * kWave * heads; };
         const bool prefetch = rows >= 589824;
-        const int heads_per_task = prefetch ? 32 : rows >= 212992 ? 64 : rows >= 57344 ? 16 : 8;
+        const int heads_per_task = fills_a_wave(64) ? 64 : rows > kWave * 64 || fills_a_wave(32) ? 32 : rows >= 14336 ? 16 : 8;
         const int64_t tasks_per_token = (num_heads + heads_per_task - 1) / heads_per_task;
         const dim3 grid(static_cast<unsigned>((num_tokens * tasks_per_token + WARPS - 1) / WARPS));
         uint32_t mul, shift;
