@@ -464,14 +464,41 @@ struct ScaleDivider {
     }
 };
 
+// The same of both halves of a bf16 pair, two values an instruction.
+template <int MODE, bool TWO_TERM>
+__device__ __forceinline__ float2 quotients(uint32_t pair, const ScaleDivider<MODE>& d) {
+    const float2 x = make_float2(bf16_lo(pair), bf16_hi(pair));
+    if (MODE != kDivideFast) return make_float2(d.template quotient<TWO_TERM>(x.x), d.template quotient<TWO_TERM>(x.y));
+    float2 q;
+    if (TWO_TERM)
+        asm("{.reg .b64 x, y, l;\n\t"
+            "mov.b64 x, {%2, %3};\n\t"
+            "mov.b64 y, {%4, %4};\n\t"
+            "mov.b64 l, {%5, %5};\n\t"
+            "mul.rn.f32x2 l, x, l;\n\t"
+            "fma.rn.f32x2 x, x, y, l;\n\t"
+            "mov.b64 {%0, %1}, x;}"
+            : "=f"(q.x), "=f"(q.y)
+            : "f"(x.x), "f"(x.y), "f"(d.recip), "f"(d.recip_lo));
+    else
+        asm("{.reg .b64 x, y, n, q, r;\n\t"
+            "mov.b64 x, {%2, %3};\n\t"
+            "mov.b64 y, {%4, %4};\n\t"
+            "mov.b64 n, {%5, %5};\n\t"
+            "mul.rn.f32x2 q, x, y;\n\t"
+            "fma.rn.f32x2 r, n, q, x;\n\t"
+            "fma.rn.f32x2 q, r, y, q;\n\t"
+            "mov.b64 {%0, %1}, q;}"
+            : "=f"(q.x), "=f"(q.y)
+            : "f"(x.x), "f"(x.y), "f"(d.recip), "f"(-d.scale));
+    return q;
+}
+
 template <int MODE, bool TWO_TERM>
 __device__ __forceinline__ uint2 quant8_by(const uint4& v, const ScaleDivider<MODE>& d) {
-    float x[8];
-    unpack8(v, x);
-    float q[8];  // the e4m3 conversion saturates at +-448
-#pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = d.template quotient<TWO_TERM>(x[i]);
-    return make_uint2(pack_e4m3x4(q[0], q[1], q[2], q[3]), pack_e4m3x4(q[4], q[5], q[6], q[7]));
+    const float2 x0 = quotients<MODE, TWO_TERM>(v.x, d), x1 = quotients<MODE, TWO_TERM>(v.y, d);
+    const float2 x2 = quotients<MODE, TWO_TERM>(v.z, d), x3 = quotients<MODE, TWO_TERM>(v.w, d);
+    return make_uint2(pack_e4m3x4(x0.x, x0.y, x1.x, x1.y), pack_e4m3x4(x2.x, x2.y, x3.x, x3.y));  // saturates at +-448
 }
 
 // Both halves of a bf16 pair times a bf16 power of two, as fp32: exact, one instruction a value (the sum with -0 keeps the sign of

@@ -133,7 +133,8 @@ void launch_vector(const GroupQuantParams& p, bool ue8m0, int division, cudaStre
 
 // HBM-bound once a lane moves 32 bytes at a time: 32768 x 7168, groups of 128, 121 -> 102 us with power-of-two scales and
 // 132 -> 102 us with fp32 scales (7.0 TB/s, the 2-read-1-write ceiling of the probe) against 16-byte loads; 4097 x 7168 16.5 /
-// 18.1 -> 12.0 / 13.4 us.  Two groups in flight per lane group: one gives 119 us and four 103 us there.  Few groups want
+// 18.1 -> 12.0 / 13.4 us (fp32 scales 12.3 us since two values are divided by an instruction, which was issue-bound at that size; 1531 x
+// 1536 2.3 -> 2.2 us, 32768 x 7168 102 -> 100 us).  Two groups in flight per lane group: one gives 119 us and four 103 us there.  Few groups want
 // as many warps as there are (1531 x 1536: 2.0 us with one, 2.3 with two; 4097 x 1536: 3.9 and 3.4 us).
 constexpr int64_t kFewGroups = 32768;
 

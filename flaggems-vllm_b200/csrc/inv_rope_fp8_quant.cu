@@ -37,7 +37,8 @@ struct InvRopeParams {
 // Two passes of U heads are in flight: the loads of the next pass go out before the current one is worked on (8192 x 128 rows:
 // 241 us, 253 us with one pass of four heads).
 // Bound by instruction issue before HBM in 16-byte pieces (253 us, fp32 scales 265 us); with 32-byte loads, 16-byte stores
-// and 6 shuffles a head 241 us = 6.7 TB/s and 247 us.  CTAs per SM: 6 247 us, 7 241 us, 8 306 us (spills).
+// and 6 shuffles a head 241 us = 6.7 TB/s and 247 us (245 us, and 61 x 128 rows 3.8 -> 3.6 us, since two values are divided by an instruction).
+// Two sets of registers that take turns instead of being copied: 61 x 128 rows 3.5 -> 3.4 us, but 8192 x 128 rows 241 -> 245 us.  CTAs per SM: 6 247 us, 7 241 us, 8 306 us (spills).
 constexpr int kMainLanes = 28;
 constexpr int kHeadsInFlight = 2;  // per pass
 constexpr int kCtasPerSm = 7;      // 72 registers
