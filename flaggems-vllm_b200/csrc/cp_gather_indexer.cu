@@ -55,7 +55,7 @@ __device__ __forceinline__ bool locate(const CpGatherParams& p, int32_t t, int32
 // 32/LANES*U <= 32 consecutive tokens.  Lane i locates token i of the warp (one bisection per token, all of them
 // side by side); the lane groups then fetch block and position of their tokens with shuffles.
 template <int WARPS, int LANES, int U>
-__global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_vec_kernel(const CpGatherParams p) {
+__global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_vec_kernel(const Launched<CpGatherParams> p) {
     begin_dependent_kernel();
     constexpr int kGroups = 32 / LANES;
     static_assert(kGroups * U <= 32, "a warp locates one token per lane");
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_vec_kernel(const
 // of about eight), every lane moves on from there to its own token, copies that token's scale, and four lanes copy the 128
 // bytes of a token with 32-byte accesses (16 sequences of up to 16384 tokens: 10.8 -> 9.7 us; 32 of up to 4096: 6.3 -> 4.1 us).
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_128_kernel(const CpGatherParams p) {
+__global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_128_kernel(const Launched<CpGatherParams> p) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int32_t first = static_cast<int32_t>((static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5)) * 32);
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_128_kernel(const
 
 // Any head_dim and any alignment: one warp per token, byte by byte.
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_bytes_kernel(const CpGatherParams p) {
+__global__ void __launch_bounds__(WARPS * 32) cp_gather_indexer_bytes_kernel(const Launched<CpGatherParams> p) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);

@@ -100,7 +100,7 @@ __device__ __forceinline__ int64_t load_index(const void* p, int64_t i, int is64
 constexpr int kE4m3Lanes = kNopeDim / 16;
 constexpr int kTokensInFlight = 4;  // per warp
 template <int WARPS, bool FAST, bool WIDE, int U>
-__global__ void __launch_bounds__(WARPS * 32) gather_dequant_requests_kernel(const GatherParams g) {
+__global__ void __launch_bounds__(WARPS * 32) gather_dequant_requests_kernel(const Launched<GatherParams> g) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t req = blockIdx.y;

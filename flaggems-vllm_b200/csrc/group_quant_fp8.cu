@@ -32,7 +32,7 @@ struct GroupQuantParams {
 // UE8M0: power-of-two scales (exact reciprocal multiply); DIVISION: how x / scale is formed otherwise
 // (IEEE division, the verified reciprocal-and-correct division for the default eps, or x * (1/scale) for `act_quant`).
 template <int WARPS, int LANES, int U, bool WIDE, bool UE8M0, int DIVISION>
-__global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_kernel(const GroupQuantParams p) {
+__global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_kernel(const Launched<GroupQuantParams> p) {
     constexpr int kGroups = 32 / LANES;
     const int lane = threadIdx.x & 31;
     const int sub = lane % LANES;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_kernel(const Group
 
 // Any group size and alignment: one warp per group, element by element.
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_scalar_kernel(const GroupQuantParams p, const int ue8m0, const int reciprocal) {
+__global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_scalar_kernel(const Launched<GroupQuantParams, 2 * sizeof(int)> p, const int ue8m0, const int reciprocal) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t g = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);

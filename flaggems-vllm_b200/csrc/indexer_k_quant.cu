@@ -49,7 +49,7 @@ __device__ __forceinline__ float group_scale(float amax, bool ue8m0) {
 }
 
 template <int WARPS, bool FP16>
-__global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_kernel(const IndexerParams p) {
+__global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_kernel(const Launched<IndexerParams> p) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_kernel(const Index
 // Fast shape for head_dim 64 / 128 / 256: a token is G = head_dim/8 lanes of 16 bytes, so one warp instruction
 // moves 32/G tokens, and U passes are loaded (slot and row) before any is used.
 template <int WARPS, int G, int U, bool FP16>
-__global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_rows_kernel(const IndexerParams p) {
+__global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_rows_kernel(const Launched<IndexerParams> p) {
     begin_dependent_kernel();
     constexpr int TOKENS = 32 / G;
     const int lane = threadIdx.x & 31, sub = lane % G, which = lane / G;
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_rows_kernel(const 
 #endif
 // UE8M0 (power-of-two scales): bf16 keys stay packed - group maximum and scaling on the bf16x2 words, as in quant8_pow2.
 template <int WARPS, int U, bool FP16, bool UE8M0>
-__global__ void __launch_bounds__(WARPS * 32, DSV4_INDEXER_K_CTAS) indexer_k_quant_128_kernel(const IndexerParams p) {
+__global__ void __launch_bounds__(WARPS * 32, DSV4_INDEXER_K_CTAS) indexer_k_quant_128_kernel(const Launched<IndexerParams> p) {
     const int lane = threadIdx.x & 31, sub = lane & 7, which = lane >> 3;
     const int64_t base = (static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5)) * (U * 4) + which;
     if (starts_early() && sub == 0) {

@@ -134,7 +134,7 @@ __device__ __forceinline__ void load_row(const uint8_t* p, float (&x)[E]) {
 }
 
 template <int WARPS, int E, bool FP4>
-__global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_kernel(const IndexerQParams p) {
+__global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_kernel(const Launched<IndexerQParams> p) {
     begin_dependent_kernel();
     constexpr int D = 32 * E;
     const int lane = threadIdx.x & 31;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_kernel(const 
 // U passes per warp are loaded before any is used.  Needs 16-byte aligned rows and a rotary tail that starts
 // on a multiple of 8 values.
 template <int WARPS, int G, int U, bool FP4>
-__global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_rows_kernel(const IndexerQParams p, const int cs_vec4) {
+__global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_rows_kernel(const Launched<IndexerQParams, 2 * sizeof(int)> p, const int cs_vec4) {
     begin_dependent_kernel();
     constexpr int D = 8 * G, ROWS = 32 / G;
     const int lane = threadIdx.x & 31, sub = lane % G, slot = lane / G;
@@ -320,7 +320,7 @@ cudaError_t launch_rows(const IndexerQParams& p, bool fp4, int64_t rows, int cs_
 // before -> after: 16384 tokens, MXFP4 61.3 -> 57.2 us (6.1 TB/s), FP8 64.4 -> 62.8 us (6.7 TB/s); 65536 tokens 227.8 -> 214.0 and
 // 238.2 -> 236.6 us; 1531 tokens, out of L2, 8.0 -> 5.8 and 6.1 us; 61 tokens 2.1 -> 2.0 us.
 template <int WARPS, bool FP4, bool WIDE, bool PREFETCH>
-__global__ void __launch_bounds__(WARPS * 32, 6) indexer_q_rope_quant_heads_kernel(const IndexerQParams p, const int heads_per_task, const uint32_t tasks_per_token,
+__global__ void __launch_bounds__(WARPS * 32, 6) indexer_q_rope_quant_heads_kernel(const Launched<IndexerQParams, 4 * sizeof(int)> p, const int heads_per_task, const uint32_t tasks_per_token,
                                                                                 const uint32_t tpt_mul, const uint32_t tpt_shift) {
     const int lane = threadIdx.x & 31, sub = lane & 3, which = lane >> 2;
     const uint32_t task = blockIdx.x * WARPS + (threadIdx.x >> 5);

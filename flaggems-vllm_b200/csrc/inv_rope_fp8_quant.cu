@@ -44,7 +44,7 @@ constexpr int kHeadsInFlight = 2;  // per pass
 constexpr int kCtasPerSm = 7;      // 72 registers
 
 template <int WARPS, bool PACKED, bool FASTDIV, int U, int MIN_CTAS, bool WIDE>
-__global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kernel(const InvRopeParams p, const int heads_per_task, const uint32_t tasks_per_token,
+__global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kernel(const Launched<InvRopeParams, 4 * sizeof(int)> p, const int heads_per_task, const uint32_t tasks_per_token,
                                                                       const uint32_t tpt_mul, const uint32_t tpt_shift) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
@@ -172,7 +172,7 @@ struct InvRopeGeometry {
 };
 
 template <int WARPS, bool PACKED>
-__global__ void __launch_bounds__(WARPS * 32) inv_rope_fp8_quant_any_kernel(const InvRopeParams p, const InvRopeGeometry geo) {
+__global__ void __launch_bounds__(WARPS * 32) inv_rope_fp8_quant_any_kernel(const Launched<InvRopeParams, sizeof(InvRopeGeometry)> p, const InvRopeGeometry geo) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t row = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);

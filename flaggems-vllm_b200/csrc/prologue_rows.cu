@@ -23,7 +23,7 @@ namespace {
 // sine i): 256 more bytes from L2 per row, but no barrier and no shared-memory round trip in the dependent chain
 // position -> table row, which is what a launch of a few waves waits for.
 template <int RPW, int WARPS, int MIN_CTAS, bool CHECKED, bool PADDED, int PDL = 0, bool STAGED = true>
-__global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) prologue_rows_kernel(const PrologueParams p, const int64_t kv_ctas) {
+__global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) prologue_rows_kernel(const Launched<PrologueParams, sizeof(int64_t)> p, const int64_t kv_ctas) {
     static_assert(STAGED || !CHECKED, "the range-checked build marks bad tokens in shared memory");
     constexpr int TILE = RPW * WARPS;
     constexpr int MAX_TOKENS = TILE + 1;  // a tile of TILE rows touches at most TILE tokens (+1 slack)
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) prologue_rows_kernel(con
 // kernels above (the sum of squares is grouped differently, within the freedom the mean has anyway); cache bytes are
 // identical.  Only this plain form exists for such pointers: no range-checked and no out-of-place variant.
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) prologue_rows_any_alignment_kernel(const PrologueParams p, const int64_t kv_ctas) {
+__global__ void __launch_bounds__(WARPS * 32) prologue_rows_any_alignment_kernel(const Launched<PrologueParams, sizeof(int64_t)> p, const int64_t kv_ctas) {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const bool is_kv = static_cast<int64_t>(blockIdx.x) < kv_ctas;

@@ -38,7 +38,7 @@ __device__ __forceinline__ float inv_rms_of(float sum, int size, float eps) {
 // access per chunk, otherwise (rows on 16-byte boundaries only) two.  EARLY: the weights are fetched before the reduction.
 template <int WARPS, int CH, bool WIDE, bool EARLY>
 __global__ void __launch_bounds__(WARPS * 32, EARLY ? 1 : CH == 1 ? 16 : CH == 2 ? 10 : CH == 3 ? 7 : 6)
-q_kv_rmsnorm_kernel(const NormRows q, const NormRows kv, int64_t num_tokens, float eps) {
+q_kv_rmsnorm_kernel(const Launched<NormRows, sizeof(NormRows) + 16> q, const NormRows kv, int64_t num_tokens, float eps) {
     const int lane = threadIdx.x & 31;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
     if (r >= 2 * num_tokens) return;
@@ -151,7 +151,7 @@ __device__ __forceinline__ void store_any(uint8_t* base, int64_t i, int dtype, f
 }
 
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) q_kv_rmsnorm_any_kernel(const AnyRows q, const AnyRows kv, int64_t num_tokens, float eps) {
+__global__ void __launch_bounds__(WARPS * 32) q_kv_rmsnorm_any_kernel(const Launched<AnyRows, sizeof(AnyRows) + 16> q, const AnyRows kv, int64_t num_tokens, float eps) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);

@@ -65,7 +65,7 @@ struct Entries {
 // in flight: 512 entries of a row in one pass where W is 8 (a decode batch of 61 rows 3.7 -> 3.1 us, bound by its three dependent
 // loads; 32768 x 2048: 86.8 -> 85.4 us, 6.3 TB/s).
 template <int WARPS, int W>
-__global__ void __launch_bounds__(WARPS * 32) global_topk_kernel(const GlobalTopkParams p) {
+__global__ void __launch_bounds__(WARPS * 32) global_topk_kernel(const Launched<GlobalTopkParams> p) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int64_t t = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
@@ -117,7 +117,7 @@ struct CombineParams {
 // W is 8.  Few requests: the token's is found by a vote instead of a bisection (1531 rows of 640: 3.2 -> 2.6 us,
 // 8192: 7.1 -> 5.7 us).
 template <int WARPS, int W>
-__global__ void __launch_bounds__(WARPS * 32) combine_topk_swa_kernel(const CombineParams p) {
+__global__ void __launch_bounds__(WARPS * 32) combine_topk_swa_kernel(const Launched<CombineParams> p) {
     begin_dependent_kernel();
     const int lane = threadIdx.x & 31;
     const int32_t token = static_cast<int32_t>(blockIdx.x * WARPS + (threadIdx.x >> 5));

@@ -631,7 +631,7 @@ __device__ __forceinline__ int32_t row_range(const TopkParams& p, int r, int64_t
 // finite values take 20 us (ranking the thousand equal values by counting took 1267 us); 61 x 1400 7.4 and 3.0 us; 4096 x 4096, where
 // they are too many for the pool, 201 and 30 us.
 template <bool DECODE, int THREADS, int QUADS>
-__global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_short_kernel(const TopkParams p) {
+__global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_short_kernel(const Launched<TopkParams> p) {
     begin_dependent_kernel();
     __shared__ Shared s;
     extern __shared__ uint2 dynamic[];
@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(THREADS, 1536 / THREADS) topk_short_kernel(con
 
 // One CTA per row, the row in registers: QUADS x 4 values per thread.  The sample is the first value of every quad.
 template <bool DECODE, int THREADS, int QUADS>
-__global__ void __launch_bounds__(THREADS) topk_registers_kernel(const TopkParams p) {
+__global__ void __launch_bounds__(THREADS) topk_registers_kernel(const Launched<TopkParams> p) {
     begin_dependent_kernel();
     __shared__ Shared s;
     extern __shared__ uint2 dynamic[];
@@ -856,7 +856,7 @@ __device__ __forceinline__ int row_at_place(Shared& s, const TopkParams& p, uint
 // order of their lengths.  CTAs of 256 threads: five per SM with 48 registers; six with 40 were up to 3 % slower (a causal chunk of
 // 4096 x 32768, k 2048 122.5 | 119 us, 1000 x 40000 30.2 | 29.6 us; the pool for k 2048 leaves room for five anyway).
 template <bool DECODE, int THREADS, bool TWO, bool LONGEST_FIRST = false>
-__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 5 : TWO ? 2 : 3) topk_stream_kernel(const TopkParams p) {
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 5 : TWO ? 2 : 3) topk_stream_kernel(const Launched<TopkParams> p) {
     constexpr int kSampleQuads = sample_quads(THREADS);
     begin_dependent_kernel();
     __shared__ Shared s;
