@@ -36,8 +36,12 @@ __device__ __forceinline__ float inv_rms_of(float sum, int size, float eps) {
 
 // CH = 32-byte chunks per lane the launch needs (1 to 4): fewer live registers for the common 1536 / 512 rows.  WIDE: one 32-byte
 // access per chunk, otherwise (rows on 16-byte boundaries only) two.  EARLY: the weights are fetched before the reduction.
+constexpr int ctas_per_sm(int chunks, bool early) {  // of 128 threads
+    return early ? (chunks == 1 ? 10 : chunks == 2 ? 7 : chunks == 3 ? 5 : 4) : (chunks == 1 ? 16 : chunks == 2 ? 10 : chunks == 3 ? 7 : 6);
+}
+
 template <int WARPS, int CH, bool WIDE, bool EARLY>
-__global__ void __launch_bounds__(WARPS * 32, EARLY ? 1 : CH == 1 ? 16 : CH == 2 ? 10 : CH == 3 ? 7 : 6)
+__global__ void __launch_bounds__(WARPS * 32, ctas_per_sm(CH, EARLY))
 q_kv_rmsnorm_kernel(const Launched<NormRows, sizeof(NormRows) + 16> q, const NormRows kv, int64_t num_tokens, float eps) {
     const int lane = threadIdx.x & 31;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
@@ -90,12 +94,22 @@ q_kv_rmsnorm_kernel(const Launched<NormRows, sizeof(NormRows) + 16> q, const Nor
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
         const float rr = inv_rms_of(acc, size, eps);
+        // two values an instruction; the same products, each rounded (32768 tokens 41.1 -> 40.7 us)
+        const auto product = [&](uint32_t xv, uint32_t wv) {
+            float2 y;
+            asm("{.reg .b64 x, r, w;\n\t"
+                "mov.b64 x, {%2, %3};\n\t"
+                "mov.b64 r, {%4, %4};\n\t"
+                "mov.b64 w, {%5, %6};\n\t"
+                "mul.rn.f32x2 x, x, r;\n\t"
+                "mul.rn.f32x2 x, x, w;\n\t"
+                "mov.b64 {%0, %1}, x;}"
+                : "=f"(y.x), "=f"(y.y)
+                : "f"(bf16_lo(xv)), "f"(bf16_hi(xv)), "f"(rr), "f"(bf16_lo(wv)), "f"(bf16_hi(wv)));
+            return pack_bf16x2(y.x, y.y);
+        };
         const auto apply = [&](const uint4& xv, const uint4& wv) {
-            float f[8], g[8];
-            unpack8(xv, f), unpack8(wv, g);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = __fmul_rn(__fmul_rn(f[i], rr), g[i]);
-            return pack8(f);
+            return make_uint4(product(xv.x, wv.x), product(xv.y, wv.y), product(xv.z, wv.z), product(xv.w, wv.w));
         };
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
@@ -181,23 +195,37 @@ bool on_boundaries(uintptr_t bytes, const NormRows& t) {
            t.out_stride % elements == 0 && t.size % elements == 0 && t.size <= kMaxChunks * 512;
 }
 
-// Up to here the weights are fetched before the reduction (90 registers for rows of 1536), above it afterwards (72, 7 CTAs per
-// SM).  Before | after, us a launch of rows of 1536 and 512: 61 tokens 1.6 | 2.1, 1100 tokens 3.2 | 3.6, 65536 tokens 91 | 80 (6.7 TB/s;
-// 85.5 with 16-byte accesses).  In between it depends on where the rows come from.  Out of L2, as a projection has just written
-// them: 1531 tokens 3.5 | 3.8, 3072 tokens 5.0 | 5.5, 4096 tokens 6.1 | 6.1, 8192 tokens 10.5 | 9.3, which is where the line lies.
-// From HBM: 1531 tokens 4.5 | 4.0, 3072 tokens 6.8 | 6.4, 4096 tokens 8.6 | 7.6.
+// Whether the weights are fetched before the reduction (96 registers for rows of 1536, five CTAs per SM) or after it (72, seven).  Before,
+// they wait for nothing; after, more rows are in flight.  Before | after, us a launch of rows of 1536 and 512, out of L2 as a projection
+// has just written them, and from HBM:
+//   tokens   61         600        1100       1480       1500       2000       2300       2960       3600       4096       8192
+//   L2       1.6|2.2    2.0|2.6    2.5|3.1    2.6|3.2    3.1|3.2    3.4|3.4    3.7|4.7    4.2|5.1    4.9|5.3    5.3|5.6    10.5|9.0
+//   HBM      1.6|2.2    2.1|2.7    2.6|3.1    2.8|3.4    3.5|3.3    4.3|3.5    4.6|5.1    5.3|5.7    6.4|6.2    7.0|6.7    - |11.7
+// So it pays up to 4096 tokens, except where the launch is one wave of the other form and no longer one of this (1481 to 2072 tokens).
+// Four CTAs per SM of 102 registers, as before: 1300 tokens 3.0 and 3.6 instead of 2.6 and 2.7, 2960 tokens 4.6 and 6.1, 4096 tokens
+// 5.8 and 8.0; 1100 tokens 2.3 and 2.4 instead of 2.5 and 2.6.  65536 tokens 80 us (6.7 TB/s), before the reduction 91 us.
 constexpr int64_t kEarlyWeightTokens = 4096;
+constexpr int64_t kSms = 148;
 
-template <bool WIDE, bool EARLY>
-void launch_rows(const NormRows& q, const NormRows& kv, int64_t num_tokens, float eps, cudaStream_t stream) {
+template <bool WIDE, int CH>
+void launch_chunks(const NormRows& q, const NormRows& kv, int64_t num_tokens, float eps, cudaStream_t stream) {
     constexpr int WARPS = 4;
-    const dim3 grid(static_cast<unsigned>((2 * num_tokens + WARPS - 1) / WARPS));
+    const int64_t ctas = (2 * num_tokens + WARPS - 1) / WARPS;
+    const auto run = [&](auto* kernel) { launch_dependent(kernel, static_cast<unsigned>(ctas), WARPS * 32, stream, q, kv, num_tokens, eps); };
+    if constexpr (WIDE) {
+        const bool one_wave_late = ctas > kSms * ctas_per_sm(CH, true) && ctas <= kSms * ctas_per_sm(CH, false);
+        if (num_tokens <= kEarlyWeightTokens && !one_wave_late) return run(q_kv_rmsnorm_kernel<WARPS, CH, WIDE, true>);
+    }
+    run(q_kv_rmsnorm_kernel<WARPS, CH, WIDE, false>);
+}
+
+template <bool WIDE>
+void launch_rows(const NormRows& q, const NormRows& kv, int64_t num_tokens, float eps, cudaStream_t stream) {
     const int32_t longest = std::max(q.vec_ok ? q.size : 0, kv.vec_ok ? kv.size : 0);
-    const auto run = [&](auto* kernel) { launch_dependent(kernel, grid, WARPS * 32, stream, q, kv, num_tokens, eps); };
-    if (longest <= 512) run(q_kv_rmsnorm_kernel<WARPS, 1, WIDE, EARLY>);
-    else if (longest <= 1024) run(q_kv_rmsnorm_kernel<WARPS, 2, WIDE, EARLY>);
-    else if (longest <= 1536) run(q_kv_rmsnorm_kernel<WARPS, 3, WIDE, EARLY>);
-    else run(q_kv_rmsnorm_kernel<WARPS, 4, WIDE, EARLY>);
+    if (longest <= 512) launch_chunks<WIDE, 1>(q, kv, num_tokens, eps, stream);
+    else if (longest <= 1024) launch_chunks<WIDE, 2>(q, kv, num_tokens, eps, stream);
+    else if (longest <= 1536) launch_chunks<WIDE, 3>(q, kv, num_tokens, eps, stream);
+    else launch_chunks<WIDE, 4>(q, kv, num_tokens, eps, stream);
 }
 
 }  // namespace
@@ -213,9 +241,8 @@ cudaError_t launch_q_kv_rmsnorm(const void* q, void* q_out, const void* q_weight
                kv_in_stride, kv_out_stride, static_cast<int32_t>(kv_size), 0};
     a.vec_ok = on_boundaries(16, a) ? 1 : 0, b.vec_ok = on_boundaries(16, b) ? 1 : 0;
     const bool wide = (!a.vec_ok || on_boundaries(32, a)) && (!b.vec_ok || on_boundaries(32, b));
-    if (!wide) launch_rows<false, false>(a, b, num_tokens, eps, stream);
-    else if (num_tokens <= kEarlyWeightTokens) launch_rows<true, true>(a, b, num_tokens, eps, stream);
-    else launch_rows<true, false>(a, b, num_tokens, eps, stream);
+    if (wide) launch_rows<true>(a, b, num_tokens, eps, stream);
+    else launch_rows<false>(a, b, num_tokens, eps, stream);
     count_launch();
     return cudaGetLastError();
 }

@@ -25,3 +25,13 @@ def test_row_sizes(q_size, kv_size, offset, tokens):
     for got, rows, w in zip(fg.fused_q_kv_rmsnorm(q, kv, wq, wk, 1e-6), (q, kv), (wq, wk)):
         want = c_oracle.weighted_rmsnorm(rows.cpu().contiguous(), w.cpu(), 1e-6)
         assert int(compare.bf16_ulp_distance(got.cpu(), want).max()) <= 1
+
+
+@pytest.mark.parametrize("tokens", [1480, 1481, 2072, 2073, 4096, 4097])
+def test_both_sides_of_the_lines(tokens):
+    """Rows of 1536 and 512 either side of the launch sizes that decide when the weights are fetched."""
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    q, kv = torch.randn(tokens, 1536, generator=g, device=DEV).bfloat16(), torch.randn(tokens, 512, generator=g, device=DEV).bfloat16()
+    wq, wk = torch.randn(1536, generator=g, device=DEV).bfloat16(), torch.randn(512, generator=g, device=DEV).bfloat16()
+    for got, rows, w in zip(fg.fused_q_kv_rmsnorm(q, kv, wq, wk, 1e-6), (q, kv), (wq, wk)):
+        assert int(compare.bf16_ulp_distance(got.cpu(), c_oracle.weighted_rmsnorm(rows.cpu(), w.cpu(), 1e-6)).max()) <= 1
