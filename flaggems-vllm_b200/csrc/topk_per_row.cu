@@ -890,12 +890,28 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 5 : TWO ? 2 : 3) top
     int32_t left = to - from - tid;  // quads from this thread's next one to the end of the share
     int32_t position = row.position(from + tid);
     const float* next = row.x + position;
-    float4 v[kStreamBatch];
-    const auto load_batch = [&]() {
-#pragma unroll
-        for (int u = 0; u < kStreamBatch; ++u) v[u] = u * THREADS < left ? load_quad(next + 4 * u * THREADS) : none;
+    // every CTA of the cluster takes the same sample: runs of 8 consecutive quads (one 128-byte line each, where the row is
+    // so aligned) spread evenly over the row
+    const int32_t base = row.stride == 1 ? begin : 0, span = row.stride == 1 ? end - begin : row.quads;
+    const auto sampled_quad = [&](int32_t j) {  // runs of 8, each on a multiple of 8
+        const int32_t run = j >> 3;
+        const int32_t at = span > kSampleQuads ? static_cast<int32_t>(static_cast<uint32_t>((static_cast<uint64_t>(run) * static_cast<uint32_t>(span)) / (kSampleQuads / 8)) & ~7u) : 8 * run;
+        return at + (j & 7);
     };
-    load_batch();
+    // The sample is asked for first: everything waits for it, and it came late behind the first batches of a full GPU.  Before -> after, k 512:
+    // 496 x 262144 ragged 59.7 -> 58.6 us, full length 92.0 -> 90.7; 592 x 100000 37.2 -> 36.2; 2000 x 17003 39.1 -> 37.6; 4096 x 20001, k 2048
+    // 92.8 -> 90.0; 290 x 200000 34.7 -> 34.1; 4096 x 32768, k 2048 118.1 and 118.3.  More batches to L2 at the start cost more than they gave:
+    // 2 | 4 | 6 instead of one, 496 x 262144 60.2 | 61.9 | 64.7 us, 4096 x 32768, k 512 102 | 109 | 112 instead of 99.
+    constexpr int kMine = kSampleQuads / THREADS;
+    float4 sample[kMine];
+#pragma unroll
+    for (int u = 0; u < kMine; ++u) {
+        const int32_t quad = sampled_quad(tid + u * THREADS);
+        sample[u] = quad >= span ? none : row.stride == 1 ? load_quad(row.x + row.position(base + quad)) : row.load(base + quad);
+    }
+    float4 v[kStreamBatch];
+#pragma unroll
+    for (int u = 0; u < kStreamBatch; ++u) v[u] = u * THREADS < left ? load_quad(next + 4 * u * THREADS) : none;
     // The up to three values in front of the first whole quad and behind the last one, one per lane of the first CTA's first warp.
     float edge_value = -INFINITY;
     int32_t edge_position = -1;
@@ -915,33 +931,16 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 5 : TWO ? 2 : 3) top
     if (tid < 4) s.counters[tid] = 0u;
     if (tid == 4) s.pooled = 0u;
     __syncthreads();
-    // every CTA of the cluster takes the same sample: runs of 8 consecutive quads (one 128-byte line each, where the row is
-    // so aligned) spread evenly over the row
-    const int32_t base = row.stride == 1 ? begin : 0, span = row.stride == 1 ? end - begin : row.quads;
-    const auto sampled_quad = [&](int32_t j) {  // runs of 8, each on a multiple of 8
-        const int32_t run = j >> 3;
-        const int32_t at = span > kSampleQuads ? static_cast<int32_t>(static_cast<uint32_t>((static_cast<uint64_t>(run) * static_cast<uint32_t>(span)) / (kSampleQuads / 8)) & ~7u) : 8 * run;
-        return at + (j & 7);
-    };
     uint32_t largest = 0u;
     float peak = -INFINITY;
-    {
-        constexpr int kMine = kSampleQuads / THREADS;
-        float4 sample[kMine];
 #pragma unroll
-        for (int u = 0; u < kMine; ++u) {
-            const int32_t quad = sampled_quad(tid + u * THREADS);
-            sample[u] = quad >= span ? none : row.stride == 1 ? load_quad(row.x + row.position(base + quad)) : row.load(base + quad);
-        }
+    for (int u = 0; u < kMine; ++u) {
+        if (sampled_quad(tid + u * THREADS) >= span) continue;
+        const float value[4] = {sample[u].x, sample[u].y, sample[u].z, sample[u].w};
 #pragma unroll
-        for (int u = 0; u < kMine; ++u) {
-            if (sampled_quad(tid + u * THREADS) >= span) continue;
-            const float value[4] = {sample[u].x, sample[u].y, sample[u].z, sample[u].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                atomicAdd(&s.hist[coarse_bin(value[e])], 1u);
-                peak = fmaxf(peak, value[e]);
-            }
+        for (int e = 0; e < 4; ++e) {
+            atomicAdd(&s.hist[coarse_bin(value[e])], 1u);
+            peak = fmaxf(peak, value[e]);
         }
     }
     largest = order_key(__float_as_uint(peak));
