@@ -430,11 +430,9 @@ __device__ __forceinline__ float abs_max8(const uint4& v) {
 }
 
 // ---- quantisation with scale = max(amax, eps) / 448 (the epilogue quantiser and the per-token-group quantiser) ----
-// Power-of-two scale >= s as (exponent byte, value): ceil(log2(max(s, 1e-10))) from the bit pattern.
-__device__ __forceinline__ uint32_t pow2_ceil_code(float s) {
-    const uint32_t u = __float_as_uint(fmaxf(s, 1e-10f));
-    return ((u >> 23) & 0xffu) + ((u & 0x7fffffu) ? 1u : 0u);
-}
+// Exponent byte of the power of two >= s: ceil(log2(max(s, 1e-10))) + 127 from the bit pattern, the exponent field, one higher where
+// any mantissa bit is set.
+__device__ __forceinline__ uint32_t pow2_ceil_code(float s) { return (__float_as_uint(fmaxf(s, 1e-10f)) + 0x7fffffu) >> 23; }
 
 // How x / scale is formed for a scale that is not a power of two.
 enum : int { kDivideIeee = 0, kDivideFast = 1, kMultiplyReciprocal = 2 };

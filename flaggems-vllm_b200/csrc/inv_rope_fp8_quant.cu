@@ -34,11 +34,15 @@ struct InvRopeParams {
 // FASTDIV (fp32-scale mode only): see ScaleDivider.
 // WIDE: one 32-byte load and one 16-byte store per lane and head; otherwise (rows on 16-byte boundaries only) two of half the
 // size.
-// Two passes of U heads are in flight: the loads of the next pass go out before the current one is worked on (8192 x 128 rows:
-// 241 us, 253 us with one pass of four heads).
-// Bound by instruction issue before HBM in 16-byte pieces (253 us, fp32 scales 265 us); with 32-byte loads, 16-byte stores
-// and 6 shuffles a head 241 us = 6.7 TB/s and 247 us (245 us, and 61 x 128 rows 3.8 -> 3.6 us, since two values are divided by an instruction).
-// Two sets of registers that take turns instead of being copied: 61 x 128 rows 3.5 -> 3.4 us, but 8192 x 128 rows 241 -> 245 us.  CTAs per SM: 6 247 us, 7 241 us, 8 306 us (spills).
+// Two passes of U heads are in flight: the loads of the next pass go out before the current one is worked on.
+// HBM-bound at full clock (8192 x 128 rows 241 us = 6.7 TB/s), but in a run of some tenths of a second the power limit takes the clock to
+// 1.58 GHz, and there the kernel is bound by instruction issue: 182 warp instructions a head took 264-268 us, and fp32 scales 286-293.  Now:
+// every lane loads 32 bytes, the last four the rotary values once more, and a mask keeps them out of the maximum (no lane-dependent branch
+// around the loads, no zeroing); the last group's scale is formed once, by its own lanes, and fetched by a shuffle.  Sustained, before ->
+// after: 8192 x 128 rows 264-268 -> 252 us, fp32 scales 286-293 -> 273-275; 16384 x 16 67 -> 65; 1531 x 128 50.5 -> 49.2; 256 x 128
+// 11.1 -> 10.9 us.  The same arithmetic with two sets of registers that take turns instead of being copied: 151 instructions, but 266 us
+// and 286-303.  Heads per pass and CTAs per SM, 8192 x 128 rows: 2, 7 252 us; 1, 10 258; 1, 8 269; 2, 6 258; 2, 8 254 (fp32 scales 298);
+// 3, 6 306.
 constexpr int kMainLanes = 28;
 constexpr int kHeadsInFlight = 2;  // per pass
 constexpr int kCtasPerSm = 7;      // 72 registers
@@ -67,25 +71,27 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kerne
         }
         return;
     }
-    const uint8_t* in_token = p.o + static_cast<int64_t>(token) * p.o_stride_token * 2;
-    Bytes32 v[U], v_next[U];
-    uint32_t tail[U], tail_next[U];
-    const auto load_pass = [&](int h0, Bytes32 (&rv)[U], uint32_t (&rt)[U]) {
+    // A pass is U heads.  Past the last head of the task its first one is loaded once more.
+    struct Pass {
+        Bytes32 v[U];
+        uint32_t tail[U];
+    };
+    const int64_t head_stride = p.o_stride_head * 2;
+    const uint8_t* in = p.o + static_cast<int64_t>(token) * p.o_stride_token * 2 + head_begin * head_stride;  // of the next pass to load
+    const auto load_pass = [&](int h0, Pass& to) {
+        if (h0 < head_end) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            rv[u].lo = rv[u].hi = make_uint4(0u, 0u, 0u, 0u);
-            rt[u] = 0u;
-            if (h0 + u < head_end) {
-                const uint8_t* in = in_token + (h0 + u) * p.o_stride_head * 2;
-                if (lane < kMainLanes) {
-                    if (WIDE) rv[u] = ld_stream32(in + 32 * lane);
-                    else rv[u].lo = ld_stream16(in + 32 * lane), rv[u].hi = ld_stream16(in + 32 * lane + 16);
-                }
-                rt[u] = ld_stream4(in + 2 * kNopeDim + 4 * lane);
+            for (int u = 0; u < U; ++u) {
+                const uint8_t* from = u == 0 || h0 + u < head_end ? in + u * head_stride : in;
+                if (WIDE) to.v[u] = ld_stream32(from + 32 * lane);
+                else to.v[u].lo = ld_stream16(from + 32 * lane), to.v[u].hi = ld_stream16(from + 32 * lane + 16);
+                to.tail[u] = ld_stream4(from + 2 * kNopeDim + 4 * lane);
             }
         }
+        in += U * head_stride;
     };
-    load_pass(head_begin, v, tail);
+    Pass first, second;
+    load_pass(head_begin, first);
     const float* cs = p.cos_sin + p.positions[token] * p.cos_sin_stride;
     const float c = cs[lane], sn = cs[32 + lane];
     // Output addresses advance by constants from one head to the next and are recomputed only where a new group of heads
@@ -100,49 +106,49 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kerne
     const auto group_scale = [&](int g) { return p.scale + (g * p.scale_stride_group + token) * 4 + lane_scale; };
     uint8_t* out = group_out(group) + static_cast<int64_t>(head_in_group) * (kRowBytes / 2);
     uint8_t* scale_at = group_scale(group) + head_in_group * scale_step;
-    for (int h0 = head_begin; h0 < head_end; h0 += U) {
-        load_pass(h0 + U, v_next, tail_next);  // past the last head of the task: nothing is loaded
+    const uint32_t main_mask = lane < kMainLanes ? 0xffffffffu : 0u;  // lanes whose 16 values are not rotary ones
+    const uint32_t rotary_mask = lane >= 24 ? 0xffff0000u : 0u;  // lanes of the last group: the pairs belong to it
+    const int scale_shift = lane & 24;                           // chunk k of the head in byte k
+    const auto finish_pass = [&](int h0, const Pass& pass) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int head = h0 + u;
-            if (head >= head_end) break;
+            if (h0 + u >= head_end) break;
             // inverse rotation of the lane's pair, products rounded separately, then to bf16 as the torch path does
-            const float e = bf16_lo(tail[u]), o = bf16_hi(tail[u]);
+            const float e = bf16_lo(pass.tail[u]), o = bf16_hi(pass.tail[u]);
             const uint32_t rot = pack_bf16x2(__fadd_rn(__fmul_rn(e, c), __fmul_rn(o, sn)), __fsub_rn(__fmul_rn(o, c), __fmul_rn(e, sn)));
-            const float te = bf16_lo(rot), to = bf16_hi(rot);
             // Group maxima on the packed words: |.| maxima of the even and the odd elements side by side (the sign bits of
             // the intermediate words are meaningless and cleared at the end), then the maximum of the lane's 16 values in
             // the low half and that of its pair in the high half of one word.
-            const uint4 &a = v[u].lo, &b = v[u].hi;
-            const uint32_t pm = max_abs_bf16x2(max_abs_bf16x2(max_abs_bf16x2(a.x, a.y), max_abs_bf16x2(a.z, a.w)),
+            const uint4 &a = pass.v[u].lo, &b = pass.v[u].hi;
+            const uint32_t all = max_abs_bf16x2(max_abs_bf16x2(max_abs_bf16x2(a.x, a.y), max_abs_bf16x2(a.z, a.w)),
                                                max_abs_bf16x2(max_abs_bf16x2(b.x, b.y), max_abs_bf16x2(b.z, b.w)));
+            const uint32_t pm = all & main_mask;
             uint32_t both = max_abs_bf16x2(__byte_perm(pm, rot, 0x5410), __byte_perm(pm, rot, 0x7632)) & 0x7fff7fffu;
 #pragma unroll
             for (int m = 1; m <= 4; m <<= 1) both = max_bf16x2(both, __shfl_xor_sync(0xffffffffu, both, m));
-            const uint32_t of_eight = both;  // low half: the group's maximum (without the pairs in lanes 24-31)
+            const uint32_t of_eight = both;  // low half: the group's maximum, in the last group without the pairs
 #pragma unroll
             for (int m = 8; m <= 16; m <<= 1) both = max_bf16x2(both, __shfl_xor_sync(0xffffffffu, both, m));
-            const float m3 = fmaxf(bf16_hi(both), bf16_lo(__shfl_sync(0xffffffffu, of_eight, 24)));
-            const float mm = lane >= 24 ? m3 : bf16_lo(of_eight);
-            const float sm = __fmul_rn(fmaxf(mm, p.eps), 1.0f / 448.0f), s3 = __fmul_rn(fmaxf(m3, p.eps), 1.0f / 448.0f);
+            const float largest = fmaxf(bf16_lo(of_eight), __uint_as_float(both & rotary_mask));
+            const float scale = __fmul_rn(fmaxf(largest, p.eps), 1.0f / 448.0f);
             uint2 qa, qb;
             uint32_t qt;
             if (PACKED) {
-                const uint32_t code_m = pow2_ceil_code(sm), code_3 = pow2_ceil_code(s3);
-                qa = quant8_pow2(a, code_m), qb = quant8_pow2(b, code_m);
-                const float inv3 = __uint_as_float((254u - code_3) << 23);
-                qt = pack_e4m3x4(__fmul_rn(te, inv3), __fmul_rn(to, inv3), 0.f, 0.f);
-                // chunk k of the head in byte k
-                const uint32_t word = __reduce_or_sync(0xffffffffu, code_m << (8 * (lane >> 3)));
+                const uint32_t code = pow2_ceil_code(scale), code_3 = __shfl_sync(0xffffffffu, code, 24);
+                qa = quant8_pow2(a, code), qb = quant8_pow2(b, code);
+                const float2 t = scaled_pair(rot, static_cast<uint16_t>((254u - code_3) << 7));
+                qt = pack_e4m3x4(t.x, t.y, 0.f, 0.f);
+                const uint32_t word = __reduce_or_sync(0xffffffffu, code << scale_shift);
                 if (lane == 0) *reinterpret_cast<uint32_t*>(scale_at) = word;
             } else {
                 // the three-instruction form of the fast division for every scale: a warp-uniform choice between it and the
                 // two-instruction form was no faster
                 constexpr int kDivision = FASTDIV ? kDivideFast : kDivideIeee;
-                const ScaleDivider<kDivision> by_m(sm), by_3(s3);
-                qa = quant8_by<kDivision, false>(a, by_m), qb = quant8_by<kDivision, false>(b, by_m);
-                qt = pack_e4m3x4(by_3.template quotient<false>(te), by_3.template quotient<false>(to), 0.f, 0.f);
-                if ((lane & 7) == 0) *reinterpret_cast<float*>(scale_at) = sm;
+                const ScaleDivider<kDivision> by(scale), by_3(__shfl_sync(0xffffffffu, scale, 24));
+                qa = quant8_by<kDivision, false>(a, by), qb = quant8_by<kDivision, false>(b, by);
+                const float2 t = quotients<kDivision, false>(rot, by_3);
+                qt = pack_e4m3x4(t.x, t.y, 0.f, 0.f);
+                if ((lane & 7) == 0) *reinterpret_cast<float*>(scale_at) = scale;
             }
             if (lane < kMainLanes) {
                 if (WIDE) st_stream16(out + 16 * lane, make_uint4(qa.x, qa.y, qb.x, qb.y));
@@ -156,8 +162,11 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kerne
                 out = group_out(group), scale_at = group_scale(group);
             }
         }
-#pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = v_next[u], tail[u] = tail_next[u];
+    };
+    for (int h0 = head_begin; h0 < head_end; h0 += U) {
+        load_pass(h0 + U, second);  // past the end of the task: nothing
+        finish_pass(h0, first);
+        first = second;
     }
 }
 

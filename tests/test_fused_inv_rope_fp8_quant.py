@@ -101,7 +101,7 @@ def test_kernel_reproduces_upstream_reference(name, packed):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("packed", [False, True])
-@pytest.mark.parametrize("tokens,heads,groups", [(1, 64, 8), (7, 64, 8), (32, 128, 8), (128, 32, 4), (1001, 16, 1), (2, 3, 3)])
+@pytest.mark.parametrize("tokens,heads,groups", [(1, 64, 8), (7, 64, 8), (32, 128, 8), (128, 32, 4), (1001, 16, 1), (2, 3, 3), (3, 1, 1), (9, 5, 1), (2500, 17, 1), (1300, 21, 3)])
 def test_kernel_matches_oracle_and_layout_contract(tokens, heads, groups, packed):
     g = torch.Generator().manual_seed(tokens * 131 + heads)
     o = torch.randn(tokens, heads, 512, generator=g).to(torch.bfloat16)
