@@ -49,6 +49,8 @@ def test_kernel_reproduces_upstream_reference(name):
 @pytest.mark.parametrize("tokens,cols,group,column_major", [
     (1, 512, 128, False), (83, 4096, 128, False), (83, 5120, 64, True), (7, 13824, 128, True), (33, 2048, 256, False), (9, 4096, 512, True),
     (5, 96, 48, False), (6, 120, 24, True),
+    # numbers of groups that end inside a warp's pass: one, 17 and 65 of them, two groups a lane group above 32768
+    (1, 128, 128, True), (17, 64, 64, False), (13, 640, 128, False), (3, 256, 256, True), (1, 512, 512, False), (4099, 1152, 128, True), (1009, 2112, 64, False),
 ])
 def test_kernel_matches_oracle(tokens, cols, group, column_major, ue8m0):
     """The upstream shape list (7 / 83 tokens, 512 ... 13824 columns, groups of 64 ... 512), both scale layouts, group
