@@ -17,13 +17,13 @@
 #include <ATen/EmptyTensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
-#include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdio>
 
 #include "../../include/dsv4_prologue.h"
+#include "current_device.h"
 
 namespace {
 
@@ -104,12 +104,12 @@ bool is(const Tensor& t, ScalarType type) { return t.scalar_type() == type; }
 bool on(const Tensor& t, const Tensor& first) { return t.is_cuda() && t.get_device() == first.get_device(); }
 
 // A contiguous, uninitialised tensor on the device of `like`.  Where that device is current, as it is in nearly every call, without the
-// look at torch's set-up and the device guard that empty_cuda() takes each time: 0.36 instead of 0.45 us a tensor, a call with two of them
-// 4.25 -> 4.0 us.
+// look at torch's set-up and the device guard that empty_cuda() takes each time.
 Tensor make_empty(at::IntArrayRef sizes, ScalarType type, const Tensor& like) {
     static const bool set_up = (at::globalContext().lazyInitDevice(at::kCUDA), true);
+    (void)set_up;
     const at::Device device = like.device();
-    if (!set_up || device.index() != c10::cuda::current_device()) return Tensor(at::detail::empty_cuda(sizes, type, device, std::nullopt));
+    if (!dsv4::is_current(device.index())) return Tensor(at::detail::empty_cuda(sizes, type, device, std::nullopt));
     return Tensor(at::detail::empty_generic(sizes, c10::cuda::CUDACachingAllocator::get(), c10::DispatchKeySet(c10::DispatchKey::CUDA), type, std::nullopt));
 }
 
@@ -123,16 +123,15 @@ void set_view(Tensor& t, at::IntArrayRef sizes, at::IntArrayRef strides) {
 template <typename Launch>
 bool launch_on(const Tensor& first, Launch&& launch) {
     const auto device = static_cast<c10::DeviceIndex>(first.get_device());
-    int code;
-    {
-        c10::cuda::OptionalCUDAGuard guard;
-        if (device != c10::cuda::current_device()) guard.set_device(at::Device(at::kCUDA, device));
+    const int code = dsv4::with_device(device, [&] {
         void* stream = c10::cuda::getCurrentCUDAStream(device).stream();
+        int result;
         // a launch can block (full launch queue): other Python threads go on meanwhile
         Py_BEGIN_ALLOW_THREADS
-        code = launch(stream);
+        result = launch(stream);
         Py_END_ALLOW_THREADS
-    }
+        return result;
+    });
     if (code == 0) return true;
     PyObject* r = PyObject_CallFunction(g_check, "i", code);
     if (r) {

@@ -26,7 +26,7 @@ HOST_SOURCES = ("host_calls.cpp",)
 PROBE_SOURCES = ("hbm_probe.cu", "division_probe.cu")
 SOURCES = ("abi.cu", "prologue_rows.cu", "prologue_bulk.cu", "gather_dequant.cu", "q_kv_rmsnorm.cu", "inv_rope_fp8_quant.cu", "indexer_k_quant.cu",
            "indexer_q_rope_quant.cu", "cp_gather_indexer.cu", "topk_indices.cu", "topk_per_row.cu", "group_quant_fp8.cu")
-HEADERS = ("dsv4_common.cuh", "../../include/dsv4_prologue.h", "../../include/dsv4_hbm_probe.h")
+HEADERS = ("dsv4_common.cuh", "current_device.h", "../../include/dsv4_prologue.h", "../../include/dsv4_hbm_probe.h")
 
 
 def nvcc_path() -> str:
