@@ -431,8 +431,11 @@ __device__ __forceinline__ float abs_max8(const uint4& v) {
 
 // ---- quantisation with scale = max(amax, eps) / 448 (the epilogue quantiser and the per-token-group quantiser) ----
 // Exponent byte of the power of two >= s: ceil(log2(max(s, 1e-10))) + 127 from the bit pattern, the exponent field, one higher where
-// any mantissa bit is set.
+// any mantissa bit is set.  255 where s is infinite.
 __device__ __forceinline__ uint32_t pow2_ceil_code(float s) { return (__float_as_uint(fmaxf(s, 1e-10f)) + 0x7fffffu) >> 23; }
+// 1 / 2^(code - 127) as the bits of a bf16.  Zero where the scale is infinite, so that x / inf is 0 for a finite x and NaN for an infinite
+// one; the codes of finite bf16 maxima end at 247.
+__device__ __forceinline__ uint32_t pow2_reciprocal(uint32_t code) { return static_cast<uint32_t>(max(254 - static_cast<int>(code), 0)) << 7; }
 
 // How x / scale is formed for a scale that is not a power of two.
 enum : int { kDivideIeee = 0, kDivideFast = 1, kMultiplyReciprocal = 2 };
@@ -527,13 +530,15 @@ __device__ __forceinline__ float2 scaled_pair(uint32_t pair, uint16_t factor) {
     return r;
 }
 
-// 8 bf16 values times the exact reciprocal of a power-of-two scale (same result as dividing by it).  The reciprocal's exponent field
-// 254 - code is in range for every bf16 maximum.
-__device__ __forceinline__ uint2 quant8_pow2(const uint4& v, uint32_t code) {
-    const auto factor = static_cast<uint16_t>((254u - code) << 7);  // 2^(127 - code)
-    const float2 x0 = scaled_pair(v.x, factor), x1 = scaled_pair(v.y, factor), x2 = scaled_pair(v.z, factor), x3 = scaled_pair(v.w, factor);
+// 8 bf16 values times a power of two, given as bf16, to e4m3.
+__device__ __forceinline__ uint2 quant8_times(const uint4& v, uint32_t factor) {
+    const auto f = static_cast<uint16_t>(factor);
+    const float2 x0 = scaled_pair(v.x, f), x1 = scaled_pair(v.y, f), x2 = scaled_pair(v.z, f), x3 = scaled_pair(v.w, f);
     return make_uint2(pack_e4m3x4(x0.x, x0.y, x1.x, x1.y), pack_e4m3x4(x2.x, x2.y, x3.x, x3.y));
 }
+
+// 8 bf16 values times the exact reciprocal of a power-of-two scale (same result as dividing by it).
+__device__ __forceinline__ uint2 quant8_pow2(const uint4& v, uint32_t code) { return quant8_times(v, pow2_reciprocal(code)); }
 
 // 8 bf16 -> 8 e4m3 bytes of value x / 2^(code-127) (division by a power of two: exact).
 __device__ __forceinline__ uint2 quant8(const uint4& v, uint32_t code) {

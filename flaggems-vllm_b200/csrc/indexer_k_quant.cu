@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_k_quant_rows_kernel(const 
 #ifndef DSV4_INDEXER_K_CTAS
 #define DSV4_INDEXER_K_CTAS 1
 #endif
-// UE8M0 (power-of-two scales): bf16 keys stay packed - group maximum and scaling on the bf16x2 words, as in quant8_pow2.
+// UE8M0 (power-of-two scales): bf16 keys stay packed up to the group maximum and are widened as they are scaled (quant8_pow2).
 template <int WARPS, int U, bool FP16, bool UE8M0>
 __global__ void __launch_bounds__(WARPS * 32, DSV4_INDEXER_K_CTAS) indexer_k_quant_128_kernel(const Launched<IndexerParams> p) {
     const int lane = threadIdx.x & 31, sub = lane & 7, which = lane >> 3;

@@ -134,9 +134,9 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kerne
             uint2 qa, qb;
             uint32_t qt;
             if (PACKED) {
-                const uint32_t code = pow2_ceil_code(scale), code_3 = __shfl_sync(0xffffffffu, code, 24);
-                qa = quant8_pow2(a, code), qb = quant8_pow2(b, code);
-                const float2 t = scaled_pair(rot, static_cast<uint16_t>((254u - code_3) << 7));
+                const uint32_t code = pow2_ceil_code(scale), factor = pow2_reciprocal(code), factor_3 = __shfl_sync(0xffffffffu, factor, 24);
+                qa = quant8_times(a, factor), qb = quant8_times(b, factor);
+                const float2 t = scaled_pair(rot, static_cast<uint16_t>(factor_3));
                 qt = pack_e4m3x4(t.x, t.y, 0.f, 0.f);
                 const uint32_t word = __reduce_or_sync(0xffffffffu, code << scale_shift);
                 if (lane == 0) *reinterpret_cast<uint32_t*>(scale_at) = word;
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(WARPS * 32) inv_rope_fp8_quant_any_kernel(cons
         if (PACKED) {
             const uint32_t code = pow2_ceil_code(scale);
             word |= code << (8 * k);
-            inv = __uint_as_float((254u - code) << 23);
+            inv = bf16_lo(pow2_reciprocal(code));
         }
         for (int pr = lane; pr < geo.group / 2; pr += 32) {
             const int e0 = k * geo.group + 2 * pr;
