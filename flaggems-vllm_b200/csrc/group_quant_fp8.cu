@@ -83,9 +83,13 @@ __global__ void __launch_bounds__(WARPS * 32) group_quant_fp8_kernel(const Launc
         } else {
             // one warp-uniform choice of the division form per pass (see ScaleDivider); lanes past the last group
             // have left the loop body above only after the vote, so every lane takes part in it
-            const ScaleDivider<DIVISION> by_scale(scale);
-            if (two_term) qa = quant8_by<DIVISION, true>(a, by_scale), qb = quant8_by<DIVISION, true>(b, by_scale);
-            else qa = quant8_by<DIVISION, false>(a, by_scale), qb = quant8_by<DIVISION, false>(b, by_scale);
+            if (two_term) {
+                const ScaleDivider<DIVISION> by_scale(scale);
+                qa = quant8_by<DIVISION, true>(a, by_scale), qb = quant8_by<DIVISION, true>(b, by_scale);
+            } else {
+                const ScaleDivider<DIVISION> by_scale(DIVISION == kDivideFast ? finite_scale(scale) : scale);
+                qa = quant8_by<DIVISION, false>(a, by_scale), qb = quant8_by<DIVISION, false>(b, by_scale);
+            }
         }
         uint8_t* dst = p.out + g * p.group_size + 16 * sub;
         if (WIDE) st_stream16(dst, make_uint4(qa.x, qa.y, qb.x, qb.y));

@@ -144,11 +144,13 @@ __global__ void __launch_bounds__(WARPS * 32, MIN_CTAS) inv_rope_fp8_quant_kerne
                 // the three-instruction form of the fast division for every scale: a warp-uniform choice between it and the
                 // two-instruction form was no faster
                 constexpr int kDivision = FASTDIV ? kDivideFast : kDivideIeee;
-                const ScaleDivider<kDivision> by(scale), by_3(__shfl_sync(0xffffffffu, scale, 24));
+                // stored before the division, which then has one register more
+                if ((lane & 7) == 0) *reinterpret_cast<float*>(scale_at) = scale;
+                const float divisor = FASTDIV ? finite_scale(scale) : scale;
+                const ScaleDivider<kDivision> by(divisor), by_3(__shfl_sync(0xffffffffu, divisor, 24));
                 qa = quant8_by<kDivision, false>(a, by), qb = quant8_by<kDivision, false>(b, by);
                 const float2 t = quotients<kDivision, false>(rot, by_3);
                 qt = pack_e4m3x4(t.x, t.y, 0.f, 0.f);
-                if ((lane & 7) == 0) *reinterpret_cast<float*>(scale_at) = scale;
             }
             if (lane < kMainLanes) {
                 if (WIDE) st_stream16(out + 16 * lane, make_uint4(qa.x, qa.y, qb.x, qb.y));
