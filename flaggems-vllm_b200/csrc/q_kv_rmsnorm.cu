@@ -195,15 +195,16 @@ bool on_boundaries(uintptr_t bytes, const NormRows& t) {
            t.out_stride % elements == 0 && t.size % elements == 0 && t.size <= kMaxChunks * 512;
 }
 
-// Whether the weights are fetched before the reduction (96 registers for rows of 1536, five CTAs per SM) or after it (72, seven).  Before,
-// they wait for nothing; after, more rows are in flight.  Before | after, us a launch of rows of 1536 and 512, out of L2 as a projection
-// has just written them, and from HBM:
-//   tokens   61         600        1100       1480       1500       2000       2300       2960       3600       4096       8192
-//   L2       1.6|2.2    2.0|2.6    2.5|3.1    2.6|3.2    3.1|3.2    3.4|3.4    3.7|4.7    4.2|5.1    4.9|5.3    5.3|5.6    10.5|9.0
-//   HBM      1.6|2.2    2.1|2.7    2.6|3.1    2.8|3.4    3.5|3.3    4.3|3.5    4.6|5.1    5.3|5.7    6.4|6.2    7.0|6.7    - |11.7
-// So it pays up to 4096 tokens, except where the launch is one wave of the other form and no longer one of this (1481 to 2072 tokens).
-// Four CTAs per SM of 102 registers, as before: 1300 tokens 3.0 and 3.6 instead of 2.6 and 2.7, 2960 tokens 4.6 and 6.1, 4096 tokens
-// 5.8 and 8.0; 1100 tokens 2.3 and 2.4 instead of 2.5 and 2.6.  65536 tokens 80 us (6.7 TB/s), before the reduction 91 us.
+// Whether the weights are fetched before the reduction or after it.  Before, they wait for nothing; after, fewer registers are held and
+// more rows are in flight.  Before | after, us a launch from a graph, rows of 1536 and 512 (96 registers and five CTAs per SM | 72 and
+// seven), out of L2 as a projection has just written them, and from HBM:
+//   tokens   61         600        1100       1480       1531       2000       2300       2960       3600       4096       8192
+//   L2       1.5|1.9    1.7|2.3    2.3|3.0    2.4|3.1    2.9|3.1    3.3|3.1    3.5|4.4    4.0|4.9    4.8|5.1    5.1|5.4    8.8|8.7
+//   HBM      1.5|1.8    1.9|2.4    2.4|2.9    2.6|3.2    3.4|3.2    4.0|3.3    4.3|4.9    5.0|5.4    6.2|6.0    6.8|6.4   12.3|11.4
+// So before up to 4096 tokens (from about 3300 on out of L2 only), except where the launch is one wave of the other form and no longer
+// one of this: 1481 to 2072 tokens (1481 tokens 2.7|3.1 and 3.0|3.2).  Other widths have such a range too, but there the other form spills, or loses out of L2 what it gains
+// from HBM: 512 + 512, 3200 tokens 2.6|3.7 and 3.4|3.6; 1024 + 512, 2073 tokens 2.4|3.2 and 2.9|3.2, 2600 tokens 3.1|3.2 and 3.8|3.4;
+// 2048 + 512, 1185 tokens 2.8|3.5 and 3.2|3.6, 1500 tokens 3.4|3.5 and 4.1|3.5.
 constexpr int64_t kEarlyWeightTokens = 4096;
 constexpr int64_t kSms = 148;
 
@@ -213,7 +214,7 @@ void launch_chunks(const NormRows& q, const NormRows& kv, int64_t num_tokens, fl
     const int64_t ctas = (2 * num_tokens + WARPS - 1) / WARPS;
     const auto run = [&](auto* kernel) { launch_dependent(kernel, static_cast<unsigned>(ctas), WARPS * 32, stream, q, kv, num_tokens, eps); };
     if constexpr (WIDE) {
-        const bool one_wave_late = ctas > kSms * ctas_per_sm(CH, true) && ctas <= kSms * ctas_per_sm(CH, false);
+        const bool one_wave_late = CH == 3 && ctas > kSms * ctas_per_sm(CH, true) && ctas <= kSms * ctas_per_sm(CH, false);
         if (num_tokens <= kEarlyWeightTokens && !one_wave_late) return run(q_kv_rmsnorm_kernel<WARPS, CH, WIDE, true>);
     }
     run(q_kv_rmsnorm_kernel<WARPS, CH, WIDE, false>);
