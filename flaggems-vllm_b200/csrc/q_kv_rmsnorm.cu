@@ -94,7 +94,9 @@ q_kv_rmsnorm_kernel(const Launched<NormRows, sizeof(NormRows) + 16> q, const Nor
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
         const float rr = inv_rms_of(acc, size, eps);
-        // two values an instruction; the same products, each rounded (32768 tokens 41.1 -> 40.7 us)
+        // Two values an instruction, the same products, each rounded: rows of 512 on 16-byte boundaries 16384 tokens 16.8 -> 15.1 us, others
+        // up to 2 %.  Not where it spills (16-byte form, rows of up to 1024 and 2048: 16384 tokens 19.2 us scalar and 21.9 packed, 32.2 and 34.3).
+        constexpr bool kPairs = WIDE || CH % 2 == 1;
         const auto product = [&](uint32_t xv, uint32_t wv) {
             float2 y;
             asm("{.reg .b64 x, r, w;\n\t"
@@ -109,6 +111,13 @@ q_kv_rmsnorm_kernel(const Launched<NormRows, sizeof(NormRows) + 16> q, const Nor
             return pack_bf16x2(y.x, y.y);
         };
         const auto apply = [&](const uint4& xv, const uint4& wv) {
+            if (!kPairs) {
+                float f[8], g[8];
+                unpack8(xv, f), unpack8(wv, g);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) f[i] = __fmul_rn(__fmul_rn(f[i], rr), g[i]);
+                return pack8(f);
+            }
             return make_uint4(product(xv.x, wv.x), product(xv.y, wv.y), product(xv.z, wv.z), product(xv.w, wv.w));
         };
 #pragma unroll
