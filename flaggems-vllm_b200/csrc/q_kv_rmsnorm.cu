@@ -40,8 +40,8 @@ constexpr int ctas_per_sm(int chunks, bool early) {  // of 128 threads
     return early ? (chunks == 1 ? 10 : chunks == 2 ? 7 : chunks == 3 ? 5 : 4) : (chunks == 1 ? 16 : chunks == 2 ? 10 : chunks == 3 ? 7 : 6);
 }
 
-template <int WARPS, int CH, bool WIDE, bool EARLY>
-__global__ void __launch_bounds__(WARPS * 32, ctas_per_sm(CH, EARLY))
+template <int WARPS, int CH, bool WIDE, bool EARLY, int CTAS = ctas_per_sm(CH, EARLY)>
+__global__ void __launch_bounds__(WARPS * 32, CTAS)
 q_kv_rmsnorm_kernel(const Launched<NormRows, sizeof(NormRows) + 16> q, const NormRows kv, int64_t num_tokens, float eps) {
     const int lane = threadIdx.x & 31;
     const int64_t r = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
@@ -215,6 +215,11 @@ bool on_boundaries(uintptr_t bytes, const NormRows& t) {
 // from HBM: 512 + 512, 3200 tokens 2.6|3.7 and 3.4|3.6; 1024 + 512, 2073 tokens 2.4|3.2 and 2.9|3.2, 2600 tokens 3.1|3.2 and 3.8|3.4;
 // 2048 + 512, 1185 tokens 2.8|3.5 and 3.2|3.6, 1500 tokens 3.4|3.5 and 4.1|3.5.
 constexpr int64_t kEarlyWeightTokens = 4096;
+// With rows of up to 1536, the early form with four CTAs per SM (102 registers) instead of five, while the launch is one wave of it and
+// two such launches, one draining and one starting, no longer fit side by side with five: 741 to 1184 tokens.  Four | five: 600 tokens
+// 2.0|1.7 and 2.0|1.9, 740 tokens 2.2|1.8 and 2.2|2.0, 780 tokens 2.2|2.2 and 2.3|2.3, 900 tokens 2.0|2.3 and 2.2|2.4, 1184 tokens 2.1|2.3
+// and 2.3|2.4, 1185 tokens 2.5|2.3 and 2.9|2.4, 2960 tokens 4.3|4.0 and 5.8|5.0.
+constexpr int kRoomyCtas = 4;
 constexpr int64_t kSms = 148;
 
 template <bool WIDE, int CH>
@@ -223,6 +228,9 @@ void launch_chunks(const NormRows& q, const NormRows& kv, int64_t num_tokens, fl
     const int64_t ctas = (2 * num_tokens + WARPS - 1) / WARPS;
     const auto run = [&](auto* kernel) { launch_dependent(kernel, static_cast<unsigned>(ctas), WARPS * 32, stream, q, kv, num_tokens, eps); };
     if constexpr (WIDE) {
+        if constexpr (CH == 3) {
+            if (2 * ctas > kSms * ctas_per_sm(CH, true) && ctas <= kSms * kRoomyCtas) return run(q_kv_rmsnorm_kernel<WARPS, CH, WIDE, true, kRoomyCtas>);
+        }
         const bool one_wave_late = CH == 3 && ctas > kSms * ctas_per_sm(CH, true) && ctas <= kSms * ctas_per_sm(CH, false);
         if (num_tokens <= kEarlyWeightTokens && !one_wave_late) return run(q_kv_rmsnorm_kernel<WARPS, CH, WIDE, true>);
     }

@@ -27,9 +27,9 @@ def test_row_sizes(q_size, kv_size, offset, tokens):
         assert int(compare.bf16_ulp_distance(got.cpu(), want).max()) <= 1
 
 
-@pytest.mark.parametrize("q_size,tokens", [(1536, n) for n in (1480, 1481, 2072, 2073, 4096, 4097)] + [(512, 2961), (512, 4097), (1024, 2073), (1024, 2961), (2048, 1185), (2048, 1777)])
+@pytest.mark.parametrize("q_size,tokens", [(1536, n) for n in (740, 741, 1184, 1185, 1480, 1481, 2072, 2073, 4096, 4097)] + [(512, 2961), (512, 4097), (1024, 2073), (1024, 2961), (2048, 1185), (2048, 1777)])
 def test_both_sides_of_the_lines(q_size, tokens):
-    """Either side of the launch sizes that decide, for rows of 1536 and 512, when the weights are fetched, and where a wave of the
+    """Either side of the launch sizes that decide, for rows of 1536 and 512, when the weights are fetched and with how many CTAs per SM, and where a wave of the
     other widths ends."""
     g = torch.Generator(device=DEV).manual_seed(tokens)
     q, kv = torch.randn(tokens, q_size, generator=g, device=DEV).bfloat16(), torch.randn(tokens, 512, generator=g, device=DEV).bfloat16()
