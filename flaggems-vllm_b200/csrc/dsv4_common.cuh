@@ -450,7 +450,7 @@ enum : int { kDivideIeee = 0, kDivideFast = 1, kMultiplyReciprocal = 2 };
 // q can differ from RN(x/scale) in the last fp32 bit, but never in the e4m3 byte of an x that is not -0: a CPU test enumerates every bf16
 // group maximum (hence every reachable scale, for the reference's eps = 1e-10) against every bf16 value below it, for
 // each of the three values y can take (the correctly rounded reciprocal and its two neighbours) and both forms -
-// 1.6e9 cases each, zero differing bytes.  The form is a template argument: a caller that uses the two-term form votes once
+// 1.6e9 cases each, zero differing bytes; a GPU test enumerates them with quotients() below and the device's own reciprocal.  The form is a template argument: a caller that uses the two-term form votes once
 // per warp on the scales' range (`__all_sync`), so the choice is a uniform branch around straight-line code; the epilogue
 // quantiser uses the corrected form throughout (no second code path measured faster there).  For any other eps the
 // kernels divide.
@@ -474,24 +474,20 @@ struct ScaleDivider {
         }
     }
     __device__ __forceinline__ bool allows_two_term() const { return scale <= kTwoTermMaxScale; }
-    // TWO_TERM is honoured in kDivideFast mode only
-    template <bool TWO_TERM>
-    __device__ __forceinline__ float quotient(float x) const {
-        if (MODE == kMultiplyReciprocal) return __fmul_rn(x, recip);
-        if (MODE == kDivideIeee) return __fdiv_rn(x, scale);
-        if (TWO_TERM) return __fmaf_rn(x, recip, __fmul_rn(x, recip_lo));
-        const float q0 = __fmul_rn(x, recip);
-        return __fmaf_rn(__fmaf_rn(-scale, q0, x), recip, q0);
+    __device__ __forceinline__ float quotient(float x) const {  // of the other two modes
+        static_assert(MODE != kDivideFast, "quotients() divides");
+        return MODE == kMultiplyReciprocal ? __fmul_rn(x, recip) : __fdiv_rn(x, scale);
     }
 };
 
-// The same of both halves of a bf16 pair, two values an instruction.
+// Both halves of a bf16 pair divided, with kDivideFast two values an instruction.  TWO_TERM is honoured in that mode only.
 template <int MODE, bool TWO_TERM>
 __device__ __forceinline__ float2 quotients(uint32_t pair, const ScaleDivider<MODE>& d) {
     const float2 x = make_float2(bf16_lo(pair), bf16_hi(pair));
-    if (MODE != kDivideFast) return make_float2(d.template quotient<TWO_TERM>(x.x), d.template quotient<TWO_TERM>(x.y));
     float2 q;
-    if (TWO_TERM)
+    if constexpr (MODE != kDivideFast)
+        q = make_float2(d.quotient(x.x), d.quotient(x.y));
+    else if constexpr (TWO_TERM)
         asm("{.reg .b64 x, y, l;\n\t"
             "mov.b64 x, {%2, %3};\n\t"
             "mov.b64 y, {%4, %4};\n\t"

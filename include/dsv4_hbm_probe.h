@@ -27,7 +27,7 @@ int dsv4_hbm_probe(int mode, void* buffer, int64_t rows, void* cuda_stream);
 /*
  * On-device check of the division shortcut the quantisers use for fp32 scales (product with a refined approximate
  * reciprocal; form 2 = two-term, scales up to 2^100, form 3 = corrected product, any scale).  For every non-negative
- * finite bf16 group maximum and every bf16 value up to it, with scale = max(amax, eps) / 448 as the operators form it,
+ * finite bf16 group maximum and every bf16 value up to it, of either sign, two at a time as the operators divide them, with scale = max(amax, eps) / 448 as the operators form it,
  * adds to counts[0] the pairs examined, to counts[1] those whose e4m3 byte differs from that of the IEEE quotient and
  * to counts[2] the scales whose refined reciprocal is more than one unit in the last place from the correctly rounded
  * one.  `counts` is caller-allocated device memory of three 64-bit words that the caller has zeroed.  A test aid: the
