@@ -456,6 +456,48 @@ cudaError_t launch_e(const IndexerQParams& p, bool fp4, unsigned grid, cudaStrea
     return cudaGetLastError();
 }
 
+// Heads per warp (a task: that many heads of one token, or what is left of them): few rows, short tasks, so that there are enough of them;
+// many rows, long ones, whose set-up more heads share; and where tasks of 64 or 32 heads make one wave that is nearly full, those.
+// FP8 / MXFP4, us a launch of 64 heads a token, from a graph with three inputs in rotation (from 3072 tokens on they come from HBM):
+//   8 | 16           200 tokens  2.4 / 2.4 | 2.5 / 2.4         256 tokens  2.7 / 2.7 | 2.5 / 2.5
+//   16 | 32 | 64      832 tokens  3.7 / 3.7 | 3.9 / 3.5 | 5.1 / 4.7        1280 tokens  5.7 / 5.6 | 5.8 / 5.5 | 6.1 / 6.0
+//                    1536 tokens  6.8 / 6.2 | 6.1 / 5.8 | 7.5 / 6.9        1800 tokens  8.8 / 8.4 | 8.9 / 8.1 | 9.0 / 8.7
+//                    2500 tokens 10.7 / 10.3 | 11.5 / 11.1 | 10.7 / 10.5   3072 tokens 13.4 / 12.9 | 12.6 / 12.2 | 12.0 / 11.7
+//                    4096 tokens 18.1 / 17.0 | 18.2 / 17.0 | 19.9 / 18.4   8192 tokens 36.2 / 33.1 | 34.5 / 31.0 | 35.4 / 31.9
+//   32 | prefetch    8192 tokens 34.5 / 31.0 | 34.0 / 31.4       9216 tokens 39.0 / 34.9 | 37.4 / 34.3     32768 tokens 127 / 113 | 121 / 109
+// (With 64 at 5500 to 6500 tokens, nearly two waves of them, 3 % less than with 32.)
+// Other numbers of heads: a short last task costs nearly a long one's place, so it is the number of tasks that decides, and tasks of one
+// length are preferred.  16 | 32 | 64:
+//    96 heads: 1979 tokens 14.3 / 13.3 | 14.0 / 12.8 | 17.7 / 16.4     75 heads: 2533 tokens 14.6 / 13.7 | 16.0 / 14.7 | 17.8 / 16.5
+//    80 heads: 1125 tokens  7.3 / 6.4 | 7.0 / 6.0 | 9.0 / 8.1          1625 tokens 10.7 / 10.1 | 11.4 / 10.6 | 11.1 / 10.1
+//    48 heads: 1875 tokens  7.3 / 6.4 | 8.5 / 7.6 | 8.4 / 7.7          3958 tokens 14.3 / 13.3 | 15.4 / 14.2 | 15.9 / 14.7
+//              3437 tokens 12.3 / 11.3 | 12.7 / 11.6 | 11.7 / 10.6     5416 tokens 18.4 / 17.0 | 19.7 / 18.1 | 18.4 / 16.7
+//             16000 tokens 49.7 / 45.0 | 46.4 / 42.1 | 47.4 / 43.2    56 heads: 5000 tokens 20.4 / 18.9 | 19.2 / 17.2 | 20.0 / 18.3
+//    40 heads: 5520 tokens 16.8 / 15.8 | 17.6 / 16.3 | 15.9 / 14.4    14746 tokens 41.0 / 37.9 | 37.5 / 34.7 | 37.0 / 34.1
+//    24 heads: 2500 tokens  5.3 / 5.1 | 5.0 / 4.6 | 5.0 / 4.6          6875 tokens 13.4 / 12.6 | 12.0 / 10.7 | 12.0 / 10.7
+constexpr int kHeadsWarps = 4;                    // per CTA
+constexpr int64_t kWave = 148 * 6 * kHeadsWarps;  // warps of a B200
+constexpr int64_t kPrefetchRows = 589824;         // from here on a task sends the rest of its rows to L2 at its start
+constexpr int heads_of_a_task(int64_t tokens, int heads) {
+    const int64_t rows = tokens * heads;
+    const auto one_length = [&](int n) { return heads <= n || heads % n == 0; };
+    const auto fills = [&](int n, int64_t waves) {
+        const int64_t tasks = tokens * ((heads + n - 1) / n);
+        return tasks <= waves * kWave && 9 * tasks >= 7 * waves * kWave;
+    };
+    if (one_length(64) && fills(64, 1)) return 64;
+    if (rows > kWave * 64) return heads > 32 && heads <= (rows >= kPrefetchRows ? 40 : 48) ? 64 : 32;
+    if (fills(32, 1) || (one_length(32) && fills(32, 2))) return 32;
+    if (rows < 14336) return 8;
+    for (int n = 32; n <= 64 && !one_length(16); n *= 2)
+        if (one_length(n) && 9 * rows >= 7 * kWave * n) return n;
+    return 16;
+}
+static_assert(heads_of_a_task(223, 64) == 8 && heads_of_a_task(224, 64) == 16 && heads_of_a_task(1381, 64) == 16 && heads_of_a_task(1382, 64) == 32);
+static_assert(heads_of_a_task(1777, 64) == 16 && heads_of_a_task(2763, 64) == 64 && heads_of_a_task(3552, 64) == 64 && heads_of_a_task(3553, 64) == 32);
+static_assert(heads_of_a_task(1979, 96) == 32 && heads_of_a_task(2533, 75) == 16 && heads_of_a_task(4600, 48) == 16 && heads_of_a_task(1875, 48) == 16);
+static_assert(heads_of_a_task(3437, 48) == 64 && heads_of_a_task(5416, 48) == 64 && heads_of_a_task(12289, 48) == 32 && heads_of_a_task(2250, 40) == 16 && heads_of_a_task(6500, 40) == 64);
+
 }  // namespace
 
 cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q, int64_t q_stride0, int64_t q_stride1,
@@ -484,21 +526,9 @@ cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q,
     const bool heads_shape = head_dim == 128 && rot_dim == 64 && rows_shape &&
                              (fp4 || (addr(out) % 16 == 0 && out_stride0 % 16 == 0 && out_stride1 % 16 == 0));
     if (heads_shape) {
-        constexpr int WARPS = 4;
-        // Heads per warp: few rows, short tasks, so that there are enough of them; many rows, long ones, whose set-up more heads
-        // share; and where 64 or 32 heads make one wave that is nearly full, those.  FP8 / MXFP4, us a launch of 64 heads a token,
-        // from a graph with three inputs in rotation (from 3072 tokens on they come from HBM):
-        //   8 | 16           200 tokens  2.4 / 2.4 | 2.5 / 2.4         256 tokens  2.7 / 2.7 | 2.5 / 2.5
-        //   16 | 32 | 64      832 tokens  3.7 / 3.7 | 3.9 / 3.5 | 5.1 / 4.7        1280 tokens  5.7 / 5.6 | 5.8 / 5.5 | 6.1 / 6.0
-        //                    1536 tokens  6.8 / 6.2 | 6.1 / 5.8 | 7.5 / 6.9        1800 tokens  8.8 / 8.4 | 8.9 / 8.1 | 9.0 / 8.7
-        //                    2500 tokens 10.7 / 10.3 | 11.5 / 11.1 | 10.7 / 10.5   3072 tokens 13.4 / 12.9 | 12.6 / 12.2 | 12.0 / 11.7
-        //                    4096 tokens 18.1 / 17.0 | 18.2 / 17.0 | 19.9 / 18.4   8192 tokens 36.2 / 33.1 | 34.5 / 31.0 | 35.4 / 31.9
-        //   32 | prefetch    8192 tokens 34.5 / 31.0 | 34.0 / 31.4       9216 tokens 39.0 / 34.9 | 37.4 / 34.3     32768 tokens 127 / 113 | 121 / 109
-        // (With 64 at 5500 to 6500 tokens, nearly two waves of them, 3 % less than with 32.)
-        constexpr int64_t kWave = 148 * 6 * WARPS;  // warps of a B200
-        const auto fills_a_wave = [&](int64_t heads) { return rows <= kWave * heads && 9 * rows >= 7 * kWave * heads; };
-        const bool prefetch = rows >= 589824;
-        const int heads_per_task = fills_a_wave(64) ? 64 : rows > kWave * 64 || fills_a_wave(32) ? 32 : rows >= 14336 ? 16 : 8;
+        constexpr int WARPS = kHeadsWarps;
+        const bool prefetch = rows >= kPrefetchRows;
+        const int heads_per_task = heads_of_a_task(num_tokens, num_heads);
         const int64_t tasks_per_token = (num_heads + heads_per_task - 1) / heads_per_task;
         const dim3 grid(static_cast<unsigned>((num_tokens * tasks_per_token + WARPS - 1) / WARPS));
         uint32_t mul, shift;

@@ -33,6 +33,13 @@ def test_both_sides_of_the_lines(tokens, heads, fp4):
 
 
 @pytest.mark.parametrize("fp4", [False, True])
+@pytest.mark.parametrize("tokens,heads", [(1979, 96), (2533, 75), (1125, 80), (1382, 48), (1875, 48), (2763, 48), (4737, 48), (12289, 48), (5520, 40), (2763, 24), (4737, 24), (14336, 1), (3001, 3)])
+def test_other_numbers_of_heads(tokens, heads, fp4):
+    """Numbers of heads that leave a short last task, one task a token, and tasks of 40 and 48 heads, with and without requests to L2."""
+    test_both_sides_of_the_lines(tokens, heads, fp4)
+
+
+@pytest.mark.parametrize("fp4", [False, True])
 def test_special_values(fp4):
     tokens, heads = 96, 64
     g = torch.Generator(device=DEV).manual_seed(7)
