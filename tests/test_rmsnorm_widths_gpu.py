@@ -27,10 +27,19 @@ def test_row_sizes(q_size, kv_size, offset, tokens):
         assert int(compare.bf16_ulp_distance(got.cpu(), want).max()) <= 1
 
 
-@pytest.mark.parametrize("q_size,tokens", [(1536, n) for n in (740, 741, 1184, 1185, 1480, 1481, 2072, 2073, 4096, 4097)] + [(512, 2961), (512, 4097), (1024, 2073), (1024, 2961), (2048, 1185), (2048, 1777)])
-def test_both_sides_of_the_lines(q_size, tokens):
-    """Either side of the launch sizes that decide, for rows of 1536 and 512, when the weights are fetched and with how many CTAs per SM, and where a wave of the
-    other widths ends."""
+@pytest.mark.parametrize("tokens", [1480, 1481, 2072, 2073, 4096, 4097])
+def test_both_sides_of_the_lines(tokens):
+    """Rows of 1536 and 512 either side of the launch sizes that decide when the weights are fetched."""
+    g = torch.Generator(device=DEV).manual_seed(tokens)
+    q, kv = torch.randn(tokens, 1536, generator=g, device=DEV).bfloat16(), torch.randn(tokens, 512, generator=g, device=DEV).bfloat16()
+    wq, wk = torch.randn(1536, generator=g, device=DEV).bfloat16(), torch.randn(512, generator=g, device=DEV).bfloat16()
+    for got, rows, w in zip(fg.fused_q_kv_rmsnorm(q, kv, wq, wk, 1e-6), (q, kv), (wq, wk)):
+        assert int(compare.bf16_ulp_distance(got.cpu(), c_oracle.weighted_rmsnorm(rows.cpu(), w.cpu(), 1e-6)).max()) <= 1
+
+
+@pytest.mark.parametrize("q_size,tokens", [(1536, 740), (1536, 741), (1536, 1184), (1536, 1185), (512, 2961), (512, 4097), (1024, 2073), (1024, 2961), (2048, 1185), (2048, 1777)])
+def test_lines_of_the_other_forms(q_size, tokens):
+    """Either side of the sizes that decide how many CTAs an SM holds with rows of 1536, and where a wave of the other widths ends."""
     g = torch.Generator(device=DEV).manual_seed(tokens)
     q, kv = torch.randn(tokens, q_size, generator=g, device=DEV).bfloat16(), torch.randn(tokens, 512, generator=g, device=DEV).bfloat16()
     wq, wk = torch.randn(q_size, generator=g, device=DEV).bfloat16(), torch.randn(512, generator=g, device=DEV).bfloat16()
