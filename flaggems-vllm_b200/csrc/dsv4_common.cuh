@@ -457,8 +457,8 @@ enum : int { kDivideIeee = 0, kDivideFast = 1, kMultiplyReciprocal = 2 };
 // kMultiplyReciprocal: x * RN(1/scale), what the statement of `act_quant` computes.
 constexpr float kTwoTermMaxScale = 0x1p100f;
 // The scale to give a kDivideFast divider that can meet an infinite one: with the largest finite scale its reciprocal and the
-// quotients of finite values are 0, with an infinite one both would be NaN.  (Epilogue, 8192 x 128 rows: 272.7 -> 275.0 us; the group
-// quantiser needs it in the form for large scales only, where it costs nothing.)
+// quotients of finite values are 0, with an infinite one both would be NaN.  (Epilogue, 8192 x 128 rows, sustained: 270.6 -> 273.1 us;
+// the group quantiser needs it in the form for large scales only, where it costs nothing.)
 __device__ __forceinline__ float finite_scale(float s) { return fminf(s, 0x1.fffffep127f); }
 
 template <int MODE>
