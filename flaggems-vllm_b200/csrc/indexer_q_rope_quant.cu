@@ -319,8 +319,8 @@ cudaError_t launch_rows(const IndexerQParams& p, bool fp4, int64_t rows, int cs_
 // of registers take turns instead of being copied, and weights and scale words are written for 32 heads at once.  64 heads a token,
 // before -> after: 16384 tokens, MXFP4 61.3 -> 57.2 us (6.1 TB/s), FP8 64.4 -> 62.8 us (6.7 TB/s); 65536 tokens 227.8 -> 214.0 and
 // 238.2 -> 236.6 us; 1531 tokens, out of L2, 8.0 -> 5.8 and 6.1 us; 61 tokens 2.1 -> 2.0 us.
-template <int WARPS, bool FP4, bool WIDE, bool PREFETCH>
-__global__ void __launch_bounds__(WARPS * 32, 6) indexer_q_rope_quant_heads_kernel(const Launched<IndexerQParams, 4 * sizeof(int)> p, const int heads_per_task, const uint32_t tasks_per_token,
+template <int WARPS, bool FP4, bool WIDE, bool PREFETCH, int CTAS = 6>
+__global__ void __launch_bounds__(WARPS * 32, CTAS) indexer_q_rope_quant_heads_kernel(const Launched<IndexerQParams, 4 * sizeof(int)> p, const int heads_per_task, const uint32_t tasks_per_token,
                                                                                 const uint32_t tpt_mul, const uint32_t tpt_shift) {
     const int lane = threadIdx.x & 31, sub = lane & 3, which = lane >> 2;
     const uint32_t task = blockIdx.x * WARPS + (threadIdx.x >> 5);
@@ -498,6 +498,27 @@ static_assert(heads_of_a_task(1777, 64) == 16 && heads_of_a_task(2763, 64) == 64
 static_assert(heads_of_a_task(1979, 96) == 32 && heads_of_a_task(2533, 75) == 16 && heads_of_a_task(4600, 48) == 16 && heads_of_a_task(1875, 48) == 16);
 static_assert(heads_of_a_task(3437, 48) == 64 && heads_of_a_task(5416, 48) == 64 && heads_of_a_task(12289, 48) == 32 && heads_of_a_task(2250, 40) == 16 && heads_of_a_task(6500, 40) == 64);
 
+// Heads per warp of the form with seven CTAs per SM (72 registers, 56 to 108 bytes a thread spilled), or 0 for that with six: seven where
+// the tasks make one or two waves of seven and a little more than as many of six.  FP8 / MXFP4, us as above, six | seven:
+//   16 heads, 1 wave:   64 heads, 889 tokens 4.3 / 4.1 | 4.8 / 4.6     950 tokens 5.2 / 4.8 | 4.9 / 4.6     1036 tokens 5.5 / 5.2 | 5.0 / 4.8
+//                       16 heads, 4000 tokens 5.6 / 5.2 | 5.1 / 4.8    32 heads, 2000 tokens 5.5 / 5.2 | 5.0 / 4.7
+//   32 heads, 1 wave:   64 heads, 1777 tokens 9.3 / 8.4 | 9.5 / 8.4    1850 tokens 10.3 / 9.6 | 9.5 / 8.6     2072 tokens 11.0 / 10.4 | 10.4 / 9.6
+//             2 waves:  64 heads, 3553 tokens 16.4 / 15.0 | 16.4 / 14.9    3700 tokens 18.0 / 16.6 | 17.2 / 15.6     4144 tokens 19.3 / 17.6 | 18.6 / 16.8
+// Rows on 16-byte boundaries spill more and gain with 16 heads only (64 heads, 1000 tokens 6.9 / 6.8 | 6.4 / 6.1; 1850 tokens 10.4 / 10.1 | 10.4 / 9.4;
+// 3700 tokens 18.5 / 17.0 | 18.6 / 16.6).  Up to 8 heads a token are one pass a task, for which the spills do not pay (8000 tokens of 8 5.8 / 5.7 | 6.0 / 5.8).
+constexpr int heads_with_seven_ctas(int64_t tokens, int heads, bool wide) {
+    for (int n = wide ? 32 : 16; n >= 16 && heads > 8; n /= 2) {
+        if (heads > n && n == 32 && heads % n != 0) continue;
+        const int64_t tasks = tokens * ((heads + n - 1) / n);
+        for (int waves = 1; waves <= (wide ? 2 : 1); ++waves)
+            if (33 * tasks > 34 * waves * kWave && 6 * tasks <= 7 * waves * kWave) return n;
+    }
+    return 0;
+}
+static_assert(heads_with_seven_ctas(914, 64, true) == 0 && heads_with_seven_ctas(915, 64, false) == 16 && heads_with_seven_ctas(1036, 64, true) == 16 && heads_with_seven_ctas(1037, 64, true) == 0);
+static_assert(heads_with_seven_ctas(1829, 64, true) == 0 && heads_with_seven_ctas(1830, 64, true) == 32 && heads_with_seven_ctas(1830, 64, false) == 0 && heads_with_seven_ctas(2072, 64, true) == 32);
+static_assert(heads_with_seven_ctas(4000, 8, true) == 0 && heads_with_seven_ctas(4000, 16, false) == 16 && heads_with_seven_ctas(3660, 64, true) == 32 && heads_with_seven_ctas(4144, 64, true) == 32 && heads_with_seven_ctas(4145, 64, true) == 0);
+
 }  // namespace
 
 cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q, int64_t q_stride0, int64_t q_stride1,
@@ -528,14 +549,17 @@ cudaError_t launch_indexer_q_rope_quant(const int64_t* positions, const void* q,
     if (heads_shape) {
         constexpr int WARPS = kHeadsWarps;
         const bool prefetch = rows >= kPrefetchRows;
-        const int heads_per_task = heads_of_a_task(num_tokens, num_heads);
+        const bool wide = addr(q) % 32 == 0 && q_stride0 % 16 == 0 && q_stride1 % 16 == 0;
+        const int with_seven = heads_with_seven_ctas(num_tokens, num_heads, wide);
+        const int heads_per_task = with_seven != 0 ? with_seven : heads_of_a_task(num_tokens, num_heads);
         const int64_t tasks_per_token = (num_heads + heads_per_task - 1) / heads_per_task;
         const dim3 grid(static_cast<unsigned>((num_tokens * tasks_per_token + WARPS - 1) / WARPS));
         uint32_t mul, shift;
         make_fast_divisor(static_cast<uint32_t>(tasks_per_token), &mul, &shift);
-        const bool wide = addr(q) % 32 == 0 && q_stride0 % 16 == 0 && q_stride1 % 16 == 0;
         const auto run = [&](auto* kernel) { launch_dependent(kernel, grid, WARPS * 32, stream, p, heads_per_task, static_cast<uint32_t>(tasks_per_token), mul, shift); };
-        if (!wide) fp4 ? run(indexer_q_rope_quant_heads_kernel<WARPS, true, false, false>) : run(indexer_q_rope_quant_heads_kernel<WARPS, false, false, false>);
+        if (with_seven != 0 && wide) fp4 ? run(indexer_q_rope_quant_heads_kernel<WARPS, true, true, false, 7>) : run(indexer_q_rope_quant_heads_kernel<WARPS, false, true, false, 7>);
+        else if (with_seven != 0) fp4 ? run(indexer_q_rope_quant_heads_kernel<WARPS, true, false, false, 7>) : run(indexer_q_rope_quant_heads_kernel<WARPS, false, false, false, 7>);
+        else if (!wide) fp4 ? run(indexer_q_rope_quant_heads_kernel<WARPS, true, false, false>) : run(indexer_q_rope_quant_heads_kernel<WARPS, false, false, false>);
         else if (!prefetch) fp4 ? run(indexer_q_rope_quant_heads_kernel<WARPS, true, true, false>) : run(indexer_q_rope_quant_heads_kernel<WARPS, false, true, false>);
         else fp4 ? run(indexer_q_rope_quant_heads_kernel<WARPS, true, true, true>) : run(indexer_q_rope_quant_heads_kernel<WARPS, false, true, true>);
         count_launch();

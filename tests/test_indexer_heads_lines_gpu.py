@@ -40,6 +40,24 @@ def test_other_numbers_of_heads(tokens, heads, fp4):
 
 
 @pytest.mark.parametrize("fp4", [False, True])
+@pytest.mark.parametrize("offset", [0, 8])
+@pytest.mark.parametrize("tokens,heads", [(914, 64), (915, 64), (1036, 64), (1037, 64), (1830, 64), (2072, 64), (3661, 64), (4144, 64), (4000, 16), (1980, 24), (1000, 50)])
+def test_one_or_two_waves_of_seven_ctas(tokens, heads, offset, fp4):
+    """Either side of the sizes that take seven CTAs per SM, on both row alignments."""
+    g = torch.Generator(device=DEV).manual_seed(tokens + offset)
+    store = torch.empty(tokens * heads * 128 + offset, device=DEV, dtype=torch.bfloat16).normal_(generator=g)
+    q = store[offset:].view(tokens, heads, 128)
+    w = torch.randn(tokens, heads, generator=g, device=DEV)
+    pos = torch.randint(0, 512, (tokens,), generator=g, device=DEV)
+    cs = workloads.cos_sin_table(512)
+    got = _bytes(fg.fused_indexer_q_rope_quant(pos, q, cs.to(DEV), w, 0.0884, 0.125, use_fp4=fp4), fp4)
+    want, want_s, want_w = c_oracle.indexer_q_rope_quant(pos.cpu(), q.cpu(), cs, w.cpu(), 0.0884, 0.125, use_fp4=fp4)
+    assert torch.equal(got[0], want.contiguous().view(torch.uint8).flatten()) and torch.equal(got[-1], want_w)
+    if fp4:
+        assert torch.equal(got[1], want_s.contiguous().view(torch.uint8).flatten())
+
+
+@pytest.mark.parametrize("fp4", [False, True])
 def test_special_values(fp4):
     tokens, heads = 96, 64
     g = torch.Generator(device=DEV).manual_seed(7)
