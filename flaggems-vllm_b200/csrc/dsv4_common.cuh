@@ -146,10 +146,11 @@ __device__ __forceinline__ void begin_dependent_kernel() {
     let_next_kernel_start();
 }
 
-// A kernel's first parameter, filled up so that the parameters of the launch take 32 bytes more than a multiple of 64.  `BEHIND`:
-// bytes of the parameters behind it.  The host's cost of a launch depends on that size and nearly nothing else of the kernel: sizes of 24
-// or 32 mod 64 bytes 1.58 us a dependent launch, every other size from 8 to 512 bytes 1.95 us (plain launches: 32 mod 64 1.85 us, 24 and
-// 40 2.0 us, others 2.45 us; driver 580.159).  With a driver that puts its lines elsewhere the filling changes nothing.
+// A kernel's first parameter, filled up so that the parameters of the launch take 32 bytes more than a multiple of 64, or 28 where the
+// last one is of 4 bytes (the filled block is a multiple of 8).  `BEHIND`: bytes of the parameters behind it, rounded up to 8.
+// The host's cost of a launch depends on that size and nearly nothing else of the kernel (80 to 288 bytes, driver 580.159): 20, 24, 28 and
+// 32 mod 64 1.68-1.81 us a dependent launch, every other size 2.02-2.25; a plain launch 1.80-1.93 us at 32, 2.1-2.3 at 20 to 28, 36 and
+// 40, others 2.5-2.7.  With a driver that puts its lines elsewhere the filling changes nothing.
 constexpr size_t launch_filling(size_t bytes) { return (32 + 64 - bytes % 64) % 64; }
 template <typename T, size_t BEHIND = 0, size_t FILL = launch_filling(sizeof(T) + BEHIND)>
 struct Launched : T {
@@ -447,13 +448,13 @@ enum : int { kDivideIeee = 0, kDivideFast = 1, kMultiplyReciprocal = 2 };
 //                  (beyond that y_lo would be subnormal), or
 //   corrected      q0 = RN(x * y), r = fma(-scale, q0, x), q = fma(r, y, q0)      three instructions, any scale.
 // (-0 becomes +0 in the corrected form, and in the two-term one where y_lo is negative: the last sum makes it so.)
-// q can differ from RN(x/scale) in the last fp32 bit, but never in the e4m3 byte of an x that is not -0: a CPU test enumerates every bf16
-// group maximum (hence every reachable scale, for the reference's eps = 1e-10) against every bf16 value below it, for
-// each of the three values y can take (the correctly rounded reciprocal and its two neighbours) and both forms -
-// 1.6e9 cases each, zero differing bytes; a GPU test enumerates them with quotients() below and the device's own reciprocal.  The form is a template argument: a caller that uses the two-term form votes once
-// per warp on the scales' range (`__all_sync`), so the choice is a uniform branch around straight-line code; the epilogue
-// quantiser uses the corrected form throughout (no second code path measured faster there).  For any other eps the
-// kernels divide.
+// q can differ from RN(x/scale) in the last fp32 bit, but never in the e4m3 byte of an x that is not -0: a CPU test enumerates
+// every bf16 group maximum (hence every reachable scale, for the reference's eps = 1e-10) against every bf16 value below it, for
+// each of the three values y can take (the correctly rounded reciprocal and its two neighbours) and both forms - 1.6e9 cases
+// each, zero differing bytes; a GPU test enumerates the pairs with quotients() below and the device's own reciprocal.  The form
+// is a template argument: a caller that uses the two-term form votes once per warp on the scales' range (`__all_sync`), so the
+// choice is a uniform branch around straight-line code; the epilogue quantiser uses the corrected form throughout (no second
+// code path measured faster there).  For any other eps the kernels divide.
 // kMultiplyReciprocal: x * RN(1/scale), what the statement of `act_quant` computes.
 constexpr float kTwoTermMaxScale = 0x1p100f;
 // The scale to give a kDivideFast divider that can meet an infinite one: with the largest finite scale its reciprocal and the

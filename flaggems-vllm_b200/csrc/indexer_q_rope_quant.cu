@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_kernel(const 
 // U passes per warp are loaded before any is used.  Needs 16-byte aligned rows and a rotary tail that starts
 // on a multiple of 8 values.
 template <int WARPS, int G, int U, bool FP4>
-__global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_rows_kernel(const Launched<IndexerQParams, 2 * sizeof(int)> p, const int cs_vec4) {
+__global__ void __launch_bounds__(WARPS * 32) indexer_q_rope_quant_rows_kernel(const Launched<IndexerQParams, 8> p, const int cs_vec4) {
     begin_dependent_kernel();
     constexpr int D = 8 * G, ROWS = 32 / G;
     const int lane = threadIdx.x & 31, sub = lane % G, slot = lane / G;
@@ -314,11 +314,13 @@ cudaError_t launch_rows(const IndexerQParams& p, bool fp4, int64_t rows, int cs_
 // 32 are 2 lanes.  WIDE: 32-byte loads, otherwise (rows on 16-byte boundaries only) two of half the size.  Two passes are in
 // flight: the loads of the next one go out before the current one is worked on.  PREFETCH: one instruction sends the rest of the
 // task's rows to L2 at its start.
-// Was bound by instruction issue: 345 warp instructions for a pass of eight heads with MXFP4, FP32 and conversion pipes apart.  Now
-// bf16 values are widened and scaled by one instruction each (scaled_pair()), two pairs rotated at a time (rotate_two()), two sets
-// of registers take turns instead of being copied, and weights and scale words are written for 32 heads at once.  64 heads a token,
-// before -> after: 16384 tokens, MXFP4 61.3 -> 57.2 us (6.1 TB/s), FP8 64.4 -> 62.8 us (6.7 TB/s); 65536 tokens 227.8 -> 214.0 and
-// 238.2 -> 236.6 us; 1531 tokens, out of L2, 8.0 -> 5.8 and 6.1 us; 61 tokens 2.1 -> 2.0 us.
+// Large batches are bound by HBM, smaller ones by instruction issue: a pass of eight heads with MXFP4 is 217 warp instructions.  For
+// that, bf16 values are widened and scaled by one instruction each (scaled_pair()), two pairs are rotated at a time (rotate_two()), two
+// sets of registers take turns, and weights and scale words are written for 32 heads at once.  Without these (345 instructions) -> with,
+// 64 heads a token, us a launch from a graph, FP8 and MXFP4:
+//   at full clock: 61 tokens 1.88 -> 1.71 and 1.94 -> 1.71; 1531 tokens 9.4 -> 8.0 and 9.2 -> 6.7; 9216 tokens 38.7 -> 36.4 and 36.9 -> 33.1;
+//     16384 tokens 63.9 -> 61.4 (6.7 TB/s) and 64-67 -> 57-59 (6.0 TB/s); 65536 tokens 238-246 -> 235 (7.0 TB/s) and 230-235 -> 207-212
+//   sustained, at the clock the power limit leaves: 16384 tokens 69.2 -> 65.2 and 65.5 -> 58.7; 65536 tokens 262 -> 244 and 250 -> 218
 template <int WARPS, bool FP4, bool WIDE, bool PREFETCH, int CTAS = 6>
 __global__ void __launch_bounds__(WARPS * 32, CTAS) indexer_q_rope_quant_heads_kernel(const Launched<IndexerQParams, 4 * sizeof(int)> p, const int heads_per_task, const uint32_t tasks_per_token,
                                                                                 const uint32_t tpt_mul, const uint32_t tpt_shift) {

@@ -35,14 +35,12 @@ struct InvRopeParams {
 // WIDE: one 32-byte load and one 16-byte store per lane and head; otherwise (rows on 16-byte boundaries only) two of half the
 // size.
 // Two passes of U heads are in flight: the loads of the next pass go out before the current one is worked on.
-// HBM-bound at full clock (8192 x 128 rows 241 us = 6.7 TB/s), but in a run of some tenths of a second the power limit takes the clock to
-// 1.58 GHz, and there the kernel is bound by instruction issue: 182 warp instructions a head took 264-268 us, and fp32 scales 286-293.  Now:
-// every lane loads 32 bytes, the last four the rotary values once more, and a mask keeps them out of the maximum (no lane-dependent branch
-// around the loads, no zeroing); the last group's scale is formed once, by its own lanes, and fetched by a shuffle.  Sustained, before ->
-// after: 8192 x 128 rows 264-268 -> 252 us, fp32 scales 286-293 -> 273-275; 16384 x 16 67 -> 65; 1531 x 128 50.5 -> 49.2; 256 x 128
-// 11.1 -> 10.9 us.  The same arithmetic with two sets of registers that take turns instead of being copied: 151 instructions, but 266 us
-// and 286-303.  Heads per pass and CTAs per SM, 8192 x 128 rows: 2, 7 252 us; 1, 10 258; 1, 8 269; 2, 6 258; 2, 8 254 (fp32 scales 298);
-// 3, 6 306.
+// HBM-bound at full clock (8192 x 128 rows 240 us = 6.7 TB/s, fp32 scales 245).  In a run of some tenths of a second the power limit takes
+// the clock to 1.58 GHz, and there instruction issue bounds it as well: 250 us, fp32 scales 273 (rows on 16-byte boundaries 278 and 298).
+// So every lane loads 32 bytes, the last four the rotary values once more, and a mask keeps them out of the maximum (no lane-dependent
+// branch around the loads, no zeroing), and the last group's scale is formed once, by its own lanes, and fetched by a shuffle: about 150
+// warp instructions a head (tasks of 16 heads; fp32 scales 168) instead of 182, with which it took 264 and 293 us (284 and 312).
+// Heads per pass and CTAs per SM, 8192 x 128 rows, sustained: 2, 7 252 us; 1, 10 258; 1, 8 269; 2, 6 258; 2, 8 254 (fp32 scales 298); 3, 6 306.
 constexpr int kMainLanes = 28;
 constexpr int kHeadsInFlight = 2;  // per pass
 constexpr int kCtasPerSm = 7;      // 72 registers
