@@ -103,13 +103,14 @@ struct Arguments {
 bool is(const Tensor& t, ScalarType type) { return t.scalar_type() == type; }
 bool on(const Tensor& t, const Tensor& first) { return t.is_cuda() && t.get_device() == first.get_device(); }
 
-// A contiguous, uninitialised tensor on the device of `like`.  Where that device is current, as it is in nearly every call, without the
-// look at torch's set-up and the device guard that empty_cuda() takes each time.
-Tensor make_empty(at::IntArrayRef sizes, ScalarType type, const Tensor& like) {
+using dsv4::OnDevice;
+OnDevice on_device_of(const Tensor& t, OnDevice::Use use = OnDevice::kAllocatesToo) { return OnDevice(static_cast<c10::DeviceIndex>(t.get_device()), use); }
+
+// A contiguous, uninitialised tensor on the device of the call, without the look at torch's set-up and the device guard that empty_cuda()
+// takes each time.
+Tensor make_empty(at::IntArrayRef sizes, ScalarType type, const OnDevice&) {
     static const bool set_up = (at::globalContext().lazyInitDevice(at::kCUDA), true);
     (void)set_up;
-    const at::Device device = like.device();
-    if (!dsv4::is_current(device.index())) return Tensor(at::detail::empty_cuda(sizes, type, device, std::nullopt));
     return Tensor(at::detail::empty_generic(sizes, c10::cuda::CUDACachingAllocator::get(), c10::DispatchKeySet(c10::DispatchKey::CUDA), type, std::nullopt));
 }
 
@@ -119,19 +120,15 @@ void set_view(Tensor& t, at::IntArrayRef sizes, at::IntArrayRef strides) {
     t.unsafeGetTensorImpl()->set_sizes_and_strides(sizes, strides);
 }
 
-// Runs `launch(stream)` with the device of `first` current.  False after a failed launch, with a Python error set.
+// Runs `launch(stream)` with the device of the call current.  False after a failed launch, with a Python error set.
 template <typename Launch>
-bool launch_on(const Tensor& first, Launch&& launch) {
-    const auto device = static_cast<c10::DeviceIndex>(first.get_device());
-    const int code = dsv4::with_device(device, [&] {
-        void* stream = c10::cuda::getCurrentCUDAStream(device).stream();
-        int result;
-        // a launch can block (full launch queue): other Python threads go on meanwhile
-        Py_BEGIN_ALLOW_THREADS
-        result = launch(stream);
-        Py_END_ALLOW_THREADS
-        return result;
-    });
+bool launch_on(const OnDevice& here, Launch&& launch) {
+    void* stream = c10::cuda::getCurrentCUDAStream(here.index).stream();
+    int code;
+    // a launch can block (full launch queue): other Python threads go on meanwhile
+    Py_BEGIN_ALLOW_THREADS
+    code = launch(stream);
+    Py_END_ALLOW_THREADS
     if (code == 0) return true;
     PyObject* r = PyObject_CallFunction(g_check, "i", code);
     if (r) {
@@ -187,7 +184,7 @@ PyObject* prologue(Arguments& a) {
     REQUIRE(on(*kv, *q) && on(*cache, *q) && on(*slots, *q) && on(*pos, *q) && on(*cs, *q));
     if (!a.ok) Py_RETURN_NONE;
     if (tokens == 0) Py_RETURN_TRUE;
-    if (!launch_on(*q, [&](void* stream) {
+    if (!launch_on(on_device_of(*q, OnDevice::kLaunchesOnly), [&](void* stream) {
             return dsv4_qnorm_rope_kv_insert(q->data_ptr(), kv->data_ptr(), cache->data_ptr(), static_cast<const int64_t*>(slots->data_ptr()),
                                              static_cast<const int64_t*>(pos->data_ptr()), static_cast<const float*>(cs->data_ptr()), eps,
                                              tokens, heads, slots->size(0), block, cache->stride(0), stream);
@@ -219,8 +216,9 @@ PyObject* q_kv_rmsnorm(Arguments& a) {
     REQUIRE(qw->dim() == 1 && qw->size(0) == qr->size(1) && kw->dim() == 1 && kw->size(0) == kv->size(1));
     if (!a.ok) Py_RETURN_NONE;
     const int64_t tokens = qr->size(0);
-    Tensor qo = make_empty(qr->sizes(), qr->scalar_type(), *qr), ko = make_empty(kv->sizes(), kv->scalar_type(), *qr);
-    if (tokens > 0 && !launch_on(*qr, [&](void* stream) {
+    const OnDevice here = on_device_of(*qr);
+    Tensor qo = make_empty(qr->sizes(), qr->scalar_type(), here), ko = make_empty(kv->sizes(), kv->scalar_type(), here);
+    if (tokens > 0 && !launch_on(here, [&](void* stream) {
             return dsv4_fused_q_kv_rmsnorm_dtypes(qr->data_ptr(), qo.data_ptr(), qw->data_ptr(), qr->stride(0), qo.stride(0), qr->size(1),
                                                   dtype_code(*qr), dtype_code(*qw), kv->data_ptr(), ko.data_ptr(), kw->data_ptr(),
                                                   kv->stride(0), ko.stride(0), kv->size(1), dtype_code(*kv), dtype_code(*kw), tokens, eps, stream);
@@ -242,17 +240,18 @@ PyObject* group_quant(Arguments& a) {
     REQUIRE(cols % group == 0 && x->stride(-1) == 1 && (x->dim() == 2 || (x->is_contiguous() && !column_major)));
     if (!a.ok) Py_RETURN_NONE;
     const int64_t rows = cols > 0 ? x->numel() / cols : 0, groups = cols / group;
-    Tensor xq = make_empty(x->sizes(), at::kFloat8_e4m3fn, *x), xs;
+    const OnDevice here = on_device_of(*x);
+    Tensor xq = make_empty(x->sizes(), at::kFloat8_e4m3fn, here), xs;
     if (column_major) {
-        xs = make_empty({groups, x->size(0)}, at::kFloat, *x);
+        xs = make_empty({groups, x->size(0)}, at::kFloat, here);
         set_view(xs, {x->size(0), groups}, {1, std::max<int64_t>(x->size(0), 1)});
     } else {
         at::DimVector sizes(x->sizes().begin(), x->sizes().end());
         sizes.back() = groups;
-        xs = make_empty(sizes, at::kFloat, *x);
+        xs = make_empty(sizes, at::kFloat, here);
     }
     const int64_t stride_row = column_major ? 1 : groups, stride_group = column_major ? x->size(0) : 1;
-    if (rows > 0 && !launch_on(*x, [&](void* stream) {
+    if (rows > 0 && !launch_on(here, [&](void* stream) {
             return dsv4_per_token_group_quant_fp8(x->data_ptr(), x->dim() == 2 ? x->stride(0) : cols, xq.data_ptr(),
                                                   static_cast<float*>(xs.data_ptr()), stride_row, stride_group, rows, cols, group, eps,
                                                   ue8m0 ? 1 : 0, stream);
@@ -270,11 +269,12 @@ PyObject* act_quant(Arguments& a) {
     REQUIRE(x->is_cuda() && is(*x, at::kBFloat16) && x->dim() >= 1 && x->is_contiguous() && block > 0 && x->size(-1) % block == 0);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t cols = x->size(-1), rows = cols > 0 ? x->numel() / cols : 0;
-    Tensor y = make_empty(x->sizes(), at::kFloat8_e4m3fn, *x);
+    const OnDevice here = on_device_of(*x);
+    Tensor y = make_empty(x->sizes(), at::kFloat8_e4m3fn, here);
     at::DimVector sizes(x->sizes().begin(), x->sizes().end());
     sizes.back() = cols / block;
-    Tensor s = make_empty(sizes, at::kFloat, *x);
-    if (rows > 0 && !launch_on(*x, [&](void* stream) {
+    Tensor s = make_empty(sizes, at::kFloat, here);
+    if (rows > 0 && !launch_on(here, [&](void* stream) {
             return dsv4_act_quant(x->data_ptr(), cols, y.data_ptr(), static_cast<float*>(s.data_ptr()), rows, cols, block, round_scale ? 1 : 0,
                                   stream);
         }))
@@ -302,9 +302,10 @@ PyObject* inv_rope_fp8_quant(Arguments& a) {
     if (!a.ok) Py_RETURN_NONE;
     const int64_t d = per_group * head_dim, padded = (tokens + 3) / 4 * 4;
     const int64_t inner = packed ? (d / group + 3) / 4 : d / group;
-    Tensor fp8 = make_empty({n_groups, tokens, d}, at::kFloat8_e4m3fn, *o);
-    Tensor scale = make_empty({n_groups * inner * padded}, packed ? at::kInt : at::kFloat, *o);
-    if (tokens > 0 && !launch_on(*o, [&](void* stream) {
+    const OnDevice here = on_device_of(*o);
+    Tensor fp8 = make_empty({n_groups, tokens, d}, at::kFloat8_e4m3fn, here);
+    Tensor scale = make_empty({n_groups * inner * padded}, packed ? at::kInt : at::kFloat, here);
+    if (tokens > 0 && !launch_on(here, [&](void* stream) {
             return dsv4_fused_inv_rope_fp8_quant_geometry(
                 o->data_ptr(), o->stride(0), o->stride(1), static_cast<const int64_t*>(pos->data_ptr()),
                 static_cast<const float*>(cs->data_ptr()), cs->stride(0), fp8.data_ptr(), scale.data_ptr(), inner * padded, tokens, padded,
@@ -331,24 +332,25 @@ PyObject* indexer_q_rope_quant(Arguments& a) {
     REQUIRE((dim == 64 || dim == 128 || dim == 256) && rot % 2 == 0 && rot <= dim && (dim - rot) % (dim / 32) == 0);
     REQUIRE(on(*pos, *q) && on(*cs, *q) && on(*w, *q));
     if (!a.ok) Py_RETURN_NONE;
-    Tensor w_out = make_empty({tokens, heads}, at::kFloat, *q), q_out, scale;
+    const OnDevice here = on_device_of(*q);
+    Tensor w_out = make_empty({tokens, heads}, at::kFloat, here), q_out, scale;
     void* scale_ptr = nullptr;
     if (fp4) {
-        q_out = make_empty({tokens, heads, dim / 2}, at::kByte, *q);
+        q_out = make_empty({tokens, heads, dim / 2}, at::kByte, here);
         // the four UE8M0 bytes of a head of 128 travel as one int32 (two for 256); a head of 64 keeps its two bytes
         const int64_t words = dim / 128;
-        if (words == 1) scale = make_empty({tokens, heads}, at::kInt, *q);
-        else if (words > 1) scale = make_empty({tokens, heads, words}, at::kInt, *q);
-        else scale = make_empty({tokens, heads, dim / 32}, at::kByte, *q);
+        if (words == 1) scale = make_empty({tokens, heads}, at::kInt, here);
+        else if (words > 1) scale = make_empty({tokens, heads, words}, at::kInt, here);
+        else scale = make_empty({tokens, heads, dim / 32}, at::kByte, here);
         scale_ptr = scale.data_ptr();
     } else if (q->is_contiguous()) {
-        q_out = make_empty(q->sizes(), at::kFloat8_e4m3fn, *q);
+        q_out = make_empty(q->sizes(), at::kFloat8_e4m3fn, here);
     } else {  // keeps the order of dimensions in memory that a dense, permuted q has
         q_out = at::empty_like(*q, q->options().dtype(at::kFloat8_e4m3fn));
         REQUIRE(q_out.stride(2) == 1);
         if (!a.ok) Py_RETURN_NONE;
     }
-    if (tokens > 0 && !launch_on(*q, [&](void* stream) {
+    if (tokens > 0 && !launch_on(here, [&](void* stream) {
             return dsv4_fused_indexer_q_rope_quant(
                 static_cast<const int64_t*>(pos->data_ptr()), q->data_ptr(), q->stride(0), q->stride(1), cs->data_ptr(), cs->stride(0),
                 is(*cs, at::kBFloat16) ? 1 : 0, rot, q_out.data_ptr(), q_out.stride(0), q_out.stride(1), scale_ptr,
@@ -384,7 +386,7 @@ PyObject* indexer_k_quant(Arguments& a) {
     REQUIRE(on(*cache, *k) && on(*slots, *k));
     if (!a.ok) Py_RETURN_NONE;
     if (tokens == 0 || cache->size(0) == 0) Py_RETURN_TRUE;
-    if (!launch_on(*k, [&](void* stream) {
+    if (!launch_on(on_device_of(*k, OnDevice::kLaunchesOnly), [&](void* stream) {
             return dsv4_indexer_k_quant_and_cache(k->data_ptr(), k->stride(0), is(*k, at::kHalf) ? 1 : 0, cache->data_ptr(), cache->stride(0),
                                                   static_cast<const int64_t*>(slots->data_ptr()), tokens, block, dim, group, ue8m0 ? 1 : 0, stream);
         }))
@@ -412,7 +414,7 @@ PyObject* cp_gather_indexer(Arguments& a) {
     REQUIRE(on(*k, *cache) && on(*scale, *cache) && on(*table, *cache) && on(*cu, *cache));
     if (!a.ok) Py_RETURN_NONE;
     if (tokens == 0 || batch == 0 || cache->size(0) == 0) Py_RETURN_TRUE;
-    if (!launch_on(*cache, [&](void* stream) {
+    if (!launch_on(on_device_of(*cache, OnDevice::kLaunchesOnly), [&](void* stream) {
             return dsv4_cp_gather_indexer_k_quant_cache(cache->data_ptr(), cache->stride(0), k->data_ptr(), k->stride(0), scale->data_ptr(),
                                                         scale->stride(0) * static_cast<int64_t>(scale->element_size()),
                                                         static_cast<const int32_t*>(table->data_ptr()), table->stride(0),
@@ -436,9 +438,10 @@ PyObject* global_topk(Arguments& a) {
     REQUIRE(!valid || (is(*valid, at::kInt) && valid->is_contiguous() && valid->dim() == 1 && valid->size(0) == tokens && on(*valid, *topk)));
     REQUIRE(on(*request, *topk) && on(*table, *topk));
     if (!a.ok) Py_RETURN_NONE;
-    Tensor out = topk->is_contiguous() ? make_empty(topk->sizes(), at::kInt, *topk) : at::empty_like(*topk);
-    Tensor lens = make_empty({tokens}, at::kInt, *topk);
-    if (tokens > 0 && !launch_on(*topk, [&](void* stream) {
+    const OnDevice here = on_device_of(*topk);
+    Tensor out = topk->is_contiguous() ? make_empty(topk->sizes(), at::kInt, here) : at::empty_like(*topk);
+    Tensor lens = make_empty({tokens}, at::kInt, here);
+    if (tokens > 0 && !launch_on(here, [&](void* stream) {
             return dsv4_compute_global_topk_indices_and_lens(
                 static_cast<const int32_t*>(topk->data_ptr()), topk->stride(0), static_cast<const int32_t*>(request->data_ptr()),
                 static_cast<const int32_t*>(table->data_ptr()), table->stride(0), valid ? static_cast<const int32_t*>(valid->data_ptr()) : nullptr,
@@ -462,8 +465,9 @@ PyObject* combine_topk_swa(Arguments& a) {
     REQUIRE(start->size(0) >= requests + 1 && gather->size(0) >= requests);
     if (!a.ok) Py_RETURN_NONE;
     const int64_t width = (k + window + kAlignment - 1) / kAlignment * kAlignment;
-    Tensor combined = make_empty({tokens, width}, at::kInt, *topk), lens = make_empty({tokens}, at::kInt, *topk);
-    if (tokens > 0 && requests > 0 && !launch_on(*topk, [&](void* stream) {
+    const OnDevice here = on_device_of(*topk);
+    Tensor combined = make_empty({tokens, width}, at::kInt, here), lens = make_empty({tokens}, at::kInt, here);
+    if (tokens > 0 && requests > 0 && !launch_on(here, [&](void* stream) {
             return dsv4_combine_topk_swa_indices(
                 static_cast<const int32_t*>(topk->data_ptr()), topk->stride(0), topk->size(1), static_cast<const int32_t*>(start->data_ptr()),
                 static_cast<const int32_t*>(seq->data_ptr()), static_cast<const int32_t*>(gather->data_ptr()),
@@ -498,7 +502,7 @@ PyObject* dequantize_and_gather(Arguments& a) {
     if (!a.ok) Py_RETURN_NONE;
     if (requests == 0 || out->size(1) == 0) Py_RETURN_TRUE;
     const int64_t pitch = cache->dim() == 3 ? cache->size(1) * cache->size(2) : cache->stride(0);
-    if (!launch_on(*out, [&](void* stream) {
+    if (!launch_on(on_device_of(*out, OnDevice::kLaunchesOnly), [&](void* stream) {
             return dsv4_dequantize_and_gather_k_cache(out->data_ptr(), out->stride(0), out->stride(1), out->size(1), cache->data_ptr(),
                                                       seq->data_ptr(), gather ? gather->data_ptr() : nullptr, table->data_ptr(), requests,
                                                       table->size(1), block, pitch, offset, static_cast<int32_t>(nope),
@@ -528,7 +532,7 @@ PyObject* top_k_decode(Arguments& a) {
     REQUIRE(seq->size(0) * next_n >= rows);
     if (!a.ok) Py_RETURN_NONE;
     if (rows == 0 || k == 0) Py_RETURN_TRUE;
-    if (!launch_on(*logits, [&](void* stream) {
+    if (!launch_on(on_device_of(*logits, OnDevice::kLaunchesOnly), [&](void* stream) {
             return dsv4_top_k_per_row_decode(static_cast<const float*>(logits->data_ptr()), stride0, stride1, next_n,
                                              static_cast<const int32_t*>(seq->data_ptr()), static_cast<int32_t*>(indices->data_ptr()), rows,
                                              logits->size(1), k, stream);
@@ -547,7 +551,7 @@ PyObject* top_k_prefill(Arguments& a) {
         REQUIRE(is(*t, at::kInt) && t->dim() == 1 && t->is_contiguous() && t->size(0) >= rows && on(*t, *logits));
     if (!a.ok) Py_RETURN_NONE;
     if (rows == 0 || k == 0) Py_RETURN_TRUE;
-    if (!launch_on(*logits, [&](void* stream) {
+    if (!launch_on(on_device_of(*logits, OnDevice::kLaunchesOnly), [&](void* stream) {
             return dsv4_top_k_per_row_prefill(static_cast<const float*>(logits->data_ptr()), stride0, stride1,
                                               static_cast<const int32_t*>(starts->data_ptr()), static_cast<const int32_t*>(ends->data_ptr()),
                                               static_cast<int32_t*>(indices->data_ptr()), rows, logits->size(1), k, stream);
@@ -569,7 +573,7 @@ PyObject* persistent_topk(Arguments& a) {
     REQUIRE(on(*lengths, *logits) && on(*output, *logits));
     if (!a.ok) Py_RETURN_NONE;
     if (rows == 0) Py_RETURN_TRUE;
-    if (!launch_on(*logits, [&](void* stream) {
+    if (!launch_on(on_device_of(*logits, OnDevice::kLaunchesOnly), [&](void* stream) {
             return dsv4_top_k_per_row_prefill(static_cast<const float*>(logits->data_ptr()), logits->stride(0), logits->stride(1), nullptr,
                                               static_cast<const int32_t*>(lengths->data_ptr()), static_cast<int32_t*>(output->data_ptr()), rows,
                                               std::min(logits->size(1), longest), k, stream);

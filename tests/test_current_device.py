@@ -26,11 +26,16 @@ extern "C" cudaError_t cudaSetDevice(int device) { runtime_device = device; retu
 extern "C" cudaError_t cudaGetDeviceCount(int* count) { *count = 4; return cudaSuccess; }
 static bool only_device_1(c10::DeviceIndex device) { return device == 1; }
 
-int main(int, char** arguments) {
+int main(int count, char** arguments) {
     const int runtime = std::atoi(arguments[1]), noted = std::atoi(arguments[2]), wanted = std::atoi(arguments[3]);
     c10::cuda::_internal::setHasPrimaryContext(only_device_1);
     runtime_device = runtime;
     if (noted >= 0) c10::cuda::MaybeSetDevice(static_cast<c10::DeviceIndex>(noted));  // what the end of a torch guard does
+    if (count > 4) {  // a call that only launches
+        const dsv4::OnDevice here(static_cast<c10::DeviceIndex>(wanted), dsv4::OnDevice::kLaunchesOnly);
+        std::printf("%d\n", runtime_device);
+        return 0;
+    }
     const bool current = dsv4::is_current(static_cast<c10::DeviceIndex>(wanted));
     const int launched_on = dsv4::with_device(static_cast<c10::DeviceIndex>(wanted), [] { return runtime_device; });
     std::printf("%d %d %d %d\n", static_cast<int>(current), launched_on, static_cast<int>(c10::cuda::current_device()), runtime_device);
@@ -63,3 +68,9 @@ def test_the_wanted_device_is_the_runtimes(program, runtime, noted, wanted, curr
     said, launched_on, torch_after, _ = map(int, subprocess.run([str(program), str(runtime), str(noted), str(wanted)], check=True, capture_output=True, text=True).stdout.split())
     assert bool(said) == current and launched_on == wanted
     assert torch_after == (noted if noted >= 0 else runtime)  # torch's device afterwards is what it was
+
+
+@pytest.mark.parametrize("runtime,noted,wanted", [(1, -1, 1), (1, 1, 1), (1, 3, 3), (1, 3, 1), (1, 0, 0), (1, -1, 0), (0, 2, 3)])
+def test_a_call_without_outputs_launches_on_the_wanted_device(program, runtime, noted, wanted):
+    said = subprocess.run([str(program), str(runtime), str(noted), str(wanted), "launch"], check=True, capture_output=True, text=True).stdout
+    assert int(said) == wanted
